@@ -582,6 +582,9 @@ static int create_impl(fg_ctx *h, const fg_mesh *m, const fg_region *regs, int n
     if (demag == FG_DEMAG_FMM) {
         int s = fmm_build(c);
         if (s != FG_OK) return s;
+    } else {
+        c.direct_nsplit = direct_splits(c);
+        CK(dalloc(&c.direct_part, (c.opts.first_order ? 1 : 2) * (size_t)c.direct_nsplit * std::max(1, c.n_mag_nodes)));
     }
     c.dinc = demag == FG_DEMAG_FMM && c.opts.precision == FG_PREC_FP32_REFINE && c.opts.demag_increment != 0 &&
             !c.batch;
@@ -721,7 +724,7 @@ void fg_destroy(fg_ctx *h) {
                     c.Sval32, c.A, c.Ainv, c.A32, c.tri, c.tri_c, c.tinc_ptr, c.tinc, c.src_xyz, c.mag_nodes, c.u[0], c.u[1],
                     c.v[0], c.v[1], c.phi[0], c.phi[1], c.phiv[0], c.phiv[1], c.ep, c.eq, c.ep32, c.eq32, c.Dl32,
                     c.slot, c.Dl, c.rhs, c.x, c.bv, c.W, c.fv, c.partial, c.bar, c.dres, c.src_q, c.tri_slot,
-                    c.pot, c.epart, c.src_dst, c.src_q2, c.tri_slot2, c.pot2, c.tri_be, c.hsp, c.da_ds, c.J_ds, c.state_ds,
+                    c.pot, c.epart, c.src_dst, c.src_q2, c.tri_slot2, c.pot2, c.direct_part, c.tri_be, c.hsp, c.da_ds, c.J_ds, c.state_ds,
                     c.dstate32, c.da32, c.cq32, c.src_qf, c.src_q2f, c.tri_ds, c.tri32};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -890,7 +893,7 @@ static int demag_into(fg_ctx *h, const double *m, double *phi_out) {
         CK(fmm_eval(c));
         c.launches += fmm_launches_per_eval(c);
     } else {
-        CK(launch_p2p_direct(c));
+        CK(launch_p2p_direct(c, 1));
         c.launches += 1;
     }
     CK(launch_phi_final(c, phi_out));
@@ -914,20 +917,20 @@ static int energy_impl(fg_ctx *h, const double Hext[3], double E[4], double avg[
     return FG_OK;
 }
 
-// Demag of m and of v (Fem::compute_all, src/fem.h): with the FMM one evaluation of both
-// charge sets (shared tree passes, one near-field pass), else one after the other.
+// Demag of m and of v (Fem::compute_all, src/fem.h): one evaluation of both charge sets (the
+// FMM shares the tree passes and the near field, the direct sum the distances).
 static int demag_pair(fg_ctx *h) {
     Ctx &c = h->c;
-    if (c.opts.demag != FG_DEMAG_FMM || !c.src_q2) {
-        int s = demag_into(h, c.u[1], c.phi[1]);
-        if (s == FG_OK) s = demag_into(h, c.v[1], c.phiv[1]);
-        return s;
-    }
     CK(launch_charges_pair(c, c.u[1], c.v[1]));
-    CK(fmm_eval(c, 2));
-    CK(launch_phi_final(c, c.phi[1], 0));
-    CK(launch_phi_final(c, c.phiv[1], 1));
-    c.launches += 3 + fmm_launches_per_eval(c, 2);
+    if (c.opts.demag == FG_DEMAG_FMM) {
+        CK(fmm_eval(c, 2));
+        c.launches += fmm_launches_per_eval(c, 2);
+    } else {
+        CK(launch_p2p_direct(c, 2));
+        c.launches += 1;
+    }
+    CK(launch_phi_final(c, c.phi[1], c.phiv[1]));
+    c.launches += 2;
     return FG_OK;
 }
 
@@ -946,18 +949,16 @@ static int demag_increment(fg_ctx *h) {
         const cudaError_t se = fmm_eval(c, nq);
         c.charges32 = false;
         CK(se);
-        CK(launch_phi_final(c, c.phi[1], 0, c.phi[0]));
-        if (nq == 2) CK(launch_phi_final(c, c.phiv[1], 1, c.phiv[0]));
-        c.launches += 2 + nq + fmm_launches_per_eval(c, nq);
+        CK(launch_phi_final(c, c.phi[1], nq == 2 ? c.phiv[1] : nullptr, c.phi[0], c.phiv[0]));
+        c.launches += 3 + fmm_launches_per_eval(c, nq);
         return FG_OK;
     }
     if (nq == 2) CK(launch_charges_pair(c, c.u[1], c.v[1]));
     else CK(launch_charges(c, c.u[1]));
     const int s = fmm_eval_fp64(c, nq);
     if (s != FG_OK) return s;
-    CK(launch_phi_final(c, c.phi[1], 0));
-    if (nq == 2) CK(launch_phi_final(c, c.phiv[1], 1));
-    c.launches += 1 + nq;
+    CK(launch_phi_final(c, c.phi[1], nq == 2 ? c.phiv[1] : nullptr));
+    c.launches += 2;
     return FG_OK;
 }
 

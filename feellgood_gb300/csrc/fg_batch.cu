@@ -229,14 +229,13 @@ static cudaError_t batch_demag_all(Ctx &c) {
     const int nq = c.opts.first_order ? 1 : 2;
     cudaError_t e = nq == 2 ? launch_charges_pair(c, c.u[1], c.v[1]) : launch_charges(c, c.u[1], 0);
     if (e == cudaSuccess) e = fmm_eval(c, nq);
-    if (e == cudaSuccess) e = launch_phi_final(c, c.phi[1], 0);
-    if (e == cudaSuccess && nq == 2) e = launch_phi_final(c, c.phiv[1], 1);
+    if (e == cudaSuccess) e = launch_phi_final(c, c.phi[1], nq == 2 ? c.phiv[1] : nullptr);
     return e;
 }
 
 static int demag_launches(const Ctx &c) {
     const int nq = c.opts.first_order ? 1 : 2;
-    return 1 + nq + fmm_launches_per_eval(c, nq);
+    return 2 + fmm_launches_per_eval(c, nq);
 }
 
 // Whether a step uses the learned guess (after its training solves; the network of a batch is

@@ -272,6 +272,9 @@ struct Ctx {
     float4 *tri_ds = nullptr;  // energies: per triangle normal and 0.5 mu0 dMs w_g as double-single pairs
     double *pot = nullptr;       // nn
     double *pot2 = nullptr;      // nn, potential of src_q2
+    // direct sum: partial sums [set][share][magnetic node] (null with the FMM), shares
+    double *direct_part = nullptr;
+    int direct_nsplit = 0;
     // incremental demag of the FP32 + refinement path (fg_opts.demag_increment): NEXT's
     // potentials = CURRENT's + the potentials of NEXT - CURRENT (the potential is linear in
     // the field), the FP32 FMM acting on the change only, the sum kept in FP64
@@ -342,9 +345,11 @@ cudaError_t launch_apply(Ctx &c, double c0, const double *x, double *y);
 // set 0: charges into src_q / tri_slot, potential from pot; set 1: src_q2 / tri_slot2 / pot2
 cudaError_t launch_charges(Ctx &c, const double *m, int set = 0);
 cudaError_t launch_charges_pair(Ctx &c, const double *m, const double *v);  // sets 0 and 1 in one pass
-cudaError_t launch_p2p_direct(Ctx &c);
-// phi_out = base + (pot + corr) / (4 pi) (base nullptr: no base)
-cudaError_t launch_phi_final(Ctx &c, double *phi_out, int set = 0, const double *base = nullptr);
+int direct_splits(const Ctx &c);                 // shares of the sources of the direct sum
+cudaError_t launch_p2p_direct(Ctx &c, int nq);  // sets 0 .. nq - 1 into direct_part
+// phi = base + (pot + corr) / (4 pi) of set 0 and, phi1 not null, of set 1 (base null: no base)
+cudaError_t launch_phi_final(Ctx &c, double *phi0, double *phi1 = nullptr, const double *base0 = nullptr,
+                             const double *base1 = nullptr);
 cudaError_t launch_state_diff(Ctx &c);  // dstate32 = NEXT - CURRENT for u and v (FP32)
 cudaError_t launch_charges32(Ctx &c, int nq);  // FP32 charges of dstate32 (incremental demag)
 cudaError_t launch_energy(Ctx &c, const double Hext[3]);

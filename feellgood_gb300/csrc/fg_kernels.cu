@@ -1179,51 +1179,95 @@ __global__ void k_charges32(int nmt, int nft, const int4 *__restrict__ tet, cons
     }
 }
 
-// Exact FP64 direct sum pot_i = sum_s q_s / |x_i - y_s| over all sources, tiled through
-// shared memory (one thread per magnetic node).
-__global__ void __launch_bounds__(256) k_p2p_direct64(int nt, const int *__restrict__ tnode,
-                                                      const double *__restrict__ xyz, int ns,
-                                                      const double *__restrict__ sxyz,
-                                                      const double *__restrict__ q, double *__restrict__ pot) {
-    __shared__ double4 tile[256];
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+// 1 / sqrt(s) in FP64: the rsqrt.approx.ftz.f64 estimate y0 (its significand ends in the high
+// word, so y0^2 is exact) and one step of the third-order iteration y0 (1 + e/2 + 3 e^2/8),
+// e = 1 - s y0^2 (|e| < 2^-20, so the next term is below 2^-60): five FP64 operations.
+// s = 0 gives inf and s = inf gives 0, as 1 / sqrt does.
+__device__ __forceinline__ double rsqrt_step3(double s) {
+    double y0;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(s));
+    const unsigned hi = (unsigned)__double2hiint(y0);
+    const double e = fma(-s, y0 * y0, 1.0);
+    const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);
+    return hi - 1u < 0x7fefffffu ? y : y0;
+}
+
+// Exact FP64 direct sum pot_i = sum_s q_s / |x_i - y_s| of NQ charge sets: one thread per
+// magnetic node, the sources of the block's share (blockIdx.y of nsplit) tiled through shared
+// memory, partial sums to part[(set * nsplit + share) * nt + k], which k_phi_final adds in
+// share order. Bound by the FP64 pipe (2 operations per clock and SM): 3 subtractions, 3 for
+// r^2, 5 for the reciprocal distance and one per set, so both sets share 11 of the 13; blocks
+// of 64 threads waste few lanes on a small mesh, and since one warp per scheduler keeps that
+// pipe busy the split only has to give every scheduler work.
+constexpr int DIRECT_TPB = 64;
+template <int NQ>
+__global__ void __launch_bounds__(DIRECT_TPB) k_p2p_direct64(int nt, const int *__restrict__ tnode,
+                                                             const double *__restrict__ xyz, int ns,
+                                                             const double *__restrict__ sxyz,
+                                                             const double *__restrict__ q0,
+                                                             const double *__restrict__ q1, double *__restrict__ part) {
+    __shared__ double4 tile[DIRECT_TPB];
+    __shared__ double tile2[NQ == 2 ? DIRECT_TPB : 1];
+    const int k = blockIdx.x * DIRECT_TPB + threadIdx.x;
+    const int nsplit = gridDim.y;
+    const int s0 = (int)((long long)ns * blockIdx.y / nsplit), s1 = (int)((long long)ns * (blockIdx.y + 1) / nsplit);
     double x = 0, y = 0, z = 0;
-    int node = -1;
     if (k < nt) {
-        node = tnode[k];
-        x = xyz[3 * node];
-        y = xyz[3 * node + 1];
-        z = xyz[3 * node + 2];
+        const size_t n = 3 * (size_t)tnode[k];
+        x = xyz[n];
+        y = xyz[n + 1];
+        z = xyz[n + 2];
     }
-    double acc = 0.0;
-    for (int base = 0; base < ns; base += 256) {
+    double a0 = 0.0, a1 = 0.0;
+    for (int base = s0; base < s1; base += DIRECT_TPB) {
         const int s = base + threadIdx.x;
-        if (s < ns) tile[threadIdx.x] = make_double4(sxyz[3 * s], sxyz[3 * s + 1], sxyz[3 * s + 2], q[s]);
-        else tile[threadIdx.x] = make_double4(0, 0, 0, 0);
+        if (s < s1) {
+            const size_t o = 3 * (size_t)s;
+            tile[threadIdx.x] = make_double4(sxyz[o], sxyz[o + 1], sxyz[o + 2], q0[s]);
+            if constexpr (NQ == 2) tile2[threadIdx.x] = q1[s];
+        }
         __syncthreads();
-        const int cnt = min(256, ns - base);
+        const int cnt = min(DIRECT_TPB, s1 - base);
+#pragma unroll 4
         for (int j = 0; j < cnt; j++) {
             const double4 t = tile[j];
             const double dx = x - t.x, dy = y - t.y, dz = z - t.z;
-            acc += t.w * rsqrt(dx * dx + dy * dy + dz * dz);
+            const double r = rsqrt_step3(fma(dx, dx, fma(dy, dy, dz * dz)));
+            a0 = fma(t.w, r, a0);
+            if constexpr (NQ == 2) a1 = fma(tile2[j], r, a1);
         }
         __syncthreads();
     }
-    if (node >= 0) pot[node] = acc;
+    if (k < nt) {
+        part[(size_t)blockIdx.y * nt + k] = a0;
+        if constexpr (NQ == 2) part[((size_t)nsplit + blockIdx.y) * nt + k] = a1;
+    }
 }
 
-// phi_i = (pot_i + corr_i) / (4 pi), src/fmm_demag.h:211-223; corr gathered per node.
+// phi_i = (pot_i + corr_i) / (4 pi), src/fmm_demag.h:211-223; corr gathered per node. The
+// potential is pot[i], or the sum of nsplit partial sums of the direct sum (pot null). Grid y
+// selects the charge set.
+struct PhiSet {
+    const double *tri_slot, *pot, *part, *base;
+    double *phi;
+};
 __global__ void k_phi_final(int nt, const int *__restrict__ tnode, const int *__restrict__ tinc_ptr,
-                            const int *__restrict__ tinc, const double *__restrict__ tri_slot,
-                            const double *__restrict__ pot, const double *__restrict__ base,
-                            double *__restrict__ phi) {
+                            const int *__restrict__ tinc, int nsplit, PhiSet set0, PhiSet set1) {
+    const PhiSet st = blockIdx.y ? set1 : set0;
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nt) return;
     const int i = tnode[k];
     double corr = 0.0;
-    for (int j = tinc_ptr[i]; j < tinc_ptr[i + 1]; j++) corr += tri_slot[tinc[j]];
-    const double p = (pot[i] + corr) / (4 * M_PI);
-    phi[i] = base ? base[i] + p : p;
+    for (int j = tinc_ptr[i]; j < tinc_ptr[i + 1]; j++) corr += st.tri_slot[tinc[j]];
+    double pot = 0.0;
+    if (st.pot) {
+        pot = st.pot[i];
+    } else {
+#pragma unroll 8
+        for (int b = 0; b < nsplit; b++) pot += st.part[(size_t)b * nt + k];
+    }
+    const double p = (pot + corr) / (4 * M_PI);
+    st.phi[i] = st.base ? st.base[i] + p : p;
 }
 
 // d = NEXT - CURRENT of u (first 3 nn) and of v (next 3 nn).
@@ -1782,19 +1826,32 @@ cudaError_t launch_charges_pair(Ctx &c, const double *m, const double *v) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_p2p_direct(Ctx &c) {
+// Shares of the sources per block of nodes: about 16 blocks per SM in all (4 warps per
+// scheduler; the FP64 pipe is full with one, the rest even out the last wave), but at least 32
+// sources in each, below which the fixed cost of a block shows.
+int direct_splits(const Ctx &c) {
+    const int tiles = nblocks(std::max(1, c.n_mag_nodes), DIRECT_TPB);
+    return std::max(1, std::min(nblocks(16 * (long)c.nsm, tiles), c.nsrc / 32));
+}
+
+cudaError_t launch_p2p_direct(Ctx &c, int nq) {
     if (c.n_mag_nodes == 0) return cudaSuccess;
-    k_p2p_direct64<<<nblocks(c.n_mag_nodes, 256), 256, 0, c.stream>>>(c.n_mag_nodes, c.mag_nodes, c.xyz, c.nsrc,
-                                                                        c.src_xyz, c.src_q, c.pot);
+    if (!c.direct_part || (nq == 2 && !c.src_q2)) return cudaErrorInvalidValue;
+    const dim3 grid(nblocks(c.n_mag_nodes, DIRECT_TPB), c.direct_nsplit);
+    (nq == 2 ? k_p2p_direct64<2> : k_p2p_direct64<1>)<<<grid, DIRECT_TPB, 0, c.stream>>>(
+        c.n_mag_nodes, c.mag_nodes, c.xyz, c.nsrc, c.src_xyz, c.src_q, c.src_q2, c.direct_part);
     return cudaGetLastError();
 }
 
-cudaError_t launch_phi_final(Ctx &c, double *phi_out, int set, const double *base) {
+cudaError_t launch_phi_final(Ctx &c, double *phi0, double *phi1, const double *base0, const double *base1) {
     if (c.n_mag_nodes == 0) return cudaSuccess;
-    const double *ts = set ? c.tri_slot2 : c.tri_slot, *pot = set ? c.pot2 : c.pot;
-    if (!ts || !pot) return cudaErrorInvalidValue;
-    k_phi_final<<<nblocks(c.n_mag_nodes, 256), 256, 0, c.stream>>>(c.n_mag_nodes, c.mag_nodes, c.tinc_ptr, c.tinc,
-                                                                     ts, pot, base, phi_out);
+    if (phi1 && (!c.tri_slot2 || !c.pot2)) return cudaErrorInvalidValue;
+    const size_t n = (size_t)c.direct_nsplit * c.n_mag_nodes;
+    const double *part = c.direct_part;
+    const PhiSet s0{c.tri_slot, part ? nullptr : c.pot, part, base0, phi0};
+    const PhiSet s1{c.tri_slot2, part ? nullptr : c.pot2, part ? part + n : nullptr, base1, phi1};
+    k_phi_final<<<dim3(nblocks(c.n_mag_nodes, 128), phi1 ? 2 : 1), 128, 0, c.stream>>>(
+        c.n_mag_nodes, c.mag_nodes, c.tinc_ptr, c.tinc, c.direct_nsplit, s0, s1);
     return cudaGetLastError();
 }
 
