@@ -724,7 +724,7 @@ void fg_destroy(fg_ctx *h) {
                     c.Sval32, c.A, c.Ainv, c.A32, c.tri, c.tri_c, c.tinc_ptr, c.tinc, c.src_xyz, c.mag_nodes, c.u[0], c.u[1],
                     c.v[0], c.v[1], c.phi[0], c.phi[1], c.phiv[0], c.phiv[1], c.ep, c.eq, c.ep32, c.eq32, c.Dl32,
                     c.slot, c.Dl, c.rhs, c.x, c.bv, c.W, c.fv, c.partial, c.bar, c.dres, c.src_q, c.tri_slot,
-                    c.pot, c.epart, c.src_dst, c.src_q2, c.tri_slot2, c.pot2, c.direct_part, c.tri_be, c.hsp, c.da_ds, c.J_ds, c.state_ds,
+                    c.pot, c.epart, c.src_dst, c.src_q2, c.tri_slot2, c.pot2, c.direct_part, c.fmm_err, c.tri_be, c.hsp, c.da_ds, c.J_ds, c.state_ds,
                     c.dstate32, c.da32, c.cq32, c.src_qf, c.src_q2f, c.tri_ds, c.tri32};
     for (void *p : ptrs)
         if (p) cudaFree(p);

@@ -96,7 +96,18 @@ struct FmmTree {
     struct TcLaunch { int unit0 = 0, nunit = 0, comb0 = 0, ncomb = 0; };
     std::vector<TcLaunch> tc_m2m, tc_l2l;        // per level
     TcLaunch tc_m2l;
-    int *tc_err = nullptr;                       // FG_ETIMEDOUT when a pipeline wait expired
+    // FP64 path: translations by exact digit products on the tensor cores (fg_fmm_oz.cu)
+    struct OzLaunch { int unit0 = 0, nunit = 0, tile0 = 0, ntile = 0, nsplit = 0; };
+    std::vector<OzLaunch> oz_m2m, oz_l2l;        // per level
+    OzLaunch oz_m2l;
+    int *oz_cells = nullptr, *oz_codes = nullptr, *oz_wexp = nullptr, *oz_leaves = nullptr;
+    int4 *oz_units = nullptr;
+    int2 *oz_fin = nullptr;
+    double *oz_scratch = nullptr;
+    unsigned char *oz_digits = nullptr;          // of M up to M2L, of F from there
+    float *oz_scale = nullptr;
+    unsigned char *oz_img[3] = {nullptr, nullptr, nullptr};  // M2M, M2L, L2L
+    float *oz_rows[3] = {nullptr, nullptr, nullptr};
     float *Mh = nullptr, *Ml = nullptr, *Fh = nullptr, *Fl = nullptr;  // hi/lo splits of M and F
     unsigned char *img_m2l = nullptr, *img_m2m = nullptr, *img_l2l = nullptr;  // operator images
     int *dst_keep = nullptr;
@@ -592,100 +603,6 @@ __global__ void __launch_bounds__(160) k_translate(int n_out, int out0, int ncod
         T *o = out + (size_t)(out0 + c) * NR + rg * RT;
 #pragma unroll
         for (int i = 0; i < RT; i++) o[i] = accumulate ? o[i] + acc[i][j] : acc[i][j];
-    }
-}
-
-// FP64-path translations in double-single arithmetic on the FP32 pipes (GB300's FP64 pipe
-// does 2 DFMA per clock and SM, 1/64 of its FP32 rate): the same batched GEMM as
-// k_translate, both charge sets of a block of DS_TB output cells as its 2 DS_TB columns, the
-// operator and the inputs split into FP32 pairs hi + lo on their way into shared memory,
-// every product exact through fma (Dekker's TwoProduct) and summed with Knuth's two-sum,
-// the running sum renormalised once per code (about 44 significant bits), the result
-// rounded to FP64 once.
-constexpr int DS_TB = 16, DS_COLS = 2 * DS_TB, DS_CT = 2, DS_BLD = DS_COLS + 1;
-constexpr int tr_ds_smem() { return (NR * NR + NR * DS_BLD) * (int)sizeof(float2); }
-
-__device__ __forceinline__ float2 ds_split(double x) {
-    const float h = (float)x;
-    return make_float2(h, (float)(x - (double)h));
-}
-
-__global__ void __launch_bounds__(160, 2) k_translate_ds(int n_out, int out0, int ncode, const int *__restrict__ tab,
-                                                         const double *__restrict__ ops, const double *in,
-                                                         double *out, int accumulate, int nset, size_t set_stride) {
-    // in and out may be the same array (M2M, L2L): the cells read and written are disjoint.
-    constexpr int RT = 10;
-    extern __shared__ unsigned char smem_raw[];
-    float2 *AT = reinterpret_cast<float2 *>(smem_raw);  // AT[k * NR + row] = Op[row][k]
-    float2 *Bs = AT + NR * NR;                           // [NR][DS_BLD]: column set * DS_TB + cell
-    __shared__ int srcs[DS_TB];
-    const int tid = threadIdx.x, rg = tid / 16, cg = tid % 16;
-    const int c_begin = blockIdx.x * DS_TB;
-    float ah[RT][DS_CT], al[RT][DS_CT];
-#pragma unroll
-    for (int i = 0; i < RT; i++)
-#pragma unroll
-        for (int j = 0; j < DS_CT; j++) ah[i][j] = al[i][j] = 0.f;
-    for (int code = 0; code < ncode; code++) {
-        int sc = -1;
-        if (tid < DS_TB && c_begin + tid < n_out) sc = tab[(size_t)(out0 + c_begin + tid) * ncode + code];
-        if (tid < DS_TB) srcs[tid] = sc;
-        if (!__syncthreads_or(sc >= 0)) continue;
-        for (int e = tid; e < NR * NR; e += blockDim.x) {
-            const int row = e / NR, k = e % NR;
-            AT[k * NR + row] = ds_split(ops[(size_t)code * NR * NR + e]);
-        }
-        for (int e = tid; e < NR * DS_COLS; e += blockDim.x) {
-            const int col = e / NR, k = e % NR, cell = col % DS_TB, set = col / DS_TB;
-            const int src = srcs[cell];
-            Bs[k * DS_BLD + col] = (src >= 0 && set < nset) ? ds_split(in[set * set_stride + (size_t)src * NR + k])
-                                                              : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-#pragma unroll 2
-        for (int k = 0; k < NR; k++) {
-            float2 a[RT], b[DS_CT];
-#pragma unroll
-            for (int i = 0; i < RT; i++) a[i] = AT[k * NR + rg * RT + i];
-#pragma unroll
-            for (int j = 0; j < DS_CT; j++) b[j] = Bs[k * DS_BLD + cg * DS_CT + j];
-#pragma unroll
-            for (int i = 0; i < RT; i++)
-#pragma unroll
-                for (int j = 0; j < DS_CT; j++) {
-                    // (ah, al) += a b: exact leading product and cross terms, two-sum into hi
-                    const float p = a[i].x * b[j].x;
-                    float e = fmaf(a[i].x, b[j].x, -p);
-                    e = fmaf(a[i].x, b[j].y, e);
-                    e = fmaf(a[i].y, b[j].x, e);
-                    const float s = ah[i][j] + p;
-                    const float bb = s - ah[i][j];
-                    const float err = (ah[i][j] - (s - bb)) + (p - bb);
-                    ah[i][j] = s;
-                    al[i][j] += e + err;
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < RT; i++)
-#pragma unroll
-            for (int j = 0; j < DS_CT; j++) {  // renormalise: |lo| back to half an ulp of hi
-                const float s = ah[i][j] + al[i][j];
-                al[i][j] = al[i][j] - (s - ah[i][j]);
-                ah[i][j] = s;
-            }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int j = 0; j < DS_CT; j++) {
-        const int col = cg * DS_CT + j, cell = col % DS_TB, set = col / DS_TB;
-        const int c = c_begin + cell;
-        if (c >= n_out || set >= nset) continue;
-        double *o = out + set * set_stride + (size_t)(out0 + c) * NR + rg * RT;
-#pragma unroll
-        for (int i = 0; i < RT; i++) {
-            const double v = (double)ah[i][j] + (double)al[i][j];
-            o[i] = accumulate ? o[i] + v : v;
-        }
     }
 }
 
@@ -1298,6 +1215,39 @@ static const FmmOps &fmm_ops() {
     return ops;
 }
 
+// Power-of-two weights of the coefficients for the digit products (fg_fmm_oz.cu): multipoles by
+// the inverse of the rms of Ups_n^m over the cell times 0.6^-n, locals by the inverse of the
+// rms of The_n^m over the M2L offsets times 2.5^n. The factors share the decay with the degree
+// between the operator and the expansion (of 1, 0.8, 0.6, 0.5 and of 1, 1.5, 2, 3 the errors were
+// smallest there: 2e-16 to 2e-14 against up to 1e-12 without).
+static void oz_weights(int *wM, int *wF) {
+    const int P = FMM_P, G = 8;
+    std::vector<double> m2(NR, 0.0), f2(NR, 0.0);
+    std::vector<cd> X;
+    for (int a = 0; a < G * G * G; a++) {
+        ups_host((a % G + 0.5) / G - 0.5, (a / G % G + 0.5) / G - 0.5, (a / G / G + 0.5) / G - 0.5, P, X);
+        for (int n = 0; n <= P; n++)
+            for (int m = 0; m <= n; m++) {
+                const cd v = X[cidx(n, m)];
+                m2[ridx(n, m, 0)] += v.real() * v.real() / (G * G * G);
+                if (m) m2[ridx(n, m, 1)] += v.imag() * v.imag() / (G * G * G);
+            }
+    }
+    for (int code = 0; code < NCODE_M2L; code++) {
+        const int d[3] = {code / 49 - 3, code / 7 % 7 - 3, code % 7 - 3};
+        if (std::abs(d[0]) <= 1 && std::abs(d[1]) <= 1 && std::abs(d[2]) <= 1) continue;
+        the_host(d[0], d[1], d[2], P, X);
+        for (int n = 0; n <= P; n++)
+            for (int m = 0; m <= n; m++)
+                for (int part = 0; part < (m ? 2 : 1); part++) f2[ridx(n, m, part)] += std::norm(X[cidx(n, m)]) / 316.0;
+    }
+    for (int n = 0; n <= P; n++)
+        for (int k = n * n; k < (n + 1) * (n + 1); k++) {
+            wM[k] = -(int)std::lrint(0.5 * std::log2(m2[k]) - n * std::log2(0.6));
+            wF[k] = -(int)std::lrint(0.5 * std::log2(f2[k]) + n * std::log2(2.5));
+        }
+}
+
 void fmm_free(Ctx &c);
 static int fmm_build_forest(Ctx &c, int L);
 template <typename T>
@@ -1354,6 +1304,10 @@ int fmm_build(Ctx &c) {
     const auto t_begin = std::chrono::steady_clock::now();
     c.tree_wall_ms = c.tree_sort_ms = 0.0;
     const std::vector<SamplePts> S = split_samples(c);
+    if (!c.fmm_err) {
+        FCK(cudaMalloc(&c.fmm_err, sizeof(int)));
+        FCK(cudaMemset(c.fmm_err, 0, sizeof(int)));
+    }
     // mean number of sources per occupied leaf at each depth, over all samples
     std::vector<double> occ(11, 0.0);
     {
@@ -1550,6 +1504,7 @@ static int fmm_build_forest(Ctx &c, int L) {
     std::vector<int> nsub_src(ncell, 0), nsub_tgt(ncell, 0);
     std::vector<int> m2m_tab((size_t)ncell * 8, -1), l2l_tab((size_t)ncell * 8, -1);
     std::vector<int> m2l_tab((size_t)ncell * NCODE_M2L, -1);
+    std::vector<unsigned char> octant(ncell, 0);  // within the parent
     std::vector<int> near_ptr(nleaf + 1, 0), near_leaf;
     size_t src_off = 0, tgt_off = 0, nm2l = 0, np2p = 0;
     int ijk[3];
@@ -1601,6 +1556,7 @@ static int fmm_build_forest(Ctx &c, int L) {
             const int n = 1 << l;
             for (size_t i = 0; i < H.keys[l].size(); i++) {
                 const int gc = base[l][g] + (int)i;
+                octant[gc] = (unsigned char)(H.keys[l][i] & 7);
                 if (nsub_tgt[gc] == 0) continue;
                 decode(H.keys[l][i], ijk);
                 const int px = ijk[0] >> 1, py = ijk[1] >> 1, pz = ijk[2] >> 1;
@@ -1710,8 +1666,6 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(up(&t->tc_comb, comb));
         t->nslot_floats = (size_t)std::max(1, nslot) * translate_tc_tile() * NR;
         FCK(cudaMalloc(&t->tc_scratch, sizeof(float) * t->nslot_floats * t->nq));
-        FCK(cudaMalloc(&t->tc_err, sizeof(int)));
-        FCK(cudaMemset(t->tc_err, 0, sizeof(int)));
         FCK(translate_tc_setup());
         const size_t nexp = (size_t)ncell * NR * t->nq;
         FCK(cudaMalloc(&t->Mh, nexp * sizeof(float)));
@@ -1729,6 +1683,124 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(up((float **)&t->img_m2m, im2m));
         FCK(up((float **)&t->img_l2l, il2l));
     }
+    t->ds = !fp32 && c.opts.fmm_native_fp64 == 0;
+    if (t->ds) {
+        std::vector<int> cells, codes;
+        std::vector<int4> units;
+        std::vector<int2> fin;
+        int nslot = 0;
+        struct Tile { std::vector<int> cells, codes; };
+        auto tiles_of = [&](const std::vector<int> &list, int ncode, const std::vector<int> &tab) {
+            std::vector<Tile> T;
+            for (size_t b = 0; b < list.size(); b += OZ_TILE) {
+                Tile x;
+                x.cells.assign(list.begin() + b, list.begin() + std::min(list.size(), b + OZ_TILE));
+                for (int code = 0; code < ncode; code++)
+                    for (int cc : x.cells)
+                        if (tab[(size_t)cc * ncode + code] >= 0) {
+                            x.codes.push_back(code);
+                            break;
+                        }
+                x.cells.resize(OZ_TILE, -1);
+                T.push_back(std::move(x));
+            }
+            return T;
+        };
+        // tiles of a level: its cells in order, or the cells of each octant apart, whichever needs
+        // fewer (tile, code) products (a tile costs about one more)
+        auto level_tiles = [&](int l, int ncode, const std::vector<int> &tab) {
+            std::vector<int> all;
+            std::vector<std::vector<int>> oct(8);
+            for (int k = t->lev_begin[l]; k < t->lev_begin[l + 1]; k++) {
+                all.push_back(k);
+                oct[octant[k]].push_back(k);
+            }
+            std::vector<Tile> A = tiles_of(all, ncode, tab), B;
+            for (const auto &o : oct)
+                for (auto &x : tiles_of(o, ncode, tab)) B.push_back(std::move(x));
+            auto cost = [](const std::vector<Tile> &T) {
+                size_t n = T.size();
+                for (const auto &x : T) n += x.codes.size();
+                return n;
+            };
+            return cost(B) < cost(A) ? B : A;
+        };
+        // units of at most mc codes: the size among the candidates whose units, handed in order to
+        // the earliest free SM, finish first (a unit costs its codes plus about 2)
+        auto plan = [&](const std::vector<Tile> &T) {
+            int mc = 64;
+            double best = 1e300;
+            for (int k : {64, 48, 32, 24, 16, 12, 8, 6, 4, 3, 2, 1}) {
+                std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+                for (int q = 0; q < std::max(1, c.nsm); q++) free_at.push(0.0);
+                double span = 0.0;
+                for (const Tile &x : T) {
+                    const int n = (int)x.codes.size(), nu = (n + k - 1) / k;
+                    for (int q = 0; q < nu; q++) {
+                        const double t1 = free_at.top() + 2.0 + ((long)n * (q + 1) / nu - (long)n * q / nu);
+                        free_at.pop();
+                        free_at.push(t1);
+                        span = std::max(span, t1);
+                    }
+                }
+                if (span < best) {
+                    best = span;
+                    mc = k;
+                }
+            }
+            FmmTree::OzLaunch l;
+            l.unit0 = (int)units.size();
+            l.tile0 = (int)fin.size();
+            int slot = 0;
+            for (const Tile &x : T) {
+                const int n = (int)x.codes.size(), nu = (n + mc - 1) / mc, first = (int)codes.size();
+                for (int q = 0; q < nu; q++)
+                    units.push_back(make_int4((int)fin.size(), first + (int)((long)n * q / nu),
+                                              first + (int)((long)n * (q + 1) / nu), slot + q));
+                fin.push_back(make_int2(slot, nu));
+                slot += nu;
+                codes.insert(codes.end(), x.codes.begin(), x.codes.end());
+                cells.insert(cells.end(), x.cells.begin(), x.cells.end());
+            }
+            l.nunit = (int)units.size() - l.unit0;
+            l.ntile = (int)fin.size() - l.tile0;
+            nslot = std::max(nslot, slot);
+            return l;
+        };
+        t->oz_m2m.assign(L + 1, FmmTree::OzLaunch());
+        t->oz_l2l.assign(L + 1, FmmTree::OzLaunch());
+        for (int l = L - 1; l >= 2; l--) t->oz_m2m[l] = plan(level_tiles(l, 8, m2m_tab));
+        std::vector<Tile> all;
+        int nsplit = 0;  // listed cells above the leaves: their locals are translated further
+        for (int l = 2; l <= L; l++) {
+            if (l == L) nsplit = OZ_TILE * (int)all.size();
+            for (auto &x : level_tiles(l, NCODE_M2L, m2l_tab)) all.push_back(std::move(x));
+        }
+        t->oz_m2l = plan(all);
+        t->oz_m2l.nsplit = nsplit;
+        for (int l = 3; l <= L; l++) t->oz_l2l[l] = plan(level_tiles(l, 8, l2l_tab));
+        std::vector<int> wexp(2 * NR), leaves(nleaf);
+        oz_weights(wexp.data(), wexp.data() + NR);
+        for (int k = 0; k < nleaf; k++) leaves[k] = t->leaf0 + k;
+        static const OzImages im[3] = {oz_images(ops.m2m, 8, wexp.data()), oz_images(ops.m2l, NCODE_M2L, wexp.data()),
+                                       oz_images(ops.l2l, 8, wexp.data() + NR)};
+        for (int k = 0; k < 3; k++) {
+            FCK(up(&t->oz_img[k], im[k].img));
+            FCK(up(&t->oz_rows[k], im[k].row_scale));
+        }
+        FCK(up(&t->oz_cells, cells));
+        FCK(up(&t->oz_codes, codes));
+        FCK(up(&t->oz_units, units));
+        FCK(up(&t->oz_fin, fin));
+        FCK(up(&t->oz_wexp, wexp));
+        FCK(up(&t->oz_leaves, leaves));
+        FCK(cudaMalloc(&t->oz_scratch, sizeof(double) * std::max(1, nslot) * OZ_TILE * NR * t->nq));
+        FCK(cudaMalloc(&t->oz_digits, (size_t)ncell * t->nq * OZ_CELL_BYTES));
+        FCK(cudaMemset(t->oz_digits, 0, (size_t)ncell * t->nq * OZ_CELL_BYTES));
+        FCK(cudaMalloc(&t->oz_scale, sizeof(float) * ncell * t->nq));
+        FCK(cudaMemset(t->oz_scale, 0, sizeof(float) * ncell * t->nq));
+        FCK(oz_setup());
+    }
     FCK(up(&t->leaf_src, leaf_src));
     FCK(up(&t->leaf_tgt, leaf_tgt));
     FCK(up(&t->tgt_node, tgt_node));
@@ -1741,7 +1813,6 @@ static int fmm_build_forest(Ctx &c, int L) {
     FCK(up(&t->near_leaf, near_leaf));
     FCK(up_as<double>(&t->sloc, sloc, fp32));
     FCK(up_as<double>(&t->tloc, tloc, fp32));
-    t->ds = !fp32 && c.opts.fmm_native_fp64 == 0;
     if (t->ds) {
         // x = hi + lo, hi on the 2^-20 grid (|x| < 4 leaf units: exact in FP32)
         auto split = [](const std::vector<double> &v, std::vector<float4> &hi, std::vector<float4> &lo) {
@@ -1768,9 +1839,11 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(up(&t->ds_tgt_hi, th));
         FCK(up(&t->ds_tgt_lo, tl));
     }
-    FCK(up_as<double>(&t->op_m2l, ops.m2l, fp32));
-    FCK(up_as<double>(&t->op_m2m, ops.m2m, fp32));
-    FCK(up_as<double>(&t->op_l2l, ops.l2l, fp32));
+    if (!t->ds) {
+        FCK(up_as<double>(&t->op_m2l, ops.m2l, fp32));
+        FCK(up_as<double>(&t->op_m2m, ops.m2m, fp32));
+        FCK(up_as<double>(&t->op_l2l, ops.l2l, fp32));
+    }
     if (c.src_dst) cudaFree(c.src_dst);
     c.src_dst = nullptr;
     FCK(up(&c.src_dst, src_dst));
@@ -1792,7 +1865,6 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(cudaFuncSetAttribute(k_translate<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<float>()));
     } else {
         FCK(cudaFuncSetAttribute(k_translate<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<double>()));
-        FCK(cudaFuncSetAttribute(k_translate_ds, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_ds_smem()));
     }
     if (c.opts.profile)
         for (auto &set : t->ev)
@@ -1812,9 +1884,11 @@ void fmm_free(Ctx &c) {
     if (!t) return;
     void *ptrs[] = {t->leaf_scale, t->leaf_src, t->leaf_tgt, t->tgt_node, t->sloc, t->tloc, t->leaf_ijk, t->m2l_tab, t->m2m_tab,
                     t->l2l_tab, t->near_ptr, t->near_leaf, t->M, t->F, t->op_m2l, t->op_m2m, t->op_l2l,
-                    t->tc_code, t->tc_units, t->tc_comb, t->tc_scratch, t->tc_err, t->Mh, t->Ml, t->Fh, t->Fl,
+                    t->tc_code, t->tc_units, t->tc_comb, t->tc_scratch, t->Mh, t->Ml, t->Fh, t->Fl,
                     t->img_m2l, t->img_m2m, t->img_l2l, t->ds_src_hi, t->ds_src_lo, t->ds_tgt_hi, t->ds_tgt_lo,
-                    t->sq2, t->ds_q2};
+                    t->sq2, t->ds_q2, t->oz_cells, t->oz_codes, t->oz_wexp, t->oz_leaves, t->oz_units, t->oz_fin,
+                    t->oz_scratch, t->oz_digits, t->oz_scale, t->oz_img[0], t->oz_img[1], t->oz_img[2], t->oz_rows[0],
+                    t->oz_rows[1], t->oz_rows[2]};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     for (auto &set : t->ev)
@@ -1941,17 +2015,12 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
             a.out_hi = kind == M2M ? t.Mh : t.Fh;
             a.out_lo = kind == M2M ? t.Ml : t.Fl;
             a.accumulate = kind == L2L;
-            a.tile_code = t.tc_code; a.err = t.tc_err; a.terms = 7;
+            a.tile_code = t.tc_code; a.err = c.fmm_err; a.terms = 7;
             a.units = t.tc_units + tl.unit0; a.nunits = tl.nunit;
             a.comb = t.tc_comb + tl.comb0; a.ncomb = tl.ncomb; a.scratch = t.tc_scratch;
             a.nset = nq; a.set_io = sstride; a.set_scratch = t.nslot_floats;
             const cudaError_t e = launch_translate_tc(c.stream, a);
             if (e != cudaSuccess && terr == cudaSuccess) terr = e;
-        } else if (sizeof(T) == 8 && t.ds) {  // FP64 path: double-single, both sets per launch
-            const double *ops = (const double *)(kind == M2M ? t.op_m2m : kind == M2L ? t.op_m2l : t.op_l2l);
-            double *in = (double *)(kind == L2L ? F : M), *out = (double *)(kind == M2M ? M : F);
-            k_translate_ds<<<(n + DS_TB - 1) / DS_TB, 160, tr_ds_smem(), c.stream>>>(n, out0, ncode, tab, ops, in, out,
-                                                                                     kind == L2L, nq, sstride);
         } else {
             const void *ops = kind == M2M ? t.op_m2m : kind == M2L ? t.op_m2l : t.op_l2l;
             for (int q = 0; q < nq; q++) {
@@ -1961,9 +2030,37 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
             }
         }
     };
+    // FP64 path: exact digit products on the tensor cores, then the sums of the units' partial
+    // results and the digits of the next translation's inputs
+    auto note = [&](cudaError_t e) {
+        if (e != cudaSuccess && terr == cudaSuccess) terr = e;
+    };
+    OzFinish fa{};
+    if (t.ds) {
+        fa.ncell = t.ncell; fa.nset = nq; fa.scratch = t.oz_scratch; fa.digits = t.oz_digits; fa.scale = t.oz_scale;
+        fa.io = (double *)M; fa.cells = t.oz_leaves; fa.nlist = t.nleaf; fa.accumulate = 1; fa.split = t.nleaf;
+        fa.wexp = t.oz_wexp;
+        note(launch_oz_finish(c.stream, fa));  // digits of the leaves' multipoles
+    }
+    auto translate_oz = [&](int kind, const FmmTree::OzLaunch &ol, int nsplit) {
+        if (!ol.ntile) return;
+        OzArgs a{};
+        a.ncode = kind == M2L ? NCODE_M2L : 8; a.ncell = t.ncell; a.nset = nq;
+        a.cells = t.oz_cells; a.codes = t.oz_codes;
+        a.tab = kind == M2M ? t.m2m_tab : kind == M2L ? t.m2l_tab : t.l2l_tab;
+        a.op_img = t.oz_img[kind]; a.row_scale = t.oz_rows[kind];
+        a.in = t.oz_digits; a.in_scale = t.oz_scale;
+        a.units = t.oz_units + ol.unit0; a.nunits = ol.nunit; a.scratch = t.oz_scratch; a.err = c.fmm_err;
+        note(launch_translate_oz(c.stream, a));
+        fa.io = (double *)(kind == M2M ? M : F);
+        fa.cells = t.oz_cells + (size_t)ol.tile0 * OZ_TILE; fa.nlist = ol.ntile * OZ_TILE; fa.fin = t.oz_fin + ol.tile0;
+        fa.accumulate = kind == L2L; fa.split = nsplit; fa.wexp = t.oz_wexp + (kind == M2M ? 0 : NR);
+        note(launch_oz_finish(c.stream, fa));
+    };
     const FmmTree::TcLaunch none;
     for (int l = L - 1; l >= 2; l--)
-        translate(M2M, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_m2m[l] : none);
+        if (t.ds) translate_oz(M2M, t.oz_m2m[l], t.oz_m2m[l].ntile * OZ_TILE);
+        else translate(M2M, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_m2m[l] : none);
     if (prof) cudaEventRecord(ev[2], c.stream);
     if (split) {  // the near field beside M2L and L2L
         cudaEventRecord(c.ev_fork, c.stream);
@@ -1975,10 +2072,12 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
         cudaEventRecord(c.ev_join, c.stream2);
         ns.near_only = 0;
     }
-    translate(M2L, t.ncell, 0, t.tc_m2l);
+    if (t.ds) translate_oz(M2L, t.oz_m2l, t.oz_m2l.nsplit);
+    else translate(M2L, t.ncell, 0, t.tc_m2l);
     if (prof) cudaEventRecord(ev[3], c.stream);
     for (int l = 3; l <= L; l++)
-        translate(L2L, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_l2l[l] : none);
+        if (t.ds) translate_oz(L2L, t.oz_l2l[l], l < L ? t.oz_l2l[l].ntile * OZ_TILE : 0);
+        else translate(L2L, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_l2l[l] : none);
     if (prof) cudaEventRecord(ev[4], c.stream);
     if (split) {
         cudaStreamWaitEvent(c.stream, c.ev_join, 0);
@@ -2055,9 +2154,16 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
     if (!t) return 0;
     int n = 2;  // P2M, L2P + P2P (both sets in one launch each)
     if (c.opts.fmm_overlap != 0 && c.stream2) n += 1;  // L2P after the overlapped near field
-    // tensor-core and double-single translations: both sets in one launch (the tensor-core
-    // form adds one combine launch); the k_translate form launches once per set
-    const int per = (t->tc || (!t->fp32 && t->ds)) ? 1 : nq;
+    if (t->ds) {  // digits of the leaves, then per translation the products and the sums
+        n += 1;
+        for (int l = 2; l <= t->L - 1; l++) n += (t->oz_m2m[l].nunit > 0) + (t->oz_m2m[l].ntile > 0);
+        n += (t->oz_m2l.nunit > 0) + (t->oz_m2l.ntile > 0);
+        for (int l = 3; l <= t->L; l++) n += (t->oz_l2l[l].nunit > 0) + (t->oz_l2l[l].ntile > 0);
+        return n;
+    }
+    // tensor-core translations: both sets in one launch and one combine launch; the k_translate
+    // form launches once per set
+    const int per = t->tc ? 1 : nq;
     for (int l = 2; l <= t->L - 1; l++) n += per + (t->tc && t->tc_m2m[l].ncomb > 0);
     n += per + (t->tc && t->tc_m2l.ncomb > 0);
     for (int l = 3; l <= t->L; l++) n += per + (t->tc && t->tc_l2l[l].ncomb > 0);
@@ -2065,8 +2171,7 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
 }
 
 int *fmm_error_flag(const Ctx &c) {
-    const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
-    return t ? t->tc_err : nullptr;
+    return c.fmm_err;
 }
 
 int fmm_info(const Ctx &c, int *L, int *nleaf, double *n_m2l, double *n_p2p) {

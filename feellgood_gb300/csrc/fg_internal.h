@@ -248,6 +248,7 @@ struct Ctx {
     std::vector<int> h_src_seg, h_node_seg;  // sample of every source / node (empty: one sample)
     int *src_dst = nullptr;      // original source index -> storage position (FMM order)
     void *fmm = nullptr;         // FMM tree and buffers (fg_fmm.cu)
+    int *fmm_err = nullptr;      // FG_ETIMEDOUT when a wait of a tensor-core translation expired
     double *src_q = nullptr;
     double *src_q2 = nullptr;    // charges of v (demag of m and v evaluated together), or nullptr
     double *tri_slot = nullptr;  // 3 x nft corrections
@@ -407,6 +408,44 @@ std::vector<float> translate_tc_images(const std::vector<double> &ops, int ncode
 // split into units of at most max_codes codes (appended to codes/units/comb; nslot grows).
 void translate_tc_units(int n_out, int ncode, const int *tab, int out0, int max_codes, std::vector<int> &codes,
                         std::vector<int4> &units, std::vector<int4> &comb, int &nslot);
+
+// Translations of the FP64 path on the tensor cores by exact digit products (fg_fmm_oz.cu)
+constexpr int OZ_TILE = 48;           // output cells per tile
+constexpr int OZ_CELL_BYTES = 1120;   // digits of one expansion: [item 7][digit 5][16] FP16
+struct OzArgs {
+    int ncode, ncell, nset;
+    const int *cells;             // [tile][48] output cell or -1
+    const int *codes;             // operator codes of each tile, tile after tile
+    const int *tab;               // [cell][ncode] input cell or -1
+    const unsigned char *op_img;  // oz_images
+    const float *row_scale;       // [code][100]
+    const unsigned char *in;      // digits of the inputs [set][cell]
+    const float *in_scale;        // [set][cell]
+    const int4 *units;            // per CTA: tile, first and end index into codes, scratch slot
+    int nunits;
+    double *scratch;              // [slot][set][48][100] partial results
+    int *err;                     // FG_ETIMEDOUT after an expired wait
+};
+struct OzFinish {
+    int nlist, ncell, nset;
+    const int *cells;       // listed cells (48 per tile) or -1
+    const int2 *fin;        // per tile: first slot, number of slots (null: split only)
+    const double *scratch;
+    double *io;             // expansions [set][cell][100]
+    int accumulate;         // 1: io += result
+    int split;              // write digits and scales of the first split listed cells
+    const int *wexp;        // weight exponents of the 100 coefficients
+    unsigned char *digits;
+    float *scale;
+};
+struct OzImages {
+    std::vector<unsigned char> img;
+    std::vector<float> row_scale;
+};
+cudaError_t oz_setup();
+cudaError_t launch_translate_oz(cudaStream_t st, const OzArgs &a);
+cudaError_t launch_oz_finish(cudaStream_t st, const OzFinish &a);
+OzImages oz_images(const std::vector<double> &ops, int ncode, const int *wexp);
 int fmm_stage_ms(const Ctx &c, double ms[5]);
 int mlp_create(Ctx &c);
 void mlp_free(Ctx &c);

@@ -1,0 +1,62 @@
+"""The FP64 path's FMM (digit-product translations on the tensor cores, double-single near field
+and P2M) against the same tree on the FP64 pipe, at the edges of its launches: a single tile and
+tiles that end inside a level or an octant, one level (no M2M or L2L), deep flat and long trees,
+leaves with few and many nodes, one and two charge sets, uneven forests."""
+import numpy as np
+import pytest
+
+import feellgood_gb300 as fg
+from tests import cases
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+# (1, 1, 1): 8 nodes; (3, 3, 3) at depth 2: one octant per leaf; (8, 8, 8) at depth 3: 64 leaves of
+# each octant, not a multiple of a 48-cell tile; plates and bars at depths whose leaves are partly
+# empty; a shallow tree with hundreds of nodes per leaf
+@pytest.mark.parametrize("shape,leaf", [((1, 1, 1), -2), ((3, 3, 3), -2), ((8, 8, 8), -3), ((30, 26, 1), -5),
+                                        ((2, 3, 60), -6), ((15, 14, 13), -2), ((11, 7, 5), -4)])
+def test_fp64_fmm_edges(shape, leaf):
+    m = cases.cuboid(*shape)
+    u = cases.perturbed_state(m["xyz"], seed=21, sigma=0.3)
+    v = cases.tangent_field(u, seed=22)
+    H = np.zeros(3)
+    pot = []
+    for native in (0, 1):
+        c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=leaf, fmm_native_fp64=native)
+        c.set_state(u, v)
+        c.compute_all(H)
+        s = c.get_state(0)
+        pot.append((s["phi"], s["phiv"], c.demag(0), c.demag(1)))
+    # digits carry 2^-46 of the largest coefficient, double-single sums about 2^-46 of the summed
+    # magnitudes, which cancel by up to two orders of magnitude for a random tangent field
+    for k in range(4):
+        assert _rel(pot[0][k], pot[1][k]) < (2e-13 if k % 2 == 0 else 1e-12)
+    # two sets in one evaluation follow the arithmetic of one
+    assert _rel(pot[0][0], pot[0][2]) < 1e-14 and _rel(pot[0][1], pot[0][3]) < 1e-14
+
+
+def test_fp64_forest_matches_single_trees():
+    meshes = [cases.cuboid(*s) for s in ((9, 9, 9), (4, 6, 5), (12, 3, 2), (2, 2, 2))]
+    us = [cases.perturbed_state(m["xyz"], seed=30 + k, sigma=0.3) for k, m in enumerate(meshes)]
+    b = fg.Context(meshes, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=-3)
+    b.set_state(np.concatenate(us))
+    pb = b.demag(0)
+    for k, m in enumerate(meshes):
+        c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=-3)
+        c.set_state(us[k])
+        assert _rel(pb[b.node_offsets[k]:b.node_offsets[k + 1]], c.demag(0)) < 1e-13
+
+
+def test_not_a_number_propagates():
+    """A magnetisation that is not a number reaches every potential that depends on it."""
+    m = cases.cuboid(6, 6, 6)
+    u = cases.perturbed_state(m["xyz"], seed=40)
+    u[5] = np.nan
+    c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=-3)
+    c.set_state(u)
+    assert np.isnan(c.demag(0)).all()
