@@ -72,12 +72,20 @@ struct FmmTree {
     double stage_sum[5] = {0, 0, 0, 0, 0};
     long long stage_n = 0;
     // device
-    int *leaf_src = nullptr, *leaf_tgt = nullptr, *tgt_node = nullptr;
+    int *leaf_src = nullptr, *leaf_tgt = nullptr, *tgt_node = nullptr, *tgt_leaf = nullptr;
+    int ntgt = 0;
     void *sloc = nullptr;  // 4 x nsrc: leaf-local source coordinates (T), w: charge of set 0
     void *tloc = nullptr;  // 4 x ntgt: leaf-local target coordinates (T)
     // FP64 path, near field in double-single arithmetic: every coordinate split as
     // hi (on a 2^-20 grid of leaf units) + lo, the charge as hi + lo; (x, y, z, q) per part
     bool ds = false;
+    // The FP64 tree of an FP32 + refinement context (full evaluations, where CURRENT has no valid
+    // potentials) keeps the kernels and the order of sums that such runs have always started
+    // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9
+    // in phiv two steps later (film), so runs repeat bit for bit only with the same last bits
+    bool repeat = false;
+    int4 *p2p_task = nullptr;  // leaf, first target, targets (at most 8) of a near-field block
+    int n_p2p_task = 0;
     float4 *ds_src_hi = nullptr, *ds_src_lo = nullptr, *ds_tgt_hi = nullptr, *ds_tgt_lo = nullptr;
     int *leaf_ijk = nullptr;  // 3 x nleaf integer leaf coordinates (within the leaf's own tree)
     double *leaf_scale = nullptr;  // 1 / physical leaf width of the leaf's tree
@@ -97,6 +105,7 @@ struct FmmTree {
     std::vector<TcLaunch> tc_m2m, tc_l2l;        // per level
     TcLaunch tc_m2l;
     // FP64 path: translations by exact digit products on the tensor cores (fg_fmm_oz.cu)
+    bool oz = false;
     struct OzLaunch { int unit0 = 0, nunit = 0, tile0 = 0, ntile = 0, nsplit = 0; };
     std::vector<OzLaunch> oz_m2m, oz_l2l;        // per level
     OzLaunch oz_m2l;
@@ -606,6 +615,100 @@ __global__ void __launch_bounds__(160) k_translate(int n_out, int out0, int ncod
     }
 }
 
+// Translations in double-single arithmetic on the FP32 pipes (the full FP64 evaluation of the
+// FP32 + refinement path, see FmmTree::repeat): the same batched GEMM as
+// k_translate, both charge sets of a block of DS_TB output cells as its 2 DS_TB columns, the
+// operator and the inputs split into FP32 pairs hi + lo on their way into shared memory,
+// every product exact through fma (Dekker's TwoProduct) and summed with Knuth's two-sum,
+// the running sum renormalised once per code (about 44 significant bits), the result
+// rounded to FP64 once.
+constexpr int DS_TB = 16, DS_COLS = 2 * DS_TB, DS_CT = 2, DS_BLD = DS_COLS + 1;
+constexpr int tr_ds_smem() { return (NR * NR + NR * DS_BLD) * (int)sizeof(float2); }
+
+__device__ __forceinline__ float2 ds_split(double x) {
+    const float h = (float)x;
+    return make_float2(h, (float)(x - (double)h));
+}
+
+__global__ void __launch_bounds__(160, 2) k_translate_ds(int n_out, int out0, int ncode, const int *__restrict__ tab,
+                                                         const double *__restrict__ ops, const double *in,
+                                                         double *out, int accumulate, int nset, size_t set_stride) {
+    // in and out may be the same array (M2M, L2L): the cells read and written are disjoint.
+    constexpr int RT = 10;
+    extern __shared__ unsigned char smem_raw[];
+    float2 *AT = reinterpret_cast<float2 *>(smem_raw);  // AT[k * NR + row] = Op[row][k]
+    float2 *Bs = AT + NR * NR;                           // [NR][DS_BLD]: column set * DS_TB + cell
+    __shared__ int srcs[DS_TB];
+    const int tid = threadIdx.x, rg = tid / 16, cg = tid % 16;
+    const int c_begin = blockIdx.x * DS_TB;
+    float ah[RT][DS_CT], al[RT][DS_CT];
+#pragma unroll
+    for (int i = 0; i < RT; i++)
+#pragma unroll
+        for (int j = 0; j < DS_CT; j++) ah[i][j] = al[i][j] = 0.f;
+    for (int code = 0; code < ncode; code++) {
+        int sc = -1;
+        if (tid < DS_TB && c_begin + tid < n_out) sc = tab[(size_t)(out0 + c_begin + tid) * ncode + code];
+        if (tid < DS_TB) srcs[tid] = sc;
+        if (!__syncthreads_or(sc >= 0)) continue;
+        for (int e = tid; e < NR * NR; e += blockDim.x) {
+            const int row = e / NR, k = e % NR;
+            AT[k * NR + row] = ds_split(ops[(size_t)code * NR * NR + e]);
+        }
+        for (int e = tid; e < NR * DS_COLS; e += blockDim.x) {
+            const int col = e / NR, k = e % NR, cell = col % DS_TB, set = col / DS_TB;
+            const int src = srcs[cell];
+            Bs[k * DS_BLD + col] = (src >= 0 && set < nset) ? ds_split(in[set * set_stride + (size_t)src * NR + k])
+                                                              : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (int k = 0; k < NR; k++) {
+            float2 a[RT], b[DS_CT];
+#pragma unroll
+            for (int i = 0; i < RT; i++) a[i] = AT[k * NR + rg * RT + i];
+#pragma unroll
+            for (int j = 0; j < DS_CT; j++) b[j] = Bs[k * DS_BLD + cg * DS_CT + j];
+#pragma unroll
+            for (int i = 0; i < RT; i++)
+#pragma unroll
+                for (int j = 0; j < DS_CT; j++) {
+                    // (ah, al) += a b: exact leading product and cross terms, two-sum into hi
+                    const float p = a[i].x * b[j].x;
+                    float e = fmaf(a[i].x, b[j].x, -p);
+                    e = fmaf(a[i].x, b[j].y, e);
+                    e = fmaf(a[i].y, b[j].x, e);
+                    const float s = ah[i][j] + p;
+                    const float bb = s - ah[i][j];
+                    const float err = (ah[i][j] - (s - bb)) + (p - bb);
+                    ah[i][j] = s;
+                    al[i][j] += e + err;
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < RT; i++)
+#pragma unroll
+            for (int j = 0; j < DS_CT; j++) {  // renormalise: |lo| back to half an ulp of hi
+                const float s = ah[i][j] + al[i][j];
+                al[i][j] = al[i][j] - (s - ah[i][j]);
+                ah[i][j] = s;
+            }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < DS_CT; j++) {
+        const int col = cg * DS_CT + j, cell = col % DS_TB, set = col / DS_TB;
+        const int c = c_begin + cell;
+        if (c >= n_out || set >= nset) continue;
+        double *o = out + set * set_stride + (size_t)(out0 + c) * NR + rg * RT;
+#pragma unroll
+        for (int i = 0; i < RT; i++) {
+            const double v = (double)ah[i][j] + (double)al[i][j];
+            o[i] = accumulate ? o[i] + v : v;
+        }
+    }
+}
+
 // 1/sqrt in the precision of the path.
 template <typename T> __device__ __forceinline__ T rsqrt_p(T x);
 template <> __device__ __forceinline__ float rsqrt_p<float>(float x) {
@@ -953,7 +1056,166 @@ __device__ __forceinline__ void ds_two_sum(float a, float b, float &s, float &e)
     e = (a - (s - bb)) + (b - bb);
 }
 
-// L2P + P2P of the FP64 path in double-single arithmetic. Coordinates are leaf-local with
+// Near field of the FP64 path in double-single arithmetic. Coordinates are leaf-local with hi
+// parts on a 2^-20 grid (|x| < 4, so hi - hi' is exact in FP32) and lo = x - hi (|lo| <= 2^-21,
+// held to 2^-45); per pair: d = (hi - hi') + (lo - lo'), r^2 as a double-single sum of the
+// squares (the leading products exact through fma), 1/r from the SFU estimate y and
+// y (1 + e/2 + 3 e^2/8), e = 1 - r^2 y^2 formed exactly to about 2^-46, q/r as a double-single
+// product, summed with two-sum: 69 FP32 operations per pair for two charge sets, 45 of them for
+// the geometry the sets share, so the FP32 pipe (128 lanes per clock and SM) bounds it.
+//
+// One block per task: up to 8 target nodes of one leaf (the leaf's targets shared out evenly),
+// held in registers by every thread; the sources of all its adjacent leaves, one list, are
+// spread over the 128 threads, so lanes idle only at the end of that list and a tree of a few
+// hundred leaves still gives every SM work. Sums over the threads in FP64 in a fixed order.
+constexpr int P2P_NT = 8;
+template <int NT, int NQ>
+__device__ __forceinline__ void p2p_ds_pass(int tb, int ntot, const int *seg_src, const int *seg_end,
+                                            const float (*seg_off)[3], const float4 *__restrict__ th4,
+                                            const float4 *__restrict__ tl4, const float4 *__restrict__ sh4,
+                                            const float4 *__restrict__ sl4, const float *__restrict__ q2h,
+                                            const float *__restrict__ q2l, double (&out)[NQ * P2P_NT]) {
+    float thx[NT], thy[NT], thz[NT], tlx[NT], tly[NT], tlz[NT], ah[NQ][NT], al[NQ][NT];
+#pragma unroll
+    for (int j = 0; j < NT; j++) {
+        const float4 h = __ldg(th4 + tb + j), l = __ldg(tl4 + tb + j);
+        thx[j] = h.x; thy[j] = h.y; thz[j] = h.z;
+        tlx[j] = l.x; tly[j] = l.y; tlz[j] = l.z;
+#pragma unroll
+        for (int k = 0; k < NQ; k++) ah[k][j] = al[k][j] = 0.f;
+    }
+    int e = 0;
+    for (int i = threadIdx.x; i < ntot; i += 128) {
+        while (i >= seg_end[e]) e++;
+        const int s = seg_src[e] + i;
+        const float4 h = sh4[s], l = sl4[s];
+        // integer offset of the adjacent leaf, added exactly to the hi parts
+        const float sx = h.x + seg_off[e][0], sy = h.y + seg_off[e][1], sz = h.z + seg_off[e][2];
+        float qh[NQ], ql[NQ];
+        qh[0] = h.w;
+        ql[0] = l.w;
+        if constexpr (NQ == 2) {
+            qh[1] = q2h[s];
+            ql[1] = q2l[s];
+        }
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            const float d1x = thx[j] - sx, d1y = thy[j] - sy, d1z = thz[j] - sz;  // exact
+            const float d2x = tlx[j] - l.x, d2y = tly[j] - l.y, d2z = tlz[j] - l.z;
+            // squares: d^2 = d1^2 + d2 (2 d1 + d2), leading products exact
+            const float px = d1x * d1x, py = d1y * d1y, pz = d1z * d1z;
+            const float ex = fmaf(d2x, fmaf(2.f, d1x, d2x), fmaf(d1x, d1x, -px));
+            const float ey = fmaf(d2y, fmaf(2.f, d1y, d2y), fmaf(d1y, d1y, -py));
+            const float ez = fmaf(d2z, fmaf(2.f, d1z, d2z), fmaf(d1z, d1z, -pz));
+            float s1_, e1, s2_, e2;
+            ds_two_sum(px, py, s1_, e1);
+            ds_two_sum(s1_, pz, s2_, e2);
+            const float eps = (e1 + e2) + ((ex + ey) + ez);
+            const float Sh = s2_ + eps, Sl = eps - (Sh - s2_);
+            const float y = rsqrt_p<float>(Sh);
+            const float p = Sh * y, pe = fmaf(Sl, y, fmaf(Sh, y, -p));  // r^2 y
+            const float del = fmaf(-pe, y, fmaf(-p, y, 1.f));
+            const float yl = (y * del) * fmaf(0.375f, del, 0.5f);
+            // q / r = (qh + ql)(y + yl), accumulated with two-sum
+#pragma unroll
+            for (int k = 0; k < NQ; k++) {
+                const float c1 = qh[k] * y;
+                const float c2 = fmaf(ql[k], y, fmaf(qh[k], yl, fmaf(qh[k], y, -c1)));
+                float sn, en;
+                ds_two_sum(ah[k][j], c1, sn, en);
+                ah[k][j] = sn;
+                al[k][j] += en + c2;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NQ; k++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) out[k * P2P_NT + j] = double(ah[k][j]) + double(al[k][j]);
+}
+
+template <int NQ>
+__global__ void __launch_bounds__(128, 4) k_p2p_ds(const int4 *__restrict__ task, const int *__restrict__ leaf_src,
+                                                   const int *__restrict__ tgt_node, const float4 *__restrict__ th4,
+                                                   const float4 *__restrict__ tl4, const float4 *__restrict__ sh4,
+                                                   const float4 *__restrict__ sl4, const float *__restrict__ q2h,
+                                                   const float *__restrict__ q2l, const int *__restrict__ leaf_ijk,
+                                                   const int *__restrict__ near_ptr, const int *__restrict__ near_leaf,
+                                                   double *__restrict__ pot0, double *__restrict__ pot1) {
+    // the adjacent leaves as one list of sources: source i of the list, seg_end[e - 1] <= i <
+    // seg_end[e], is source seg_src[e] + i
+    __shared__ int seg_src[28], seg_end[28];
+    __shared__ float seg_off[28][3];
+    constexpr int NV = NQ * P2P_NT;
+    __shared__ double red[4][NV];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int4 t = task[blockIdx.x];
+    const int leaf = t.x, tb = t.y, nt = t.z;
+    const int e0 = near_ptr[leaf], ne = near_ptr[leaf + 1] - e0;
+    if (warp == 0) {
+        int s0 = 0, n = 0;
+        if (lane < ne) {
+            const int nl = near_leaf[e0 + lane];
+            s0 = leaf_src[nl];
+            n = leaf_src[nl + 1] - s0;
+#pragma unroll
+            for (int d = 0; d < 3; d++) seg_off[lane][d] = float(leaf_ijk[3 * nl + d] - leaf_ijk[3 * leaf + d]);
+        }
+        int end = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, end, o);
+            if (lane >= o) end += x;
+        }
+        if (lane < 28) {
+            seg_src[lane] = s0 - (end - n);
+            seg_end[lane] = end;
+        }
+    }
+    __syncthreads();
+    const int ntot = ne > 0 ? seg_end[ne - 1] : 0;
+    double v[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) v[k] = 0.0;
+#define FG_P2P(N)                                                                                                  \
+    case N:                                                                                                        \
+        p2p_ds_pass<N, NQ>(tb, ntot, seg_src, seg_end, seg_off, th4, tl4, sh4, sl4, q2h, q2l, v);                  \
+        break;
+    switch (nt) {
+        FG_P2P(1) FG_P2P(2) FG_P2P(3) FG_P2P(4) FG_P2P(5) FG_P2P(6) FG_P2P(7) FG_P2P(8)
+    }
+#undef FG_P2P
+    // sums over the warp: the halves of the values are exchanged until each lane holds one, in the
+    // order of a butterfly over lane bits 4 to 0 for every value
+    int n = NV;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        if (n > 1) {
+            n >>= 1;
+            const bool hi = lane & o;
+#pragma unroll
+            for (int k = 0; k < NV / 2; k++)
+                if (k < n) {
+                    const double send = hi ? v[k] : v[k + n], keep = hi ? v[k + n] : v[k];
+                    v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    constexpr int DUP = 32 / NV;  // lanes holding each value
+    if (lane % DUP == 0) red[warp][lane / DUP] = v[0];
+    __syncthreads();
+    if (threadIdx.x < NV) {
+        const int k = threadIdx.x / P2P_NT, j = threadIdx.x % P2P_NT;
+        if (j < nt)
+            (k ? pot1 : pot0)[tgt_node[tb + j]] =
+                ((red[0][threadIdx.x] + red[1][threadIdx.x]) + red[2][threadIdx.x]) + red[3][threadIdx.x];
+    }
+}
+
+// L2P + P2P in double-single arithmetic of the full FP64 evaluation of the FP32 + refinement path
+// (FmmTree::repeat). Coordinates are leaf-local with
 // hi parts on a 2^-20 grid (|x| < 4, so hi - hi' is exact in FP32) and lo = x - hi
 // (|lo| <= 2^-21, held to 2^-45); per pair: dx = (hi - hi') + (lo - lo'), r^2 as a
 // double-single sum of the squares (the leading products exact through fma), 1/r from the
@@ -1090,37 +1352,46 @@ __global__ void __launch_bounds__(128) k_l2p_p2p_ds(int nleaf, const int *__rest
     }
 }
 
-// L2P after a near-field-only pass: one warp per target leaf, lane j of a pass evaluates
-// the local expansion(s) at target j and forms the potential from the stored near sum with
-// the same operations as the fused pass, pot = (far + near) * scale.
+// L2P after a near field that stored its sums: one thread per target evaluates its leaf's local
+// expansion(s) and forms the potential from the stored near sum with the operations of the fused
+// FP32 pass, pot = (far + near) * scale. Threads of a warp are targets of one or two leaves, so
+// every lane works (one warp per leaf left lanes idle, which on the 1/64-rate FP64 pipe that
+// bounds the FP64 form costs as much as work). The loads are volatile so that they stay beside
+// their use: hoisted together they spilled.
+__device__ __forceinline__ float ld_here(const float *p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ld_here(const double *p) {
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+    return v;
+}
 template <typename T, int NQ>
-__global__ void __launch_bounds__(128) k_l2p(int nleaf, const int *__restrict__ leaf_tgt,
-                                             const int *__restrict__ tgt_node, const T *__restrict__ tloc,
-                                             int leaf0, const double *__restrict__ leaf_scale, NearSets<T> sets) {
-    const int lane = threadIdx.x & 31;
-    const int leaf = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (leaf >= nleaf) return;
-    const int t0 = leaf_tgt[leaf], t1 = leaf_tgt[leaf + 1];
+__global__ void __launch_bounds__(128) k_l2p(int ntgt, const int *__restrict__ tgt_leaf,
+                                             const int *__restrict__ tgt_node, const T *__restrict__ tloc, int leaf0,
+                                             const double *__restrict__ leaf_scale, NearSets<T> sets) {
+    const int ti = blockIdx.x * 128 + threadIdx.x;
+    if (ti >= ntgt) return;
+    const int leaf = tgt_leaf[ti];
     const size_t fbase = (size_t)(leaf0 + leaf) * NR;
     const double sc = leaf_scale[leaf];
-    const T *__restrict__ Fa = sets.F[0] + fbase;
-    const T *__restrict__ Fb = sets.F[NQ - 1] + fbase;
-    for (int ti = t0 + lane; ti < t1; ti += 32) {
-        const T x = tloc[4 * (size_t)ti], y = tloc[4 * (size_t)ti + 1], z = tloc[4 * (size_t)ti + 2];
-        T fa = 0, fb = 0;
-        ups_cols<T>(x, y, z, [&](int n, int m, T re, T im) {
-            if (m == 0) {
-                fa += Fa[ridx(n, 0, 0)] * re;
-                if constexpr (NQ == 2) fb += Fb[ridx(n, 0, 0)] * re;
-            } else {
-                fa += T(2) * (Fa[ridx(n, m, 0)] * re + Fa[ridx(n, m, 1)] * im);
-                if constexpr (NQ == 2) fb += T(2) * (Fb[ridx(n, m, 0)] * re + Fb[ridx(n, m, 1)] * im);
-            }
-        });
-        const int node = tgt_node[ti];
-        sets.pot[0][node] = (double(fa) + sets.pot[0][node]) * sc;
-        if constexpr (NQ == 2) sets.pot[1][node] = (double(fb) + sets.pot[1][node]) * sc;
-    }
+    const T *Fa = sets.F[0] + fbase, *Fb = sets.F[NQ - 1] + fbase;
+    const T x = tloc[4 * (size_t)ti], y = tloc[4 * (size_t)ti + 1], z = tloc[4 * (size_t)ti + 2];
+    T fa = 0, fb = 0;
+    ups_cols<T>(x, y, z, [&](int n, int m, T re, T im) {
+        if (m == 0) {
+            fa += ld_here(Fa + ridx(n, 0, 0)) * re;
+            if constexpr (NQ == 2) fb += ld_here(Fb + ridx(n, 0, 0)) * re;
+        } else {
+            fa += T(2) * (ld_here(Fa + ridx(n, m, 0)) * re + ld_here(Fa + ridx(n, m, 1)) * im);
+            if constexpr (NQ == 2) fb += T(2) * (ld_here(Fb + ridx(n, m, 0)) * re + ld_here(Fb + ridx(n, m, 1)) * im);
+        }
+    });
+    const int node = tgt_node[ti];
+    sets.pot[0][node] = (double(fa) + sets.pot[0][node]) * sc;
+    if constexpr (NQ == 2) sets.pot[1][node] = (double(fb) + sets.pot[1][node]) * sc;
 }
 
 // ---------------------------------------------------------------------------------
@@ -1684,7 +1955,9 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(up((float **)&t->img_l2l, il2l));
     }
     t->ds = !fp32 && c.opts.fmm_native_fp64 == 0;
-    if (t->ds) {
+    t->repeat = t->ds && c.opts.precision == FG_PREC_FP32_REFINE;
+    t->oz = t->ds && !t->repeat;
+    if (t->oz) {
         std::vector<int> cells, codes;
         std::vector<int4> units;
         std::vector<int2> fin;
@@ -1804,6 +2077,10 @@ static int fmm_build_forest(Ctx &c, int L) {
     FCK(up(&t->leaf_src, leaf_src));
     FCK(up(&t->leaf_tgt, leaf_tgt));
     FCK(up(&t->tgt_node, tgt_node));
+    t->ntgt = (int)tgt_node.size();
+    std::vector<int> tgt_leaf(tgt_node.size());
+    for (int l = 0; l < nleaf; l++) std::fill(tgt_leaf.begin() + leaf_tgt[l], tgt_leaf.begin() + leaf_tgt[l + 1], l);
+    FCK(up(&t->tgt_leaf, tgt_leaf));
     FCK(up(&t->leaf_ijk, leaf_ijk));
     FCK(up(&t->leaf_scale, leaf_scale));
     FCK(up(&t->m2l_tab, m2l_tab));
@@ -1834,12 +2111,36 @@ static int fmm_build_forest(Ctx &c, int L) {
         std::vector<float4> sh, sl, th, tl;
         split(sloc, sh, sl);
         split(tloc, th, tl);
+        std::vector<int4> task;
+        std::vector<long> cost;
+        for (int l = 0; l < nleaf; l++) {
+            const int n = leaf_tgt[l + 1] - leaf_tgt[l], groups = (n + P2P_NT - 1) / P2P_NT;
+            long src = 0;
+            for (int e = near_ptr[l]; e < near_ptr[l + 1]; e++) src += leaf_src[near_leaf[e] + 1] - leaf_src[near_leaf[e]];
+            for (int g = 0; g < groups; g++) {
+                const int b = (int)((long)n * g / groups), e = (int)((long)n * (g + 1) / groups);
+                task.push_back(make_int4(l, leaf_tgt[l] + b, e - b, 0));
+                cost.push_back(src * (e - b));
+            }
+        }
+        // where the sources fit in L2 the expensive blocks go first, which evens out the last wave;
+        // else the leaf order keeps neighbouring blocks on the same sources
+        if ((size_t)c.nsrc * 40 < ((size_t)64 << 20)) {
+            std::vector<int> order(task.size());
+            for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+            std::vector<int4> sorted;
+            for (int k : order) sorted.push_back(task[k]);
+            task.swap(sorted);
+        }
+        t->n_p2p_task = (int)task.size();
+        FCK(up(&t->p2p_task, task));
         FCK(up(&t->ds_src_hi, sh));
         FCK(up(&t->ds_src_lo, sl));
         FCK(up(&t->ds_tgt_hi, th));
         FCK(up(&t->ds_tgt_lo, tl));
     }
-    if (!t->ds) {
+    if (!t->oz) {
         FCK(up_as<double>(&t->op_m2l, ops.m2l, fp32));
         FCK(up_as<double>(&t->op_m2m, ops.m2m, fp32));
         FCK(up_as<double>(&t->op_l2l, ops.l2l, fp32));
@@ -1865,6 +2166,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(cudaFuncSetAttribute(k_translate<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<float>()));
     } else {
         FCK(cudaFuncSetAttribute(k_translate<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<double>()));
+        FCK(cudaFuncSetAttribute(k_translate_ds, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_ds_smem()));
     }
     if (c.opts.profile)
         for (auto &set : t->ev)
@@ -1882,11 +2184,11 @@ static int fmm_build_forest(Ctx &c, int L) {
 void fmm_free(Ctx &c) {
     FmmTree *t = static_cast<FmmTree *>(c.fmm);
     if (!t) return;
-    void *ptrs[] = {t->leaf_scale, t->leaf_src, t->leaf_tgt, t->tgt_node, t->sloc, t->tloc, t->leaf_ijk, t->m2l_tab, t->m2m_tab,
+    void *ptrs[] = {t->leaf_scale, t->leaf_src, t->leaf_tgt, t->tgt_node, t->tgt_leaf, t->sloc, t->tloc, t->leaf_ijk, t->m2l_tab, t->m2m_tab,
                     t->l2l_tab, t->near_ptr, t->near_leaf, t->M, t->F, t->op_m2l, t->op_m2m, t->op_l2l,
                     t->tc_code, t->tc_units, t->tc_comb, t->tc_scratch, t->Mh, t->Ml, t->Fh, t->Fl,
                     t->img_m2l, t->img_m2m, t->img_l2l, t->ds_src_hi, t->ds_src_lo, t->ds_tgt_hi, t->ds_tgt_lo,
-                    t->sq2, t->ds_q2, t->oz_cells, t->oz_codes, t->oz_wexp, t->oz_leaves, t->oz_units, t->oz_fin,
+                    t->sq2, t->ds_q2, t->p2p_task, t->oz_cells, t->oz_codes, t->oz_wexp, t->oz_leaves, t->oz_units, t->oz_fin,
                     t->oz_scratch, t->oz_digits, t->oz_scale, t->oz_img[0], t->oz_img[1], t->oz_img[2], t->oz_rows[0],
                     t->oz_rows[1], t->oz_rows[2]};
     for (void *p : ptrs)
@@ -1971,13 +2273,16 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     const int nb = (t.nleaf + 3) / 4;
     auto near_field = [&](cudaStream_t st) {
         if constexpr (sizeof(T) == 8) {
-            if (t.ds) {
+            if (t.repeat) {
                 auto k = nq == 2 ? k_l2p_p2p_ds<2> : k_l2p_p2p_ds<1>;
                 k<<<nb, 128, 0, st>>>(t.nleaf, t.leaf_src, t.leaf_tgt, t.tgt_node, (const double *)t.tloc, t.ds_tgt_hi,
                                       t.ds_tgt_lo, t.ds_src_hi, t.ds_src_lo, t.ds_q2,
                                       t.ds_q2 ? t.ds_q2 + t.nsrc : nullptr, t.leaf_ijk, t.leaf0, t.leaf_scale,
                                       t.near_ptr, t.near_leaf, ns);
-            }
+            } else if (t.ds && t.n_p2p_task > 0)
+                (nq == 2 ? k_p2p_ds<2> : k_p2p_ds<1>)<<<t.n_p2p_task, 128, 0, st>>>(
+                    t.p2p_task, t.leaf_src, t.tgt_node, t.ds_tgt_hi, t.ds_tgt_lo, t.ds_src_hi, t.ds_src_lo, t.ds_q2,
+                    t.ds_q2 ? t.ds_q2 + t.nsrc : nullptr, t.leaf_ijk, t.near_ptr, t.near_leaf, ns.pot[0], ns.pot[1]);
         }
         if (!t.ds) {
             auto k = nq == 2 ? k_l2p_p2p<T, 2> : k_l2p_p2p<T, 1>;
@@ -2021,6 +2326,11 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
             a.nset = nq; a.set_io = sstride; a.set_scratch = t.nslot_floats;
             const cudaError_t e = launch_translate_tc(c.stream, a);
             if (e != cudaSuccess && terr == cudaSuccess) terr = e;
+        } else if (sizeof(T) == 8 && t.ds) {  // double-single, both sets per launch
+            const double *ops = (const double *)(kind == M2M ? t.op_m2m : kind == M2L ? t.op_m2l : t.op_l2l);
+            double *in = (double *)(kind == L2L ? F : M), *out = (double *)(kind == M2M ? M : F);
+            k_translate_ds<<<(n + DS_TB - 1) / DS_TB, 160, tr_ds_smem(), c.stream>>>(n, out0, ncode, tab, ops, in, out,
+                                                                                     kind == L2L, nq, sstride);
         } else {
             const void *ops = kind == M2M ? t.op_m2m : kind == M2L ? t.op_m2l : t.op_l2l;
             for (int q = 0; q < nq; q++) {
@@ -2036,7 +2346,7 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
         if (e != cudaSuccess && terr == cudaSuccess) terr = e;
     };
     OzFinish fa{};
-    if (t.ds) {
+    if (t.oz) {
         fa.ncell = t.ncell; fa.nset = nq; fa.scratch = t.oz_scratch; fa.digits = t.oz_digits; fa.scale = t.oz_scale;
         fa.io = (double *)M; fa.cells = t.oz_leaves; fa.nlist = t.nleaf; fa.accumulate = 1; fa.split = t.nleaf;
         fa.wexp = t.oz_wexp;
@@ -2059,7 +2369,7 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     };
     const FmmTree::TcLaunch none;
     for (int l = L - 1; l >= 2; l--)
-        if (t.ds) translate_oz(M2M, t.oz_m2m[l], t.oz_m2m[l].ntile * OZ_TILE);
+        if (t.oz) translate_oz(M2M, t.oz_m2m[l], t.oz_m2m[l].ntile * OZ_TILE);
         else translate(M2M, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_m2m[l] : none);
     if (prof) cudaEventRecord(ev[2], c.stream);
     if (split) {  // the near field beside M2L and L2L
@@ -2072,17 +2382,20 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
         cudaEventRecord(c.ev_join, c.stream2);
         ns.near_only = 0;
     }
-    if (t.ds) translate_oz(M2L, t.oz_m2l, t.oz_m2l.nsplit);
+    if (t.oz) translate_oz(M2L, t.oz_m2l, t.oz_m2l.nsplit);
     else translate(M2L, t.ncell, 0, t.tc_m2l);
     if (prof) cudaEventRecord(ev[3], c.stream);
     for (int l = 3; l <= L; l++)
-        if (t.ds) translate_oz(L2L, t.oz_l2l[l], l < L ? t.oz_l2l[l].ntile * OZ_TILE : 0);
+        if (t.oz) translate_oz(L2L, t.oz_l2l[l], l < L ? t.oz_l2l[l].ntile * OZ_TILE : 0);
         else translate(L2L, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_l2l[l] : none);
     if (prof) cudaEventRecord(ev[4], c.stream);
-    if (split) {
-        cudaStreamWaitEvent(c.stream, c.ev_join, 0);
+    if (split || t.oz) {  // L2P apart: the double-single near field stores its sums
+        if (split) cudaStreamWaitEvent(c.stream, c.ev_join, 0);
+        else near_field(c.stream);
         auto k = nq == 2 ? k_l2p<T, 2> : k_l2p<T, 1>;
-        k<<<nb, 128, 0, c.stream>>>(t.nleaf, t.leaf_tgt, t.tgt_node, (const T *)t.tloc, t.leaf0, t.leaf_scale, ns);
+        if (t.ntgt > 0)
+            k<<<(t.ntgt + 127) / 128, 128, 0, c.stream>>>(t.ntgt, t.tgt_leaf, t.tgt_node, (const T *)t.tloc, t.leaf0,
+                                                          t.leaf_scale, ns);
     } else {
         near_field(c.stream);
     }
@@ -2153,8 +2466,8 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
     const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
     if (!t) return 0;
     int n = 2;  // P2M, L2P + P2P (both sets in one launch each)
-    if (c.opts.fmm_overlap != 0 && c.stream2) n += 1;  // L2P after the overlapped near field
-    if (t->ds) {  // digits of the leaves, then per translation the products and the sums
+    if ((c.opts.fmm_overlap != 0 && c.stream2) || t->oz) n += 1;  // L2P apart from the near field
+    if (t->oz) {  // digits of the leaves, then per translation the products and the sums
         n += 1;
         for (int l = 2; l <= t->L - 1; l++) n += (t->oz_m2m[l].nunit > 0) + (t->oz_m2m[l].ntile > 0);
         n += (t->oz_m2l.nunit > 0) + (t->oz_m2l.ntile > 0);
@@ -2163,7 +2476,7 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
     }
     // tensor-core translations: both sets in one launch and one combine launch; the k_translate
     // form launches once per set
-    const int per = t->tc ? 1 : nq;
+    const int per = t->tc || t->ds ? 1 : nq;
     for (int l = 2; l <= t->L - 1; l++) n += per + (t->tc && t->tc_m2m[l].ncomb > 0);
     n += per + (t->tc && t->tc_m2l.ncomb > 0);
     for (int l = 3; l <= t->L; l++) n += per + (t->tc && t->tc_l2l[l].ncomb > 0);
