@@ -283,11 +283,6 @@ __global__ void __launch_bounds__(128) k_p2m(int nleaf, const int *__restrict__ 
         const T x = sloc[4 * (size_t)s], y = sloc[4 * (size_t)s + 1], z = sloc[4 * (size_t)s + 2];
         const T qq = T(q[s]);
         st.qn[(size_t)s * st.qn_stride] = qq;
-        if (st.qh) {  // charge as hi + lo for the double-single near field
-            const float qh = (float)q[s];
-            st.qh[(size_t)s * st.qd_stride] = qh;
-            st.ql[(size_t)s * st.qd_stride] = (float)(q[s] - (double)qh);
-        }
         ups_cols<T>(x, y, z, [&](int n, int m, T re, T im) {
             acc[ridx(n, m, 0)] += qq * re;
             if (m) acc[ridx(n, m, 1)] -= qq * im;
@@ -430,16 +425,211 @@ __global__ void __launch_bounds__(128) k_p2m2(int nleaf, const int *__restrict__
 }
 
 // ---- P2M of the FP64 path in double-single arithmetic -------------------------------
-// The harmonics and the accumulation of k_p2m's FP64 form on the FP32 pipes (GB300's FP64
-// pipe, 2 DFMA per clock and SM, made the FP64 P2M 9.9 ms of the film's FP64 evaluation):
-// the recurrences of ups_cols with every operation a double-single one (about 48 bits), the
-// coordinates as the normalised pair of their stored hi + lo parts, the charge split once.
+// The harmonics and their sums on the FP32 pipes (GB300's FP64 pipe runs at 1/64 of their rate).
+// A column m is formed without divisions as V_n = k_n Ups_n^m,
+//   V_m = (x + i y)^m, V_{m+1} = z V_m, V_n = (2n-1) z V_{n-1} - g r^2 V_{n-2},
+// g = 1 for n = m + 2 and (n-1+m)(n-1-m) above, k_m = k_{m+1} = 2^m m!, k_n = k_{n-1} (n+m)(n-m),
+// and the leaf's sums are multiplied by 1 / k_n once.
 
 __device__ __forceinline__ dsf dsc(double x) {  // a double constant as a double-single pair
     const float h = (float)x;
     return {h, (float)(x - (double)h)};
 }
 
+// A warp forms two columns of a leaf: (0, 5), (1, 9), (2, 8), (3, 7) or (4, 6), 20 reals every pair
+// (80 registers of sums for two sets) and nearly the same work.
+constexpr int P2M_COL[5][2] = {{0, 5}, {1, 9}, {2, 8}, {3, 7}, {4, 6}};
+struct P2mTab {
+    int idx[5][20];     // real index of each of a warp's 20 sums
+    double fac[5][20];  // 1 / k_n, negative for imaginary parts (M = sum q conj(Ups))
+};
+constexpr P2mTab make_p2m_tab() {
+    P2mTab t{};
+    for (int w = 0; w < 5; w++) {
+        int r = 0;
+        for (int h = 0; h < 2; h++) {
+            const int m = P2M_COL[w][h];
+            double k = 1.0;
+            for (int i = 1; i <= m; i++) k *= 2.0 * i;
+            for (int n = m; n <= FMM_P; n++) {
+                if (n >= m + 2) k *= double((n + m) * (n - m));
+                for (int part = 0; part < (m ? 2 : 1); part++, r++) {
+                    t.idx[w][r] = ridx(n, m, part);
+                    t.fac[w][r] = (part ? -1.0 : 1.0) / k;
+                }
+            }
+        }
+    }
+    return t;
+}
+__constant__ P2mTab c_p2m = make_p2m_tab();
+
+// products and sums of normalised pairs; a product left unnormalised (hi, lo) keeps |lo| below
+// 2^-22 |hi|
+__device__ __forceinline__ dsf ds_prod(dsf x, dsf y) {
+    const float p = x.h * y.h;
+    return {p, fmaf(x.l, y.h, fmaf(x.h, y.l, fmaf(x.h, y.h, -p)))};
+}
+__device__ __forceinline__ dsf ds_diff(dsf x, dsf y) {  // of unnormalised products, normalised
+    const dsf s = ds_two_sum_f(x.h, -y.h);
+    return ds_quick(s.h, s.l + (x.l - y.l));
+}
+__device__ __forceinline__ dsf ds_sum(dsf x, dsf y) {
+    const dsf s = ds_two_sum_f(x.h, y.h);
+    return ds_quick(s.h, s.l + (x.l + y.l));
+}
+__device__ __forceinline__ dsf ds_scale(dsf x, float c) {  // times a small integer, unnormalised
+    const float p = x.h * c;
+    return {p, fmaf(x.l, c, fmaf(x.h, c, -p))};
+}
+struct dsc2 { dsf re, im; };
+__device__ __forceinline__ dsc2 ds_cmul(dsc2 a, dsc2 b) {
+    return {ds_diff(ds_prod(a.re, b.re), ds_prod(a.im, b.im)), ds_sum(ds_prod(a.re, b.im), ds_prod(a.im, b.re))};
+}
+template <int M>
+__device__ __forceinline__ dsc2 ds_cpow(dsc2 w) {  // w^M, M >= 1
+    if constexpr (M == 1) return w;
+    else if constexpr (M % 2 == 0) {
+        const dsc2 h = ds_cpow<M / 2>(w);
+        return ds_cmul(h, h);
+    } else return ds_cmul(ds_cpow<M - 1>(w), w);
+}
+
+// Column M of one source: f(n, V_n); the imaginary parts of column 0 are zero and unused.
+template <int M, typename Fn>
+__device__ __forceinline__ void p2m_column(dsc2 d, dsf z, dsf r2, Fn &&f) {
+    f(M, d);
+    if constexpr (M < FMM_P) {
+        auto mul = [](dsf a, dsf b) {
+            const dsf p = ds_prod(a, b);
+            return ds_quick(p.h, p.l);
+        };
+        dsc2 p2 = d, p1;
+        if constexpr (M == 0) p1 = {z, {0.f, 0.f}};
+        else p1 = {mul(z, d.re), mul(z, d.im)};
+        f(M + 1, p1);
+#pragma unroll
+        for (int n = M + 2; n <= FMM_P; n++) {
+            const dsf az = ds_scale(z, float(2 * n - 1));
+            const dsf gr = n == M + 2 ? r2 : ds_scale(r2, float((n - 1 + M) * (n - 1 - M)));
+            dsc2 c;
+            c.re = ds_diff(ds_prod(az, p1.re), ds_prod(gr, p2.re));
+            if constexpr (M > 0) c.im = ds_diff(ds_prod(az, p1.im), ds_prod(gr, p2.im));
+            else c.im = {0.f, 0.f};
+            f(n, c);
+            p2 = p1;
+            p1 = c;
+        }
+    }
+}
+
+template <int NS, int W>
+__device__ __forceinline__ void p2m_ds_warp(int lane, int s0, int s1, const float4 *__restrict__ shi,
+                                            const float4 *__restrict__ slo, size_t base, const P2mSet<double> &a,
+                                            const P2mSet<double> &b) {
+    constexpr int MA = P2M_COL[W][0], MB = P2M_COL[W][1], NA = MA ? 2 * (FMM_P + 1 - MA) : FMM_P + 1;
+    dsf acc[20 * NS];
+#pragma unroll
+    for (int k = 0; k < 20 * NS; k++) acc[k] = dsf{0.f, 0.f};
+    int since = 0;
+    for (int s = s0 + lane; s < s1; s += 32) {
+        const float4 h = shi[s], l = slo[s];
+        const dsf x = ds_two_sum_f(h.x, l.x), y = ds_two_sum_f(h.y, l.y), z = ds_two_sum_f(h.z, l.z);
+        const double qa_d = a.q[s], qb_d = NS == 2 ? b.q[s] : 0.0;
+        const dsf qa = dsc(qa_d), qb = dsc(qb_d);
+        if constexpr (W == 0) {  // the charges for the near field, once
+            a.qh[(size_t)s * a.qd_stride] = qa.h;
+            a.ql[(size_t)s * a.qd_stride] = qa.l;
+            if constexpr (NS == 2) {
+                b.qh[(size_t)s * b.qd_stride] = qb.h;
+                b.ql[(size_t)s * b.qd_stride] = qb.l;
+            }
+        }
+        const dsf r2 = ds_sum(ds_sum(ds_prod(x, x), ds_prod(y, y)), ds_prod(z, z));
+        auto add = [&](int k, dsf q, dsf v) {
+            const dsf p = ds_prod(q, v), t = ds_two_sum_f(acc[k].h, p.h);
+            acc[k].h = t.h;
+            acc[k].l += t.l + p.l;
+        };
+        auto col = [&](int m, int k0, int n, dsc2 v) {
+            const int k = k0 + (m ? 2 * (n - m) : n);
+            add(k, qa, v.re);
+            if (m) add(k + 1, qa, v.im);
+            if constexpr (NS == 2) {
+                add(20 + k, qb, v.re);
+                if (m) add(20 + k + 1, qb, v.im);
+            }
+        };
+        const dsc2 w{x, y};
+        if constexpr (MA == 0) {
+            p2m_column<0>({{1.f, 0.f}, {0.f, 0.f}}, z, r2, [&](int n, dsc2 v) { col(0, 0, n, v); });
+            p2m_column<MB>(ds_cpow<MB>(w), z, r2, [&](int n, dsc2 v) { col(MB, NA, n, v); });
+        } else {
+            const dsc2 wa = ds_cpow<MA>(w);
+            p2m_column<MA>(wa, z, r2, [&](int n, dsc2 v) { col(MA, 0, n, v); });
+            // w^MB from w^MA: 9 = 8 + 1, 8 = 4 x 2, 7 = 4 + 3, 6 = 4 + 2
+            dsc2 wb;
+            if constexpr (MB == 9) wb = ds_cpow<9>(w);
+            else if constexpr (MB == 8) wb = ds_cpow<4>(wa);
+            else wb = ds_cmul(wa, ds_cpow<MB - MA>(w));
+            p2m_column<MB>(wb, z, r2, [&](int n, dsc2 v) { col(MB, NA, n, v); });
+        }
+        if (++since == 16) {  // |lo| back to half an ulp of hi
+            since = 0;
+#pragma unroll
+            for (int k = 0; k < 20 * NS; k++) acc[k] = ds_quick(acc[k].h, acc[k].l);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 20 * NS; k++) acc[k] = ds_quick(acc[k].h, acc[k].l);
+    // sums over the warp: the halves of the values are exchanged while their number is even (lane
+    // bit 4 keeps the set of two), each value by the butterfly over lane bits 4 to 0
+    int n = 20 * NS;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const bool halve = n % 2 == 0, hi = lane & o;
+        if (halve) n >>= 1;
+#pragma unroll
+        for (int k = 0; k < 10 * NS; k++)
+            if (k < n) {
+                const dsf keep = halve && hi ? acc[k + n] : acc[k], send = halve && !hi ? acc[k + n] : acc[k];
+                acc[k] = ds_add(keep, dsf{__shfl_xor_sync(0xffffffffu, send.h, o), __shfl_xor_sync(0xffffffffu, send.l, o)});
+            }
+    }
+    // five values left: of lanes that differ in bits 0 and 1 (two sets) or 0 to 2 the same ones
+    const int sub = NS == 2 ? lane & 3 : lane & 7, set = NS == 2 ? lane >> 4 : 0;
+    const int r0 = NS == 2 ? 10 * (lane >> 3 & 1) + 5 * (lane >> 2 & 1) : 10 * (lane >> 4) + 5 * (lane >> 3 & 1);
+#pragma unroll
+    for (int k = 0; k < 5; k++)
+        if ((k & 3) == sub) (set ? b : a).M[base + c_p2m.idx[W][r0 + k]] = ds_to(acc[k]) * c_p2m.fac[W][r0 + k];
+}
+
+// P2M of the FP64 path: one warp per leaf and pair of columns (grid y) over the leaf's sources, the
+// NS charge sets in one pass (the harmonics of a source are formed once for both; one set and two
+// run the same arithmetic). About 5,400 FP32 operations per source for two sets. The loop bodies
+// are straight-line code of some 20 KB each: the column pair is the slow grid index, so
+// that an SM runs one of them at a time (with the five pairs side by side in a block, 18 of 20
+// cycles went to instruction fetch: wire 2.77 ms).
+template <int NS>
+__global__ void __launch_bounds__(128, 4) k_p2m_ds(int nleaf, const int *__restrict__ leaf_src,
+                                                   const float4 *__restrict__ shi, const float4 *__restrict__ slo,
+                                                   int leaf0, P2mSet<double> set0, P2mSet<double> set1) {
+    const int lane = threadIdx.x & 31, leaf = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (leaf >= nleaf) return;
+    const int s0 = leaf_src[leaf], s1 = leaf_src[leaf + 1];
+    const size_t base = (size_t)(leaf0 + leaf) * NR;
+    switch (blockIdx.y) {
+        case 0: p2m_ds_warp<NS, 0>(lane, s0, s1, shi, slo, base, set0, set1); break;
+        case 1: p2m_ds_warp<NS, 1>(lane, s0, s1, shi, slo, base, set0, set1); break;
+        case 2: p2m_ds_warp<NS, 2>(lane, s0, s1, shi, slo, base, set0, set1); break;
+        case 3: p2m_ds_warp<NS, 3>(lane, s0, s1, shi, slo, base, set0, set1); break;
+        default: p2m_ds_warp<NS, 4>(lane, s0, s1, shi, slo, base, set0, set1); break;
+    }
+}
+
+// ---- P2M of the full FP64 evaluation of the FP32 + refinement path (FmmTree::repeat) ----
+// The recurrences of ups_cols with every operation a double-single one, the coordinates as the
+// normalised pair of their stored hi + lo parts, the charge split once.
 template <int M, int M0, int M1, typename Fn>
 __device__ __forceinline__ void ups_col_ds(dsf x, dsf y, dsf z, dsf r2, dsf &dre, dsf &dim, Fn &f) {
     if constexpr (M > 0) {
@@ -485,18 +675,12 @@ __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, const floa
         const dsf x = ds_two_sum_f(h.x, l.x), y = ds_two_sum_f(h.y, l.y), z = ds_two_sum_f(h.z, l.z);
         const double qa_d = a.q[s], qb_d = NS == 2 ? b.q[s] : 0.0;
         const dsf qa = dsc(qa_d), qb = dsc(qb_d);
-        if constexpr (M0 == 0) {  // the charges for the near field, as k_p2m stores them
-            a.qn[(size_t)s * a.qn_stride] = qa_d;
-            if (a.qh) {
-                a.qh[(size_t)s * a.qd_stride] = qa.h;
-                a.ql[(size_t)s * a.qd_stride] = (float)(qa_d - (double)qa.h);
-            }
+        if constexpr (M0 == 0) {  // the charges for the near field
+            a.qh[(size_t)s * a.qd_stride] = qa.h;
+            a.ql[(size_t)s * a.qd_stride] = qa.l;
             if constexpr (NS == 2) {
-                b.qn[(size_t)s * b.qn_stride] = qb_d;
-                if (b.qh) {
-                    b.qh[(size_t)s * b.qd_stride] = qb.h;
-                    b.ql[(size_t)s * b.qd_stride] = (float)(qb_d - (double)qb.h);
-                }
+                b.qh[(size_t)s * b.qd_stride] = qb.h;
+                b.ql[(size_t)s * b.qd_stride] = qb.l;
             }
         }
         const dsf r2 = ds_add(ds_add(ds_mul(x, x), ds_mul(y, y)), ds_mul(z, z));
@@ -541,7 +725,7 @@ __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, const floa
 // of accumulators for two sets); one set and two run the same code, so a set's expansion
 // does not depend on whether the other is evaluated beside it.
 template <int NS>
-__global__ void __launch_bounds__(128) k_p2m_ds(int nleaf, const int *__restrict__ leaf_src,
+__global__ void __launch_bounds__(128) k_p2m_ds_repeat(int nleaf, const int *__restrict__ leaf_src,
                                                 const float4 *__restrict__ shi, const float4 *__restrict__ slo,
                                                 int leaf0, P2mSet<double> set0, P2mSet<double> set1) {
     const int lane = threadIdx.x & 31;
@@ -2049,7 +2233,11 @@ static int fmm_build_forest(Ctx &c, int L) {
             if (l == L) nsplit = OZ_TILE * (int)all.size();
             for (auto &x : level_tiles(l, NCODE_M2L, m2l_tab)) all.push_back(std::move(x));
         }
+        const size_t codes0 = codes.size();
         t->oz_m2l = plan(all);
+        if (c.opts.verbose)
+            fprintf(stderr, "fmm: m2l %zu (tile, code) products in %d tiles, %d units\n", codes.size() - codes0,
+                    t->oz_m2l.ntile, t->oz_m2l.nunit);
         t->oz_m2l.nsplit = nsplit;
         for (int l = 3; l <= L; l++) t->oz_l2l[l] = plan(level_tiles(l, 8, l2l_tab));
         std::vector<int> wexp(2 * NR), leaves(nleaf);
@@ -2088,7 +2276,7 @@ static int fmm_build_forest(Ctx &c, int L) {
     FCK(up(&t->l2l_tab, l2l_tab));
     FCK(up(&t->near_ptr, near_ptr));
     FCK(up(&t->near_leaf, near_leaf));
-    FCK(up_as<double>(&t->sloc, sloc, fp32));
+    if (!t->ds) FCK(up_as<double>(&t->sloc, sloc, fp32));
     FCK(up_as<double>(&t->tloc, tloc, fp32));
     if (t->ds) {
         // x = hi + lo, hi on the 2^-20 grid (|x| < 4 leaf units: exact in FP32)
@@ -2155,9 +2343,10 @@ static int fmm_build_forest(Ctx &c, int L) {
     FCK(cudaMemset(t->M, 0, nexp_all * esz));
     FCK(cudaMemset(t->F, 0, nexp_all * esz));
     if (t->nq == 2) {
-        FCK(cudaMalloc(&t->sq2, std::max(1, c.nsrc) * esz));
-        FCK(cudaMemset(t->sq2, 0, std::max(1, c.nsrc) * esz));
-        if (t->ds) {
+        if (!t->ds) {
+            FCK(cudaMalloc(&t->sq2, std::max(1, c.nsrc) * esz));
+            FCK(cudaMemset(t->sq2, 0, std::max(1, c.nsrc) * esz));
+        } else {
             FCK(cudaMalloc(&t->ds_q2, 2 * sizeof(float) * std::max(1, c.nsrc)));
             FCK(cudaMemset(t->ds_q2, 0, 2 * sizeof(float) * std::max(1, c.nsrc)));
         }
@@ -2247,7 +2436,7 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
         p.M = M + q * sstride;
         p.Mh = tc ? t.Mh + q * sstride : nullptr;
         p.Ml = tc ? t.Ml + q * sstride : nullptr;
-        p.qn = q ? (T *)t.sq2 : (T *)t.sloc + 3;
+        p.qn = t.ds ? nullptr : q ? (T *)t.sq2 : (T *)t.sloc + 3;
         p.qn_stride = q ? 1 : 4;
         p.qh = p.ql = nullptr;
         p.qd_stride = q ? 1 : 4;
@@ -2294,8 +2483,11 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     if constexpr (sizeof(T) == 4) {
         (nq == 2 ? k_p2m2<2> : k_p2m2<1>)<<<(t.nleaf + 3) / 4, 128, 0, c.stream>>>(
             t.nleaf, t.leaf_src, (const float *)t.sloc, t.leaf0, ps[0], ps[1]);
+    } else if (t.oz) {
+        (nq == 2 ? k_p2m_ds<2> : k_p2m_ds<1>)<<<dim3((t.nleaf + 3) / 4, 5), 128, 0, c.stream>>>(
+            t.nleaf, t.leaf_src, (const float4 *)t.ds_src_hi, (const float4 *)t.ds_src_lo, t.leaf0, ps[0], ps[1]);
     } else if (t.ds) {
-        (nq == 2 ? k_p2m_ds<2> : k_p2m_ds<1>)<<<(t.nleaf + 3) / 4, 128, 0, c.stream>>>(
+        (nq == 2 ? k_p2m_ds_repeat<2> : k_p2m_ds_repeat<1>)<<<(t.nleaf + 3) / 4, 128, 0, c.stream>>>(
             t.nleaf, t.leaf_src, (const float4 *)t.ds_src_hi, (const float4 *)t.ds_src_lo, t.leaf0, ps[0], ps[1]);
     } else {
         k_p2m<T><<<dim3((t.nleaf + 3) / 4, nq), 128, 0, c.stream>>>(t.nleaf, t.leaf_src, (const T *)t.sloc, t.leaf0,
