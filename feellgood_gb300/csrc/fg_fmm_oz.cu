@@ -70,9 +70,9 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // 32,000 (the M = 128 MMA reads
 constexpr int ITEM_BYTES = ND * KI * 2;         // digits of one expansion and item (160)
 static_assert(OZ_CELL_BYTES == IPC * ITEM_BYTES, "digit layout");
 constexpr int TMEM_COLS = 512;
-constexpr int LAG = NSTAGE - 1;
+constexpr int LAG = 3;  // items whose gathers are in flight; an item's arrival then waits for the MMAs of the
+                        // fourth item before it only (M2L of the wire, LAG 3 / 4 / 5 / 6: 0.80 / 0.80 / 0.83 / 0.87 ms)
 constexpr int NPROD = 96, NDRAIN = 384, NTHREAD = NPROD + 32 + NDRAIN;
-constexpr int NTASK = NCOL / 16 * ND / 3;  // 16-column copies per producer warp and item
 constexpr int DCOL = 32;  // columns per drain warp
 
 __device__ __forceinline__ uint64_t sdesc(uint32_t saddr) { return sdesc_kmajor(saddr, LBO, SBO); }
@@ -114,9 +114,11 @@ __global__ void __launch_bounds__(NTHREAD, 1) k_translate_oz(OzArgs a) {
     const uint32_t tmem = tmem_base;
 
     if (warp < 3) {
-        // lane pairs copy the two 16-byte halves of one column's digit, 16 columns per warp copy
-        const int half = lane & 1, csub = lane >> 1;
-        const int ngroup = ns * NCELL / 16, ntask = ngroup * ND;
+        // lane pairs copy the two 16-byte halves of one column's digit, 16 columns per copy; warp w
+        // copies columns 16 w .. 16 w + 15 of every set, all digits
+        const int half = lane & 1, ccell = 16 * warp + (lane >> 1);
+        const uint32_t dst = A_BYTES + (ccell >> 3) * SBO + half * LBO + (ccell & 7) * 16;
+        const size_t set_bytes = (size_t)a.ncell * OZ_CELL_BYTES;
         bool live = true;
         const int pc = tid % NCELL, py = tid / NCELL;  // cell and set whose scale this thread reads
         const int mycell = py < ns ? cells[pc] : -1;
@@ -126,7 +128,8 @@ __global__ void __launch_bounds__(NTHREAD, 1) k_translate_oz(OzArgs a) {
         auto scale_of = [&](int sc) { return sc >= 0 ? __ldg(a.in_scale + (size_t)py * a.ncell + sc) : 0.f; };
         int s_cur = src_of(0), s_next = src_of(1);
         float f_cur = scale_of(s_cur);
-        size_t src[NTASK];
+        const unsigned char *src = nullptr;
+        uint32_t bytes = 0;
         int armed = 0;
         for (int it = 0; it < nitems + LAG; it++) {
             if (it >= LAG) {  // the copies of item it - LAG have landed
@@ -143,13 +146,9 @@ __global__ void __launch_bounds__(NTHREAD, 1) k_translate_oz(OzArgs a) {
                     s_next = src_of(ci + 2);
                     f_cur = scale_of(s_cur);
                     asm volatile("bar.sync 1, %0;" ::"n"(NPROD) : "memory");
-#pragma unroll
-                    for (int i = 0; i < NTASK; i++) {
-                        const int task = warp + 3 * i, col = (task % ngroup) * 16 + csub, d = task / ngroup;
-                        const int y = col >= NCELL ? 1 : 0, sc = task < ntask ? scell[ring][col - NCELL * y] : -1;
-                        src[i] = sc >= 0 ? ((size_t)y * a.ncell + sc) * OZ_CELL_BYTES + d * (KI * 2) + half * 16
-                                         : ~(size_t)0;
-                    }
+                    const int sc = scell[ring][ccell];
+                    bytes = sc >= 0 ? 16u : 0u;  // 0: zero fill where the code brings the cell nothing
+                    src = a.in + (sc >= 0 ? (size_t)sc * OZ_CELL_BYTES : 0) + half * 16;
                 }
                 const int s = it % NSTAGE;
                 if (live && it >= NSTAGE && !mbar_wait(&empty[s], ((it / NSTAGE) - 1) & 1, err, &bail)) live = false;
@@ -160,16 +159,11 @@ __global__ void __launch_bounds__(NTHREAD, 1) k_translate_oz(OzArgs a) {
                         bulk_g2s(st, a.op_img + ((size_t)codes[ci] * IPC + q) * A_BYTES, A_BYTES, &bfull[s]);
                         armed = it + 1;
                     }
+                    const unsigned char *from = src + q * ITEM_BYTES;
+                    unsigned char *to = st + dst;
+                    for (int y = 0; y < ns; y++, from += set_bytes, to += (NCELL / 8) * SBO)
 #pragma unroll
-                    for (int i = 0; i < NTASK; i++) {
-                        const int task = warp + 3 * i;
-                        if (task < ntask) {
-                            const int col = (task % ngroup) * 16 + csub, d = task / ngroup;
-                            const bool ok = src[i] != ~(size_t)0;
-                            cp16(st + A_BYTES + d * B_DIGIT + (col >> 3) * SBO + half * LBO + (col & 7) * 16,
-                                 a.in + (ok ? src[i] + (size_t)q * ITEM_BYTES : 0), ok ? 16u : 0u);
-                        }
-                    }
+                        for (int d = 0; d < ND; d++) cp16(to + d * B_DIGIT, from + d * (KI * 2), bytes);
                 }
             }
             cp_commit();
@@ -193,13 +187,14 @@ __global__ void __launch_bounds__(NTHREAD, 1) k_translate_oz(OzArgs a) {
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t base = smem_u32(sm + s * STAGE_BYTES);
+                    // the address is the low field of the descriptor, in units of 16 bytes
+                    const uint64_t da = sdesc(smem_u32(sm + s * STAGE_BYTES)), db = da + A_BYTES / 16;
 #pragma unroll
                     for (int i = 0; i < ND; i++)
 #pragma unroll
                         for (int j = 0; i + j < ND; j++)
-                            mma_f16(tmem + (i + j) * NCOL, sdesc(base + i * A_DIGIT),
-                                    sdesc(base + A_BYTES + j * B_DIGIT), idesc, (q == 0 && i == 0) ? 0u : 1u);
+                            mma_f16(tmem + (i + j) * NCOL, da + i * (A_DIGIT / 16), db + j * (B_DIGIT / 16), idesc,
+                                    (q == 0 && i == 0) ? 0u : 1u);
                     mma_commit(&empty[s]);
                 }
                 mma_commit(&tfull);
