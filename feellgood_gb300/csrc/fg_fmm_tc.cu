@@ -69,7 +69,10 @@ constexpr int B_BYTES = (NB / 8) * SBO;                 // 8 KB per part
 constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // 32 KB
 constexpr int TMEM_COLS = 512;  // 2 buffers x (main, corr) x 128 columns: all of an SM's TMEM
 constexpr int IMG_BYTES = 13 * SBO;  // one operator image part: rows 0..103 (13 groups of 8)
-constexpr int LAG = NSTAGE - 1;      // items whose gathers may still be in flight
+// items whose gathers may still be in flight: an item's arrival follows its thread's wait for the
+// stage LAG - 1 items later, so fewer leave the MMAs more slack (film / platelet M2L with 5: 0.47 / 1.73
+// ms, 3: 0.455 / 1.64, 2: 0.45 / 1.64; two would not cover the gathers' latency on a busy L2)
+constexpr int LAG = 3;
 
 using namespace tc;
 
