@@ -583,8 +583,11 @@ static int create_impl(fg_ctx *h, const fg_mesh *m, const fg_region *regs, int n
         int s = fmm_build(c);
         if (s != FG_OK) return s;
     } else {
-        c.direct_nsplit = direct_splits(c);
-        CK(dalloc(&c.direct_part, (c.opts.first_order ? 1 : 2) * (size_t)c.direct_nsplit * std::max(1, c.n_mag_nodes)));
+        CK(dense_build(c, R));
+        if (!c.direct_mat) {
+            c.direct_nsplit = direct_splits(c);
+            CK(dalloc(&c.direct_part, (c.opts.first_order ? 1 : 2) * (size_t)c.direct_nsplit * std::max(1, c.n_mag_nodes)));
+        }
     }
     c.dinc = demag == FG_DEMAG_FMM && c.opts.precision == FG_PREC_FP32_REFINE && c.opts.demag_increment != 0 &&
             !c.batch;
@@ -724,7 +727,7 @@ void fg_destroy(fg_ctx *h) {
                     c.Sval32, c.A, c.Ainv, c.A32, c.tri, c.tri_c, c.tinc_ptr, c.tinc, c.src_xyz, c.mag_nodes, c.u[0], c.u[1],
                     c.v[0], c.v[1], c.phi[0], c.phi[1], c.phiv[0], c.phiv[1], c.ep, c.eq, c.ep32, c.eq32, c.Dl32,
                     c.slot, c.Dl, c.rhs, c.x, c.bv, c.W, c.fv, c.partial, c.bar, c.dres, c.src_q, c.tri_slot,
-                    c.pot, c.epart, c.src_dst, c.src_q2, c.tri_slot2, c.pot2, c.direct_part, c.fmm_err, c.tri_be, c.hsp, c.da_ds, c.J_ds, c.state_ds,
+                    c.pot, c.epart, c.src_dst, c.src_q2, c.tri_slot2, c.pot2, c.direct_part, c.direct_mat, c.fmm_err, c.tri_be, c.hsp, c.da_ds, c.J_ds, c.state_ds,
                     c.dstate32, c.da32, c.cq32, c.src_qf, c.src_q2f, c.tri_ds, c.tri32};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -888,6 +891,11 @@ int fg_step(fg_ctx *h, double dt, double prefactor, const double Hext[3], double
 
 static int demag_into(fg_ctx *h, const double *m, double *phi_out) {
     Ctx &c = h->c;
+    if (c.direct_mat) {
+        CK(launch_dense(c, m, nullptr, phi_out, nullptr));
+        c.launches += 1 + (c.dense_nshare > 1);
+        return FG_OK;
+    }
     CK(launch_charges(c, m));
     if (c.opts.demag == FG_DEMAG_FMM) {
         CK(fmm_eval(c));
@@ -918,9 +926,14 @@ static int energy_impl(fg_ctx *h, const double Hext[3], double E[4], double avg[
 }
 
 // Demag of m and of v (Fem::compute_all, src/fem.h): one evaluation of both charge sets (the
-// FMM shares the tree passes and the near field, the direct sum the distances).
+// FMM shares the tree passes and the near field, the direct sum its matrix or the distances).
 static int demag_pair(fg_ctx *h) {
     Ctx &c = h->c;
+    if (c.direct_mat) {
+        CK(launch_dense(c, c.u[1], c.v[1], c.phi[1], c.phiv[1]));
+        c.launches += 1 + (c.dense_nshare > 1);
+        return FG_OK;
+    }
     CK(launch_charges_pair(c, c.u[1], c.v[1]));
     if (c.opts.demag == FG_DEMAG_FMM) {
         CK(fmm_eval(c, 2));

@@ -276,6 +276,8 @@ struct Ctx {
     // direct sum: partial sums [set][share][magnetic node] (null with the FMM), shares
     double *direct_part = nullptr;
     int direct_nsplit = 0;
+    double *direct_mat = nullptr;  // direct sum as a matrix over the magnetic nodes (fg_dense.cu), or null
+    int dense_nshare = 0;
     // incremental demag of the FP32 + refinement path (fg_opts.demag_increment): NEXT's
     // potentials = CURRENT's + the potentials of NEXT - CURRENT (the potential is linear in
     // the field), the FP32 FMM acting on the change only, the sum kept in FP64
@@ -346,6 +348,9 @@ cudaError_t launch_apply(Ctx &c, double c0, const double *x, double *y);
 // set 0: charges into src_q / tri_slot, potential from pot; set 1: src_q2 / tri_slot2 / pot2
 cudaError_t launch_charges(Ctx &c, const double *m, int set = 0);
 cudaError_t launch_charges_pair(Ctx &c, const double *m, const double *v);  // sets 0 and 1 in one pass
+// direct sum as a matrix over the nodes (fg_dense.cu)
+cudaError_t dense_build(Ctx &c, const Rules &R);  // direct_mat stays null where it does not fit
+cudaError_t launch_dense(Ctx &c, const double *m0, const double *m1, double *phi0, double *phi1);
 int direct_splits(const Ctx &c);                 // shares of the sources of the direct sum
 cudaError_t launch_p2p_direct(Ctx &c, int nq);  // sets 0 .. nq - 1 into direct_part
 // phi = base + (pot + corr) / (4 pi) of set 0 and, phi1 not null, of set 1 (base null: no base)

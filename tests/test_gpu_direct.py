@@ -1,6 +1,7 @@
-"""The exact direct sum of the demag potential at the edges of its launch: node counts at, below
-and above a block of 64, fewer sources than one share of the split, one and several blocks, one
-and two charge sets, both Gauss rules."""
+"""The exact direct sum of the demag potential at the edges of its launches: as a matrix over the
+nodes (one and several blocks of rows, node counts at, below and above their multiples, one and
+several shares of the columns, one and two fields, both Gauss rules) and, where the matrix would be
+too large, as the sum over Gauss points."""
 import numpy as np
 import pytest
 
@@ -33,3 +34,22 @@ def test_direct_sum_edges(shape, one_point, first_order):
     assert np.linalg.norm(c.demag(0) - po) < 4e-12 * np.linalg.norm(po)
     if not first_order:
         assert np.linalg.norm(s["phiv"] - pv) < 1e-11 * np.linalg.norm(pv)
+
+
+def test_direct_sum_over_gauss_points_where_the_matrix_does_not_fit():
+    """45,000 nodes (a matrix of 48 GB): the potentials of a few nodes against their sums."""
+    m = cases.cuboid(74, 74, 7)
+    u = cases.perturbed_state(m["xyz"], seed=13, sigma=0.3)
+    v = cases.tangent_field(u, seed=14)
+    c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_DIRECT)
+    c.set_state(u, v)
+    c.compute_all(np.zeros(3))
+    s = c.get_state(0)
+    o = fgo.Oracle(m, cases.oracle_regions())
+    o.set_state(u, v)
+    pick = np.linspace(0, len(m["xyz"]) - 1, 12).astype(int)
+    for which, got in ((0, s["phi"]), (1, s["phiv"])):
+        pts, q, corr = o.charges(which)
+        ref = np.array([((q / np.linalg.norm(pts - m["xyz"][i], axis=1)).sum() + corr[i]) / (4 * np.pi) for i in pick])
+        # 1.4 million FP64 terms on either side, summed in shares of thousands
+        assert np.linalg.norm(got[pick] - ref) < 1e-11 * np.linalg.norm(ref) * (1 if which == 0 else 10)
