@@ -898,14 +898,15 @@ static int demag_into(fg_ctx *h, const double *m, double *phi_out) {
     }
     CK(launch_charges(c, m));
     if (c.opts.demag == FG_DEMAG_FMM) {
-        CK(fmm_eval(c));
-        c.launches += fmm_launches_per_eval(c);
+        CK(fmm_eval(c, 1, {{m, nullptr}, {phi_out, nullptr}}));
+        c.launches += 1 + fmm_launches_per_eval(c);
+        if (fmm_whole(c)) return FG_OK;
     } else {
         CK(launch_p2p_direct(c, 1));
-        c.launches += 1;
+        c.launches += 2;
     }
     CK(launch_phi_final(c, phi_out));
-    c.launches += 2;
+    c.launches += 1;
     return FG_OK;
 }
 
@@ -936,14 +937,15 @@ static int demag_pair(fg_ctx *h) {
     }
     CK(launch_charges_pair(c, c.u[1], c.v[1]));
     if (c.opts.demag == FG_DEMAG_FMM) {
-        CK(fmm_eval(c, 2));
-        c.launches += fmm_launches_per_eval(c, 2);
+        CK(fmm_eval(c, 2, {{c.u[1], c.v[1]}, {c.phi[1], c.phiv[1]}}));
+        c.launches += 1 + fmm_launches_per_eval(c, 2);
+        if (fmm_whole(c)) return FG_OK;
     } else {
         CK(launch_p2p_direct(c, 2));
-        c.launches += 1;
+        c.launches += 2;
     }
     CK(launch_phi_final(c, c.phi[1], c.phiv[1]));
-    c.launches += 2;
+    c.launches += 1;
     return FG_OK;
 }
 
@@ -959,7 +961,7 @@ static int demag_increment(fg_ctx *h) {
         CK(launch_state_diff(c));
         CK(launch_charges32(c, nq));
         c.charges32 = true;  // the FP32 FMM reads the FP32 charges of the change
-        const cudaError_t se = fmm_eval(c, nq);
+        const cudaError_t se = fmm_eval(c, nq, FmmFields{});
         c.charges32 = false;
         CK(se);
         CK(launch_phi_final(c, c.phi[1], nq == 2 ? c.phiv[1] : nullptr, c.phi[0], c.phiv[0]));

@@ -13,7 +13,9 @@
 // nodes 0.061 ms, 180 nodes 0.013. Forming B costs about one such sum. Against quadruple
 // precision the potentials are as exact as those sums (6e-16 for a smooth field of 1,680 nodes).
 #include <algorithm>
+#include <vector>
 
+#include "fg_ds.cuh"
 #include "fg_internal.h"
 
 namespace fg {
@@ -201,6 +203,445 @@ cudaError_t launch_dense(Ctx &c, const double *m0, const double *m1, double *phi
     if (c.dense_nshare > 1)
         k_dense_sum<<<dim3((n + 127) / 128, m1 ? 2 : 1), 128, 0, c.stream>>>(n, c.mag_nodes, c.dense_nshare, c.direct_part,
                                                                             phi0, phi1);
+    return cudaGetLastError();
+}
+
+}  // namespace fg
+
+// ---------------------------------------------------------------------------------
+// Near field of the FP64 FMM as dense blocks over the nodes.
+//
+// The same linearity holds leaf by leaf: the potentials of a leaf's target nodes from the Gauss
+// points of its adjacent leaves, plus the triangles' self-corrections, are a block of
+// [targets][3 column nodes], the columns being the nodes of every element with a Gauss point
+// there (an element whose points lie in near and far leaves contributes its near points only).
+// Formed once in FP64, stored as double-single pairs (48 bits, the arithmetic of the pair sum it
+// replaces), 8 bytes per entry: film of 1.2M tets 4.1 GB, read once per evaluation of both fields.
+
+namespace fg {
+
+namespace {
+
+constexpr int HASH = 8192;      // slots of a leaf's tables in shared memory
+constexpr int MAX_NODE = 4096;  // column nodes and elements a leaf may have
+constexpr int MAX_ELEM = 6144;
+constexpr int TG = 8;           // targets formed together
+
+__device__ __forceinline__ int hash_of(int key) { return (int)(((unsigned)key * 2654435761u) >> 19); }
+
+// Adds key to the table unless it holds more than `most` keys (the caller then gives the leaf up).
+__device__ __forceinline__ int hash_add(int *tab, int key, int *count, int most) {
+    int h = hash_of(key);
+    for (;;) {
+        if (*(volatile int *)count > most) return -1;
+        const int prev = atomicCAS(&tab[h], -1, key);
+        if (prev == -1) atomicAdd(count, 1);
+        if (prev == -1 || prev == key) return h;
+        h = (h + 1) & (HASH - 1);
+    }
+}
+__device__ __forceinline__ int hash_find(const int *tab, int key) {
+    for (int h = hash_of(key);; h = (h + 1) & (HASH - 1)) {
+        const int k = tab[h];
+        if (k == key) return h;
+        if (k == -1) return -1;
+    }
+}
+
+struct NearArgs {
+    int nleaf, nmt, npi_t, npi_f;
+    const int *leaf_src, *leaf_tgt, *tgt_node, *near_ptr, *near_leaf, *src_orig;
+    const int4 *tet, *tri;
+    const int *tinc_ptr, *tinc;
+};
+
+// f(element, Gauss point) for every source of the leaf's adjacent leaves; elements are the
+// magnetic tetrahedra, then the triangles. Every thread of the block takes part.
+template <typename Fn>
+__device__ __forceinline__ void near_sources(const NearArgs &a, int leaf, Fn &&f) {
+    for (int e = a.near_ptr[leaf]; e < a.near_ptr[leaf + 1]; e++) {
+        const int nl = a.near_leaf[e];
+        for (int s = a.leaf_src[nl] + threadIdx.x; s < a.leaf_src[nl + 1]; s += blockDim.x) {
+            const int o = a.src_orig[s], nt = a.nmt * a.npi_t;
+            if (o < nt) f(o / a.npi_t, o % a.npi_t);
+            else f(a.nmt + (o - nt) / a.npi_f, (o - nt) % a.npi_f);
+        }
+    }
+}
+
+// The column nodes of a leaf into the table `nodes`, its elements into `elems`.
+__device__ __forceinline__ void near_tables(const NearArgs &a, int leaf, int *nodes, int *elems, int *nn, int *ne) {
+    for (int k = threadIdx.x; k < HASH; k += blockDim.x) nodes[k] = elems[k] = -1;
+    if (threadIdx.x == 0) *nn = *ne = 0;
+    __syncthreads();
+    near_sources(a, leaf, [&](int el, int) { hash_add(elems, el, ne, MAX_ELEM); });
+    __syncthreads();
+    auto add_tri = [&](int f) {
+        const int4 v = a.tri[f];
+        hash_add(nodes, v.x, nn, MAX_NODE);
+        hash_add(nodes, v.y, nn, MAX_NODE);
+        hash_add(nodes, v.z, nn, MAX_NODE);
+    };
+    for (int k = threadIdx.x; k < HASH; k += blockDim.x) {
+        const int el = elems[k];
+        if (el < 0) continue;
+        if (el < a.nmt) {
+            const int4 v = a.tet[el];
+            hash_add(nodes, v.x, nn, MAX_NODE);
+            hash_add(nodes, v.y, nn, MAX_NODE);
+            hash_add(nodes, v.z, nn, MAX_NODE);
+            hash_add(nodes, v.w, nn, MAX_NODE);
+        } else {
+            add_tri(el - a.nmt);
+        }
+    }
+    // the self-corrections reach the nodes of every triangle of a target
+    for (int t = a.leaf_tgt[leaf] + threadIdx.x; t < a.leaf_tgt[leaf + 1]; t += blockDim.x) {
+        const int i = a.tgt_node[t];
+        for (int k = a.tinc_ptr[i]; k < a.tinc_ptr[i + 1]; k++) add_tri(a.tinc[k] / 3);
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) k_near_count(NearArgs a, int *ncol, int *over) {
+    extern __shared__ int tab[];
+    __shared__ int nn, ne;
+    const int leaf = blockIdx.x;
+    if (a.leaf_tgt[leaf] == a.leaf_tgt[leaf + 1]) {
+        if (threadIdx.x == 0) ncol[leaf] = 0;
+        return;
+    }
+    near_tables(a, leaf, tab, tab + HASH, &nn, &ne);
+    if (threadIdx.x == 0) {
+        ncol[leaf] = nn;
+        if (nn > MAX_NODE || ne > MAX_ELEM) *over = 1;
+    }
+}
+
+// The columns of every leaf in ascending order (cptr: first column, padded to an even number with -1).
+__global__ void __launch_bounds__(256) k_near_cols(NearArgs a, const int *cptr, const int *ncol, int *col) {
+    extern __shared__ int tab[];
+    __shared__ int nn, ne, cnt;
+    const int leaf = blockIdx.x, n = ncol[leaf];
+    if (n == 0) return;
+    near_tables(a, leaf, tab, tab + HASH, &nn, &ne);
+    if (threadIdx.x == 0) cnt = 0;
+    int *list = tab + HASH;
+    int m = 1;
+    while (m < n) m <<= 1;
+    for (int k = threadIdx.x; k < m; k += 256) list[k] = 0x7fffffff;
+    __syncthreads();
+    for (int k = threadIdx.x; k < HASH; k += 256)
+        if (tab[k] >= 0) list[atomicAdd(&cnt, 1)] = tab[k];
+    for (int size = 2; size <= m; size <<= 1)
+        for (int s = size >> 1; s > 0; s >>= 1) {
+            __syncthreads();
+            for (int k = threadIdx.x; k < m; k += 256) {
+                const int p = k ^ s;
+                if (p > k && (list[k] > list[p]) == ((k & size) == 0)) {
+                    const int t = list[k];
+                    list[k] = list[p];
+                    list[p] = t;
+                }
+            }
+        }
+    __syncthreads();
+    for (int k = threadIdx.x; k < cptr[leaf + 1] - cptr[leaf]; k += 256) col[cptr[leaf] + k] = k < n ? list[k] : -1;
+}
+
+// The entries of every leaf's block, 8 targets at a time: G[slot][target] = sum over a tetrahedron's
+// near Gauss points of w_g / r, then a thread per column node gathers its tetrahedra (in the
+// order of its incidence list) and triangles.
+__global__ void __launch_bounds__(256) k_near_fill(NearArgs a, Rules R, const int *__restrict__ cptr,
+                                                   const int *__restrict__ col, const size_t *__restrict__ boff,
+                                                   const double *__restrict__ xyz, const double *__restrict__ src,
+                                                   const double *__restrict__ da, const double *__restrict__ detJ,
+                                                   const int *__restrict__ treg, const DevRegion *__restrict__ regs,
+                                                   const int *__restrict__ inc_ptr, const int *__restrict__ inc,
+                                                   const DevTri *__restrict__ tc, double *__restrict__ scratch,
+                                                   float2 *__restrict__ B) {
+    extern __shared__ int tab[];
+    int *mask = tab + HASH;
+    __shared__ double tx[TG][3];
+    __shared__ int tn[TG], ne;
+    double *G = scratch + (size_t)blockIdx.x * HASH * TG;
+    for (int leaf = blockIdx.x; leaf < a.nleaf; leaf += gridDim.x) {
+        const int t0 = a.leaf_tgt[leaf], t1 = a.leaf_tgt[leaf + 1], c0 = cptr[leaf], nc = cptr[leaf + 1] - c0;
+        if (t0 == t1) continue;
+        __syncthreads();
+        for (int k = threadIdx.x; k < HASH; k += 256) {
+            tab[k] = -1;
+            mask[k] = 0;
+        }
+        if (threadIdx.x == 0) ne = 0;
+        __syncthreads();
+        near_sources(a, leaf, [&](int el, int g) {
+            const int h = hash_add(tab, el, &ne, MAX_ELEM);
+            if (h >= 0) atomicOr(&mask[h], 1 << g);
+        });
+        for (int tb = t0; tb < t1; tb += TG) {
+            const int nt = min(TG, t1 - tb);
+            __syncthreads();
+            if (threadIdx.x < TG) {
+                const int i = a.tgt_node[tb + min((int)threadIdx.x, nt - 1)];
+                tn[threadIdx.x] = i;
+                for (int d = 0; d < 3; d++) tx[threadIdx.x][d] = xyz[3 * (size_t)i + d];
+            }
+            __syncthreads();
+            for (int k = threadIdx.x; k < HASH; k += 256) {
+                const int el = tab[k], mk = mask[k];
+                if (el < 0 || el >= a.nmt) continue;
+                double s[TG];
+#pragma unroll
+                for (int t = 0; t < TG; t++) s[t] = 0.0;
+                for (int g = 0; g < R.npi_t; g++) {
+                    if (!(mk >> g & 1)) continue;
+                    const double *p = src + 3 * ((size_t)el * R.npi_t + g);
+                    const double px = p[0], py = p[1], pz = p[2], w = R.tp[g];
+#pragma unroll
+                    for (int t = 0; t < TG; t++) {
+                        const double dx = tx[t][0] - px, dy = tx[t][1] - py, dz = tx[t][2] - pz;
+                        s[t] += w * rsqrt(dx * dx + dy * dy + dz * dz);
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < TG; t++) G[(size_t)k * TG + t] = s[t];
+            }
+            __syncthreads();
+            for (int j = threadIdx.x; j < nc; j += 256) {
+                const int node = col[c0 + j];
+                double b[TG][3];
+#pragma unroll
+                for (int t = 0; t < TG; t++) b[t][0] = b[t][1] = b[t][2] = 0.0;
+                if (node >= 0) {
+                    for (int q = inc_ptr[node]; q < inc_ptr[node + 1]; q++) {
+                        const int el = inc[q] >> 2, v = inc[q] & 3, h = hash_find(tab, el);
+                        if (h < 0) continue;
+                        const double w = -regs[treg[el]].Ms * detJ[el];
+                        double k[3];
+#pragma unroll
+                        for (int c = 0; c < 3; c++) k[c] = w * da[(3 * v + c) * (size_t)a.nmt + el];
+#pragma unroll
+                        for (int t = 0; t < TG; t++) {
+                            const double g = G[(size_t)h * TG + t];
+#pragma unroll
+                            for (int c = 0; c < 3; c++) b[t][c] += k[c] * g;
+                        }
+                    }
+                    for (int q = a.tinc_ptr[node]; q < a.tinc_ptr[node + 1]; q++) {
+                        const int f = a.tinc[q] / 3, v = a.tinc[q] % 3, h = hash_find(tab, a.nmt + f);
+                        const int mk = h >= 0 ? mask[h] : 0;
+                        const DevTri &T = tc[f];
+                        const int4 vt = a.tri[f];
+#pragma unroll
+                        for (int t = 0; t < TG; t++) {
+                            double g = 0.0;
+                            for (int p = 0; p < R.npi_f; p++) {
+                                if (!(mk >> p & 1)) continue;
+                                const double *y = src + 3 * ((size_t)a.nmt * R.npi_t + (size_t)f * R.npi_f + p);
+                                const double dx = tx[t][0] - y[0], dy = tx[t][1] - y[1], dz = tx[t][2] - y[2];
+                                g += T.w[p] * R.fa[v][p] * rsqrt(dx * dx + dy * dy + dz * dz);
+                            }
+                            const int own = tn[t] == vt.x ? 0 : tn[t] == vt.y ? 1 : tn[t] == vt.z ? 2 : -1;
+                            if (own >= 0) g += T.beta[3 * own + v];
+                            g *= T.dMs;
+#pragma unroll
+                            for (int c = 0; c < 3; c++) b[t][c] += g * T.n[c];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int t = 0; t < TG; t++) {
+                    if (t >= nt) break;
+                    float2 *o = B + boff[leaf] + (size_t)(tb + t - t0) * 3 * nc + 3 * j;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        const double v = b[t][c] / (4 * M_PI);
+                        const float h = (float)v;
+                        o[c] = make_float2(h, (float)(v - (double)h));
+                    }
+                }
+            }
+        }
+    }
+}
+
+// The fields as double-single pairs: (u hi, u lo, v hi, v lo) per component.
+__global__ void k_field_pairs(size_t n3, const double *__restrict__ u, const double *__restrict__ v,
+                              float4 *__restrict__ m) {
+    const size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (k >= n3) return;
+    const double x = u[k], y = v ? v[k] : 0.0;
+    const float xh = (float)x, yh = (float)y;
+    m[k] = make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
+}
+
+// Near potentials of NQ fields: a block per task (up to 16 targets of a leaf, two per warp), the
+// column nodes' fields staged in shared memory in tiles of NEAR_TILE entries, two entries of a
+// row per 16-byte load. 12 FP32 operations per entry and field (product with its rounding error
+// and cross terms, two-sum), 8 bytes of the block: HBM bounds it.
+constexpr int NEAR_TILE = 1536;
+template <int NQ>
+__global__ void __launch_bounds__(256) k_near_mv(const int4 *__restrict__ task, const int *__restrict__ leaf_tgt,
+                                                 const int *__restrict__ tgt_node, const int *__restrict__ cptr,
+                                                 const int *__restrict__ col, const size_t *__restrict__ boff,
+                                                 const float2 *__restrict__ B, const float4 *__restrict__ m,
+                                                 double *__restrict__ pot0, double *__restrict__ pot1) {
+    __shared__ float4 sm[NEAR_TILE];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int4 t = task[blockIdx.x];  // leaf, first target, targets
+    const int c0 = cptr[t.x], ne = 3 * (cptr[t.x + 1] - c0);
+    const int r0 = 2 * warp, row = t.y - leaf_tgt[t.x];
+    const bool on0 = r0 < t.z, on1 = r0 + 1 < t.z;
+    const float2 *b0 = B + boff[t.x] + (size_t)(row + (on0 ? r0 : 0)) * ne;
+    const float2 *b1 = on1 ? b0 + ne : b0;
+    float h[2][NQ], l[2][NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) h[0][q] = h[1][q] = l[0][q] = l[1][q] = 0.f;
+    auto add = [&](float &hi, float &lo, float bh, float bl, float mh, float ml) {
+        const float p = bh * mh;
+        const float e = fmaf(bl, mh, fmaf(bh, ml, fmaf(bh, mh, -p)));
+        const float s = hi + p, x = s - hi;
+        lo += ((hi - (s - x)) + (p - x)) + e;
+        hi = s;
+    };
+    for (int base = 0; base < ne; base += NEAR_TILE) {
+        const int len = min(NEAR_TILE, ne - base);
+        __syncthreads();
+        for (int e = threadIdx.x; e < len; e += 256) {
+            const int node = col[c0 + (base + e) / 3];
+            sm[e] = node >= 0 ? m[3 * (size_t)node + (base + e) % 3] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncthreads();
+        if (!on0) continue;
+        const float4 *p0 = reinterpret_cast<const float4 *>(b0 + base), *p1 = reinterpret_cast<const float4 *>(b1 + base);
+#pragma unroll 2
+        for (int e = lane; e < len / 2; e += 32) {
+            const float4 x0 = __ldcs(p0 + e), x1 = __ldcs(p1 + e), ma = sm[2 * e], mb = sm[2 * e + 1];
+            add(h[0][0], l[0][0], x0.x, x0.y, ma.x, ma.y);
+            add(h[1][0], l[1][0], x1.x, x1.y, ma.x, ma.y);
+            add(h[0][0], l[0][0], x0.z, x0.w, mb.x, mb.y);
+            add(h[1][0], l[1][0], x1.z, x1.w, mb.x, mb.y);
+            if constexpr (NQ == 2) {
+                add(h[0][1], l[0][1], x0.x, x0.y, ma.z, ma.w);
+                add(h[1][1], l[1][1], x1.x, x1.y, ma.z, ma.w);
+                add(h[0][1], l[0][1], x0.z, x0.w, mb.z, mb.w);
+                add(h[1][1], l[1][1], x1.z, x1.w, mb.z, mb.w);
+            }
+        }
+    }
+    if (!on0) return;
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            dsf s = ds_quick(h[r][q], l[r][q]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1)
+                s = ds_add(s, dsf{__shfl_xor_sync(0xffffffffu, s.h, o), __shfl_xor_sync(0xffffffffu, s.l, o)});
+            if (lane == 0 && (r == 0 || on1)) (q ? pot1 : pot0)[tgt_node[t.y + r0 + r]] = ds_to(s);
+        }
+}
+
+}  // namespace
+
+// Forms the blocks where they fit (1/8 of the device's memory, half of what is free; at most
+// MAX_NODE columns and MAX_ELEM elements per leaf); without them (N.B null) the pair sum runs.
+cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
+    size_t free_b = 0, total_b = 0;
+    cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
+    if (e != cudaSuccess) return e;
+    NearArgs a{t.nleaf, c.nmt, R.npi_t, R.npi_f, t.leaf_src, t.leaf_tgt, t.tgt_node, t.near_ptr, t.near_leaf, nullptr,
+               c.tet, c.tri, c.tinc_ptr, c.tinc};
+    int *orig = nullptr, *ncol = nullptr;
+    double *scratch = nullptr;
+    const int smem = 2 * HASH * (int)sizeof(int), blocks = std::min(t.nleaf, 2 * std::max(1, c.nsm));
+    auto done = [&](cudaError_t r) {
+        for (void *p : {(void *)orig, (void *)ncol, (void *)scratch})
+            if (p) cudaFree(p);
+        if (r != cudaSuccess || !N.B) near_free(N);
+        cudaGetLastError();
+        // what does not fit is no error: the pair sum needs none of it
+        return r == cudaErrorMemoryAllocation ? cudaSuccess : r;
+    };
+#define NCK(call)                              \
+    do {                                       \
+        const cudaError_t r_ = (call);         \
+        if (r_ != cudaSuccess) return done(r_); \
+    } while (0)
+    NCK(cudaFuncSetAttribute(k_near_count, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NCK(cudaFuncSetAttribute(k_near_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NCK(cudaFuncSetAttribute(k_near_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    NCK(cudaMalloc(&orig, sizeof(int) * std::max(1, c.nsrc)));
+    NCK(cudaMemcpyAsync(orig, t.src_orig, sizeof(int) * c.nsrc, cudaMemcpyHostToDevice, c.stream));
+    NCK(cudaMalloc(&ncol, sizeof(int) * (t.nleaf + 1)));
+    NCK(cudaMemsetAsync(ncol, 0, sizeof(int) * (t.nleaf + 1), c.stream));
+    a.src_orig = orig;
+    k_near_count<<<t.nleaf, 256, smem, c.stream>>>(a, ncol, ncol + t.nleaf);
+    std::vector<int> hn(t.nleaf + 1);
+    NCK(cudaMemcpyAsync(hn.data(), ncol, sizeof(int) * (t.nleaf + 1), cudaMemcpyDeviceToHost, c.stream));
+    NCK(cudaStreamSynchronize(c.stream));
+    if (hn[t.nleaf]) return done(cudaSuccess);
+    std::vector<int> cptr(t.nleaf + 1, 0);
+    std::vector<size_t> boff(t.nleaf, 0);
+    std::vector<int4> task;
+    size_t entries = 0;
+    for (int l = 0; l < t.nleaf; l++) {
+        const int nc = (hn[l] + 1) & ~1, nt = t.h_leaf_tgt[l + 1] - t.h_leaf_tgt[l];
+        if ((size_t)cptr[l] + nc > 0x7fffffff) return done(cudaSuccess);
+        cptr[l + 1] = cptr[l] + nc;
+        boff[l] = entries;
+        entries += (size_t)nt * 3 * nc;
+        const int groups = (nt + 15) / 16;
+        for (int g = 0; g < groups; g++) {
+            const int b = (int)((long)nt * g / groups), f = (int)((long)nt * (g + 1) / groups);
+            task.push_back(make_int4(l, t.h_leaf_tgt[l] + b, f - b, 0));
+        }
+    }
+    if (entries == 0 || entries * sizeof(float2) > std::min(total_b / 8, free_b / 2)) return done(cudaSuccess);
+    N.ntask = (int)task.size();
+    NCK(cudaMalloc(&scratch, sizeof(double) * HASH * TG * (size_t)blocks));
+    NCK(cudaMalloc(&N.cptr, sizeof(int) * (t.nleaf + 1)));
+    NCK(cudaMalloc(&N.boff, sizeof(size_t) * t.nleaf));
+    NCK(cudaMalloc(&N.task, sizeof(int4) * N.ntask));
+    NCK(cudaMalloc(&N.col, sizeof(int) * cptr[t.nleaf]));
+    NCK(cudaMalloc(&N.field, sizeof(float4) * 3 * (size_t)c.nn));
+    NCK(cudaMalloc(&N.B, sizeof(float2) * entries));
+    auto filled = [&]() -> cudaError_t {
+        cudaError_t r = cudaMemcpyAsync(N.cptr, cptr.data(), sizeof(int) * (t.nleaf + 1), cudaMemcpyHostToDevice, c.stream);
+        if (r == cudaSuccess)
+            r = cudaMemcpyAsync(N.boff, boff.data(), sizeof(size_t) * t.nleaf, cudaMemcpyHostToDevice, c.stream);
+        if (r == cudaSuccess)
+            r = cudaMemcpyAsync(N.task, task.data(), sizeof(int4) * N.ntask, cudaMemcpyHostToDevice, c.stream);
+        if (r != cudaSuccess) return r;
+        k_near_cols<<<t.nleaf, 256, smem, c.stream>>>(a, N.cptr, ncol, N.col);
+        k_near_fill<<<blocks, 256, smem, c.stream>>>(a, R, N.cptr, N.col, N.boff, c.xyz, c.src_xyz, c.da, c.detJ, c.treg,
+                                                     c.regs, c.inc_ptr, c.inc, c.tri_c, scratch, N.B);
+        r = cudaGetLastError();
+        return r == cudaSuccess ? cudaStreamSynchronize(c.stream) : r;
+    };
+    const cudaError_t r = filled();
+    if (r != cudaSuccess) {
+        cudaFree(N.B);
+        N.B = nullptr;
+    }
+#undef NCK
+    return done(r);
+}
+
+void near_free(NearMat &N) {
+    for (void *p : {(void *)N.cptr, (void *)N.boff, (void *)N.task, (void *)N.col, (void *)N.field, (void *)N.B})
+        if (p) cudaFree(p);
+    N = NearMat();
+}
+
+cudaError_t launch_near(Ctx &c, const NearTree &t, const NearMat &N, cudaStream_t st, const double *m0, const double *m1,
+                        double *pot0, double *pot1) {
+    if (N.ntask == 0) return cudaSuccess;
+    const size_t n3 = 3 * (size_t)c.nn;
+    k_field_pairs<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(n3, m0, m1, N.field);
+    (m1 ? k_near_mv<2> : k_near_mv<1>)<<<N.ntask, 256, 0, st>>>(N.task, t.leaf_tgt, t.tgt_node, N.cptr, N.col, N.boff, N.B,
+                                                               N.field, pot0, pot1);
     return cudaGetLastError();
 }
 

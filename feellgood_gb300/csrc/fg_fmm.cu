@@ -84,6 +84,7 @@ struct FmmTree {
     // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9
     // in phiv two steps later (film), so runs repeat bit for bit only with the same last bits
     bool repeat = false;
+    NearMat near;              // oz: the near field as dense blocks, where they fit
     int4 *p2p_task = nullptr;  // leaf, first target, targets (at most 8) of a near-field block
     int n_p2p_task = 0;
     float4 *ds_src_hi = nullptr, *ds_src_lo = nullptr, *ds_tgt_hi = nullptr, *ds_tgt_lo = nullptr;
@@ -917,6 +918,7 @@ struct NearSets {
     const T *F[2];          // local expansions per set
     double *pot[2];         // potentials per set
     int near_only;          // 1: write the near-field sums only (k_l2p adds the far field later)
+    double *phi[2];         // k_l2p: not null: finished potentials, the near sums being theirs already
 };
 
 // One pass of the near field and L2P over up to NT targets tb.. of a leaf (nt of them real,
@@ -1574,6 +1576,12 @@ __global__ void __launch_bounds__(128) k_l2p(int ntgt, const int *__restrict__ t
         }
     });
     const int node = tgt_node[ti];
+    if (sets.phi[0]) {
+        const double f = sc / (4 * M_PI);
+        sets.phi[0][node] = fma(double(fa), f, sets.pot[0][node]);
+        if constexpr (NQ == 2) sets.phi[1][node] = fma(double(fb), f, sets.pot[1][node]);
+        return;
+    }
     sets.pot[0][node] = (double(fa) + sets.pot[0][node]) * sc;
     if constexpr (NQ == 2) sets.pot[1][node] = (double(fb) + sets.pot[1][node]) * sc;
 }
@@ -1706,7 +1714,11 @@ static void oz_weights(int *wM, int *wF) {
 void fmm_free(Ctx &c);
 static int fmm_build_forest(Ctx &c, int L);
 template <typename T>
-static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq);
+static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f);
+static FmmFields tuning_fields(const Ctx &c) { return {{c.u[1], c.v[1]}, {c.pot, c.pot2}}; }
+static NearTree near_tree(const FmmTree &t) {
+    return {t.nleaf, t.leaf_src, t.leaf_tgt, t.tgt_node, t.near_ptr, t.near_leaf, nullptr, nullptr};
+}
 
 // Points of each sample (sources and target nodes) and the sample's root cube. A batch of
 // independent meshes gets one octree per sample (a forest); a single mesh is one tree.
@@ -1840,10 +1852,10 @@ int fmm_build(Ctx &c) {
         cudaEvent_t a, b;
         FCK(cudaEventCreate(&a));
         FCK(cudaEventCreate(&b));
-        FCK(fp32 ? fmm_eval_t<float>(c, *t, t->nq) : fmm_eval_t<double>(c, *t, t->nq));
+        FCK(fp32 ? fmm_eval_t<float>(c, *t, t->nq, tuning_fields(c)) : fmm_eval_t<double>(c, *t, t->nq, tuning_fields(c)));
         FCK(cudaEventRecord(a, c.stream));
         for (int r = 0; r < 2; r++)
-            FCK(fp32 ? fmm_eval_t<float>(c, *t, t->nq) : fmm_eval_t<double>(c, *t, t->nq));
+            FCK(fp32 ? fmm_eval_t<float>(c, *t, t->nq, tuning_fields(c)) : fmm_eval_t<double>(c, *t, t->nq, tuning_fields(c)));
         FCK(cudaEventRecord(b, c.stream));
         FCK(cudaEventSynchronize(b));
         float ms = 0;
@@ -2323,6 +2335,14 @@ static int fmm_build_forest(Ctx &c, int L) {
         }
         t->n_p2p_task = (int)task.size();
         FCK(up(&t->p2p_task, task));
+        if (t->oz) {
+            std::vector<int> orig(c.nsrc);
+            for (int k = 0; k < c.nsrc; k++) orig[src_dst[k]] = k;
+            NearTree nt = near_tree(*t);
+            nt.src_orig = orig.data();
+            nt.h_leaf_tgt = leaf_tgt.data();
+            FCK(near_build(c, make_rules(c.opts.one_gauss_point != 0), nt, t->near));
+        }
         FCK(up(&t->ds_src_hi, sh));
         FCK(up(&t->ds_src_lo, sl));
         FCK(up(&t->ds_tgt_hi, th));
@@ -2382,6 +2402,7 @@ void fmm_free(Ctx &c) {
                     t->oz_rows[1], t->oz_rows[2]};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    near_free(t->near);
     for (auto &set : t->ev)
         for (auto &e : set)
             if (e) cudaEventDestroy(e);
@@ -2414,7 +2435,7 @@ static void harvest_set(FmmTree &t, int k) {
 // c.src_q2 into c.pot2. The sets share every table, operator image and launch (grid y of
 // P2M and of the tensor-core translations; one near-field pass computes both).
 template <typename T>
-static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
+static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
     if (nq < 1 || nq > t.nq || (nq == 2 && (!c.src_q2 || !c.pot2))) return cudaErrorInvalidValue;
     const int L = t.L;
     T *M = (T *)t.M, *F = (T *)t.F;
@@ -2459,8 +2480,18 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     ns.pot[0] = c.pot;
     ns.pot[1] = nq == 2 ? c.pot2 : c.pot;
     ns.near_only = 0;
+    const bool whole = t.near.B != nullptr;
+    for (int k = 0; k < 2; k++) ns.phi[k] = whole ? f.phi[k < nq ? k : 0] : nullptr;
     const int nb = (t.nleaf + 3) / 4;
+    cudaError_t terr = cudaSuccess;  // first failed launch of a translation or of the near field
+    auto note = [&](cudaError_t e) {
+        if (e != cudaSuccess && terr == cudaSuccess) terr = e;
+    };
     auto near_field = [&](cudaStream_t st) {
+        if (whole) {
+            note(launch_near(c, near_tree(t), t.near, st, f.m[0], nq == 2 ? f.m[1] : nullptr, c.pot, c.pot2));
+            return;
+        }
         if constexpr (sizeof(T) == 8) {
             if (t.repeat) {
                 auto k = nq == 2 ? k_l2p_p2p_ds<2> : k_l2p_p2p_ds<1>;
@@ -2497,7 +2528,6 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     // out (+)= sum_code Op[code] in[tab[cell][code]] over n output cells from out0; the
     // tensor-core form reads the inputs' hi/lo split and writes the outputs' split
     enum { M2M, M2L, L2L };
-    cudaError_t terr = cudaSuccess;  // first failed translation launch
     auto translate = [&](int kind, int n, int out0, const FmmTree::TcLaunch &tl) {
         if (!n) return;
         const int ncode = kind == M2L ? NCODE_M2L : 8;
@@ -2534,9 +2564,6 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     };
     // FP64 path: exact digit products on the tensor cores, then the sums of the units' partial
     // results and the digits of the next translation's inputs
-    auto note = [&](cudaError_t e) {
-        if (e != cudaSuccess && terr == cudaSuccess) terr = e;
-    };
     OzFinish fa{};
     if (t.oz) {
         fa.ncell = t.ncell; fa.nset = nq; fa.scratch = t.oz_scratch; fa.digits = t.oz_digits; fa.scale = t.oz_scale;
@@ -2600,10 +2627,15 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq) {
     return terr != cudaSuccess ? terr : e;
 }
 
-cudaError_t fmm_eval(Ctx &c, int nq) {
+bool fmm_whole(const Ctx &c) {
+    const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
+    return t && t->near.B;
+}
+
+cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f) {
     FmmTree *t = static_cast<FmmTree *>(c.fmm);
     if (!t) return cudaErrorNotSupported;
-    return t->fp32 ? fmm_eval_t<float>(c, *t, nq) : fmm_eval_t<double>(c, *t, nq);
+    return t->fp32 ? fmm_eval_t<float>(c, *t, nq, f) : fmm_eval_t<double>(c, *t, nq, f);
 }
 
 int fmm_eval_fp64(Ctx &c, int nq) {
@@ -2613,7 +2645,7 @@ int fmm_eval_fp64(Ctx &c, int nq) {
         return FG_EINVAL;
     }
     if (!t32->fp32) {
-        FCK(fmm_eval_t<double>(c, *t32, nq));
+        FCK(fmm_eval_t<double>(c, *t32, nq, FmmFields{}));
         return FG_OK;
     }
     if (!c.fmm64) {
@@ -2630,7 +2662,7 @@ int fmm_eval_fp64(Ctx &c, int nq) {
         c.fmm64 = t;
         c.fmm = t32;
     }
-    FCK(fmm_eval_t<double>(c, *static_cast<FmmTree *>(c.fmm64), nq));
+    FCK(fmm_eval_t<double>(c, *static_cast<FmmTree *>(c.fmm64), nq, FmmFields{}));
     return FG_OK;
 }
 
@@ -2659,6 +2691,7 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
     if (!t) return 0;
     int n = 2;  // P2M, L2P + P2P (both sets in one launch each)
     if ((c.opts.fmm_overlap != 0 && c.stream2) || t->oz) n += 1;  // L2P apart from the near field
+    if (t->near.B) n += 1;  // the fields as pairs
     if (t->oz) {  // digits of the leaves, then per translation the products and the sums
         n += 1;
         for (int l = 2; l <= t->L - 1; l++) n += (t->oz_m2m[l].nunit > 0) + (t->oz_m2m[l].ntile > 0);

@@ -351,6 +351,24 @@ cudaError_t launch_charges_pair(Ctx &c, const double *m, const double *v);  // s
 // direct sum as a matrix over the nodes (fg_dense.cu)
 cudaError_t dense_build(Ctx &c, const Rules &R);  // direct_mat stays null where it does not fit
 cudaError_t launch_dense(Ctx &c, const double *m0, const double *m1, double *phi0, double *phi1);
+// near field of the FP64 FMM as dense blocks over the nodes (fg_dense.cu)
+struct NearMat {
+    int *cptr = nullptr, *col = nullptr;  // columns (node ids, ascending, -1 padding) of each leaf
+    size_t *boff = nullptr;               // first entry of each leaf's block
+    float2 *B = nullptr;                  // [target][3 columns] double-single; null: no blocks
+    int4 *task = nullptr;                 // leaf, first target, targets (at most 16)
+    float4 *field = nullptr;              // the fields as pairs, 3 per node
+    int ntask = 0;
+};
+struct NearTree {
+    int nleaf;
+    const int *leaf_src, *leaf_tgt, *tgt_node, *near_ptr, *near_leaf;  // device tables
+    const int *src_orig, *h_leaf_tgt;                                  // host: source of each position
+};
+cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N);
+void near_free(NearMat &N);
+cudaError_t launch_near(Ctx &c, const NearTree &t, const NearMat &N, cudaStream_t st, const double *m0, const double *m1,
+                        double *pot0, double *pot1);
 int direct_splits(const Ctx &c);                 // shares of the sources of the direct sum
 cudaError_t launch_p2p_direct(Ctx &c, int nq);  // sets 0 .. nq - 1 into direct_part
 // phi = base + (pot + corr) / (4 pi) of set 0 and, phi1 not null, of set 1 (base null: no base)
@@ -378,7 +396,14 @@ cudaError_t launch_mbar_timeout_probe(cudaStream_t st, int *err);
 cudaError_t launch_peak_mma_tf32(cudaStream_t st, int grid, int n, int iters, long long *cyc, int *err);
 int fmm_info(const Ctx &c, int *L, int *nleaf, double *n_m2l, double *n_p2p);
 int *fmm_error_flag(const Ctx &c);
-cudaError_t fmm_eval(Ctx &c, int nq = 1);  // nq 2: c.src_q2 -> c.pot2 beside c.src_q -> c.pot
+// The fields of an evaluation and where their finished potentials go: with fmm_whole() the FMM
+// forms its near field from m and writes phi itself, else it leaves the sums in c.pot, c.pot2.
+struct FmmFields {
+    const double *m[2];
+    double *phi[2];
+};
+bool fmm_whole(const Ctx &c);
+cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f);  // nq 2: c.src_q2 -> c.pot2 beside c.src_q -> c.pot
 // The same evaluation with an FP64 tree of the FP32 tree's depth (built on first use; the
 // FP32 tree itself when the context is FP64); FG_* status
 int fmm_eval_fp64(Ctx &c, int nq);
