@@ -85,7 +85,7 @@ struct FmmTree {
     // in phiv two steps later (film), so runs repeat bit for bit only with the same last bits
     bool repeat = false;
     NearMat near;              // oz: the near field as dense blocks, where they fit
-    int4 *p2p_task = nullptr;  // leaf, first target, targets (at most 8) of a near-field block
+    int4 *p2p_task = nullptr;  // leaf, first target, targets of a near-field task
     int n_p2p_task = 0;
     float4 *ds_src_hi = nullptr, *ds_src_lo = nullptr, *ds_tgt_hi = nullptr, *ds_tgt_lo = nullptr;
     int *leaf_ijk = nullptr;  // 3 x nleaf integer leaf coordinates (within the leaf's own tree)
@@ -1188,15 +1188,42 @@ __device__ __forceinline__ void l2p_p2p_pass_x2(int leaf, int tb, int nt, int la
     }
 }
 
-// L2P + P2P: one warp per target leaf, its targets in passes of 16 and a tail pass of 8
-// or 4 (a leaf of the film holds 18 to 64 nodes: fixed passes of 16 would spend about a
-// fifth of the pair work on padding).
-template <typename T, int NQ>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 2)  // FP32: 128 registers, 4 blocks per SM
-    k_l2p_p2p(int nleaf, const int *__restrict__ leaf_src, const int *__restrict__ leaf_tgt,
-              const int *__restrict__ tgt_node, const T *__restrict__ tloc, const T *__restrict__ sloc,
+// L2P + P2P of the FP32 path: one warp per task, up to 16 targets of a leaf (the leaf's targets
+// shared out in pairs as evenly as they go, the pass instantiated for every number of pairs, so
+// at most one target of a leaf is padding). Sources, lanes and sums are those of a warp that walks
+// the whole leaf: the potentials do not depend on the tasks. Bound by the FP32 and SFU pipes, each
+// at 16 pairs per clock and SM.
+constexpr int P2P32_NT = 16;
+template <int NQ>
+__global__ void __launch_bounds__(128, 4)  // 128 registers, 4 blocks per SM
+    k_l2p_p2p(int ntask, const int4 *__restrict__ task, const int *__restrict__ leaf_src,
+              const int *__restrict__ tgt_node, const float *__restrict__ tloc, const float *__restrict__ sloc,
               const int *__restrict__ leaf_ijk, int leaf0, const double *__restrict__ leaf_scale,
-              const int *__restrict__ near_ptr, const int *__restrict__ near_leaf, NearSets<T> sets) {
+              const int *__restrict__ near_ptr, const int *__restrict__ near_leaf, NearSets<float> sets) {
+    const int lane = threadIdx.x & 31, k = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (k >= ntask) return;
+    const int4 t = task[k];  // leaf, first target, targets
+    const int leaf = t.x, li = leaf_ijk[3 * leaf], lj = leaf_ijk[3 * leaf + 1], lk = leaf_ijk[3 * leaf + 2];
+    const size_t fbase = (size_t)(leaf0 + leaf) * NR;
+#define FG_PASS(N)                                                                                                  \
+    case N:                                                                                                         \
+        l2p_p2p_pass_x2<2 * N, NQ>(leaf, t.y, t.z, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,      \
+                                   leaf_scale, near_ptr, near_leaf, fbase, sets);                                   \
+        break;
+    switch ((t.z + 1) / 2) {
+        FG_PASS(1) FG_PASS(2) FG_PASS(3) FG_PASS(4) FG_PASS(5) FG_PASS(6) FG_PASS(7) FG_PASS(8)
+    }
+#undef FG_PASS
+}
+
+// L2P + P2P on the FP64 pipe (fmm_native_fp64): one warp per target leaf, its targets in passes of 16
+// and a tail pass of 8 or 4.
+template <int NQ>
+__global__ void __launch_bounds__(128, 2)
+    k_l2p_p2p_fp64(int nleaf, const int *__restrict__ leaf_src, const int *__restrict__ leaf_tgt,
+                   const int *__restrict__ tgt_node, const double *__restrict__ tloc, const double *__restrict__ sloc,
+                   const int *__restrict__ leaf_ijk, int leaf0, const double *__restrict__ leaf_scale,
+                   const int *__restrict__ near_ptr, const int *__restrict__ near_leaf, NearSets<double> sets) {
     const int lane = threadIdx.x & 31;
     const int leaf = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (leaf >= nleaf) return;
@@ -1207,27 +1234,15 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? 4 : 2)  // FP32: 128 reg
     for (int tb = t0; tb < t1;) {
         const int r = t1 - tb;
         const int nt = r > 8 ? 16 : r > 4 ? 8 : 4;
-        if constexpr (sizeof(T) == 4) {
-            if (nt == 16)
-                l2p_p2p_pass_x2<16, NQ>(leaf, tb, min(16, r), lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc,
-                                        leaf_ijk, leaf_scale, near_ptr, near_leaf, fbase, sets);
-            else if (nt == 8)
-                l2p_p2p_pass_x2<8, NQ>(leaf, tb, r, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,
-                                       leaf_scale, near_ptr, near_leaf, fbase, sets);
-            else
-                l2p_p2p_pass_x2<4, NQ>(leaf, tb, r, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,
-                                       leaf_scale, near_ptr, near_leaf, fbase, sets);
-        } else {
-            if (nt == 16)
-                l2p_p2p_pass<T, 16, NQ>(leaf, tb, min(16, r), lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc,
-                                        leaf_ijk, leaf_scale, near_ptr, near_leaf, fbase, sets);
-            else if (nt == 8)
-                l2p_p2p_pass<T, 8, NQ>(leaf, tb, r, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,
-                                       leaf_scale, near_ptr, near_leaf, fbase, sets);
-            else
-                l2p_p2p_pass<T, 4, NQ>(leaf, tb, r, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,
-                                       leaf_scale, near_ptr, near_leaf, fbase, sets);
-        }
+        if (nt == 16)
+            l2p_p2p_pass<double, 16, NQ>(leaf, tb, min(16, r), lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc,
+                                         leaf_ijk, leaf_scale, near_ptr, near_leaf, fbase, sets);
+        else if (nt == 8)
+            l2p_p2p_pass<double, 8, NQ>(leaf, tb, r, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,
+                                        leaf_scale, near_ptr, near_leaf, fbase, sets);
+        else
+            l2p_p2p_pass<double, 4, NQ>(leaf, tb, r, lane, li, lj, lk, leaf_src, tgt_node, tloc, sloc, leaf_ijk,
+                                        leaf_scale, near_ptr, near_leaf, fbase, sets);
         tb += nt;
     }
 }
@@ -2290,6 +2305,35 @@ static int fmm_build_forest(Ctx &c, int L) {
     FCK(up(&t->near_leaf, near_leaf));
     if (!t->ds) FCK(up_as<double>(&t->sloc, sloc, fp32));
     FCK(up_as<double>(&t->tloc, tloc, fp32));
+    // near-field tasks of at most `most` targets: each leaf's targets shared out evenly, in multiples
+    // of `step`. Where the sources (src_bytes each) fit in L2 the expensive tasks go first, which
+    // evens out the last wave; else the leaf order keeps neighbouring tasks on the same sources
+    auto near_tasks = [&](int most, int step, int src_bytes) -> cudaError_t {
+        std::vector<int4> task;
+        std::vector<long> cost;
+        for (int l = 0; l < nleaf; l++) {
+            const int n = leaf_tgt[l + 1] - leaf_tgt[l], groups = (n + most - 1) / most, units = (n + step - 1) / step;
+            long src = 0;
+            for (int e = near_ptr[l]; e < near_ptr[l + 1]; e++) src += leaf_src[near_leaf[e] + 1] - leaf_src[near_leaf[e]];
+            for (int g = 0; g < groups; g++) {
+                const int b = step * (int)((long)units * g / groups);
+                const int e = std::min(n, step * (int)((long)units * (g + 1) / groups));
+                task.push_back(make_int4(l, leaf_tgt[l] + b, e - b, 0));
+                cost.push_back(src * (e - b));
+            }
+        }
+        if ((size_t)c.nsrc * src_bytes < ((size_t)64 << 20)) {
+            std::vector<int> order(task.size());
+            for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
+            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+            std::vector<int4> sorted;
+            for (int k : order) sorted.push_back(task[k]);
+            task.swap(sorted);
+        }
+        t->n_p2p_task = (int)task.size();
+        return up(&t->p2p_task, task);
+    };
+    if (fp32) FCK(near_tasks(P2P32_NT, 2, 20));
     if (t->ds) {
         // x = hi + lo, hi on the 2^-20 grid (|x| < 4 leaf units: exact in FP32)
         auto split = [](const std::vector<double> &v, std::vector<float4> &hi, std::vector<float4> &lo) {
@@ -2311,30 +2355,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         std::vector<float4> sh, sl, th, tl;
         split(sloc, sh, sl);
         split(tloc, th, tl);
-        std::vector<int4> task;
-        std::vector<long> cost;
-        for (int l = 0; l < nleaf; l++) {
-            const int n = leaf_tgt[l + 1] - leaf_tgt[l], groups = (n + P2P_NT - 1) / P2P_NT;
-            long src = 0;
-            for (int e = near_ptr[l]; e < near_ptr[l + 1]; e++) src += leaf_src[near_leaf[e] + 1] - leaf_src[near_leaf[e]];
-            for (int g = 0; g < groups; g++) {
-                const int b = (int)((long)n * g / groups), e = (int)((long)n * (g + 1) / groups);
-                task.push_back(make_int4(l, leaf_tgt[l] + b, e - b, 0));
-                cost.push_back(src * (e - b));
-            }
-        }
-        // where the sources fit in L2 the expensive blocks go first, which evens out the last wave;
-        // else the leaf order keeps neighbouring blocks on the same sources
-        if ((size_t)c.nsrc * 40 < ((size_t)64 << 20)) {
-            std::vector<int> order(task.size());
-            for (size_t k = 0; k < order.size(); k++) order[k] = (int)k;
-            std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
-            std::vector<int4> sorted;
-            for (int k : order) sorted.push_back(task[k]);
-            task.swap(sorted);
-        }
-        t->n_p2p_task = (int)task.size();
-        FCK(up(&t->p2p_task, task));
+        FCK(near_tasks(P2P_NT, 1, 40));
         if (t->oz) {
             std::vector<int> orig(c.nsrc);
             for (int k = 0; k < c.nsrc; k++) orig[src_dst[k]] = k;
@@ -2504,10 +2525,15 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
                     t.p2p_task, t.leaf_src, t.tgt_node, t.ds_tgt_hi, t.ds_tgt_lo, t.ds_src_hi, t.ds_src_lo, t.ds_q2,
                     t.ds_q2 ? t.ds_q2 + t.nsrc : nullptr, t.leaf_ijk, t.near_ptr, t.near_leaf, ns.pot[0], ns.pot[1]);
         }
-        if (!t.ds) {
-            auto k = nq == 2 ? k_l2p_p2p<T, 2> : k_l2p_p2p<T, 1>;
-            k<<<nb, 128, 0, st>>>(t.nleaf, t.leaf_src, t.leaf_tgt, t.tgt_node, (const T *)t.tloc, (const T *)t.sloc,
-                                  t.leaf_ijk, t.leaf0, t.leaf_scale, t.near_ptr, t.near_leaf, ns);
+        if constexpr (sizeof(T) == 4) {
+            if (t.n_p2p_task > 0)
+                (nq == 2 ? k_l2p_p2p<2> : k_l2p_p2p<1>)<<<(t.n_p2p_task + 3) / 4, 128, 0, st>>>(
+                    t.n_p2p_task, t.p2p_task, t.leaf_src, t.tgt_node, (const float *)t.tloc, (const float *)t.sloc,
+                    t.leaf_ijk, t.leaf0, t.leaf_scale, t.near_ptr, t.near_leaf, ns);
+        } else if (!t.ds) {
+            (nq == 2 ? k_l2p_p2p_fp64<2> : k_l2p_p2p_fp64<1>)<<<nb, 128, 0, st>>>(
+                t.nleaf, t.leaf_src, t.leaf_tgt, t.tgt_node, (const double *)t.tloc, (const double *)t.sloc, t.leaf_ijk,
+                t.leaf0, t.leaf_scale, t.near_ptr, t.near_leaf, ns);
         }
     };
     t.ev_split[t.ev_next] = split && prof;
