@@ -896,10 +896,10 @@ static int demag_into(fg_ctx *h, const double *m, double *phi_out) {
         c.launches += 1 + (c.dense_nshare > 1);
         return FG_OK;
     }
-    CK(launch_charges(c, m));
+    if (c.opts.demag != FG_DEMAG_FMM || fmm_charges(c)) CK(launch_charges(c, m));
     if (c.opts.demag == FG_DEMAG_FMM) {
         CK(fmm_eval(c, 1, {{m, nullptr}, {phi_out, nullptr}}));
-        c.launches += 1 + fmm_launches_per_eval(c);
+        c.launches += fmm_charges(c) + fmm_launches_per_eval(c);
         if (fmm_whole(c)) return FG_OK;
     } else {
         CK(launch_p2p_direct(c, 1));
@@ -935,10 +935,10 @@ static int demag_pair(fg_ctx *h) {
         c.launches += 1 + (c.dense_nshare > 1);
         return FG_OK;
     }
-    CK(launch_charges_pair(c, c.u[1], c.v[1]));
+    if (c.opts.demag != FG_DEMAG_FMM || fmm_charges(c)) CK(launch_charges_pair(c, c.u[1], c.v[1]));
     if (c.opts.demag == FG_DEMAG_FMM) {
         CK(fmm_eval(c, 2, {{c.u[1], c.v[1]}, {c.phi[1], c.phiv[1]}}));
-        c.launches += 1 + fmm_launches_per_eval(c, 2);
+        c.launches += fmm_charges(c) + fmm_launches_per_eval(c, 2);
         if (fmm_whole(c)) return FG_OK;
     } else {
         CK(launch_p2p_direct(c, 2));

@@ -227,7 +227,8 @@ static cudaError_t batch_solve(Ctx &c) {
 // Demag of m (and of v beside it, one FMM evaluation of both charge sets).
 static cudaError_t batch_demag_all(Ctx &c) {
     const int nq = c.opts.first_order ? 1 : 2;
-    cudaError_t e = nq == 2 ? launch_charges_pair(c, c.u[1], c.v[1]) : launch_charges(c, c.u[1], 0);
+    cudaError_t e = cudaSuccess;
+    if (fmm_charges(c)) e = nq == 2 ? launch_charges_pair(c, c.u[1], c.v[1]) : launch_charges(c, c.u[1], 0);
     if (e == cudaSuccess) e = fmm_eval(c, nq, {{c.u[1], c.v[1]}, {c.phi[1], c.phiv[1]}});
     if (e == cudaSuccess && !fmm_whole(c)) e = launch_phi_final(c, c.phi[1], nq == 2 ? c.phiv[1] : nullptr);
     return e;
@@ -235,7 +236,7 @@ static cudaError_t batch_demag_all(Ctx &c) {
 
 static int demag_launches(const Ctx &c) {
     const int nq = c.opts.first_order ? 1 : 2;
-    return 1 + !fmm_whole(c) + fmm_launches_per_eval(c, nq);
+    return fmm_charges(c) + !fmm_whole(c) + fmm_launches_per_eval(c, nq);
 }
 
 // Whether a step uses the learned guess (after its training solves; the network of a batch is

@@ -225,7 +225,9 @@ namespace {
 constexpr int HASH = 8192;      // slots of a leaf's tables in shared memory
 constexpr int MAX_NODE = 4096;  // column nodes and elements a leaf may have
 constexpr int MAX_ELEM = 6144;
+constexpr int MAX_OWN = 1024;   // elements with a Gauss point in one leaf (P2M)
 constexpr int TG = 8;           // targets formed together
+constexpr int NRM = 100;        // reals per expansion
 
 __device__ __forceinline__ int hash_of(int key) { return (int)(((unsigned)key * 2654435761u) >> 19); }
 
@@ -249,18 +251,20 @@ __device__ __forceinline__ int hash_find(const int *tab, int key) {
 }
 
 struct NearArgs {
+    int own;  // 1: the sources of the leaf itself only (P2M), 0: those of its adjacent leaves
     int nleaf, nmt, npi_t, npi_f;
     const int *leaf_src, *leaf_tgt, *tgt_node, *near_ptr, *near_leaf, *src_orig;
     const int4 *tet, *tri;
     const int *tinc_ptr, *tinc;
 };
 
-// f(element, Gauss point) for every source of the leaf's adjacent leaves; elements are the
-// magnetic tetrahedra, then the triangles. Every thread of the block takes part.
+// f(element, Gauss point) for every source of the leaf's adjacent leaves (or its own); elements are
+// the magnetic tetrahedra, then the triangles. Every thread of the block takes part.
 template <typename Fn>
 __device__ __forceinline__ void near_sources(const NearArgs &a, int leaf, Fn &&f) {
-    for (int e = a.near_ptr[leaf]; e < a.near_ptr[leaf + 1]; e++) {
-        const int nl = a.near_leaf[e];
+    const int e0 = a.own ? 0 : a.near_ptr[leaf], e1 = a.own ? 1 : a.near_ptr[leaf + 1];
+    for (int e = e0; e < e1; e++) {
+        const int nl = a.own ? leaf : a.near_leaf[e];
         for (int s = a.leaf_src[nl] + threadIdx.x; s < a.leaf_src[nl + 1]; s += blockDim.x) {
             const int o = a.src_orig[s], nt = a.nmt * a.npi_t;
             if (o < nt) f(o / a.npi_t, o % a.npi_t);
@@ -296,7 +300,7 @@ __device__ __forceinline__ void near_tables(const NearArgs &a, int leaf, int *no
         }
     }
     // the self-corrections reach the nodes of every triangle of a target
-    for (int t = a.leaf_tgt[leaf] + threadIdx.x; t < a.leaf_tgt[leaf + 1]; t += blockDim.x) {
+    for (int t = a.leaf_tgt[leaf] + threadIdx.x; !a.own && t < a.leaf_tgt[leaf + 1]; t += blockDim.x) {
         const int i = a.tgt_node[t];
         for (int k = a.tinc_ptr[i]; k < a.tinc_ptr[i + 1]; k++) add_tri(a.tinc[k] / 3);
     }
@@ -307,14 +311,15 @@ __global__ void __launch_bounds__(256) k_near_count(NearArgs a, int *ncol, int *
     extern __shared__ int tab[];
     __shared__ int nn, ne;
     const int leaf = blockIdx.x;
-    if (a.leaf_tgt[leaf] == a.leaf_tgt[leaf + 1]) {
+    const int *range = a.own ? a.leaf_src : a.leaf_tgt;
+    if (range[leaf] == range[leaf + 1]) {
         if (threadIdx.x == 0) ncol[leaf] = 0;
         return;
     }
     near_tables(a, leaf, tab, tab + HASH, &nn, &ne);
     if (threadIdx.x == 0) {
         ncol[leaf] = nn;
-        if (nn > MAX_NODE || ne > MAX_ELEM) *over = 1;
+        if (nn > MAX_NODE || ne > (a.own ? MAX_OWN : MAX_ELEM)) *over = 1;
     }
 }
 
@@ -466,6 +471,140 @@ __global__ void __launch_bounds__(256) k_near_fill(NearArgs a, Rules R, const in
     }
 }
 
+// The multipoles of a leaf as a block [100][3 columns] over the nodes of its own sources' elements:
+// W[slot][k] = sum over the element's Gauss points in the leaf of w_g conj(Ups_k)(y_g) (a triangle
+// counts as three elements, one per shape function), then a warp per column node gathers its
+// elements, lanes = coefficients. One thread forms one harmonic column of one element.
+constexpr int OWN_HASH = 4096;
+__global__ void __launch_bounds__(256) k_p2m_fill(NearArgs a, Rules R, const int *__restrict__ cptr,
+                                                  const int *__restrict__ col, const size_t *__restrict__ boff,
+                                                  const int *__restrict__ src_pos, const double4 *__restrict__ sloc,
+                                                  const double *__restrict__ da, const double *__restrict__ detJ,
+                                                  const int *__restrict__ treg, const DevRegion *__restrict__ regs,
+                                                  const int *__restrict__ inc_ptr, const int *__restrict__ inc,
+                                                  const DevTri *__restrict__ tc, double *__restrict__ scratch,
+                                                  float2 *__restrict__ B) {
+    constexpr int P = 9;
+    extern __shared__ int tab[];
+    int *mask = tab + HASH, *list = mask + HASH;  // the table, its masks, the occupied slots
+    __shared__ int ne, nl;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double *W = scratch + (size_t)blockIdx.x * OWN_HASH * NRM;
+    for (int leaf = blockIdx.x; leaf < a.nleaf; leaf += gridDim.x) {
+        const int c0 = cptr[leaf], nc = cptr[leaf + 1] - c0;
+        if (nc == 0) continue;
+        __syncthreads();
+        for (int k = threadIdx.x; k < HASH; k += 256) {
+            tab[k] = -1;
+            mask[k] = 0;
+        }
+        if (threadIdx.x == 0) ne = nl = 0;
+        __syncthreads();
+        near_sources(a, leaf, [&](int el, int g) {
+            const bool tet = el < a.nmt;
+            for (int k = 0; k < (tet ? 1 : 3); k++) {
+                const int h = hash_add(tab, tet ? el : a.nmt + 3 * (el - a.nmt) + k, &ne, 3 * MAX_OWN);
+                if (h >= 0) atomicOr(&mask[h], 1 << g);
+            }
+        });
+        __syncthreads();
+        for (int k = threadIdx.x; k < HASH; k += 256)
+            if (tab[k] >= 0) {
+                const int n = atomicAdd(&nl, 1);
+                list[n] = k;
+                mask[k] |= n << 8;  // row of W
+            }
+        __syncthreads();
+        for (int q = threadIdx.x; q < nl * (P + 1); q += 256) {
+            const int k = list[q / (P + 1)], m = q % (P + 1), el = tab[k], mk = mask[k] & 255;
+            const bool tet = el < a.nmt;
+            const int f = (el - a.nmt) / 3, v = (el - a.nmt) % 3, np = tet ? R.npi_t : R.npi_f;
+            double re[P + 1], im[P + 1];
+#pragma unroll
+            for (int n = 0; n <= P; n++) re[n] = im[n] = 0.0;
+            for (int g = 0; g < np; g++) {
+                if (!(mk >> g & 1)) continue;
+                const size_t o = tet ? (size_t)el * R.npi_t + g : (size_t)a.nmt * R.npi_t + (size_t)f * R.npi_f + g;
+                const double4 y = sloc[src_pos[o]];
+                const double w = tet ? R.tp[g] : tc[f].w[g] * R.fa[v][g];
+                double dr = w, di = 0.0;  // the column's diagonal, times the weight
+                for (int i = 1; i <= m; i++) {
+                    const double t = (y.x * dr - y.y * di) / (2 * i);
+                    di = (y.x * di + y.y * dr) / (2 * i);
+                    dr = t;
+                }
+                const double r2 = y.x * y.x + y.y * y.y + y.z * y.z;
+                double p2r = 0.0, p2i = 0.0, p1r = dr, p1i = di;
+#pragma unroll
+                for (int n = 0; n <= P; n++) {  // degree n >= m
+                    if (n < m) continue;
+                    re[n] += p1r;
+                    im[n] += p1i;
+                    const int d = n + 1;
+                    const double b = d == m + 1 ? 1.0 : 1.0 / double((d + m) * (d - m));
+                    const double az = (d == m + 1 ? 1.0 : 2 * d - 1) * y.z;
+                    const double nr = (az * p1r - r2 * p2r) * b, ni = (az * p1i - r2 * p2i) * b;
+                    p2r = p1r; p2i = p1i;
+                    p1r = nr; p1i = ni;
+                }
+            }
+            double *w = W + (size_t)(mask[k] >> 8) * NRM;
+#pragma unroll
+            for (int n = 0; n <= P; n++) {
+                if (n < m) continue;
+                if (m == 0) w[n * n] = re[n];
+                else {
+                    w[n * n + 2 * m - 1] = re[n];
+                    w[n * n + 2 * m] = -im[n];
+                }
+            }
+        }
+        __syncthreads();
+        for (int j = warp; j < nc; j += 8) {
+            const int node = col[c0 + j];
+            double b[4][3];
+#pragma unroll
+            for (int i = 0; i < 4; i++) b[i][0] = b[i][1] = b[i][2] = 0.0;
+            auto gather = [&](int key, double kx, double ky, double kz) {
+                const int h = hash_find(tab, key);
+                if (h < 0) return;
+                const double *w = W + (size_t)(mask[h] >> 8) * NRM;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const int k = lane + 32 * i;
+                    const double x = k < NRM ? w[k] : 0.0;
+                    b[i][0] += kx * x;
+                    b[i][1] += ky * x;
+                    b[i][2] += kz * x;
+                }
+            };
+            if (node >= 0) {
+                for (int q = inc_ptr[node]; q < inc_ptr[node + 1]; q++) {
+                    const int el = inc[q] >> 2, v = inc[q] & 3;
+                    const double w = -regs[treg[el]].Ms * detJ[el];
+                    gather(el, w * da[(3 * v) * (size_t)a.nmt + el], w * da[(3 * v + 1) * (size_t)a.nmt + el],
+                           w * da[(3 * v + 2) * (size_t)a.nmt + el]);
+                }
+                for (int q = a.tinc_ptr[node]; q < a.tinc_ptr[node + 1]; q++) {
+                    const DevTri &T = tc[a.tinc[q] / 3];
+                    gather(a.nmt + a.tinc[q], T.dMs * T.n[0], T.dMs * T.n[1], T.dMs * T.n[2]);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int k = lane + 32 * i;
+                if (k >= NRM) continue;
+                float2 *o = B + boff[leaf] + (size_t)k * 3 * nc + 3 * j;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const float h = (float)b[i][c];
+                    o[c] = make_float2(h, (float)(b[i][c] - (double)h));
+                }
+            }
+        }
+    }
+}
+
 // The fields as double-single pairs: (u hi, u lo, v hi, v lo) per component.
 __global__ void k_field_pairs(size_t n3, const double *__restrict__ u, const double *__restrict__ v,
                               float4 *__restrict__ m) {
@@ -476,28 +615,22 @@ __global__ void k_field_pairs(size_t n3, const double *__restrict__ u, const dou
     m[k] = make_float4(xh, (float)(x - (double)xh), yh, (float)(y - (double)yh));
 }
 
-// Near potentials of NQ fields: a block per task (up to 16 targets of a leaf, two per warp), the
-// column nodes' fields staged in shared memory in tiles of NEAR_TILE entries, two entries of a
-// row per 16-byte load. 12 FP32 operations per entry and field (product with its rounding error
-// and cross terms, two-sum), 8 bytes of the block: HBM bounds it.
-constexpr int NEAR_TILE = 1536;
+// Rows of the blocks times NQ fields: a block per task (some rows of a leaf), two rows per warp at a
+// time, the column nodes' fields staged in shared memory in tiles of TILE entries (once where one
+// tile holds them), two entries of a row per 16-byte load. 12 FP32 operations per entry and field
+// (product with its rounding error and cross terms, two-sum), 8 bytes of the block: HBM bounds
+// it. Row r goes to out[rows ? rows[first + r] : first + r].
+constexpr int TILE = 1536;
 template <int NQ>
-__global__ void __launch_bounds__(256) k_near_mv(const int4 *__restrict__ task, const int *__restrict__ leaf_tgt,
-                                                 const int *__restrict__ tgt_node, const int *__restrict__ cptr,
-                                                 const int *__restrict__ col, const size_t *__restrict__ boff,
-                                                 const float2 *__restrict__ B, const float4 *__restrict__ m,
-                                                 double *__restrict__ pot0, double *__restrict__ pot1) {
-    __shared__ float4 sm[NEAR_TILE];
+__global__ void __launch_bounds__(256) k_block_mv(const int4 *__restrict__ task, const int *__restrict__ rows,
+                                                  const int *__restrict__ cptr, const int *__restrict__ col,
+                                                  const size_t *__restrict__ boff, const float2 *__restrict__ B,
+                                                  const float4 *__restrict__ m, double *__restrict__ out0,
+                                                  double *__restrict__ out1) {
+    __shared__ float4 sm[TILE];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int4 t = task[blockIdx.x];  // leaf, first target, targets
+    const int4 t = task[blockIdx.x];  // leaf, first row of its block, rows, first output
     const int c0 = cptr[t.x], ne = 3 * (cptr[t.x + 1] - c0);
-    const int r0 = 2 * warp, row = t.y - leaf_tgt[t.x];
-    const bool on0 = r0 < t.z, on1 = r0 + 1 < t.z;
-    const float2 *b0 = B + boff[t.x] + (size_t)(row + (on0 ? r0 : 0)) * ne;
-    const float2 *b1 = on1 ? b0 + ne : b0;
-    float h[2][NQ], l[2][NQ];
-#pragma unroll
-    for (int q = 0; q < NQ; q++) h[0][q] = h[1][q] = l[0][q] = l[1][q] = 0.f;
     auto add = [&](float &hi, float &lo, float bh, float bl, float mh, float ml) {
         const float p = bh * mh;
         const float e = fmaf(bl, mh, fmaf(bh, ml, fmaf(bh, mh, -p)));
@@ -505,78 +638,146 @@ __global__ void __launch_bounds__(256) k_near_mv(const int4 *__restrict__ task, 
         lo += ((hi - (s - x)) + (p - x)) + e;
         hi = s;
     };
-    for (int base = 0; base < ne; base += NEAR_TILE) {
-        const int len = min(NEAR_TILE, ne - base);
-        __syncthreads();
-        for (int e = threadIdx.x; e < len; e += 256) {
-            const int node = col[c0 + (base + e) / 3];
-            sm[e] = node >= 0 ? m[3 * (size_t)node + (base + e) % 3] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        __syncthreads();
-        if (!on0) continue;
-        const float4 *p0 = reinterpret_cast<const float4 *>(b0 + base), *p1 = reinterpret_cast<const float4 *>(b1 + base);
+    for (int r0 = 0; r0 < t.z; r0 += 16) {
+        const int r = r0 + 2 * warp;
+        const bool on0 = r < t.z, on1 = r + 1 < t.z;
+        const float2 *b0 = B + boff[t.x] + (size_t)(t.y + (on0 ? r : 0)) * ne;
+        const float2 *b1 = on1 ? b0 + ne : b0;
+        float h[2][NQ], l[2][NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; q++) h[0][q] = h[1][q] = l[0][q] = l[1][q] = 0.f;
+        for (int base = 0; base < ne; base += TILE) {
+            const int len = min(TILE, ne - base);
+            if (r0 == 0 || ne > TILE) {
+                __syncthreads();
+                for (int e = threadIdx.x; e < len; e += 256) {
+                    const int node = col[c0 + (base + e) / 3];
+                    sm[e] = node >= 0 ? m[3 * (size_t)node + (base + e) % 3] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                __syncthreads();
+            }
+            if (!on0) continue;
+            const float4 *p0 = reinterpret_cast<const float4 *>(b0 + base), *p1 = reinterpret_cast<const float4 *>(b1 + base);
 #pragma unroll 2
-        for (int e = lane; e < len / 2; e += 32) {
-            const float4 x0 = __ldcs(p0 + e), x1 = __ldcs(p1 + e), ma = sm[2 * e], mb = sm[2 * e + 1];
-            add(h[0][0], l[0][0], x0.x, x0.y, ma.x, ma.y);
-            add(h[1][0], l[1][0], x1.x, x1.y, ma.x, ma.y);
-            add(h[0][0], l[0][0], x0.z, x0.w, mb.x, mb.y);
-            add(h[1][0], l[1][0], x1.z, x1.w, mb.x, mb.y);
-            if constexpr (NQ == 2) {
-                add(h[0][1], l[0][1], x0.x, x0.y, ma.z, ma.w);
-                add(h[1][1], l[1][1], x1.x, x1.y, ma.z, ma.w);
-                add(h[0][1], l[0][1], x0.z, x0.w, mb.z, mb.w);
-                add(h[1][1], l[1][1], x1.z, x1.w, mb.z, mb.w);
+            for (int e = lane; e < len / 2; e += 32) {
+                const float4 x0 = __ldcs(p0 + e), x1 = __ldcs(p1 + e), ma = sm[2 * e], mb = sm[2 * e + 1];
+                add(h[0][0], l[0][0], x0.x, x0.y, ma.x, ma.y);
+                add(h[1][0], l[1][0], x1.x, x1.y, ma.x, ma.y);
+                add(h[0][0], l[0][0], x0.z, x0.w, mb.x, mb.y);
+                add(h[1][0], l[1][0], x1.z, x1.w, mb.x, mb.y);
+                if constexpr (NQ == 2) {
+                    add(h[0][1], l[0][1], x0.x, x0.y, ma.z, ma.w);
+                    add(h[1][1], l[1][1], x1.x, x1.y, ma.z, ma.w);
+                    add(h[0][1], l[0][1], x0.z, x0.w, mb.z, mb.w);
+                    add(h[1][1], l[1][1], x1.z, x1.w, mb.z, mb.w);
+                }
             }
         }
+        if (!on0) continue;
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+            for (int q = 0; q < NQ; q++) {
+                dsf s = ds_quick(h[i][q], l[i][q]);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    s = ds_add(s, dsf{__shfl_xor_sync(0xffffffffu, s.h, o), __shfl_xor_sync(0xffffffffu, s.l, o)});
+                if (lane == 0 && (i == 0 || on1)) {
+                    const size_t k = (size_t)t.w + r + i;
+                    (q ? out1 : out0)[rows ? rows[k] : k] = ds_to(s);
+                }
+            }
     }
-    if (!on0) return;
-#pragma unroll
-    for (int r = 0; r < 2; r++)
-#pragma unroll
-        for (int q = 0; q < NQ; q++) {
-            dsf s = ds_quick(h[r][q], l[r][q]);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-                s = ds_add(s, dsf{__shfl_xor_sync(0xffffffffu, s.h, o), __shfl_xor_sync(0xffffffffu, s.l, o)});
-            if (lane == 0 && (r == 0 || on1)) (q ? pot1 : pot0)[tgt_node[t.y + r0 + r]] = ds_to(s);
+}
+
+// Local expansions at the targets from a table of the harmonics: T[k][target] = Ups_k of the
+// target (doubled for m > 0), one thread per target, so the FP64 pipe does 100 operations per field
+// instead of forming the harmonics (film: L2P 0.37 ms). phi = sum_k F_k T_k scale / (4 pi) + near.
+__global__ void __launch_bounds__(128) k_l2p_table(int ntgt, const double4 *__restrict__ tloc, double *__restrict__ T) {
+    constexpr int P = 9;
+    const int t = blockIdx.x * 128 + threadIdx.x;
+    if (t >= ntgt) return;
+    const double4 y = tloc[t];
+    const double r2 = y.x * y.x + y.y * y.y + y.z * y.z;
+    double dr = 1.0, di = 0.0;
+    for (int m = 0; m <= P; m++) {
+        if (m) {
+            const double s = (y.x * dr - y.y * di) / (2 * m);
+            di = (y.x * di + y.y * dr) / (2 * m);
+            dr = s;
         }
+        double p2r = 0.0, p2i = 0.0, p1r = dr, p1i = di;
+        for (int n = m; n <= P; n++) {
+            if (m == 0) T[(size_t)(n * n) * ntgt + t] = p1r;
+            else {
+                T[(size_t)(n * n + 2 * m - 1) * ntgt + t] = 2.0 * p1r;
+                T[(size_t)(n * n + 2 * m) * ntgt + t] = 2.0 * p1i;
+            }
+            const int d = n + 1;
+            const double b = d == m + 1 ? 1.0 : 1.0 / double((d + m) * (d - m)), az = (d == m + 1 ? 1.0 : 2 * d - 1) * y.z;
+            const double nr = (az * p1r - r2 * p2r) * b, ni = (az * p1i - r2 * p2i) * b;
+            p2r = p1r; p2i = p1i;
+            p1r = nr; p1i = ni;
+        }
+    }
+}
+template <int NQ>
+__global__ void __launch_bounds__(128) k_l2p_apply(int ntgt, const int *__restrict__ tgt_leaf,
+                                                   const int *__restrict__ tgt_node, const double *__restrict__ T,
+                                                   const double *__restrict__ leaf_scale, const double *__restrict__ F0,
+                                                   const double *__restrict__ F1, const double *__restrict__ near0,
+                                                   const double *__restrict__ near1, double *__restrict__ phi0,
+                                                   double *__restrict__ phi1) {
+    const int t = blockIdx.x * 128 + threadIdx.x;
+    if (t >= ntgt) return;
+    const int leaf = tgt_leaf[t], node = tgt_node[t];
+    const double *a = F0 + (size_t)leaf * NRM, *b = NQ == 2 ? F1 + (size_t)leaf * NRM : nullptr;
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll 10
+    for (int k = 0; k < NRM; k++) {
+        const double x = __ldcs(T + (size_t)k * ntgt + t);
+        s0 = fma(a[k], x, s0);
+        if constexpr (NQ == 2) s1 = fma(b[k], x, s1);
+    }
+    const double f = leaf_scale[leaf] / (4 * M_PI);
+    phi0[node] = fma(s0, f, near0[node]);
+    if constexpr (NQ == 2) phi1[node] = fma(s1, f, near1[node]);
 }
 
 }  // namespace
 
-// Forms the blocks where they fit (1/8 of the device's memory, half of what is free; at most
-// MAX_NODE columns and MAX_ELEM elements per leaf); without them (N.B null) the pair sum runs.
-cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
+// Forms the blocks of one kind (own: P2M, else near field) where they fit: at most 1/8 of the
+// device's memory, half of what is free, MAX_NODE columns and MAX_ELEM (MAX_OWN) elements per leaf.
+// Without them (N.B null) the sums over Gauss points run.
+static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool own, DenseBlocks &N) {
     size_t free_b = 0, total_b = 0;
     cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
     if (e != cudaSuccess) return e;
-    NearArgs a{t.nleaf, c.nmt, R.npi_t, R.npi_f, t.leaf_src, t.leaf_tgt, t.tgt_node, t.near_ptr, t.near_leaf, nullptr,
+    NearArgs a{own, t.nleaf, c.nmt, R.npi_t, R.npi_f, t.leaf_src, t.leaf_tgt, t.tgt_node, t.near_ptr, t.near_leaf, t.src_orig,
                c.tet, c.tri, c.tinc_ptr, c.tinc};
-    int *orig = nullptr, *ncol = nullptr;
+    int *ncol = nullptr;
     double *scratch = nullptr;
-    const int smem = 2 * HASH * (int)sizeof(int), blocks = std::min(t.nleaf, 2 * std::max(1, c.nsm));
+    const int smem = 2 * HASH * (int)sizeof(int), smem_own = 3 * HASH * (int)sizeof(int);
+    const int blocks = std::min(t.nleaf, 2 * std::max(1, c.nsm));
     auto done = [&](cudaError_t r) {
-        for (void *p : {(void *)orig, (void *)ncol, (void *)scratch})
-            if (p) cudaFree(p);
-        if (r != cudaSuccess || !N.B) near_free(N);
+        if (ncol) cudaFree(ncol);
+        if (scratch) cudaFree(scratch);
+        if (r != cudaSuccess || !N.B) blocks_free(N);
         cudaGetLastError();
-        // what does not fit is no error: the pair sum needs none of it
+        // what does not fit is no error: the sums over Gauss points need none of it
         return r == cudaErrorMemoryAllocation ? cudaSuccess : r;
     };
-#define NCK(call)                              \
-    do {                                       \
-        const cudaError_t r_ = (call);         \
+#define NCK(call)                               \
+    do {                                        \
+        const cudaError_t r_ = (call);          \
         if (r_ != cudaSuccess) return done(r_); \
     } while (0)
     NCK(cudaFuncSetAttribute(k_near_count, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     NCK(cudaFuncSetAttribute(k_near_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     NCK(cudaFuncSetAttribute(k_near_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    NCK(cudaMalloc(&orig, sizeof(int) * std::max(1, c.nsrc)));
-    NCK(cudaMemcpyAsync(orig, t.src_orig, sizeof(int) * c.nsrc, cudaMemcpyHostToDevice, c.stream));
+    NCK(cudaFuncSetAttribute(k_p2m_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_own));
     NCK(cudaMalloc(&ncol, sizeof(int) * (t.nleaf + 1)));
     NCK(cudaMemsetAsync(ncol, 0, sizeof(int) * (t.nleaf + 1), c.stream));
-    a.src_orig = orig;
     k_near_count<<<t.nleaf, 256, smem, c.stream>>>(a, ncol, ncol + t.nleaf);
     std::vector<int> hn(t.nleaf + 1);
     NCK(cudaMemcpyAsync(hn.data(), ncol, sizeof(int) * (t.nleaf + 1), cudaMemcpyDeviceToHost, c.stream));
@@ -585,27 +786,30 @@ cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
     std::vector<int> cptr(t.nleaf + 1, 0);
     std::vector<size_t> boff(t.nleaf, 0);
     std::vector<int4> task;
-    size_t entries = 0;
+    size_t entries = 0, cols = 0;
     for (int l = 0; l < t.nleaf; l++) {
-        const int nc = (hn[l] + 1) & ~1, nt = t.h_leaf_tgt[l + 1] - t.h_leaf_tgt[l];
-        if ((size_t)cptr[l] + nc > 0x7fffffff) return done(cudaSuccess);
-        cptr[l + 1] = cptr[l] + nc;
+        const int nc = (hn[l] + 1) & ~1, nt = own ? NRM : t.h_leaf_tgt[l + 1] - t.h_leaf_tgt[l];
+        cols += nc;
+        if (cols > 0x7fffffff || (own && (size_t)t.nleaf * NRM > 0x7fffffff)) return done(cudaSuccess);
+        cptr[l + 1] = (int)cols;
         boff[l] = entries;
+        if (nc == 0 && !own) continue;
         entries += (size_t)nt * 3 * nc;
-        const int groups = (nt + 15) / 16;
+        // near field: up to 16 rows; P2M: all rows of a leaf (few columns), or 16 where a tile of
+        // columns does not hold them
+        const int most = own && 3 * nc <= TILE ? NRM : 16, groups = (nt + most - 1) / most;
         for (int g = 0; g < groups; g++) {
             const int b = (int)((long)nt * g / groups), f = (int)((long)nt * (g + 1) / groups);
-            task.push_back(make_int4(l, t.h_leaf_tgt[l] + b, f - b, 0));
+            task.push_back(make_int4(l, b, f - b, (own ? NRM * l : t.h_leaf_tgt[l]) + b));
         }
     }
     if (entries == 0 || entries * sizeof(float2) > std::min(total_b / 8, free_b / 2)) return done(cudaSuccess);
     N.ntask = (int)task.size();
-    NCK(cudaMalloc(&scratch, sizeof(double) * HASH * TG * (size_t)blocks));
+    NCK(cudaMalloc(&scratch, sizeof(double) * (own ? (size_t)OWN_HASH * NRM : (size_t)HASH * TG) * blocks));
     NCK(cudaMalloc(&N.cptr, sizeof(int) * (t.nleaf + 1)));
     NCK(cudaMalloc(&N.boff, sizeof(size_t) * t.nleaf));
     NCK(cudaMalloc(&N.task, sizeof(int4) * N.ntask));
-    NCK(cudaMalloc(&N.col, sizeof(int) * cptr[t.nleaf]));
-    NCK(cudaMalloc(&N.field, sizeof(float4) * 3 * (size_t)c.nn));
+    NCK(cudaMalloc(&N.col, sizeof(int) * cols));
     NCK(cudaMalloc(&N.B, sizeof(float2) * entries));
     auto filled = [&]() -> cudaError_t {
         cudaError_t r = cudaMemcpyAsync(N.cptr, cptr.data(), sizeof(int) * (t.nleaf + 1), cudaMemcpyHostToDevice, c.stream);
@@ -615,8 +819,12 @@ cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
             r = cudaMemcpyAsync(N.task, task.data(), sizeof(int4) * N.ntask, cudaMemcpyHostToDevice, c.stream);
         if (r != cudaSuccess) return r;
         k_near_cols<<<t.nleaf, 256, smem, c.stream>>>(a, N.cptr, ncol, N.col);
-        k_near_fill<<<blocks, 256, smem, c.stream>>>(a, R, N.cptr, N.col, N.boff, c.xyz, c.src_xyz, c.da, c.detJ, c.treg,
-                                                     c.regs, c.inc_ptr, c.inc, c.tri_c, scratch, N.B);
+        if (own)
+            k_p2m_fill<<<blocks, 256, smem_own, c.stream>>>(a, R, N.cptr, N.col, N.boff, t.src_pos, t.sloc, c.da, c.detJ,
+                                                            c.treg, c.regs, c.inc_ptr, c.inc, c.tri_c, scratch, N.B);
+        else
+            k_near_fill<<<blocks, 256, smem, c.stream>>>(a, R, N.cptr, N.col, N.boff, c.xyz, c.src_xyz, c.da, c.detJ, c.treg,
+                                                         c.regs, c.inc_ptr, c.inc, c.tri_c, scratch, N.B);
         r = cudaGetLastError();
         return r == cudaSuccess ? cudaStreamSynchronize(c.stream) : r;
     };
@@ -629,19 +837,54 @@ cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
     return done(r);
 }
 
-void near_free(NearMat &N) {
-    for (void *p : {(void *)N.cptr, (void *)N.boff, (void *)N.task, (void *)N.col, (void *)N.field, (void *)N.B})
+// The near field's blocks, the P2M blocks beside them, the fields' pairs and the L2P table.
+cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
+    cudaError_t e = blocks_build(c, R, t, false, N.near);
+    if (e != cudaSuccess || !N.near.B) return e;
+    e = blocks_build(c, R, t, true, N.p2m);
+    if (e != cudaSuccess) return e;
+    if (cudaMalloc(&N.field, sizeof(float4) * 3 * (size_t)c.nn) != cudaSuccess ||
+        cudaMalloc(&N.l2p, sizeof(double) * NRM * (size_t)std::max(1, t.ntgt)) != cudaSuccess) {
+        cudaGetLastError();
+        near_free(N);
+        return cudaSuccess;
+    }
+    if (t.ntgt > 0) k_l2p_table<<<(t.ntgt + 127) / 128, 128, 0, c.stream>>>(t.ntgt, t.tloc, N.l2p);
+    return cudaGetLastError();
+}
+
+void blocks_free(DenseBlocks &N) {
+    for (void *p : {(void *)N.cptr, (void *)N.boff, (void *)N.task, (void *)N.col, (void *)N.B})
         if (p) cudaFree(p);
+    N = DenseBlocks();
+}
+void near_free(NearMat &N) {
+    blocks_free(N.near);
+    blocks_free(N.p2m);
+    if (N.field) cudaFree(N.field);
+    if (N.l2p) cudaFree(N.l2p);
     N = NearMat();
 }
 
-cudaError_t launch_near(Ctx &c, const NearTree &t, const NearMat &N, cudaStream_t st, const double *m0, const double *m1,
-                        double *pot0, double *pot1) {
-    if (N.ntask == 0) return cudaSuccess;
+cudaError_t launch_field_pairs(Ctx &c, const NearMat &N, const double *m0, const double *m1) {
     const size_t n3 = 3 * (size_t)c.nn;
-    k_field_pairs<<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(n3, m0, m1, N.field);
-    (m1 ? k_near_mv<2> : k_near_mv<1>)<<<N.ntask, 256, 0, st>>>(N.task, t.leaf_tgt, t.tgt_node, N.cptr, N.col, N.boff, N.B,
-                                                               N.field, pot0, pot1);
+    k_field_pairs<<<(unsigned)((n3 + 255) / 256), 256, 0, c.stream>>>(n3, m0, m1, N.field);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_blocks(const DenseBlocks &N, const NearMat &M, cudaStream_t st, int nq, const int *rows, double *out0,
+                          double *out1) {
+    if (N.ntask == 0) return cudaSuccess;
+    (nq == 2 ? k_block_mv<2> : k_block_mv<1>)<<<N.ntask, 256, 0, st>>>(N.task, rows, N.cptr, N.col, N.boff, N.B, M.field,
+                                                                      out0, out1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_l2p_table(Ctx &c, const NearTree &t, const NearMat &N, int nq, const double *F0, const double *F1,
+                             const double *near0, const double *near1, double *phi0, double *phi1) {
+    if (t.ntgt == 0) return cudaSuccess;
+    (nq == 2 ? k_l2p_apply<2> : k_l2p_apply<1>)<<<(t.ntgt + 127) / 128, 128, 0, c.stream>>>(
+        t.ntgt, t.tgt_leaf, t.tgt_node, N.l2p, t.leaf_scale, F0, F1, near0, near1, phi0, phi1);
     return cudaGetLastError();
 }
 

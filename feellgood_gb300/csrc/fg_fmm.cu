@@ -84,7 +84,7 @@ struct FmmTree {
     // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9
     // in phiv two steps later (film), so runs repeat bit for bit only with the same last bits
     bool repeat = false;
-    NearMat near;              // oz: the near field as dense blocks, where they fit
+    NearMat near;              // oz: P2M and near field as dense blocks, where they fit
     int4 *p2p_task = nullptr;  // leaf, first target, targets of a near-field task
     int n_p2p_task = 0;
     float4 *ds_src_hi = nullptr, *ds_src_lo = nullptr, *ds_tgt_hi = nullptr, *ds_tgt_lo = nullptr;
@@ -918,7 +918,6 @@ struct NearSets {
     const T *F[2];          // local expansions per set
     double *pot[2];         // potentials per set
     int near_only;          // 1: write the near-field sums only (k_l2p adds the far field later)
-    double *phi[2];         // k_l2p: not null: finished potentials, the near sums being theirs already
 };
 
 // One pass of the near field and L2P over up to NT targets tb.. of a leaf (nt of them real,
@@ -1591,12 +1590,6 @@ __global__ void __launch_bounds__(128) k_l2p(int ntgt, const int *__restrict__ t
         }
     });
     const int node = tgt_node[ti];
-    if (sets.phi[0]) {
-        const double f = sc / (4 * M_PI);
-        sets.phi[0][node] = fma(double(fa), f, sets.pot[0][node]);
-        if constexpr (NQ == 2) sets.phi[1][node] = fma(double(fb), f, sets.pot[1][node]);
-        return;
-    }
     sets.pot[0][node] = (double(fa) + sets.pot[0][node]) * sc;
     if constexpr (NQ == 2) sets.pot[1][node] = (double(fb) + sets.pot[1][node]) * sc;
 }
@@ -1732,7 +1725,12 @@ template <typename T>
 static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f);
 static FmmFields tuning_fields(const Ctx &c) { return {{c.u[1], c.v[1]}, {c.pot, c.pot2}}; }
 static NearTree near_tree(const FmmTree &t) {
-    return {t.nleaf, t.leaf_src, t.leaf_tgt, t.tgt_node, t.near_ptr, t.near_leaf, nullptr, nullptr};
+    NearTree n{};
+    n.nleaf = t.nleaf; n.ntgt = t.ntgt;
+    n.leaf_src = t.leaf_src; n.leaf_tgt = t.leaf_tgt; n.tgt_node = t.tgt_node; n.tgt_leaf = t.tgt_leaf;
+    n.near_ptr = t.near_ptr; n.near_leaf = t.near_leaf; n.leaf_scale = t.leaf_scale;
+    n.tloc = (const double4 *)t.tloc;
+    return n;
 }
 
 // Points of each sample (sources and target nodes) and the sample's root cube. A batch of
@@ -2356,14 +2354,6 @@ static int fmm_build_forest(Ctx &c, int L) {
         split(sloc, sh, sl);
         split(tloc, th, tl);
         FCK(near_tasks(P2P_NT, 1, 40));
-        if (t->oz) {
-            std::vector<int> orig(c.nsrc);
-            for (int k = 0; k < c.nsrc; k++) orig[src_dst[k]] = k;
-            NearTree nt = near_tree(*t);
-            nt.src_orig = orig.data();
-            nt.h_leaf_tgt = leaf_tgt.data();
-            FCK(near_build(c, make_rules(c.opts.one_gauss_point != 0), nt, t->near));
-        }
         FCK(up(&t->ds_src_hi, sh));
         FCK(up(&t->ds_src_lo, sl));
         FCK(up(&t->ds_tgt_hi, th));
@@ -2377,6 +2367,25 @@ static int fmm_build_forest(Ctx &c, int L) {
     if (c.src_dst) cudaFree(c.src_dst);
     c.src_dst = nullptr;
     FCK(up(&c.src_dst, src_dst));
+    if (t->oz) {
+        std::vector<int> orig(c.nsrc);
+        for (int k = 0; k < c.nsrc; k++) orig[src_dst[k]] = k;
+        int *d_orig = nullptr;
+        double *d_sloc = nullptr;
+        cudaError_t e = up(&d_orig, orig);
+        if (e == cudaSuccess) e = up(&d_sloc, sloc);
+        if (e == cudaSuccess) {
+            NearTree nt = near_tree(*t);
+            nt.src_orig = d_orig;
+            nt.src_pos = c.src_dst;
+            nt.sloc = (const double4 *)d_sloc;
+            nt.h_leaf_tgt = leaf_tgt.data();
+            e = near_build(c, make_rules(c.opts.one_gauss_point != 0), nt, t->near);
+        }
+        if (d_orig) cudaFree(d_orig);
+        if (d_sloc) cudaFree(d_sloc);
+        FCK(e);
+    }
     const size_t esz = fp32 ? sizeof(float) : sizeof(double);
     const size_t nexp_all = (size_t)ncell * NR * t->nq;
     FCK(cudaMalloc(&t->M, nexp_all * esz));
@@ -2501,8 +2510,7 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
     ns.pot[0] = c.pot;
     ns.pot[1] = nq == 2 ? c.pot2 : c.pot;
     ns.near_only = 0;
-    const bool whole = t.near.B != nullptr;
-    for (int k = 0; k < 2; k++) ns.phi[k] = whole ? f.phi[k < nq ? k : 0] : nullptr;
+    const bool whole = t.near.near.B != nullptr;
     const int nb = (t.nleaf + 3) / 4;
     cudaError_t terr = cudaSuccess;  // first failed launch of a translation or of the near field
     auto note = [&](cudaError_t e) {
@@ -2510,7 +2518,7 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
     };
     auto near_field = [&](cudaStream_t st) {
         if (whole) {
-            note(launch_near(c, near_tree(t), t.near, st, f.m[0], nq == 2 ? f.m[1] : nullptr, c.pot, c.pot2));
+            note(launch_blocks(t.near.near, t.near, st, nq, t.tgt_node, c.pot, c.pot2));
             return;
         }
         if constexpr (sizeof(T) == 8) {
@@ -2537,9 +2545,13 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
         }
     };
     t.ev_split[t.ev_next] = split && prof;
+    if (whole) note(launch_field_pairs(c, t.near, f.m[0], nq == 2 ? f.m[1] : nullptr));
     if constexpr (sizeof(T) == 4) {
         (nq == 2 ? k_p2m2<2> : k_p2m2<1>)<<<(t.nleaf + 3) / 4, 128, 0, c.stream>>>(
             t.nleaf, t.leaf_src, (const float *)t.sloc, t.leaf0, ps[0], ps[1]);
+    } else if (t.near.p2m.B) {
+        const size_t l0 = (size_t)t.leaf0 * NR;
+        note(launch_blocks(t.near.p2m, t.near, c.stream, nq, nullptr, (double *)M + l0, (double *)M + l0 + sstride));
     } else if (t.oz) {
         (nq == 2 ? k_p2m_ds<2> : k_p2m_ds<1>)<<<dim3((t.nleaf + 3) / 4, 5), 128, 0, c.stream>>>(
             t.nleaf, t.leaf_src, (const float4 *)t.ds_src_hi, (const float4 *)t.ds_src_lo, t.leaf0, ps[0], ps[1]);
@@ -2637,8 +2649,12 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
     if (split || t.oz) {  // L2P apart: the double-single near field stores its sums
         if (split) cudaStreamWaitEvent(c.stream, c.ev_join, 0);
         else near_field(c.stream);
+        if (whole) {
+            const double *Fl = (const double *)F + (size_t)t.leaf0 * NR;
+            note(launch_l2p_table(c, near_tree(t), t.near, nq, Fl, Fl + sstride, c.pot, c.pot2, f.phi[0], f.phi[1]));
+        }
         auto k = nq == 2 ? k_l2p<T, 2> : k_l2p<T, 1>;
-        if (t.ntgt > 0)
+        if (t.ntgt > 0 && !whole)
             k<<<(t.ntgt + 127) / 128, 128, 0, c.stream>>>(t.ntgt, t.tgt_leaf, t.tgt_node, (const T *)t.tloc, t.leaf0,
                                                           t.leaf_scale, ns);
     } else {
@@ -2655,7 +2671,12 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
 
 bool fmm_whole(const Ctx &c) {
     const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
-    return t && t->near.B;
+    return t && t->near.near.B;
+}
+
+bool fmm_charges(const Ctx &c) {
+    const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
+    return !t || !t->near.near.B || !t->near.p2m.B;
 }
 
 cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f) {
@@ -2717,7 +2738,7 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
     if (!t) return 0;
     int n = 2;  // P2M, L2P + P2P (both sets in one launch each)
     if ((c.opts.fmm_overlap != 0 && c.stream2) || t->oz) n += 1;  // L2P apart from the near field
-    if (t->near.B) n += 1;  // the fields as pairs
+    if (t->near.near.B) n += 1;  // the fields as pairs
     if (t->oz) {  // digits of the leaves, then per translation the products and the sums
         n += 1;
         for (int l = 2; l <= t->L - 1; l++) n += (t->oz_m2m[l].nunit > 0) + (t->oz_m2m[l].ntile > 0);

@@ -351,24 +351,35 @@ cudaError_t launch_charges_pair(Ctx &c, const double *m, const double *v);  // s
 // direct sum as a matrix over the nodes (fg_dense.cu)
 cudaError_t dense_build(Ctx &c, const Rules &R);  // direct_mat stays null where it does not fit
 cudaError_t launch_dense(Ctx &c, const double *m0, const double *m1, double *phi0, double *phi1);
-// near field of the FP64 FMM as dense blocks over the nodes (fg_dense.cu)
-struct NearMat {
+// P2M and near field of the FP64 FMM as dense blocks over the nodes (fg_dense.cu)
+struct DenseBlocks {
     int *cptr = nullptr, *col = nullptr;  // columns (node ids, ascending, -1 padding) of each leaf
     size_t *boff = nullptr;               // first entry of each leaf's block
-    float2 *B = nullptr;                  // [target][3 columns] double-single; null: no blocks
-    int4 *task = nullptr;                 // leaf, first target, targets (at most 16)
-    float4 *field = nullptr;              // the fields as pairs, 3 per node
+    float2 *B = nullptr;                  // [row][3 columns] double-single; null: no blocks
+    int4 *task = nullptr;                 // leaf, first row, rows, first output
     int ntask = 0;
 };
+struct NearMat {
+    DenseBlocks near, p2m;
+    float4 *field = nullptr;  // the fields as pairs, 3 per node
+    double *l2p = nullptr;    // harmonics at the targets [100][target]
+};
 struct NearTree {
-    int nleaf;
-    const int *leaf_src, *leaf_tgt, *tgt_node, *near_ptr, *near_leaf;  // device tables
-    const int *src_orig, *h_leaf_tgt;                                  // host: source of each position
+    int nleaf, ntgt;
+    // device tables; src_orig: source of each position, src_pos its inverse
+    const int *leaf_src, *leaf_tgt, *tgt_node, *tgt_leaf, *near_ptr, *near_leaf, *src_orig, *src_pos;
+    const double4 *sloc, *tloc;  // leaf-local coordinates of the sources (for the build only) and targets
+    const double *leaf_scale;
+    const int *h_leaf_tgt;       // host
 };
 cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N);
+void blocks_free(DenseBlocks &N);
 void near_free(NearMat &N);
-cudaError_t launch_near(Ctx &c, const NearTree &t, const NearMat &N, cudaStream_t st, const double *m0, const double *m1,
-                        double *pot0, double *pot1);
+cudaError_t launch_field_pairs(Ctx &c, const NearMat &N, const double *m0, const double *m1);
+cudaError_t launch_blocks(const DenseBlocks &N, const NearMat &M, cudaStream_t st, int nq, const int *rows, double *out0,
+                          double *out1);
+cudaError_t launch_l2p_table(Ctx &c, const NearTree &t, const NearMat &N, int nq, const double *F0, const double *F1,
+                             const double *near0, const double *near1, double *phi0, double *phi1);
 int direct_splits(const Ctx &c);                 // shares of the sources of the direct sum
 cudaError_t launch_p2p_direct(Ctx &c, int nq);  // sets 0 .. nq - 1 into direct_part
 // phi = base + (pot + corr) / (4 pi) of set 0 and, phi1 not null, of set 1 (base null: no base)
@@ -403,6 +414,7 @@ struct FmmFields {
     double *phi[2];
 };
 bool fmm_whole(const Ctx &c);
+bool fmm_charges(const Ctx &c);  // the evaluation reads charges (else it starts from the fields)
 cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f);  // nq 2: c.src_q2 -> c.pot2 beside c.src_q -> c.pot
 // The same evaluation with an FP64 tree of the FP32 tree's depth (built on first use; the
 // FP32 tree itself when the context is FP64); FG_* status
