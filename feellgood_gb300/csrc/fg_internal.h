@@ -93,12 +93,10 @@ struct SegAcc {
     double v2max;    // max over steps of max |v|^2 / gamma0^2 (bit pattern compared as unsigned)
 };
 
-// Grid-wide barrier state of the persistent kernels (bounded wait, no hang).
+// Grid-wide barrier state of the persistent kernels (bounded wait, no hang), zero at each launch.
 struct GridBar {
-    unsigned int count;
-    unsigned int gen;
-    int err;
-    int pad;
+    unsigned int count;  // arrivals since the launch
+    int err;             // FG_ETIMEDOUT once a wait expired
 };
 
 // Arguments of the FP64 BiCGSTAB persistent kernel (bicg_dir, src/algebra/bicg.h:163-234).

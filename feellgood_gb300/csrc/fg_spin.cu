@@ -1019,6 +1019,7 @@ cudaError_t launch_spin(Ctx &c) {
     }
     a.scale = S->scale; a.inner_tol = c.opts.inner_tol; a.refine_max = c.opts.refine_max;
     cudaError_t e = cudaMemsetAsync(S->res, 0, sizeof(SolveResult), c.stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(S->bar, 0, sizeof(GridBar), c.stream);
     if (e != cudaSuccess) return e;
     void *args[] = {&a};
     return cudaLaunchCooperativeKernel(S->mixed ? (void *)k_spin_mixed : (void *)k_spin_bicg, dim3(S->grid),
