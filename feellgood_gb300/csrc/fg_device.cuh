@@ -132,6 +132,40 @@ __device__ __forceinline__ void grid_sum(const double *partial, int G, double (&
     __syncthreads();
 }
 
+// The sums of blocks [b0, b1) and NX scalars that f forms from them (f(sums, x), by one thread: a
+// division or square root in every thread would queue on the 1/64-rate FP64 pipe), for every
+// thread of the block.
+template <int NV, int NX, typename F>
+__device__ __forceinline__ void sum_scalars(const double *partial, int G, int b0, int b1, double (&out)[NV],
+                                            double (&x)[NX], F f) {
+    __shared__ double res[NV + NX];
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        double s[NV];
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            double v = 0.0;
+            for (int b = b0 + lane; b < b1; b += 32) v += *(volatile const double *)&partial[k * G + b];
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            s[k] = v;
+        }
+        if (lane == 0) {
+            double y[NX];
+            f(s, y);
+#pragma unroll
+            for (int k = 0; k < NV; k++) res[k] = s[k];
+#pragma unroll
+            for (int k = 0; k < NX; k++) res[NV + k] = y[k];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; k++) out[k] = res[k];
+#pragma unroll
+    for (int k = 0; k < NX; k++) x[k] = res[NV + k];
+    __syncthreads();
+}
+
 // Sum of the partials of blocks [b0, b1) only (one sample of a batch), same fixed order.
 template <int NV>
 __device__ __forceinline__ void range_sum(const double *partial, int G, int b0, int b1, double (&out)[NV]) {

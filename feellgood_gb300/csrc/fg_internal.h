@@ -387,7 +387,7 @@ cudaError_t launch_state_diff(Ctx &c);  // dstate32 = NEXT - CURRENT for u and v
 cudaError_t launch_charges32(Ctx &c, int nq);  // FP32 charges of dstate32 (incremental demag)
 cudaError_t launch_energy(Ctx &c, const double Hext[3]);
 cudaError_t launch_energy_into(Ctx &c, const double Hext[3], double *partial);
-int bicg_grid_size(Ctx &c, bool mixed);
+int bicg_grid_size(Ctx &c);  // and c.bicg_block
 cudaError_t morton_sort(Ctx &c, int n, int L, int nseg, const double *xyz, const int *seg,
                         const std::vector<double4> &roots, const unsigned char *keep, std::vector<uint64_t> &keys,
                         std::vector<int> &idx, double *dev_ms);

@@ -546,11 +546,15 @@ __global__ void k_node64(int nn, const int *__restrict__ inc_ptr, const int *__r
 // bounded grid barriers and the dot products are deterministic two-level reductions.
 // On success the node update of LinAlgebra::solve (src/solver.cpp:74-88) is fused.
 
-__global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
+// Consecutive reductions use two buffers in turn, so that no block overwrites sums that another
+// still reads. Five barriers per iteration: s, shat = M s and its tangent vector are formed in one
+// phase, before |s| is known (a converged half step does not read the latter two).
+__global__ void __launch_bounds__(256, 4) k_bicg64(BicgArgs a) {
     const int G = gridDim.x;
     const int nn = a.nn;
     const int stride = G * blockDim.x;
     const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    double *part[2] = {a.partial, a.partial + 2 * (size_t)G};
     // phase 0: r = b - K x (masked), rt = r, p = r; |b|^2, |r|^2
     {
         double bb = 0.0, rr = 0.0;
@@ -568,18 +572,20 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
             rr += r0 * r0 + r1 * r1;
         }
         double v2[2] = {bb, rr};
-        block_store<2>(v2, a.partial, G);
+        block_store<2>(v2, part[0], G);
     }
     if (!grid_sync(a.bar)) goto timeout;
     {
-        double s2[2];
-        grid_sum<2>(a.partial, G, s2);
-        const double rhsn = sqrt(fabs(s2[0]));
-        const double resmax = a.tol;
-        double rr = s2[1], rtr = s2[1];
+        double s2[2], x2[2];
+        sum_scalars(part[0], G, 0, G, s2, x2, [](const double *s, double *x) {
+            x[0] = sqrt(fabs(s[0]));
+            x[1] = sqrt(fabs(s[1]));
+        });
+        const double rhsn = x2[0], resmax = a.tol, limit = rhsn * resmax;
+        double rnorm = x2[1], rtr = s2[1];
         double rho1 = 0.0, rho2 = 0.0, alpha = 0.0, beta = 0.0, omega = 0.0;
         int status = -1, nit = 0;
-        double res = sqrt(fabs(rr));
+        double res = rnorm;
         const double res0 = res;
         // iteration::finished
         auto finished = [&](double nr) {
@@ -588,18 +594,15 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
                 status = 2;
                 return false;
             }
-            const bool cv = res <= rhsn * resmax;
+            const bool cv = res <= limit;
             if (cv) status = 0;
             return cv;
         };
-        while (!finished(sqrt(fabs(rr)))) {
+        while (!finished(rnorm)) {
             rho1 = rtr;
-            if (nit > 0) {
-                if (rho2 == 0.0 || omega == 0.0) {
-                    status = 2;
-                    break;
-                }
-                beta = (rho1 / rho2) * (alpha / omega);
+            if (nit > 0 && (rho2 == 0.0 || omega == 0.0)) {
+                status = 2;
+                break;
             }
             // phase 1: p = r + beta (p - omega v); phat = M p; W = tangent(phat)
             for (int i = i0; i < nn; i += stride) {
@@ -626,15 +629,15 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
                     vr += y0 * a.rt[2 * i] + y1 * a.rt[2 * i + 1];
                 }
                 double v1[1] = {vr};
-                block_store<1>(v1, a.partial, G);
+                block_store<1>(v1, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s1[1];
-                grid_sum<1>(a.partial, G, s1);
-                alpha = rho1 / s1[0];
+                double s1[1], x1[1];
+                sum_scalars(part[1], G, 0, G, s1, x1, [=](const double *s, double *x) { x[0] = rho1 / s[0]; });
+                alpha = x1[0];
             }
-            // phase 3: s = r - alpha v; shat = M s; |s|^2
+            // phase 3: s = r - alpha v; |s|^2; shat = M s, W = tangent(shat)
             {
                 double ss = 0.0;
                 for (int i = i0; i < nn; i += stride) {
@@ -642,15 +645,18 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
                     const double s1 = a.r[2 * i + 1] + (-alpha) * a.v[2 * i + 1];
                     a.s[2 * i] = s0; a.s[2 * i + 1] = s1;
                     ss += s0 * s0 + s1 * s1;
+                    const double h0 = a.Minv[2 * i] * s0, h1 = a.Minv[2 * i + 1] * s1;
+                    a.shat[2 * i] = h0; a.shat[2 * i + 1] = h1;
+                    tangent(i, a.ep, a.eq, h0, h1, a.W);
                 }
                 double v1[1] = {ss};
-                block_store<1>(v1, a.partial, G);
+                block_store<1>(v1, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s1[1];
-                grid_sum<1>(a.partial, G, s1);
-                if (finished(sqrt(fabs(s1[0])))) {
+                double s1[1], x1[1];
+                sum_scalars(part[0], G, 0, G, s1, x1, [](const double *s, double *x) { x[0] = sqrt(fabs(s[0])); });
+                if (finished(x1[0])) {
                     for (int i = i0; i < nn; i += stride) {
                         a.x[2 * i] += alpha * a.phat[2 * i];
                         a.x[2 * i + 1] += alpha * a.phat[2 * i + 1];
@@ -660,14 +666,7 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
                     break;
                 }
             }
-            // phase 4: shat = M s, W = tangent(shat) ... needs a barrier before the SpMV
-            for (int i = i0; i < nn; i += stride) {
-                const double h0 = a.Minv[2 * i] * a.s[2 * i], h1 = a.Minv[2 * i + 1] * a.s[2 * i + 1];
-                a.shat[2 * i] = h0; a.shat[2 * i + 1] = h1;
-                tangent(i, a.ep, a.eq, h0, h1, a.W);
-            }
-            if (!grid_sync(a.bar)) goto timeout;
-            // phase 5: t = K shat (masked); t.s, t.t
+            // phase 4: t = K shat (masked); t.s, t.t
             {
                 double ts = 0.0, tt = 0.0;
                 for (int i = i0; i < nn; i += stride) {
@@ -680,15 +679,15 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
                     tt += y0 * y0 + y1 * y1;
                 }
                 double v2[2] = {ts, tt};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s2b[2];
-                grid_sum<2>(a.partial, G, s2b);
-                omega = s2b[0] / s2b[1];
+                double s2b[2], x1[1];
+                sum_scalars(part[1], G, 0, G, s2b, x1, [](const double *s, double *x) { x[0] = s[0] / s[1]; });
+                omega = x1[0];
             }
-            // phase 6: x += alpha phat + omega shat; r = s - omega t; |r|^2, rt.r
+            // phase 5: x += alpha phat + omega shat; r = s - omega t; |r|^2, rt.r
             {
                 double r2 = 0.0, rtr2 = 0.0;
                 for (int i = i0; i < nn; i += stride) {
@@ -705,14 +704,18 @@ __global__ void __launch_bounds__(256) k_bicg64(BicgArgs a) {
                     }
                 }
                 double v2[2] = {r2, rtr2};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s2c[2];
-                grid_sum<2>(a.partial, G, s2c);
-                rr = s2c[0];
+                double s2c[2], xn[2];
+                sum_scalars(part[0], G, 0, G, s2c, xn, [=](const double *s, double *x) {
+                    x[0] = sqrt(fabs(s[0]));
+                    x[1] = (s[1] / rho1) * (alpha / omega);
+                });
+                rnorm = xn[0];
                 rtr = s2c[1];
+                beta = xn[1];
             }
             rho2 = rho1;
             nit++;
@@ -773,6 +776,7 @@ timeout:
 // pass (slot 1, summed over the whole grid).
 __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
     const int G = gridDim.x;
+    double *part[2] = {a.partial, a.partial + 2 * (size_t)G};
     int g = 0;
     {
         int lo = 0, hi = a.nseg - 1;
@@ -804,18 +808,20 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
             rr += r0 * r0 + r1 * r1;
         }
         double v2[2] = {bb, rr};
-        block_store<2>(v2, a.partial, G);
+        block_store<2>(v2, part[0], G);
     }
     if (!grid_sync(a.bar)) goto timeout;
     {
-        double s2[2];
-        range_sum<2>(a.partial, G, b0, b1, s2);
-        const double rhsn = sqrt(fabs(s2[0]));
-        const double resmax = a.tol;
-        double rr = s2[1], rtr = s2[1];
+        double s2[2], x2[2];
+        sum_scalars(part[0], G, b0, b1, s2, x2, [](const double *s, double *x) {
+            x[0] = sqrt(fabs(s[0]));
+            x[1] = sqrt(fabs(s[1]));
+        });
+        const double rhsn = x2[0], resmax = a.tol, limit = rhsn * resmax;
+        double rnorm = x2[1], rtr = s2[1];
         double rho1 = 0.0, rho2 = 0.0, alpha = 0.0, beta = 0.0, omega = 0.0;
         int status = -1, nit = 0;
-        double res = sqrt(fabs(rr));
+        double res = rnorm;
         const double res0 = res;
         auto finished = [&](double nr) {
             res = fabs(nr);
@@ -823,22 +829,18 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
                 status = 2;
                 return false;
             }
-            const bool cv = res <= rhsn * resmax;
+            const bool cv = res <= limit;
             if (cv) status = 0;
             return cv;
         };
         bool act = true;
         for (;;) {
-            if (act && finished(sqrt(fabs(rr)))) act = false;
+            if (act && finished(rnorm)) act = false;
             if (act) {
                 rho1 = rtr;
-                if (nit > 0) {
-                    if (rho2 == 0.0 || omega == 0.0) {
-                        status = 2;
-                        act = false;
-                    } else {
-                        beta = (rho1 / rho2) * (alpha / omega);
-                    }
+                if (nit > 0 && (rho2 == 0.0 || omega == 0.0)) {
+                    status = 2;
+                    act = false;
                 }
             }
             if (act)
@@ -866,15 +868,15 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
                         vr += y0 * a.rt[2 * i] + y1 * a.rt[2 * i + 1];
                     }
                 double v2[2] = {vr, (threadIdx.x == 0 && act) ? 1.0 : 0.0};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s1[1], f[1];
-                range_sum<1>(a.partial, G, b0, b1, s1);
-                grid_sum<1>(a.partial + G, G, f);
+                double s1[1], x1[1], f[1];
+                sum_scalars(part[1], G, b0, b1, s1, x1, [=](const double *s, double *x) { x[0] = rho1 / s[0]; });
+                grid_sum<1>(part[1] + G, G, f);
                 if (f[0] == 0.0) break;  // every sample has ended
-                if (act) alpha = rho1 / s1[0];
+                if (act) alpha = x1[0];
             }
             {
                 double ss = 0.0;
@@ -884,16 +886,19 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
                         const double s1 = a.r[2 * i + 1] + (-alpha) * a.v[2 * i + 1];
                         a.s[2 * i] = s0; a.s[2 * i + 1] = s1;
                         ss += s0 * s0 + s1 * s1;
+                        const double h0 = a.Minv[2 * i] * s0, h1 = a.Minv[2 * i + 1] * s1;
+                        a.shat[2 * i] = h0; a.shat[2 * i + 1] = h1;
+                        tangent(i, a.ep, a.eq, h0, h1, a.W);
                     }
                 double v1[1] = {ss};
-                block_store<1>(v1, a.partial, G);
+                block_store<1>(v1, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s1[1];
-                range_sum<1>(a.partial, G, b0, b1, s1);
+                double s1[1], x1[1];
+                sum_scalars(part[0], G, b0, b1, s1, x1, [](const double *s, double *x) { x[0] = sqrt(fabs(s[0])); });
                 if (act) {
-                    if (finished(sqrt(fabs(s1[0])))) {
+                    if (finished(x1[0])) {
                         for (int i = i0; i < r_hi; i += stride) {
                             a.x[2 * i] += alpha * a.phat[2 * i];
                             a.x[2 * i + 1] += alpha * a.phat[2 * i + 1];
@@ -904,13 +909,6 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
                     }
                 }
             }
-            if (act)
-                for (int i = i0; i < r_hi; i += stride) {
-                    const double h0 = a.Minv[2 * i] * a.s[2 * i], h1 = a.Minv[2 * i + 1] * a.s[2 * i + 1];
-                    a.shat[2 * i] = h0; a.shat[2 * i + 1] = h1;
-                    tangent(i, a.ep, a.eq, h0, h1, a.W);
-                }
-            if (!grid_sync(a.bar)) goto timeout;
             {
                 double ts = 0.0, tt = 0.0;
                 if (act)
@@ -924,13 +922,13 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
                         tt += y0 * y0 + y1 * y1;
                     }
                 double v2[2] = {ts, tt};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s2b[2];
-                range_sum<2>(a.partial, G, b0, b1, s2b);
-                if (act) omega = s2b[0] / s2b[1];
+                double s2b[2], x1[1];
+                sum_scalars(part[1], G, b0, b1, s2b, x1, [](const double *s, double *x) { x[0] = s[0] / s[1]; });
+                if (act) omega = x1[0];
             }
             {
                 double r2 = 0.0, rtr2 = 0.0;
@@ -949,15 +947,19 @@ __global__ void __launch_bounds__(256) k_bicg64_seg(BicgArgs a) {
                         }
                     }
                 double v2[2] = {r2, rtr2};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
-                double s2c[2];
-                range_sum<2>(a.partial, G, b0, b1, s2c);
+                double s2c[2], xn[2];
+                sum_scalars(part[0], G, b0, b1, s2c, xn, [=](const double *s, double *x) {
+                    x[0] = sqrt(fabs(s[0]));
+                    x[1] = (s[1] / rho1) * (alpha / omega);
+                });
                 if (act) {
-                    rr = s2c[0];
+                    rnorm = xn[0];
                     rtr = s2c[1];
+                    beta = xn[1];
                     rho2 = rho1;
                     nit++;
                     if (nit >= a.maxiter) status = 1;
@@ -1740,16 +1742,15 @@ int bicg_seg_max_blocks(Ctx &c) {
     return std::max(1, per_sm) * c.nsm;
 }
 
-int bicg_grid_size(Ctx &c, bool mixed) {
+// Blocks of 64 threads where that gives every SM one, of 128 where 64 would give it more, then of
+// 256: the FP64 pipe (2 per clock and SM) bounds the rows of a block, so a mesh of a few thousand
+// nodes has to reach all SMs, and each further block costs at the barriers. One block of 256 meets
+// itself without a barrier.
+int bicg_grid_size(Ctx &c) {
+    c.bicg_block = c.nn <= 256 ? 256 : c.nn <= 64 * c.nsm ? 64 : c.nn <= 128 * c.nsm ? 128 : 256;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bicg64, 256, 0);
-    (void)mixed;
-    if (per_sm < 1) per_sm = 1;
-    int g = per_sm * c.nsm;
-    const int need = nblocks(c.nn, 256);
-    if (need < g) g = need;
-    if (g < 1) g = 1;
-    return g;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bicg64, c.bicg_block, 0);
+    return std::max(1, std::min(std::max(1, per_sm) * c.nsm, nblocks(c.nn, c.bicg_block)));
 }
 
 cudaError_t launch_bicg64(Ctx &c, double dt, double prefactor) {
@@ -1787,7 +1788,7 @@ cudaError_t launch_bicg64(Ctx &c, double dt, double prefactor) {
     void *args[] = {&a};
     if (multi)
         return cudaLaunchCooperativeKernel((void *)k_bicg64_seg, dim3(c.seg_grid), dim3(256), args, 0, c.stream);
-    return cudaLaunchCooperativeKernel((void *)k_bicg64, dim3(c.bicg_grid), dim3(256), args, 0, c.stream);
+    return cudaLaunchCooperativeKernel((void *)k_bicg64, dim3(c.bicg_grid), dim3(c.bicg_block), args, 0, c.stream);
 }
 
 cudaError_t launch_apply(Ctx &c, double c0, const double *x, double *y) {
