@@ -118,6 +118,9 @@ struct FmmTree {
     float *oz_scale = nullptr;
     unsigned char *oz_img[3] = {nullptr, nullptr, nullptr};  // M2M, M2L, L2L
     float *oz_rows[3] = {nullptr, nullptr, nullptr};
+    // repeat: the lists (oz_cells, oz_codes, oz_units) are those of k_translate_ds, the images its
+    // split operators, M holds pairs hi + lo, and F_split those of the locals above the leaves
+    void *F_split = nullptr;
     float *Mh = nullptr, *Ml = nullptr, *Fh = nullptr, *Fl = nullptr;  // hi/lo splits of M and F
     unsigned char *img_m2l = nullptr, *img_m2m = nullptr, *img_l2l = nullptr;  // operator images
     int *dst_keep = nullptr;
@@ -628,6 +631,11 @@ __global__ void __launch_bounds__(128, 4) k_p2m_ds(int nleaf, const int *__restr
     }
 }
 
+__device__ __forceinline__ float2 ds_split(double x) {
+    const float h = (float)x;
+    return make_float2(h, (float)(x - (double)h));
+}
+
 // ---- P2M of the full FP64 evaluation of the FP32 + refinement path (FmmTree::repeat) ----
 // The recurrences of ups_cols with every operation a double-single one, the coordinates as the
 // normalised pair of their stored hi + lo parts, the charge split once.
@@ -662,7 +670,7 @@ __device__ __forceinline__ void ups_col_ds(dsf x, dsf y, dsf z, dsf r2, dsf &dre
 }
 
 template <int NS, int M0, int M1>
-__device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, const float4 *__restrict__ shi,
+__device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, int rounds, const float4 *__restrict__ shi,
                                             const float4 *__restrict__ slo, size_t base, const P2mSet<double> &a,
                                             const P2mSet<double> &b) {
     constexpr int NPR = lidx(M0, FMM_P, M1, 1) + 1;
@@ -671,7 +679,10 @@ __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, const floa
     for (int k = 0; k < NPR; k++) acc0[k] = dsf{0.f, 0.f};
 #pragma unroll
     for (int k = 0; k < (NS == 2 ? NPR : 1); k++) acc1[k] = dsf{0.f, 0.f};
-    for (int s = s0 + lane; s < s1; s += 32) {
+    for (int q = 0; q < rounds; q++) {
+        __syncthreads();  // the block's warps in step, on the same instructions
+        const int s = s0 + lane + 32 * q;
+        if (s >= s1) continue;
         const float4 h = shi[s], l = slo[s];
         const dsf x = ds_two_sum_f(h.x, l.x), y = ds_two_sum_f(h.y, l.y), z = ds_two_sum_f(h.z, l.z);
         const double qa_d = a.q[s], qb_d = NS == 2 ? b.q[s] : 0.0;
@@ -713,33 +724,40 @@ __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, const floa
                 const dsf v0 = red(acc0[k]);
                 dsf v1 = {0.f, 0.f};
                 if constexpr (NS == 2) v1 = red(acc1[k]);
-                if ((g & 31) == lane) {
-                    a.M[base + g] = ds_to(v0);
-                    if constexpr (NS == 2) b.M[base + g] = ds_to(v1);
+                if ((g & 31) == lane && s0 >= 0) {
+                    // rounded to FP64, then the pair that the translations read
+                    reinterpret_cast<float2 *>(a.M)[base + g] = ds_split(ds_to(v0));
+                    if constexpr (NS == 2) reinterpret_cast<float2 *>(b.M)[base + g] = ds_split(ds_to(v1));
                 }
             }
 }
 
-// One warp per leaf, the NS charge sets in one pass over the sources (the FP64 tree's
-// sources as hi/lo float4 pairs): the harmonics of a source are formed once for both sets,
-// in six passes over the harmonic columns (0, 1, 2, 3, 4-5, 6-9: at most 22 reals, 88 floats
-// of accumulators for two sets); one set and two run the same code, so a set's expansion
-// does not depend on whether the other is evaluated beside it.
+// One warp per leaf and range of harmonic columns (0, 1, 2, 3, 4-5, 6-9: at most 22 reals, 88 floats
+// of accumulators for two sets), the NS charge sets together (the FP64 tree's sources as hi/lo
+// float4 pairs): the harmonics of a source are formed once for both sets; one set and two run the
+// same code, so a set's expansion does not depend on whether the other is evaluated beside it. The
+// range is the slow grid index and the block's warps keep in step: bound by fetching the unrolled
+// instructions, which six passes by each warp at its own pace made worse (294k tets, two sets: six
+// passes per warp 1.45 ms, a range per block 0.87, in step 0.73).
 template <int NS>
-__global__ void __launch_bounds__(128) k_p2m_ds_repeat(int nleaf, const int *__restrict__ leaf_src,
+__global__ void __launch_bounds__(128, 3) k_p2m_ds_repeat(int nleaf, const int *__restrict__ leaf_src,
                                                 const float4 *__restrict__ shi, const float4 *__restrict__ slo,
                                                 int leaf0, P2mSet<double> set0, P2mSet<double> set1) {
     const int lane = threadIdx.x & 31;
     const int leaf = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (leaf >= nleaf) return;
-    const int s0 = leaf_src[leaf], s1 = leaf_src[leaf + 1];
+    const int s0 = leaf < nleaf ? leaf_src[leaf] : -1, s1 = leaf < nleaf ? leaf_src[leaf + 1] : -1;  // -1: no leaf
+    int rounds = 0;  // of the block's longest leaf
+    for (int k = blockIdx.x * 4; k < min(nleaf, (int)blockIdx.x * 4 + 4); k++)
+        rounds = max(rounds, (leaf_src[k + 1] - leaf_src[k] + 31) / 32);
     const size_t base = (size_t)(leaf0 + leaf) * NR;
-    p2m_ds_pass<NS, 0, 0>(lane, s0, s1, shi, slo, base, set0, set1);
-    p2m_ds_pass<NS, 1, 1>(lane, s0, s1, shi, slo, base, set0, set1);
-    p2m_ds_pass<NS, 2, 2>(lane, s0, s1, shi, slo, base, set0, set1);
-    p2m_ds_pass<NS, 3, 3>(lane, s0, s1, shi, slo, base, set0, set1);
-    p2m_ds_pass<NS, 4, 5>(lane, s0, s1, shi, slo, base, set0, set1);
-    p2m_ds_pass<NS, 6, FMM_P>(lane, s0, s1, shi, slo, base, set0, set1);
+    switch (blockIdx.y) {
+        case 0: p2m_ds_pass<NS, 6, FMM_P>(lane, s0, s1, rounds, shi, slo, base, set0, set1); break;
+        case 1: p2m_ds_pass<NS, 4, 5>(lane, s0, s1, rounds, shi, slo, base, set0, set1); break;
+        case 2: p2m_ds_pass<NS, 3, 3>(lane, s0, s1, rounds, shi, slo, base, set0, set1); break;
+        case 3: p2m_ds_pass<NS, 2, 2>(lane, s0, s1, rounds, shi, slo, base, set0, set1); break;
+        case 4: p2m_ds_pass<NS, 1, 1>(lane, s0, s1, rounds, shi, slo, base, set0, set1); break;
+        default: p2m_ds_pass<NS, 0, 0>(lane, s0, s1, rounds, shi, slo, base, set0, set1); break;
+    }
 }
 
 // Batched translation out[c] (+)= sum_code Op[code] in[tab[c][code]] for TB output cells
@@ -801,96 +819,144 @@ __global__ void __launch_bounds__(160) k_translate(int n_out, int out0, int ncod
 }
 
 // Translations in double-single arithmetic on the FP32 pipes (the full FP64 evaluation of the
-// FP32 + refinement path, see FmmTree::repeat): the same batched GEMM as
-// k_translate, both charge sets of a block of DS_TB output cells as its 2 DS_TB columns, the
-// operator and the inputs split into FP32 pairs hi + lo on their way into shared memory,
-// every product exact through fma (Dekker's TwoProduct) and summed with Knuth's two-sum,
-// the running sum renormalised once per code (about 44 significant bits), the result
-// rounded to FP64 once.
-constexpr int DS_TB = 16, DS_COLS = 2 * DS_TB, DS_CT = 2, DS_BLD = DS_COLS + 1;
-constexpr int tr_ds_smem() { return (NR * NR + NR * DS_BLD) * (int)sizeof(float2); }
+// FP32 + refinement path, see FmmTree::repeat): per output and code the products in the order of
+// k, every product exact through fma (Dekker's TwoProduct) and summed with Knuth's two-sum, the
+// running sum renormalised once per code (about 44 significant bits), the result rounded to FP64
+// once. 12 FP32 operations per product bound it.
+//
+// A block takes DS_ROWS rows of the operators for a tile of DS_TILE output cells that share their
+// codes (the cells of one octant, in lists made with the tree), a lane per cell and DS_RT rows per
+// warp; the tile's codes run one after the other, as the order of the sums is fixed. Operators
+// (split when the tree is made, in the order in which the block reads them) and inputs (split by
+// the kernel that forms them) come through a ring of DS_STAGE pieces of DS_KC columns by cp.async.
+// Before, a block held all 100 rows of 16 neighbouring cells: most (cell, code) columns were zero,
+// each block split 10,000 FP64 operator entries per code again, and 128 blocks left SMs idle (294k
+// tets, two sets: M2L 6.24 -> 1.66 ms, FMA pipe busy 71% of the time; M2M 0.74 -> 0.12, L2L 0.66 -> 0.09).
+constexpr int DS_TILE = 32, DS_RT = 5, DS_ROWS = 4 * DS_RT, DS_PARTS = NR / DS_ROWS, DS_KC = 20, DS_STAGE = 4;
+constexpr int DS_CHUNKS = NR / DS_KC, DS_A4 = DS_ROWS * DS_KC / 2;  // float4 of operator per piece
+constexpr int DS_B4 = DS_KC / 2 + 1;  // float4 per cell and piece, one of padding against bank conflicts
+static_assert(DS_PARTS * DS_ROWS == NR && DS_CHUNKS * DS_KC == NR && DS_KC % 2 == 0);
 
-__device__ __forceinline__ float2 ds_split(double x) {
-    const float h = (float)x;
-    return make_float2(h, (float)(x - (double)h));
+// float4 of the operator image holding entries (row, k) and (row, k + 1), k even
+__host__ __device__ constexpr size_t ds_image_at(int code, int row, int k) {
+    return ((size_t)(code * DS_PARTS + row / DS_ROWS) * DS_CHUNKS + k / DS_KC) * DS_A4 + (k % DS_KC / 2) * DS_ROWS +
+           row % DS_ROWS;
+}
+__global__ void k_ds_image(int ncode, const double *__restrict__ ops, float4 *__restrict__ img) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // (code, row, k / 2)
+    if (i >= ncode * NR * NR / 2) return;
+    const int k = i % (NR / 2) * 2, row = i / (NR / 2) % NR, code = i / (NR * NR / 2);
+    const float2 a = ds_split(ops[2 * (size_t)i]), b = ds_split(ops[2 * (size_t)i + 1]);
+    img[ds_image_at(code, row, k)] = make_float4(a.x, a.y, b.x, b.y);
 }
 
-__global__ void __launch_bounds__(160, 2) k_translate_ds(int n_out, int out0, int ncode, const int *__restrict__ tab,
-                                                         const double *__restrict__ ops, const double *in,
-                                                         double *out, int accumulate, int nset, size_t set_stride) {
-    // in and out may be the same array (M2M, L2L): the cells read and written are disjoint.
-    constexpr int RT = 10;
-    extern __shared__ unsigned char smem_raw[];
-    float2 *AT = reinterpret_cast<float2 *>(smem_raw);  // AT[k * NR + row] = Op[row][k]
-    float2 *Bs = AT + NR * NR;                           // [NR][DS_BLD]: column set * DS_TB + cell
-    __shared__ int srcs[DS_TB];
-    const int tid = threadIdx.x, rg = tid / 16, cg = tid % 16;
-    const int c_begin = blockIdx.x * DS_TB;
-    float ah[RT][DS_CT], al[RT][DS_CT];
-#pragma unroll
-    for (int i = 0; i < RT; i++)
-#pragma unroll
-        for (int j = 0; j < DS_CT; j++) ah[i][j] = al[i][j] = 0.f;
-    for (int code = 0; code < ncode; code++) {
-        int sc = -1;
-        if (tid < DS_TB && c_begin + tid < n_out) sc = tab[(size_t)(out0 + c_begin + tid) * ncode + code];
-        if (tid < DS_TB) srcs[tid] = sc;
-        if (!__syncthreads_or(sc >= 0)) continue;
-        for (int e = tid; e < NR * NR; e += blockDim.x) {
-            const int row = e / NR, k = e % NR;
-            AT[k * NR + row] = ds_split(ops[(size_t)code * NR * NR + e]);
-        }
-        for (int e = tid; e < NR * DS_COLS; e += blockDim.x) {
-            const int col = e / NR, k = e % NR, cell = col % DS_TB, set = col / DS_TB;
-            const int src = srcs[cell];
-            Bs[k * DS_BLD + col] = (src >= 0 && set < nset) ? ds_split(in[set * set_stride + (size_t)src * NR + k])
-                                                              : make_float2(0.f, 0.f);
-        }
-        __syncthreads();
-#pragma unroll 2
-        for (int k = 0; k < NR; k++) {
-            float2 a[RT], b[DS_CT];
-#pragma unroll
-            for (int i = 0; i < RT; i++) a[i] = AT[k * NR + rg * RT + i];
-#pragma unroll
-            for (int j = 0; j < DS_CT; j++) b[j] = Bs[k * DS_BLD + cg * DS_CT + j];
-#pragma unroll
-            for (int i = 0; i < RT; i++)
-#pragma unroll
-                for (int j = 0; j < DS_CT; j++) {
-                    // (ah, al) += a b: exact leading product and cross terms, two-sum into hi
-                    const float p = a[i].x * b[j].x;
-                    float e = fmaf(a[i].x, b[j].x, -p);
-                    e = fmaf(a[i].x, b[j].y, e);
-                    e = fmaf(a[i].y, b[j].x, e);
-                    const float s = ah[i][j] + p;
-                    const float bb = s - ah[i][j];
-                    const float err = (ah[i][j] - (s - bb)) + (p - bb);
-                    ah[i][j] = s;
-                    al[i][j] += e + err;
-                }
-        }
-#pragma unroll
-        for (int i = 0; i < RT; i++)
-#pragma unroll
-            for (int j = 0; j < DS_CT; j++) {  // renormalise: |lo| back to half an ulp of hi
-                const float s = ah[i][j] + al[i][j];
-                al[i][j] = al[i][j] - (s - ah[i][j]);
-                ah[i][j] = s;
-            }
-        __syncthreads();
+__device__ __forceinline__ void ds_cp16(void *dst, const void *src, int bytes) {  // the rest of the 16 is zero
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+                 "r"(bytes) : "memory");
+}
+
+__global__ void __launch_bounds__(128, 5) k_translate_ds(const int4 *__restrict__ tiles, const int *__restrict__ cells,
+                                                         const int *__restrict__ codes, int ncode,
+                                                         const int *__restrict__ tab, const float4 *__restrict__ img,
+                                                         const float2 *in, size_t in_stride, double *out,
+                                                         size_t out_stride, float2 *split, size_t split_stride,
+                                                         int nsplit, int accumulate) {
+    // in and split may be the same array (M2M, L2L): the cells read and written are disjoint.
+    __shared__ float4 As[DS_STAGE][DS_A4], Bs[DS_STAGE][DS_TILE][DS_B4];
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    const int4 t = tiles[blockIdx.x / DS_PARTS];  // first cell of the list, codes from and to
+    const int part = blockIdx.x % DS_PARTS, set = blockIdx.y, nch = (t.z - t.y) * DS_CHUNKS;
+    in += set * in_stride;
+    // copies: thread 4 i + j brings 16-byte pieces j, j + 4, j + 8 of cell i; the source cell is
+    // read one code, the code two codes ahead
+    const int cc = tid / 4, cj = tid % 4, ccell = cells[t.x + cc];
+    auto code_at = [&](int q) { return codes[min(q, t.z - 1)]; };
+    auto src_at = [&](int code) { return ccell >= 0 ? tab[(size_t)ccell * ncode + code] : -1; };
+    int iq = t.y, ich = 0, code0 = 0, code1 = 0, code2 = 0, src0 = -1, src1 = -1;
+    if (nch) {
+        code0 = code_at(iq);
+        code1 = code_at(iq + 1);
+        code2 = code_at(iq + 2);
+        src0 = src_at(code0);
+        src1 = src_at(code1);
     }
+    auto issue = [&](int st) {
+        if (iq < t.z) {
+            const float4 *a = img + ((size_t)(code0 * DS_PARTS + part) * DS_CHUNKS + ich) * DS_A4;
+            for (int i = tid; i < DS_A4; i += 128) ds_cp16(&As[st][i], a + i, 16);
+            const float4 *b = reinterpret_cast<const float4 *>(in + (src0 >= 0 ? (size_t)src0 * NR + ich * DS_KC : 0));
 #pragma unroll
-    for (int j = 0; j < DS_CT; j++) {
-        const int col = cg * DS_CT + j, cell = col % DS_TB, set = col / DS_TB;
-        const int c = c_begin + cell;
-        if (c >= n_out || set >= nset) continue;
-        double *o = out + set * set_stride + (size_t)(out0 + c) * NR + rg * RT;
-#pragma unroll
-        for (int i = 0; i < RT; i++) {
-            const double v = (double)ah[i][j] + (double)al[i][j];
-            o[i] = accumulate ? o[i] + v : v;
+            for (int j = cj; j < DS_KC / 2; j += 4) ds_cp16(&Bs[st][cc][j], b + (src0 >= 0 ? j : 0), src0 >= 0 ? 16 : 0);
+            if (++ich == DS_CHUNKS) {
+                ich = 0;
+                iq++;
+                code0 = code1;
+                src0 = src1;
+                code1 = code2;
+                src1 = src_at(code1);
+                code2 = code_at(iq + 2);
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    float ah[DS_RT], al[DS_RT];
+#pragma unroll
+    for (int i = 0; i < DS_RT; i++) ah[i] = al[i] = 0.f;
+    for (int st = 0; st < DS_STAGE - 1; st++) issue(st);
+    int ch = 0;
+    for (int c = 0; c < nch; c++) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(DS_STAGE - 2) : "memory");
+        __syncthreads();  // piece c is there, and every warp is done with piece c - 1
+        issue((c + DS_STAGE - 1) % DS_STAGE);
+        const float4 *A = As[c % DS_STAGE] + warp * DS_RT, *B = Bs[c % DS_STAGE][lane];
+#pragma unroll 5
+        for (int k = 0; k < DS_KC / 2; k++) {
+            const float4 b2 = B[k];
+            float4 a2[DS_RT];
+#pragma unroll
+            for (int i = 0; i < DS_RT; i++) a2[i] = A[k * DS_ROWS + i];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const float bx = h ? b2.z : b2.x, by = h ? b2.w : b2.y;
+#pragma unroll
+                for (int i = 0; i < DS_RT; i++) {
+                    // (ah, al) += a b: exact leading product and cross terms, two-sum into hi
+                    const float ax = h ? a2[i].z : a2[i].x, ay = h ? a2[i].w : a2[i].y;
+                    const float p = __fmul_rn(ax, bx);
+                    float e = fmaf(ax, bx, -p);
+                    e = fmaf(ax, by, e);
+                    e = fmaf(ay, bx, e);
+                    const float s = __fadd_rn(ah[i], p);
+                    const float bb = s - ah[i];
+                    const float err = (ah[i] - (s - bb)) + (p - bb);
+                    ah[i] = s;
+                    al[i] += e + err;
+                }
+            }
+        }
+        if (++ch == DS_CHUNKS) {  // renormalise: |lo| back to half an ulp of hi
+            ch = 0;
+#pragma unroll
+            for (int i = 0; i < DS_RT; i++) {
+                const float s = ah[i] + al[i];
+                al[i] = al[i] - (s - ah[i]);
+                ah[i] = s;
+            }
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    const int cell = cells[t.x + lane];
+    if (cell < 0) return;
+    const size_t row0 = (size_t)cell * NR + part * DS_ROWS + warp * DS_RT;
+#pragma unroll
+    for (int i = 0; i < DS_RT; i++) {
+        double v = (double)ah[i] + (double)al[i];
+        if (out) {
+            double *o = out + set * out_stride + row0 + i;
+            if (accumulate) v = *o + v;
+            *o = v;
+        }
+        if (cell < nsplit) split[set * split_stride + row0 + i] = ds_split(v);
     }
 }
 
@@ -1414,142 +1480,113 @@ __global__ void __launch_bounds__(128, 4) k_p2p_ds(const int4 *__restrict__ task
     }
 }
 
-// L2P + P2P in double-single arithmetic of the full FP64 evaluation of the FP32 + refinement path
-// (FmmTree::repeat). Coordinates are leaf-local with
-// hi parts on a 2^-20 grid (|x| < 4, so hi - hi' is exact in FP32) and lo = x - hi
-// (|lo| <= 2^-21, held to 2^-45); per pair: dx = (hi - hi') + (lo - lo'), r^2 as a
-// double-single sum of the squares (the leading products exact through fma), 1/r from the
-// SFU estimate and one Newton step evaluated in double-single (error ~1e-13), q/r as a
-// double-single product, summed with two-sum. One warp per target leaf, 8 targets per
-// lane pass, sources spread over the lanes; per-lane sums reduced over the warp in FP64.
-// NQ charge sets share the pair geometry and 1/r (the second set's charge hi/lo in q2h/q2l).
-template <int NQ>
-__global__ void __launch_bounds__(128) k_l2p_p2p_ds(int nleaf, const int *__restrict__ leaf_src,
-                                                    const int *__restrict__ leaf_tgt,
-                                                    const int *__restrict__ tgt_node,
-                                                    const double *__restrict__ tloc,
-                                                    const float4 *__restrict__ th4, const float4 *__restrict__ tl4,
-                                                    const float4 *__restrict__ sh4, const float4 *__restrict__ sl4,
-                                                    const float *__restrict__ q2h, const float *__restrict__ q2l,
-                                                    const int *__restrict__ leaf_ijk, int leaf0,
-                                                    const double *__restrict__ leaf_scale,
-                                                    const int *__restrict__ near_ptr,
-                                                    const int *__restrict__ near_leaf, NearSets<double> sets) {
-    constexpr int NT = 8;
-    const int lane = threadIdx.x & 31;
-    const int leaf = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (leaf >= nleaf) return;
-    const int t0 = leaf_tgt[leaf], t1 = leaf_tgt[leaf + 1];
-    if (t0 == t1) return;
+// P2P in double-single arithmetic of the full FP64 evaluation of the FP32 + refinement path
+// (FmmTree::repeat): the operations of k_p2p_ds but for 1/r (one Newton step evaluated in
+// double-single, error ~1e-13) and the order of the sums: sources of each adjacent leaf spread over
+// the lanes of one warp, per-lane sums reduced over the warp in FP64. A warp takes a task of up to 8
+// targets of a leaf, the leaf's targets shared out evenly (a warp per leaf, in passes of 8 targets
+// whatever was left, with the local expansions behind them, gave each SM a dozen unequal warps;
+// 294k tets, two sets: 4.85 -> 2.23 ms and 0.09 for the local expansions, FMA pipe 76%).
+template <int NT, int NQ>
+__device__ __forceinline__ void p2p_repeat_pass(int lane, int leaf, int tb, const int *__restrict__ leaf_src,
+                                                const int *__restrict__ tgt_node, const float4 *__restrict__ th4,
+                                                const float4 *__restrict__ tl4, const float4 *__restrict__ sh4,
+                                                const float4 *__restrict__ sl4, const float *__restrict__ q2h,
+                                                const float *__restrict__ q2l, const int *__restrict__ leaf_ijk,
+                                                const int *__restrict__ near_ptr, const int *__restrict__ near_leaf,
+                                                double *__restrict__ pot0, double *__restrict__ pot1) {
     const int li = leaf_ijk[3 * leaf], lj = leaf_ijk[3 * leaf + 1], lk = leaf_ijk[3 * leaf + 2];
-    const size_t fbase = (size_t)(leaf0 + leaf) * NR;
-    for (int tb = t0; tb < t1; tb += NT) {
-        const int nt = min(NT, t1 - tb);
-        float thx[NT], thy[NT], thz[NT], tlx[NT], tly[NT], tlz[NT], ah[NQ][NT], al[NQ][NT];
+    float thx[NT], thy[NT], thz[NT], tlx[NT], tly[NT], tlz[NT], ah[NQ][NT], al[NQ][NT];
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            const int ti = tb + (j < nt ? j : 0);
-            const float4 h = th4[ti], l = tl4[ti];
-            thx[j] = h.x; thy[j] = h.y; thz[j] = h.z;
-            tlx[j] = l.x; tly[j] = l.y; tlz[j] = l.z;
+    for (int j = 0; j < NT; j++) {
+        const float4 h = th4[tb + j], l = tl4[tb + j];
+        thx[j] = h.x; thy[j] = h.y; thz[j] = h.z;
+        tlx[j] = l.x; tly[j] = l.y; tlz[j] = l.z;
 #pragma unroll
-            for (int k = 0; k < NQ; k++) ah[k][j] = al[k][j] = 0.f;
-        }
-        for (int e = near_ptr[leaf]; e < near_ptr[leaf + 1]; e++) {
-            const int nl = near_leaf[e];
-            // integer offset of the adjacent leaf, added exactly to the hi parts
-            const float ox = float(leaf_ijk[3 * nl] - li), oy = float(leaf_ijk[3 * nl + 1] - lj),
-                        oz = float(leaf_ijk[3 * nl + 2] - lk);
-            const int s0 = leaf_src[nl], s1 = leaf_src[nl + 1];
-            for (int s = s0 + lane; s < s1; s += 32) {
-                const float4 h = sh4[s], l = sl4[s];
-                const float sx = h.x + ox, sy = h.y + oy, sz = h.z + oz;
-                float qh[NQ], ql[NQ];
-                qh[0] = h.w;
-                ql[0] = l.w;
-                if constexpr (NQ == 2) {
-                    qh[1] = q2h[s];
-                    ql[1] = q2l[s];
-                }
-#pragma unroll
-                for (int j = 0; j < NT; j++) {
-                    const float d1x = thx[j] - sx, d1y = thy[j] - sy, d1z = thz[j] - sz;  // exact
-                    const float d2x = tlx[j] - l.x, d2y = tly[j] - l.y, d2z = tlz[j] - l.z;
-                    // squares: d^2 = d1^2 + d2 (2 d1 + d2), leading products exact
-                    const float px = d1x * d1x, py = d1y * d1y, pz = d1z * d1z;
-                    float ex = fmaf(d1x, d1x, -px), ey = fmaf(d1y, d1y, -py), ez = fmaf(d1z, d1z, -pz);
-                    ex = fmaf(d2x, 2.f * d1x + d2x, ex);
-                    ey = fmaf(d2y, 2.f * d1y + d2y, ey);
-                    ez = fmaf(d2z, 2.f * d1z + d2z, ez);
-                    float s1_, e1, s2_, e2;
-                    ds_two_sum(px, py, s1_, e1);
-                    ds_two_sum(s1_, pz, s2_, e2);
-                    const float el = (e1 + e2) + (ex + ey + ez);
-                    const float Sh = s2_ + el, Sl = el - (Sh - s2_);
-                    // 1/sqrt(S): SFU estimate y, then y (1 + (1 - S y^2) / 2) with S y^2 in
-                    // double-single (1 - S y^2 is small and exact to ~2^-46)
-                    float y;
-                    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(Sh));
-                    const float t1_ = y * y, t2_ = fmaf(y, y, -t1_);
-                    const float u1 = Sh * t1_;
-                    const float u2 = fmaf(Sh, t1_, -u1) + fmaf(Sh, t2_, Sl * t1_);
-                    const float delta = (1.f - u1) - u2;
-                    const float yl = 0.5f * y * delta;
-                    // q / r = (qh + ql)(y + yl), accumulated with two-sum
-#pragma unroll
-                    for (int k = 0; k < NQ; k++) {
-                        const float c1 = qh[k] * y;
-                        const float c2 = fmaf(qh[k], y, -c1) + fmaf(qh[k], yl, ql[k] * y);
-                        float sn, en;
-                        ds_two_sum(ah[k][j], c1, sn, en);
-                        ah[k][j] = sn;
-                        al[k][j] += en + c2;
-                    }
-                }
+        for (int k = 0; k < NQ; k++) ah[k][j] = al[k][j] = 0.f;
+    }
+    for (int e = near_ptr[leaf]; e < near_ptr[leaf + 1]; e++) {
+        const int nl = near_leaf[e];
+        // integer offset of the adjacent leaf, added exactly to the hi parts
+        const float ox = float(leaf_ijk[3 * nl] - li), oy = float(leaf_ijk[3 * nl + 1] - lj),
+                    oz = float(leaf_ijk[3 * nl + 2] - lk);
+        const int s0 = leaf_src[nl], s1 = leaf_src[nl + 1];
+        for (int s = s0 + lane; s < s1; s += 32) {
+            const float4 h = sh4[s], l = sl4[s];
+            const float sx = h.x + ox, sy = h.y + oy, sz = h.z + oz;
+            float qh[NQ], ql[NQ];
+            qh[0] = h.w;
+            ql[0] = l.w;
+            if constexpr (NQ == 2) {
+                qh[1] = q2h[s];
+                ql[1] = q2l[s];
             }
-        }
-        double near[NQ][NT];
-#pragma unroll
-        for (int k = 0; k < NQ; k++)
 #pragma unroll
             for (int j = 0; j < NT; j++) {
-                near[k][j] = double(ah[k][j]) + double(al[k][j]);
-                for (int o = 16; o > 0; o >>= 1) near[k][j] += __shfl_xor_sync(0xffffffffu, near[k][j], o);
-            }
-        // L2P in FP64: lane j evaluates target j
-        if (lane < nt) {
-            double nr[NQ];
+                const float d1x = thx[j] - sx, d1y = thy[j] - sy, d1z = thz[j] - sz;  // exact
+                const float d2x = tlx[j] - l.x, d2y = tly[j] - l.y, d2z = tlz[j] - l.z;
+                // squares: d^2 = d1^2 + d2 (2 d1 + d2), leading products exact
+                const float px = d1x * d1x, py = d1y * d1y, pz = d1z * d1z;
+                float ex = fmaf(d1x, d1x, -px), ey = fmaf(d1y, d1y, -py), ez = fmaf(d1z, d1z, -pz);
+                ex = fmaf(d2x, 2.f * d1x + d2x, ex);
+                ey = fmaf(d2y, 2.f * d1y + d2y, ey);
+                ez = fmaf(d2z, 2.f * d1z + d2z, ez);
+                float s1_, e1, s2_, e2;
+                ds_two_sum(px, py, s1_, e1);
+                ds_two_sum(s1_, pz, s2_, e2);
+                const float el = (e1 + e2) + (ex + ey + ez);
+                const float Sh = s2_ + el, Sl = el - (Sh - s2_);
+                // 1/sqrt(S): SFU estimate y, then y (1 + (1 - S y^2) / 2) with S y^2 in
+                // double-single (1 - S y^2 is small and exact to ~2^-46)
+                float y;
+                asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(Sh));
+                const float t1_ = y * y, t2_ = fmaf(y, y, -t1_);
+                const float u1 = Sh * t1_;
+                const float u2 = fmaf(Sh, t1_, -u1) + fmaf(Sh, t2_, Sl * t1_);
+                const float delta = (1.f - u1) - u2;
+                const float yl = 0.5f * y * delta;
+                // q / r = (qh + ql)(y + yl), accumulated with two-sum
 #pragma unroll
-            for (int k = 0; k < NQ; k++) nr[k] = 0;
-#pragma unroll
-            for (int j = 0; j < NT; j++)
-                if (j == lane)
-#pragma unroll
-                    for (int k = 0; k < NQ; k++) nr[k] = near[k][j];
-            const int ti = tb + lane;
-            if (sets.near_only) {
-#pragma unroll
-                for (int k = 0; k < NQ; k++) sets.pot[k][tgt_node[ti]] = nr[k];
-                continue;
-            }
-            const double x = tloc[4 * (size_t)ti], y = tloc[4 * (size_t)ti + 1], z = tloc[4 * (size_t)ti + 2];
-            const double *__restrict__ Fa = sets.F[0] + fbase;
-            const double *__restrict__ Fb = sets.F[NQ - 1] + fbase;
-            double fa = 0, fb = 0;
-            ups_cols<double>(x, y, z, [&](int n, int m, double re, double im) {
-                if (m == 0) {
-                    fa += Fa[ridx(n, 0, 0)] * re;
-                    if constexpr (NQ == 2) fb += Fb[ridx(n, 0, 0)] * re;
-                } else {
-                    fa += 2.0 * (Fa[ridx(n, m, 0)] * re + Fa[ridx(n, m, 1)] * im);
-                    if constexpr (NQ == 2) fb += 2.0 * (Fb[ridx(n, m, 0)] * re + Fb[ridx(n, m, 1)] * im);
+                for (int k = 0; k < NQ; k++) {
+                    const float c1 = qh[k] * y;
+                    const float c2 = fmaf(qh[k], y, -c1) + fmaf(qh[k], yl, ql[k] * y);
+                    float sn, en;
+                    ds_two_sum(ah[k][j], c1, sn, en);
+                    ah[k][j] = sn;
+                    al[k][j] += en + c2;
                 }
-            });
-            const double sc = leaf_scale[leaf];
-            sets.pot[0][tgt_node[ti]] = (fa + nr[0]) * sc;
-            if constexpr (NQ == 2) sets.pot[1][tgt_node[ti]] = (fb + nr[NQ - 1]) * sc;
+            }
         }
     }
+#pragma unroll
+    for (int k = 0; k < NQ; k++)
+#pragma unroll
+        for (int j = 0; j < NT; j++) {
+            double v = double(ah[k][j]) + double(al[k][j]);
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == j) (k ? pot1 : pot0)[tgt_node[tb + j]] = v;
+        }
+}
+
+template <int NQ>
+__global__ void __launch_bounds__(128, 4)
+    k_p2p_ds_repeat(int ntask, const int4 *__restrict__ task, const int *__restrict__ leaf_src,
+                    const int *__restrict__ tgt_node, const float4 *__restrict__ th4, const float4 *__restrict__ tl4,
+                    const float4 *__restrict__ sh4, const float4 *__restrict__ sl4, const float *__restrict__ q2h,
+                    const float *__restrict__ q2l, const int *__restrict__ leaf_ijk, const int *__restrict__ near_ptr,
+                    const int *__restrict__ near_leaf, double *__restrict__ pot0, double *__restrict__ pot1) {
+    const int lane = threadIdx.x & 31, w = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (w >= ntask) return;
+    const int4 t = task[w];
+#define FG_P2P(N)                                                                                                   \
+    case N:                                                                                                         \
+        p2p_repeat_pass<N, NQ>(lane, t.x, t.y, leaf_src, tgt_node, th4, tl4, sh4, sl4, q2h, q2l, leaf_ijk, near_ptr, \
+                               near_leaf, pot0, pot1);                                                              \
+        break;
+    switch (t.z) {
+        FG_P2P(1) FG_P2P(2) FG_P2P(3) FG_P2P(4) FG_P2P(5) FG_P2P(6) FG_P2P(7) FG_P2P(8)
+    }
+#undef FG_P2P
 }
 
 // L2P after a near field that stored its sums: one thread per target evaluates its leaf's local
@@ -2166,7 +2203,8 @@ static int fmm_build_forest(Ctx &c, int L) {
     t->ds = !fp32 && c.opts.fmm_native_fp64 == 0;
     t->repeat = t->ds && c.opts.precision == FG_PREC_FP32_REFINE;
     t->oz = t->ds && !t->repeat;
-    if (t->oz) {
+    if (t->ds) {
+        const int tile = t->oz ? OZ_TILE : DS_TILE;
         std::vector<int> cells, codes;
         std::vector<int4> units;
         std::vector<int2> fin;
@@ -2174,16 +2212,16 @@ static int fmm_build_forest(Ctx &c, int L) {
         struct Tile { std::vector<int> cells, codes; };
         auto tiles_of = [&](const std::vector<int> &list, int ncode, const std::vector<int> &tab) {
             std::vector<Tile> T;
-            for (size_t b = 0; b < list.size(); b += OZ_TILE) {
+            for (size_t b = 0; b < list.size(); b += tile) {
                 Tile x;
-                x.cells.assign(list.begin() + b, list.begin() + std::min(list.size(), b + OZ_TILE));
+                x.cells.assign(list.begin() + b, list.begin() + std::min(list.size(), b + tile));
                 for (int code = 0; code < ncode; code++)
                     for (int cc : x.cells)
                         if (tab[(size_t)cc * ncode + code] >= 0) {
                             x.codes.push_back(code);
                             break;
                         }
-                x.cells.resize(OZ_TILE, -1);
+                x.cells.resize(tile, -1);
                 T.push_back(std::move(x));
             }
             return T;
@@ -2209,7 +2247,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         };
         // units of at most mc codes: the size among the candidates whose units, handed in order to
         // the earliest free SM, finish first (a unit costs its codes plus about 2)
-        auto plan = [&](const std::vector<Tile> &T) {
+        auto plan_oz = [&](const std::vector<Tile> &T) {
             int mc = 64;
             double best = 1e300;
             for (int k : {64, 48, 32, 24, 16, 12, 8, 6, 4, 3, 2, 1}) {
@@ -2249,13 +2287,28 @@ static int fmm_build_forest(Ctx &c, int L) {
             nslot = std::max(nslot, slot);
             return l;
         };
+        // double-single: one unit per tile (a sum's codes stay in order), the longest first
+        auto plan_ds = [&](std::vector<Tile> T) {
+            std::stable_sort(T.begin(), T.end(), [](const Tile &x, const Tile &y) { return x.codes.size() > y.codes.size(); });
+            FmmTree::OzLaunch l;
+            l.unit0 = (int)units.size();
+            l.nunit = l.ntile = (int)T.size();
+            for (const Tile &x : T) {
+                const int first = (int)codes.size();
+                units.push_back(make_int4((int)cells.size(), first, first + (int)x.codes.size(), 0));
+                codes.insert(codes.end(), x.codes.begin(), x.codes.end());
+                cells.insert(cells.end(), x.cells.begin(), x.cells.end());
+            }
+            return l;
+        };
+        auto plan = [&](const std::vector<Tile> &T) { return t->oz ? plan_oz(T) : plan_ds(T); };
         t->oz_m2m.assign(L + 1, FmmTree::OzLaunch());
         t->oz_l2l.assign(L + 1, FmmTree::OzLaunch());
         for (int l = L - 1; l >= 2; l--) t->oz_m2m[l] = plan(level_tiles(l, 8, m2m_tab));
         std::vector<Tile> all;
         int nsplit = 0;  // listed cells above the leaves: their locals are translated further
         for (int l = 2; l <= L; l++) {
-            if (l == L) nsplit = OZ_TILE * (int)all.size();
+            if (l == L) nsplit = tile * (int)all.size();
             for (auto &x : level_tiles(l, NCODE_M2L, m2l_tab)) all.push_back(std::move(x));
         }
         const size_t codes0 = codes.size();
@@ -2265,27 +2318,42 @@ static int fmm_build_forest(Ctx &c, int L) {
                     t->oz_m2l.ntile, t->oz_m2l.nunit);
         t->oz_m2l.nsplit = nsplit;
         for (int l = 3; l <= L; l++) t->oz_l2l[l] = plan(level_tiles(l, 8, l2l_tab));
-        std::vector<int> wexp(2 * NR), leaves(nleaf);
-        oz_weights(wexp.data(), wexp.data() + NR);
-        for (int k = 0; k < nleaf; k++) leaves[k] = t->leaf0 + k;
-        static const OzImages im[3] = {oz_images(ops.m2m, 8, wexp.data()), oz_images(ops.m2l, NCODE_M2L, wexp.data()),
-                                       oz_images(ops.l2l, 8, wexp.data() + NR)};
-        for (int k = 0; k < 3; k++) {
-            FCK(up(&t->oz_img[k], im[k].img));
-            FCK(up(&t->oz_rows[k], im[k].row_scale));
-        }
         FCK(up(&t->oz_cells, cells));
         FCK(up(&t->oz_codes, codes));
         FCK(up(&t->oz_units, units));
-        FCK(up(&t->oz_fin, fin));
-        FCK(up(&t->oz_wexp, wexp));
-        FCK(up(&t->oz_leaves, leaves));
-        FCK(cudaMalloc(&t->oz_scratch, sizeof(double) * std::max(1, nslot) * OZ_TILE * NR * t->nq));
-        FCK(cudaMalloc(&t->oz_digits, (size_t)ncell * t->nq * OZ_CELL_BYTES));
-        FCK(cudaMemset(t->oz_digits, 0, (size_t)ncell * t->nq * OZ_CELL_BYTES));
-        FCK(cudaMalloc(&t->oz_scale, sizeof(float) * ncell * t->nq));
-        FCK(cudaMemset(t->oz_scale, 0, sizeof(float) * ncell * t->nq));
-        FCK(oz_setup());
+        if (t->oz) {
+            std::vector<int> wexp(2 * NR), leaves(nleaf);
+            oz_weights(wexp.data(), wexp.data() + NR);
+            for (int k = 0; k < nleaf; k++) leaves[k] = t->leaf0 + k;
+            static const OzImages im[3] = {oz_images(ops.m2m, 8, wexp.data()), oz_images(ops.m2l, NCODE_M2L, wexp.data()),
+                                           oz_images(ops.l2l, 8, wexp.data() + NR)};
+            for (int k = 0; k < 3; k++) {
+                FCK(up(&t->oz_img[k], im[k].img));
+                FCK(up(&t->oz_rows[k], im[k].row_scale));
+            }
+            FCK(up(&t->oz_fin, fin));
+            FCK(up(&t->oz_wexp, wexp));
+            FCK(up(&t->oz_leaves, leaves));
+            FCK(cudaMalloc(&t->oz_scratch, sizeof(double) * std::max(1, nslot) * OZ_TILE * NR * t->nq));
+            FCK(cudaMalloc(&t->oz_digits, (size_t)ncell * t->nq * OZ_CELL_BYTES));
+            FCK(cudaMemset(t->oz_digits, 0, (size_t)ncell * t->nq * OZ_CELL_BYTES));
+            FCK(cudaMalloc(&t->oz_scale, sizeof(float) * ncell * t->nq));
+            FCK(cudaMemset(t->oz_scale, 0, sizeof(float) * ncell * t->nq));
+            FCK(oz_setup());
+        } else {
+            const std::vector<double> *op[3] = {&ops.m2m, &ops.m2l, &ops.l2l};
+            for (int k = 0; k < 3; k++) {
+                const int n = k == 1 ? NCODE_M2L : 8;
+                double *d = nullptr;
+                FCK(cudaMalloc(&t->oz_img[k], (size_t)n * NR * NR * sizeof(float2)));
+                FCK(up(&d, *op[k]));
+                k_ds_image<<<(n * NR * NR / 2 + 255) / 256, 256, 0, c.stream>>>(n, d, (float4 *)t->oz_img[k]);
+                const cudaError_t e = cudaStreamSynchronize(c.stream);
+                cudaFree(d);
+                FCK(e);
+            }
+            FCK(cudaMalloc(&t->F_split, sizeof(float2) * std::max(1, t->leaf0) * NR * t->nq));
+        }
     }
     FCK(up(&t->leaf_src, leaf_src));
     FCK(up(&t->leaf_tgt, leaf_tgt));
@@ -2359,7 +2427,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(up(&t->ds_tgt_hi, th));
         FCK(up(&t->ds_tgt_lo, tl));
     }
-    if (!t->oz) {
+    if (!t->ds) {
         FCK(up_as<double>(&t->op_m2l, ops.m2l, fp32));
         FCK(up_as<double>(&t->op_m2m, ops.m2m, fp32));
         FCK(up_as<double>(&t->op_l2l, ops.l2l, fp32));
@@ -2405,7 +2473,6 @@ static int fmm_build_forest(Ctx &c, int L) {
         FCK(cudaFuncSetAttribute(k_translate<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<float>()));
     } else {
         FCK(cudaFuncSetAttribute(k_translate<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_smem<double>()));
-        FCK(cudaFuncSetAttribute(k_translate_ds, cudaFuncAttributeMaxDynamicSharedMemorySize, tr_ds_smem()));
     }
     if (c.opts.profile)
         for (auto &set : t->ev)
@@ -2429,7 +2496,7 @@ void fmm_free(Ctx &c) {
                     t->img_m2l, t->img_m2m, t->img_l2l, t->ds_src_hi, t->ds_src_lo, t->ds_tgt_hi, t->ds_tgt_lo,
                     t->sq2, t->ds_q2, t->p2p_task, t->oz_cells, t->oz_codes, t->oz_wexp, t->oz_leaves, t->oz_units, t->oz_fin,
                     t->oz_scratch, t->oz_digits, t->oz_scale, t->oz_img[0], t->oz_img[1], t->oz_img[2], t->oz_rows[0],
-                    t->oz_rows[1], t->oz_rows[2]};
+                    t->oz_rows[1], t->oz_rows[2], t->F_split};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     near_free(t->near);
@@ -2523,11 +2590,11 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
         }
         if constexpr (sizeof(T) == 8) {
             if (t.repeat) {
-                auto k = nq == 2 ? k_l2p_p2p_ds<2> : k_l2p_p2p_ds<1>;
-                k<<<nb, 128, 0, st>>>(t.nleaf, t.leaf_src, t.leaf_tgt, t.tgt_node, (const double *)t.tloc, t.ds_tgt_hi,
-                                      t.ds_tgt_lo, t.ds_src_hi, t.ds_src_lo, t.ds_q2,
-                                      t.ds_q2 ? t.ds_q2 + t.nsrc : nullptr, t.leaf_ijk, t.leaf0, t.leaf_scale,
-                                      t.near_ptr, t.near_leaf, ns);
+                if (t.n_p2p_task > 0)
+                    (nq == 2 ? k_p2p_ds_repeat<2> : k_p2p_ds_repeat<1>)<<<(t.n_p2p_task + 3) / 4, 128, 0, st>>>(
+                        t.n_p2p_task, t.p2p_task, t.leaf_src, t.tgt_node, t.ds_tgt_hi, t.ds_tgt_lo, t.ds_src_hi,
+                        t.ds_src_lo, t.ds_q2, t.ds_q2 ? t.ds_q2 + t.nsrc : nullptr, t.leaf_ijk, t.near_ptr,
+                        t.near_leaf, ns.pot[0], ns.pot[1]);
             } else if (t.ds && t.n_p2p_task > 0)
                 (nq == 2 ? k_p2p_ds<2> : k_p2p_ds<1>)<<<t.n_p2p_task, 128, 0, st>>>(
                     t.p2p_task, t.leaf_src, t.tgt_node, t.ds_tgt_hi, t.ds_tgt_lo, t.ds_src_hi, t.ds_src_lo, t.ds_q2,
@@ -2556,7 +2623,7 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
         (nq == 2 ? k_p2m_ds<2> : k_p2m_ds<1>)<<<dim3((t.nleaf + 3) / 4, 5), 128, 0, c.stream>>>(
             t.nleaf, t.leaf_src, (const float4 *)t.ds_src_hi, (const float4 *)t.ds_src_lo, t.leaf0, ps[0], ps[1]);
     } else if (t.ds) {
-        (nq == 2 ? k_p2m_ds_repeat<2> : k_p2m_ds_repeat<1>)<<<(t.nleaf + 3) / 4, 128, 0, c.stream>>>(
+        (nq == 2 ? k_p2m_ds_repeat<2> : k_p2m_ds_repeat<1>)<<<dim3((t.nleaf + 3) / 4, 6), 128, 0, c.stream>>>(
             t.nleaf, t.leaf_src, (const float4 *)t.ds_src_hi, (const float4 *)t.ds_src_lo, t.leaf0, ps[0], ps[1]);
     } else {
         k_p2m<T><<<dim3((t.nleaf + 3) / 4, nq), 128, 0, c.stream>>>(t.nleaf, t.leaf_src, (const T *)t.sloc, t.leaf0,
@@ -2586,11 +2653,6 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
             a.nset = nq; a.set_io = sstride; a.set_scratch = t.nslot_floats;
             const cudaError_t e = launch_translate_tc(c.stream, a);
             if (e != cudaSuccess && terr == cudaSuccess) terr = e;
-        } else if (sizeof(T) == 8 && t.ds) {  // double-single, both sets per launch
-            const double *ops = (const double *)(kind == M2M ? t.op_m2m : kind == M2L ? t.op_m2l : t.op_l2l);
-            double *in = (double *)(kind == L2L ? F : M), *out = (double *)(kind == M2M ? M : F);
-            k_translate_ds<<<(n + DS_TB - 1) / DS_TB, 160, tr_ds_smem(), c.stream>>>(n, out0, ncode, tab, ops, in, out,
-                                                                                     kind == L2L, nq, sstride);
         } else {
             const void *ops = kind == M2M ? t.op_m2m : kind == M2L ? t.op_m2l : t.op_l2l;
             for (int q = 0; q < nq; q++) {
@@ -2624,9 +2686,21 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
         fa.accumulate = kind == L2L; fa.split = nsplit; fa.wexp = t.oz_wexp + (kind == M2M ? 0 : NR);
         note(launch_oz_finish(c.stream, fa));
     };
+    // FP32 + refinement path's FP64 tree: double-single; M and the locals above the leaves as pairs
+    auto translate_ds = [&](int kind, const FmmTree::OzLaunch &ol) {
+        if (!ol.ntile) return;
+        const size_t fstride = (size_t)t.leaf0 * NR;
+        float2 *Ms = (float2 *)M, *Fs = (float2 *)t.F_split;
+        k_translate_ds<<<dim3(ol.nunit * DS_PARTS, nq), 128, 0, c.stream>>>(
+            t.oz_units + ol.unit0, t.oz_cells, t.oz_codes, kind == M2L ? NCODE_M2L : 8,
+            kind == M2M ? t.m2m_tab : kind == M2L ? t.m2l_tab : t.l2l_tab, (const float4 *)t.oz_img[kind],
+            kind == L2L ? Fs : Ms, kind == L2L ? fstride : sstride, kind == M2M ? nullptr : (double *)F, sstride,
+            kind == M2M ? Ms : Fs, kind == M2M ? sstride : fstride, t.leaf0, kind == L2L);
+    };
     const FmmTree::TcLaunch none;
     for (int l = L - 1; l >= 2; l--)
-        if (t.oz) translate_oz(M2M, t.oz_m2m[l], t.oz_m2m[l].ntile * OZ_TILE);
+        if (t.repeat) translate_ds(M2M, t.oz_m2m[l]);
+        else if (t.oz) translate_oz(M2M, t.oz_m2m[l], t.oz_m2m[l].ntile * OZ_TILE);
         else translate(M2M, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_m2m[l] : none);
     if (prof) cudaEventRecord(ev[2], c.stream);
     if (split) {  // the near field beside M2L and L2L
@@ -2639,14 +2713,16 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
         cudaEventRecord(c.ev_join, c.stream2);
         ns.near_only = 0;
     }
-    if (t.oz) translate_oz(M2L, t.oz_m2l, t.oz_m2l.nsplit);
+    if (t.repeat) translate_ds(M2L, t.oz_m2l);
+    else if (t.oz) translate_oz(M2L, t.oz_m2l, t.oz_m2l.nsplit);
     else translate(M2L, t.ncell, 0, t.tc_m2l);
     if (prof) cudaEventRecord(ev[3], c.stream);
     for (int l = 3; l <= L; l++)
-        if (t.oz) translate_oz(L2L, t.oz_l2l[l], l < L ? t.oz_l2l[l].ntile * OZ_TILE : 0);
+        if (t.repeat) translate_ds(L2L, t.oz_l2l[l]);
+        else if (t.oz) translate_oz(L2L, t.oz_l2l[l], l < L ? t.oz_l2l[l].ntile * OZ_TILE : 0);
         else translate(L2L, t.lev_begin[l + 1] - t.lev_begin[l], t.lev_begin[l], t.tc ? t.tc_l2l[l] : none);
     if (prof) cudaEventRecord(ev[4], c.stream);
-    if (split || t.oz) {  // L2P apart: the double-single near field stores its sums
+    if (split || t.ds) {  // L2P apart: the double-single near field stores its sums
         if (split) cudaStreamWaitEvent(c.stream, c.ev_join, 0);
         else near_field(c.stream);
         if (whole) {
@@ -2737,7 +2813,7 @@ int fmm_launches_per_eval(const Ctx &c, int nq) {
     const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
     if (!t) return 0;
     int n = 2;  // P2M, L2P + P2P (both sets in one launch each)
-    if ((c.opts.fmm_overlap != 0 && c.stream2) || t->oz) n += 1;  // L2P apart from the near field
+    if ((c.opts.fmm_overlap != 0 && c.stream2) || t->ds) n += 1;  // L2P apart from the near field
     if (t->near.near.B) n += 1;  // the fields as pairs
     if (t->oz) {  // digits of the leaves, then per translation the products and the sums
         n += 1;

@@ -40,6 +40,27 @@ def test_fp64_fmm_edges(shape, leaf):
     assert _rel(pot[0][0], pot[0][2]) < 1e-14 and _rel(pot[0][1], pot[0][3]) < 1e-14
 
 
+# the FP64 tree of the FP32 + refinement path: one level; tiles of 32 cells that are full, ragged or
+# one cell; near-field tasks of 1 to 8 targets; 64 leaves of each octant; few blocks of P2M
+@pytest.mark.parametrize("shape,leaf", [((1, 1, 1), -2), ((3, 3, 3), -2), ((8, 8, 8), -3), ((30, 26, 1), -5),
+                                        ((2, 3, 60), -6), ((15, 14, 13), -2), ((11, 7, 5), -4)])
+@pytest.mark.parametrize("overlap", [0, 1])
+def test_refinement_fp64_tree_edges(shape, leaf, overlap):
+    m = cases.cuboid(*shape)
+    u = cases.perturbed_state(m["xyz"], seed=23, sigma=0.3)
+    v = cases.tangent_field(u, seed=24)
+    pot = []
+    for o in (dict(precision=fg.FG_PREC_FP32_REFINE, fmm_overlap=overlap), dict(fmm_native_fp64=1)):
+        c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=leaf, **o)
+        c.set_state(u, v)
+        c.compute_all(np.zeros(3))
+        s = c.get_state(0)
+        pot.append((s["phi"], s["phiv"]))
+    # 1/r to 1e-13 and sums to 2^-44 of the summed magnitudes, which cancel by up to one order of
+    # magnitude for the magnetisation and two for a random tangent field
+    assert _rel(pot[0][0], pot[1][0]) < 1e-12 and _rel(pot[0][1], pot[1][1]) < 1e-11
+
+
 def test_fp64_forest_matches_single_trees():
     meshes = [cases.cuboid(*s) for s in ((9, 9, 9), (4, 6, 5), (12, 3, 2), (2, 2, 2))]
     us = [cases.perturbed_state(m["xyz"], seed=30 + k, sigma=0.3) for k, m in enumerate(meshes)]
