@@ -17,30 +17,36 @@
 // translation.
 //
 // Pipeline (one CTA of 9 warps per tile, one CTA per SM, 6 shared-memory stages of K = 16):
-//   warps 0-3  fill one stage per item: thread 0 starts two bulk copies
+//   warps 0-3  fill one stage per item: one lane, of each warp in turn, starts two bulk copies
 //              (cp.async.bulk, completion counted in bytes on bfull[s]) of the operator
 //              item, stored pre-split (hi, lo) in global memory in exactly the shared-memory
 //              image the MMA reads (no-swizzle K-major core matrices, 8 rows x 16 bytes);
 //              all 128 threads gather the 64 ns input expansions' item with 16-byte cp.async
 //              from pre-split hi/lo arrays into the same layout (zero fill where a cell has
-//              no input). A thread arrives on full[s] once its copies for that item have
-//              landed, LAG items later and before it waits for the next free stage, so
-//              LAG items per CTA are in flight and the MMAs of an item never wait for those
-//              of the item before it to complete;
-//   warp 4     one lane waits full[s] and bfull[s], issues the MMAs of each K-step of 8 and
+//              no input), and leave an arrival on full[s] that takes effect once their copies
+//              have landed (cp.async.mbarrier.arrive), so they go on to the next free stage at
+//              once;
+//   warp 4     waits full[s] and bfull[s] as a whole (warp-uniform code keeps descriptors in uniform
+//              registers), orders the gathered pieces before the tensor core's reads
+//              (fence.proxy.async); one elected lane issues the MMAs of each K-step of 8, and
 //              tcgen05.commit arrives on empty[s] when they have read the stage; each code
 //              accumulates into its own TMEM buffer (two, used in turn), committed to tfull;
 //   warps 5-8  drain a finished code buffer with tcgen05.ld (warp w owns TMEM lanes
 //              32(w%4)..+31 = coefficient rows), add it to FP32 registers with round to
 //              nearest, release it (tfree), and finally store (or add to) the outputs and
 //              their hi/lo split for the next translation.
+// An item costs about 750 clocks (its MMAs 320, its shared-memory traffic about 600): each stage goes
+// around a ring of hand-overs of some 1,500. Producers that waited for their copies and arrived
+// for them three items later left two of the six stages to cover it: 1,100 clocks (M2L of the
+// 1.2M-tet film 0.455 -> 0.387 ms, of the 3.8M-tet platelet 1.64 -> 1.36, of 24 samples of 13k tets
+// each 250 -> 188 us).
 // The tensor core's FP32 accumulation rounds toward zero, so an accumulator summed over
 // all codes in place drifts by about 2.4e-7 per 13 K-steps (measured); one accumulator per
 // code and per term group keeps the translation at FP32 rounding level.
 // Every wait on an mbarrier is bounded (about 1 s): on expiry the CTA records FG_ETIMEDOUT
 // in *err and stops issuing work; before it frees its TMEM and returns, the issuer waits
-// (bounded) for the MMAs it started (tcgen05.commit on tdone) and thread 0 for the bytes of
-// the bulk copies it started (bfull), so no asynchronous write is left in flight.
+// (bounded) for the MMAs it started (tcgen05.commit on tdone) and each producer warp for the bytes
+// of the bulk copies it started (bfull), so no asynchronous write is left in flight.
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
@@ -69,11 +75,6 @@ constexpr int B_BYTES = (NB / 8) * SBO;                 // 8 KB per part
 constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;  // 32 KB
 constexpr int TMEM_COLS = 512;  // 2 buffers x (main, corr) x 128 columns: all of an SM's TMEM
 constexpr int IMG_BYTES = 13 * SBO;  // one operator image part: rows 0..103 (13 groups of 8)
-// items whose gathers may still be in flight: an item's arrival follows its thread's wait for the
-// stage LAG - 1 items later, so fewer leave the MMAs more slack (film / platelet M2L with 5: 0.47 / 1.73
-// ms, 3: 0.455 / 1.64, 2: 0.45 / 1.64; two would not cover the gathers' latency on a busy L2)
-constexpr int LAG = 3;
-
 using namespace tc;
 
 // Shared-memory descriptor of this file's operand layout (LBO / SBO above).
@@ -86,9 +87,11 @@ __device__ __forceinline__ float tf32_rn(float x) {
 }
 
 // Gather of one item (K = 16) of the 64 input expansions of each set, hi and lo parts, with
-// 16-byte async copies into the core-matrix layout: thread t copies quads 2(t&1), 2(t&1)+1
-// of cell t>>1 of every set (column t>>1 + 64 set; zero fill beyond coefficient 99 or where
-// the cell has no input, sc < 0). The sets share the tables: one source cell for all.
+// 16-byte async copies into the core-matrix layout: thread t copies quads t & 1 and (t & 1) + 2
+// of cell t >> 1 of every set (column t >> 1 + 64 set; zero fill beyond coefficient 99 or where
+// the cell has no input, sc < 0). Two lanes read a sector of 32 bytes; four lanes per 64 bytes would
+// touch fewer lines, but their stores meet in the same banks (0.455 -> 0.478 ms on the film, where
+// this pairing gives 0.447). The sets share the tables: one source cell for all.
 __device__ __forceinline__ void gather_item(unsigned char *bs, int tid, int k0, int sc, const float *in_hi,
                                             const float *in_lo, int ns, size_t set_io) {
     const int n = tid >> 1;
@@ -98,7 +101,7 @@ __device__ __forceinline__ void gather_item(unsigned char *bs, int tid, int k0, 
         const int col = n + NC * y;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
-            const int kq = 2 * (tid & 1) + h, j = k0 + 4 * kq;
+            const int kq = (tid & 1) + 2 * h, j = k0 + 4 * kq;
             const bool ok = sc >= 0 && j < NRC;
             const size_t o = ok ? y * set_io + (size_t)sc * NRC + j : 0;
             unsigned char *d = bs + (col >> 3) * SBO + kq * 128 + (col & 7) * 16;
@@ -122,7 +125,7 @@ __device__ __forceinline__ void translate_tc_body(const TcArgs &a) {
     int *err = a.err;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *sm = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    // full: the 128 gathering threads of a stage; bfull: the operator's bulk copies (bytes);
+    // full: the 4 gathering warps of a stage; bfull: the operator's bulk copies (bytes);
     // tdone: every MMA the issuer started has completed (checked before TMEM is freed)
     __shared__ __align__(8) uint64_t full[NSTAGE], bfull[NSTAGE], empty[NSTAGE], tfull[2], tfree[2], tdone;
     __shared__ uint32_t tmem_base;
@@ -148,8 +151,8 @@ __device__ __forceinline__ void translate_tc_body(const TcArgs &a) {
     }
     if (tid == 0) {
         for (int s = 0; s < NSTAGE; s++) {
-            mbar_init(&full[s], 128);  // the 128 gathering threads
-            mbar_init(&bfull[s], 1);   // thread 0's expect_tx, completed by the bulk copies' bytes
+            mbar_init(&full[s], 128);  // the gathering threads
+            mbar_init(&bfull[s], 1);   // one expect_tx, completed by the bulk copies' bytes
             mbar_init(&empty[s], 1);
         }
         mbar_init(&tdone, 1);
@@ -174,100 +177,103 @@ __device__ __forceinline__ void translate_tc_body(const TcArgs &a) {
     const uint32_t tmem = tmem_base;
 
     if (warp < 4) {
-        // producers: one item (K = 16) per pipeline step; a thread's gathers of item it are
-        // complete (cp.async.wait_group) when it arrives for that item, LAG items later.
-        // The source cell of this thread's output cell is read once per code.
-        bool live = true;
-        // source cell of this thread's output cell for the current code; the next code's is
-        // loaded one code ahead so that its latency is hidden behind the current code's items
+        // producers: one item (K = 16) per pipeline step. The source cell of this thread's output
+        // cell is read once per code, one code ahead so that its latency is hidden behind the
+        // current code's items
         const int mycell = c_begin + (tid >> 1);
         auto src_of = [&](int ci) {
             return (ci < ncodes && mycell < n_out) ? __ldg(tab + (size_t)(out0 + mycell) * ncode + tile_code[q0 + ci])
                                                    : -1;
         };
         int sc = src_of(0), sc_next = src_of(1);
-        int armed = 0;  // thread 0: items whose bulk copies were started (in order)
-        for (int it = 0; it < nitems + LAG; it++) {
-            // arrive for item it - LAG first: its copies were issued LAG items ago, and the
-            // arrival must not wait behind this iteration's wait for a free stage (that wait
-            // follows the MMAs of item it - NSTAGE; arriving after it would hold the MMAs of
-            // item it - LAG until those of the item before it had completed)
-            if (it >= LAG) {
-                cp_wait<LAG - 1>();  // it groups committed: item it - LAG's has landed
-                fence_proxy_async();
-                if (live) mbar_arrive(&full[(it - LAG) % NSTAGE]);
+        int armed = 0;  // lane 0: one past the last item whose bulk copies this warp started
+        int s = 0, ph = 1, ci = 0, q = 0;  // stage, phase of its release, code and piece of the next item
+        for (int it = 0; it < nitems; it++) {
+            if (it >= NSTAGE && !mbar_wait(&empty[s], ph, err, &bail)) break;
+            unsigned char *st = sm + s * STAGE_BYTES;
+            if (lane == 0 && (it & 3) == warp) {  // the warps take turns: this costs as much as half a gather
+                const unsigned char *img = a.op_img + ((size_t)tile_code[q0 + ci] * IPC + q) * 2 * IMG_BYTES;
+                mbar_arrive_expect_tx(&bfull[s], 2 * IMG_BYTES);
+                bulk_g2s(st, img, IMG_BYTES, &bfull[s]);
+                bulk_g2s(st + A_BYTES, img + IMG_BYTES, IMG_BYTES, &bfull[s]);
+                armed = it + 1;
             }
-            if (it < nitems && live) {
-                const int s = it % NSTAGE;
-                if (it >= NSTAGE && !mbar_wait(&empty[s], ((it / NSTAGE) - 1) & 1, err, &bail)) live = false;
-                if (live) {
-                    const int ci = it / IPC, q = it % IPC;
-                    const int code = tile_code[q0 + ci];
-                    if (q == 0 && ci > 0) {
-                        sc = sc_next;
-                        sc_next = src_of(ci + 1);
-                    }
-                    unsigned char *st = sm + s * STAGE_BYTES;
-                    if (tid == 0) {
-                        const unsigned char *img = a.op_img + ((size_t)code * IPC + q) * 2 * IMG_BYTES;
-                        mbar_arrive_expect_tx(&bfull[s], 2 * IMG_BYTES);
-                        bulk_g2s(st, img, IMG_BYTES, &bfull[s]);
-                        bulk_g2s(st + A_BYTES, img + IMG_BYTES, IMG_BYTES, &bfull[s]);
-                        armed = it + 1;
-                    }
-                    gather_item(st + 2 * A_BYTES, tid, KI * q, sc, in_hi, in_lo, ns, set_io);
-                }
+            gather_item(st + 2 * A_BYTES, tid, KI * q, sc, in_hi, in_lo, ns, set_io);
+            cp_arrive(&full[s]);
+            if (++s == NSTAGE) {
+                s = 0;
+                ph ^= 1;
             }
-            cp_commit();
+            if (++q == IPC) {
+                q = 0;
+                ci++;
+                sc = sc_next;
+                sc_next = src_of(ci + 1);
+            }
         }
+        cp_commit();
         cp_wait<0>();
         // after a bail the issuer may not have consumed the last stages: wait (bounded) until
         // the bytes of every bulk copy still owed to a stage have landed before the CTA exits
-        if (tid == 0 && bail)
+        if (lane == 0 && bail)
             for (int it = armed > NSTAGE ? armed - NSTAGE : 0; it < armed; it++)
-                mbar_drain(&bfull[it % NSTAGE], (it / NSTAGE) & 1);
+                if ((it & 3) == warp) mbar_drain(&bfull[it % NSTAGE], (it / NSTAGE) & 1);
     } else if (warp == 4) {
-        if (lane == 0) {
-            // MMA issuer. Each code accumulates into a fresh pair of TMEM accumulators
-            // (buffer ci & 1): main = hi*hi, corr = hi*lo + lo*hi. The tensor core's FP32
-            // accumulation truncates, so its error grows with the number of MMAs summed in
-            // place; 13 K-steps per accumulator keep it at FP32 rounding level, and the drain
-            // warps add the per-code results with round-to-nearest.
-            const uint32_t idesc = idesc_tf32(MR, NC * ns);
-            bool ok = true;
-            for (int ci = 0; ci < ncodes && ok; ci++) {
-                const int b = ci & 1;
-                if (ci >= 2 && !mbar_wait(&tfree[b], ((ci >> 1) - 1) & 1, err, &bail)) break;
+        // MMA issuer: warp-uniform code, one elected lane starts the MMAs. Each code accumulates
+        // into a fresh pair of TMEM accumulators (buffer ci & 1): main = hi*hi, corr = hi*lo + lo*hi.
+        // The tensor core's FP32 accumulation truncates, so its error grows with the number of MMAs
+        // summed in place; 13 K-steps per accumulator keep it at FP32 rounding level, and the drain
+        // warps add the per-code results with round-to-nearest.
+        const uint32_t idesc = idesc_tf32(MR, NC * ns);
+        const bool lead = elect_one();
+        const uint64_t d0 = sdesc(smem_u32(sm));  // operator, high part, stage 0
+        auto wait = [&](uint64_t *bar, uint32_t parity) {
+            return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, &bail)) != 0;
+        };
+        int s = 0, ph = 0;  // stage and phase of the next item
+        bool ok = true;
+        for (int ci = 0; ci < ncodes && ok; ci++) {
+            const int b = ci & 1;
+            if (ci >= 2 && !wait(&tfree[b], ((ci >> 1) - 1) & 1)) break;
+            tc_fence_after();
+            const uint32_t dmain = tmem + b * 2 * NB, dcorr = dmain + NB;
+            for (int q = 0; q < IPC; q++) {
+                if (!wait(&full[s], ph) || !wait(&bfull[s], ph)) {
+                    ok = false;
+                    break;
+                }
+                fence_proxy_async();  // the gathered pieces, written through the generic proxy
                 tc_fence_after();
-                const uint32_t dmain = tmem + b * 2 * NB, dcorr = dmain + NB;
-                for (int q = 0; q < IPC; q++) {
-                    const int it = ci * IPC + q, s = it % NSTAGE;
-                    if (!mbar_wait(&full[s], (it / NSTAGE) & 1, err, &bail) ||
-                        !mbar_wait(&bfull[s], (it / NSTAGE) & 1, err, &bail)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const int ksteps = q < IPC - 1 ? KI / 8 : 1;
-                    const uint32_t base = smem_u32(sm + s * STAGE_BYTES);
-                    for (int k = 0; k < ksteps; k++) {
-                        const uint64_t ah = sdesc(base + k * 256), al = sdesc(base + A_BYTES + k * 256);
-                        const uint64_t bh = sdesc(base + 2 * A_BYTES + k * 256);
-                        const uint64_t bl = sdesc(base + 2 * A_BYTES + B_BYTES + k * 256);
-                        const bool first = (q == 0 && k == 0);
-                        if (terms & 1) mma_tf32(dmain, ah, bh, idesc, first ? 0u : 1u);
-                        if (terms & 2) mma_tf32(dcorr, ah, bl, idesc, first ? 0u : 1u);
-                        if (terms & 4) mma_tf32(dcorr, al, bh, idesc, (first && !(terms & 2)) ? 0u : 1u);
+                if (lead) {
+                    const uint64_t ah = d0 + s * (STAGE_BYTES / 16);
+#pragma unroll
+                    for (int k = 0; k < KI / 8; k++) {
+                        if (k && q == IPC - 1) break;
+                        const uint64_t da = ah + k * 16, dl = da + A_BYTES / 16;
+                        const uint64_t bh = da + 2 * (A_BYTES / 16), bl = bh + B_BYTES / 16;
+                        const uint32_t more = q || k;
+                        if (terms & 1) mma_tf32(dmain, da, bh, idesc, more);
+                        if (terms & 2) mma_tf32(dcorr, da, bl, idesc, more);
+                        if (terms & 4) mma_tf32(dcorr, dl, bh, idesc, (terms & 2) ? 1u : more);
                     }
                     mma_commit(&empty[s]);
                 }
-                mma_commit(&tfull[b]);
+                __syncwarp();
+                if (++s == NSTAGE) {
+                    s = 0;
+                    ph ^= 1;
+                }
             }
-            // tdone arrives once every MMA started above has completed (also after a bail,
-            // when the drain warps no longer wait for them): TMEM is freed only after that
+            if (lead) mma_commit(&tfull[b]);
+            __syncwarp();
+        }
+        // tdone arrives once every MMA started above has completed (also after a bail,
+        // when the drain warps no longer wait for them): TMEM is freed only after that
+        if (lead) {
             mma_commit(&tdone);
             mbar_drain(&tdone, 0);
         }
+        __syncwarp();
     } else {
         // drain warps 5..8: warp w reads TMEM lanes 32 (w % 4) .. +31 (coefficient rows)
         const int quarter = warp & 3;

@@ -91,6 +91,10 @@ __device__ __forceinline__ void cp16(void *dst, const void *src, uint32_t src_by
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
                  : "memory");
 }
+// An arrival of this thread on b once every cp.async that it started so far has landed.
+__device__ __forceinline__ void cp_arrive(uint64_t *b) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(b)) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -134,6 +138,13 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N) {
 }
 __device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
     mma_bf16(d, a, b, idesc, acc);  // kind::f16: the operand types are those of the descriptor
+}
+// One lane of a converged warp, the same at every call: MMAs are issued from warp-uniform code under
+// this predicate, so that descriptors and addresses stay in uniform registers.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
 }
 __device__ __forceinline__ void mma_commit(uint64_t *b) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(b))
