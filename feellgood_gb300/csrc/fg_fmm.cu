@@ -2374,13 +2374,24 @@ static int fmm_build_forest(Ctx &c, int L) {
     // near-field tasks of at most `most` targets: each leaf's targets shared out evenly, in multiples
     // of `step`. Where the sources (src_bytes each) fit in L2 the expensive tasks go first, which
     // evens out the last wave; else the leaf order keeps neighbouring tasks on the same sources
-    auto near_tasks = [&](int most, int step, int src_bytes) -> cudaError_t {
+    auto near_tasks = [&](int most, int step, int src_bytes, bool warps) -> cudaError_t {
         std::vector<int4> task;
-        std::vector<long> cost;
+        std::vector<long> cost, leaf_near(nleaf, 0);
+        long pairs = 0;
         for (int l = 0; l < nleaf; l++) {
-            const int n = leaf_tgt[l + 1] - leaf_tgt[l], groups = (n + most - 1) / most, units = (n + step - 1) / step;
-            long src = 0;
-            for (int e = near_ptr[l]; e < near_ptr[l + 1]; e++) src += leaf_src[near_leaf[e] + 1] - leaf_src[near_leaf[e]];
+            for (int e = near_ptr[l]; e < near_ptr[l + 1]; e++)
+                leaf_near[l] += leaf_src[near_leaf[e] + 1] - leaf_src[near_leaf[e]];
+            pairs += leaf_near[l] * (leaf_tgt[l + 1] - leaf_tgt[l]);
+        }
+        // a warp per task: none longer than what each resident warp (sixteen per SM) has to do on
+        // average, else the longest task sets the time (24 uneven samples of up to 13k tets: near field
+        // 210 -> 147 us; a cap of twice and of 0.7 times the average gave half of that)
+        const double share = warps ? (double)pairs / (16.0 * std::max(1, c.nsm)) : 1e300;
+        for (int l = 0; l < nleaf; l++) {
+            const int n = leaf_tgt[l + 1] - leaf_tgt[l], units = (n + step - 1) / step;
+            const long src = leaf_near[l];
+            const int groups =
+                std::min(units, std::max((n + most - 1) / most, (int)std::ceil((double)src * n / std::max(1.0, share))));
             for (int g = 0; g < groups; g++) {
                 const int b = step * (int)((long)units * g / groups);
                 const int e = std::min(n, step * (int)((long)units * (g + 1) / groups));
@@ -2399,7 +2410,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         t->n_p2p_task = (int)task.size();
         return up(&t->p2p_task, task);
     };
-    if (fp32) FCK(near_tasks(P2P32_NT, 2, 20));
+    if (fp32) FCK(near_tasks(P2P32_NT, 2, 20, true));
     if (t->ds) {
         // x = hi + lo, hi on the 2^-20 grid (|x| < 4 leaf units: exact in FP32)
         auto split = [](const std::vector<double> &v, std::vector<float4> &hi, std::vector<float4> &lo) {
@@ -2421,7 +2432,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         std::vector<float4> sh, sl, th, tl;
         split(sloc, sh, sl);
         split(tloc, th, tl);
-        FCK(near_tasks(P2P_NT, 1, 40));
+        FCK(near_tasks(P2P_NT, 1, 40, t->repeat));
         FCK(up(&t->ds_src_hi, sh));
         FCK(up(&t->ds_src_lo, sl));
         FCK(up(&t->ds_tgt_hi, th));

@@ -73,6 +73,23 @@ def test_fp64_forest_matches_single_trees():
         assert _rel(pb[b.node_offsets[k]:b.node_offsets[k + 1]], c.demag(0)) < 1e-13
 
 
+# uneven leaves: the tasks of the large samples' leaves are cut down to a single pair of targets
+@pytest.mark.parametrize("shapes,leaf", [([(12, 12, 12), (2, 2, 2)], -2), ([(16, 3, 2), (1, 1, 1), (5, 5, 5)], -3)])
+def test_refinement_forest_of_uneven_leaves(shapes, leaf):
+    meshes = [cases.cuboid(*s) for s in shapes]
+    us = [cases.perturbed_state(m["xyz"], seed=50 + k, sigma=0.3) for k, m in enumerate(meshes)]
+    phi = {}
+    for p in (fg.FG_PREC_FP32_REFINE, fg.FG_PREC_FP64):
+        c = fg.Context(meshes, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=leaf, precision=p)
+        c.set_state(np.concatenate(us))
+        phi[p] = c.demag(0)
+        o = c.node_offsets
+    # FP32 products and sums of some thousand terms that cancel by one to two orders of magnitude
+    for k in range(len(meshes)):
+        a, b = (x[o[k]:o[k + 1]] for x in (phi[fg.FG_PREC_FP32_REFINE], phi[fg.FG_PREC_FP64]))
+        assert _rel(a, b) < 2e-5
+
+
 def test_not_a_number_propagates():
     """A magnetisation that is not a number reaches every potential that depends on it."""
     m = cases.cuboid(6, 6, 6)
