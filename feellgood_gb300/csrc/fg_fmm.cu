@@ -32,6 +32,7 @@
 #include <cstring>
 #include <unordered_map>
 #include <queue>
+#include <type_traits>
 #include <vector>
 
 #include "fg_ds.cuh"
@@ -639,46 +640,59 @@ __device__ __forceinline__ float2 ds_split(double x) {
 // ---- P2M of the full FP64 evaluation of the FP32 + refinement path (FmmTree::repeat) ----
 // The recurrences of ups_cols with every operation a double-single one, the coordinates as the
 // normalised pair of their stored hi + lo parts, the charge split once.
-template <int M, int M0, int M1, typename Fn>
-__device__ __forceinline__ void ups_col_ds(dsf x, dsf y, dsf z, dsf r2, dsf &dre, dsf &dim, Fn &f) {
-    if constexpr (M > 0) {
-        const dsf s = dsc(1.0 / (2 * M));
-        const dsf nre = ds_mul(ds_sub(ds_mul(x, dre), ds_mul(y, dim)), s);
-        const dsf nim = ds_mul(ds_add(ds_mul(x, dim), ds_mul(y, dre)), s);
-        dre = nre;
-        dim = nim;
+// The columns above 0 with real and imaginary parts as the lanes of packed pairs.
+__device__ __forceinline__ ds2 ds2_dup(dsf a) { return {pk2(a.h, a.h), pk2(a.l, a.l)}; }
+__device__ __forceinline__ ds2 ds2_neg(ds2 a) { return {neg2(a.h), neg2(a.l)}; }
+__device__ __forceinline__ u64 swap2(u64 a) { return a >> 32 | a << 32; }
+
+// Column 0 of one source: f(n, V_n), real.
+template <typename Fn>
+__device__ __forceinline__ void ups_col0_ds(dsf z, dsf r2, Fn &f) {
+    dsf p2 = {1.f, 0.f}, p1 = ds_mul(z, p2);
+    f(0, p2);
+    f(1, p1);
+#pragma unroll
+    for (int n = 2; n <= FMM_P; n++) {
+        const dsf az = ds_mul(dsf{(float)(2 * n - 1), 0.f}, z);
+        const dsf c = ds_mul(ds_sub(ds_mul(az, p1), ds_mul(r2, p2)), dsc(1.0 / (n * n)));
+        f(n, c);
+        p2 = p1;
+        p1 = c;
     }
+}
+
+// Columns M (1 first) to M1, f from column M0 on; d: the diagonal of column M - 1, X = (x, x),
+// Y = (-y, y), Z = (z, z), R2 = (r2, r2).
+template <int M, int M0, int M1, typename Fn>
+__device__ __forceinline__ void ups_col_ds(ds2 X, ds2 Y, dsf z, ds2 Z, ds2 R2, ds2 d, Fn &f) {
+    d = ds2_mul(ds2_add(ds2_mul(X, d), ds2_mul(Y, ds2{swap2(d.h), swap2(d.l)})), ds2_dup(dsc(1.0 / (2 * M))));
     if constexpr (M >= M0) {
-        f(M, M, dre, dim);
+        f(M, M, d);
         if constexpr (M + 1 <= FMM_P) {
-            dsf p2re = dre, p2im = dim;
-            dsf p1re = ds_mul(z, dre), p1im = ds_mul(z, dim);
-            f(M + 1, M, p1re, p1im);
+            ds2 p2 = d, p1 = ds2_mul(Z, d);
+            f(M + 1, M, p1);
 #pragma unroll
             for (int n = M + 2; n <= FMM_P; n++) {
                 const dsf az = ds_mul(dsf{(float)(2 * n - 1), 0.f}, z);
-                const dsf b = dsc(1.0 / ((n + M) * (n - M)));
-                const dsf cre = ds_mul(ds_sub(ds_mul(az, p1re), ds_mul(r2, p2re)), b);
-                const dsf cim = ds_mul(ds_sub(ds_mul(az, p1im), ds_mul(r2, p2im)), b);
-                f(n, M, cre, cim);
-                p2re = p1re; p2im = p1im;
-                p1re = cre; p1im = cim;
+                const ds2 c = ds2_mul(ds2_add(ds2_mul(ds2_dup(az), p1), ds2_neg(ds2_mul(R2, p2))),
+                                      ds2_dup(dsc(1.0 / ((n + M) * (n - M)))));
+                f(n, M, c);
+                p2 = p1;
+                p1 = c;
             }
         }
     }
-    if constexpr (M < M1) ups_col_ds<M + 1, M0, M1>(x, y, z, r2, dre, dim, f);
+    if constexpr (M < M1) ups_col_ds<M + 1, M0, M1>(X, Y, z, Z, R2, d, f);
 }
 
 template <int NS, int M0, int M1>
 __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, int rounds, const float4 *__restrict__ shi,
                                             const float4 *__restrict__ slo, size_t base, const P2mSet<double> &a,
                                             const P2mSet<double> &b) {
-    constexpr int NPR = lidx(M0, FMM_P, M1, 1) + 1;
-    dsf acc0[NPR], acc1[NS == 2 ? NPR : 1];
-#pragma unroll
-    for (int k = 0; k < NPR; k++) acc0[k] = dsf{0.f, 0.f};
-#pragma unroll
-    for (int k = 0; k < (NS == 2 ? NPR : 1); k++) acc1[k] = dsf{0.f, 0.f};
+    constexpr int NPR = lidx(M0, FMM_P, M1, 1) + 1, NV = M0 == 0 ? NPR : NPR / 2;  // column 0, or pairs
+    using Acc = std::conditional_t<M0 == 0, dsf, ds2>;
+    static_assert(M0 > 0 || M1 == 0, "column 0 alone");
+    Acc acc0[NV] = {}, acc1[NS == 2 ? NV : 1] = {};
     for (int q = 0; q < rounds; q++) {
         __syncthreads();  // the block's warps in step, on the same instructions
         const int s = s0 + lane + 32 * q;
@@ -687,49 +701,61 @@ __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, int rounds
         const dsf x = ds_two_sum_f(h.x, l.x), y = ds_two_sum_f(h.y, l.y), z = ds_two_sum_f(h.z, l.z);
         const double qa_d = a.q[s], qb_d = NS == 2 ? b.q[s] : 0.0;
         const dsf qa = dsc(qa_d), qb = dsc(qb_d);
-        if constexpr (M0 == 0) {  // the charges for the near field
-            a.qh[(size_t)s * a.qd_stride] = qa.h;
+        const dsf r2 = ds_add(ds_add(ds_mul(x, x), ds_mul(y, y)), ds_mul(z, z));
+        if constexpr (M0 == 0) {
+            a.qh[(size_t)s * a.qd_stride] = qa.h;  // the charges for the near field
             a.ql[(size_t)s * a.qd_stride] = qa.l;
             if constexpr (NS == 2) {
                 b.qh[(size_t)s * b.qd_stride] = qb.h;
                 b.ql[(size_t)s * b.qd_stride] = qb.l;
             }
+            auto f = [&](int n, dsf re) {
+                acc0[n] = ds_add(acc0[n], ds_mul(qa, re));
+                if constexpr (NS == 2) acc1[n] = ds_add(acc1[n], ds_mul(qb, re));
+            };
+            ups_col0_ds(z, r2, f);
+        } else {  // M = sum q conj(Ups): charges (q, -q)
+            const ds2 QA = {pk2(qa.h, -qa.h), pk2(qa.l, -qa.l)}, QB = {pk2(qb.h, -qb.h), pk2(qb.l, -qb.l)};
+            auto f = [&](int n, int m, ds2 v) {
+                const int k = lidx(M0, n, m, 0) / 2;
+                acc0[k] = ds2_add(acc0[k], ds2_mul(QA, v));
+                if constexpr (NS == 2) acc1[k] = ds2_add(acc1[k], ds2_mul(QB, v));
+            };
+            const ds2 Y = {pk2(-y.h, y.h), pk2(-y.l, y.l)};
+            ups_col_ds<1, M0, M1>(ds2_dup(x), Y, z, ds2_dup(z), ds2_dup(r2), ds2{pk2(1.f, 0.f), 0ull}, f);
         }
-        const dsf r2 = ds_add(ds_add(ds_mul(x, x), ds_mul(y, y)), ds_mul(z, z));
-        dsf dre = {1.f, 0.f}, dim = {0.f, 0.f};
-        auto f = [&](int n, int m, dsf re, dsf im) {
-            const int k = lidx(M0, n, m, 0);
-            acc0[k] = ds_add(acc0[k], ds_mul(qa, re));
-            if constexpr (NS == 2) acc1[k] = ds_add(acc1[k], ds_mul(qb, re));
-            if (m) {
-                acc0[k + 1] = ds_sub(acc0[k + 1], ds_mul(qa, im));
-                if constexpr (NS == 2) acc1[k + 1] = ds_sub(acc1[k + 1], ds_mul(qb, im));
-            }
-        };
-        ups_col_ds<0, M0, M1>(x, y, z, r2, dre, dim, f);
     }
-    auto red = [&](dsf v) {
+    auto red = [&](Acc v) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-            v = ds_add(v, dsf{__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)});
+        for (int o = 16; o > 0; o >>= 1) {
+            const Acc w = {__shfl_xor_sync(0xffffffffu, v.h, o), __shfl_xor_sync(0xffffffffu, v.l, o)};
+            if constexpr (M0 == 0) v = ds_add(v, w);
+            else v = ds2_add(v, w);
+        }
         return v;
+    };
+    // rounded to FP64, then the pair that the translations read
+    auto put = [&](const P2mSet<double> &st, int g, dsf v) {
+        if ((g & 31) == lane && s0 >= 0) reinterpret_cast<float2 *>(st.M)[base + g] = ds_split(ds_to(v));
+    };
+    auto store = [&](const P2mSet<double> &st, int n, int m, Acc v) {
+        if constexpr (M0 == 0) put(st, ridx(n, m, 0), v);
+        else {
+            dsf re, im;
+            upk2(v.h, re.h, im.h);
+            upk2(v.l, re.l, im.l);
+            put(st, ridx(n, m, 0), re);
+            put(st, ridx(n, m, 1), im);
+        }
     };
 #pragma unroll
     for (int m = M0; m <= M1; m++)
 #pragma unroll
-        for (int n = m; n <= FMM_P; n++)
-#pragma unroll
-            for (int part = 0; part < (m ? 2 : 1); part++) {
-                const int k = lidx(M0, n, m, part), g = ridx(n, m, part);
-                const dsf v0 = red(acc0[k]);
-                dsf v1 = {0.f, 0.f};
-                if constexpr (NS == 2) v1 = red(acc1[k]);
-                if ((g & 31) == lane && s0 >= 0) {
-                    // rounded to FP64, then the pair that the translations read
-                    reinterpret_cast<float2 *>(a.M)[base + g] = ds_split(ds_to(v0));
-                    if constexpr (NS == 2) reinterpret_cast<float2 *>(b.M)[base + g] = ds_split(ds_to(v1));
-                }
-            }
+        for (int n = m; n <= FMM_P; n++) {
+            const int k = M0 == 0 ? n : lidx(M0, n, m, 0) / 2;
+            store(a, n, m, red(acc0[k]));
+            if constexpr (NS == 2) store(b, n, m, red(acc1[k]));
+        }
 }
 
 // One warp per leaf and range of harmonic columns (0, 1, 2, 3, 4-5, 6-9: at most 22 reals, 88 floats
@@ -738,7 +764,8 @@ __device__ __forceinline__ void p2m_ds_pass(int lane, int s0, int s1, int rounds
 // same code, so a set's expansion does not depend on whether the other is evaluated beside it. The
 // range is the slow grid index and the block's warps keep in step: bound by fetching the unrolled
 // instructions, which six passes by each warp at its own pace made worse (294k tets, two sets: six
-// passes per warp 1.45 ms, a range per block 0.87, in step 0.73).
+// passes per warp 1.45 ms, a range per block 0.87, in step 0.73, real and imaginary parts as the lanes
+// of packed FP32 operations 0.58).
 template <int NS>
 __global__ void __launch_bounds__(128, 3) k_p2m_ds_repeat(int nleaf, const int *__restrict__ leaf_src,
                                                 const float4 *__restrict__ shi, const float4 *__restrict__ slo,
@@ -1486,9 +1513,9 @@ __global__ void __launch_bounds__(128, 4) k_p2p_ds(const int4 *__restrict__ task
 // the lanes of one warp, per-lane sums reduced over the warp in FP64. A warp takes a task of up to 8
 // targets of a leaf, the leaf's targets shared out evenly (a warp per leaf, in passes of 8 targets
 // whatever was left, with the local expansions behind them, gave each SM a dozen unequal warps;
-// 294k tets, two sets: 4.85 -> 2.23 ms and 0.09 for the local expansions, FMA pipe 76%).
-template <int NT, int NQ>
-__device__ __forceinline__ void p2p_repeat_pass(int lane, int leaf, int tb, const int *__restrict__ leaf_src,
+// 294k tets, two sets: 4.85 -> 2.23 ms and 0.09 for the local expansions; packed pairs of targets 2.14).
+template <int NP, int NQ>
+__device__ __forceinline__ void p2p_repeat_pass(int lane, int leaf, int tb, int nt, const int *__restrict__ leaf_src,
                                                 const int *__restrict__ tgt_node, const float4 *__restrict__ th4,
                                                 const float4 *__restrict__ tl4, const float4 *__restrict__ sh4,
                                                 const float4 *__restrict__ sl4, const float *__restrict__ q2h,
@@ -1496,15 +1523,17 @@ __device__ __forceinline__ void p2p_repeat_pass(int lane, int leaf, int tb, cons
                                                 const int *__restrict__ near_ptr, const int *__restrict__ near_leaf,
                                                 double *__restrict__ pot0, double *__restrict__ pot1) {
     const int li = leaf_ijk[3 * leaf], lj = leaf_ijk[3 * leaf + 1], lk = leaf_ijk[3 * leaf + 2];
-    float thx[NT], thy[NT], thz[NT], tlx[NT], tly[NT], tlz[NT], ah[NQ][NT], al[NQ][NT];
+    u64 thx[NP], thy[NP], thz[NP], tlx[NP], tly[NP], tlz[NP], ah[NQ][NP], al[NQ][NP];
 #pragma unroll
-    for (int j = 0; j < NT; j++) {
-        const float4 h = th4[tb + j], l = tl4[tb + j];
-        thx[j] = h.x; thy[j] = h.y; thz[j] = h.z;
-        tlx[j] = l.x; tly[j] = l.y; tlz[j] = l.z;
+    for (int j = 0; j < NP; j++) {
+        const int t0 = tb + 2 * j, t1 = tb + min(2 * j + 1, nt - 1);
+        const float4 h = th4[t0], l = tl4[t0], h1 = th4[t1], l1 = tl4[t1];
+        thx[j] = pk2(h.x, h1.x); thy[j] = pk2(h.y, h1.y); thz[j] = pk2(h.z, h1.z);
+        tlx[j] = pk2(l.x, l1.x); tly[j] = pk2(l.y, l1.y); tlz[j] = pk2(l.z, l1.z);
 #pragma unroll
-        for (int k = 0; k < NQ; k++) ah[k][j] = al[k][j] = 0.f;
+        for (int k = 0; k < NQ; k++) ah[k][j] = al[k][j] = 0ull;
     }
+    const u64 two = pk2(2.f, 2.f), one = pk2(1.f, 1.f), half = pk2(0.5f, 0.5f);
     for (int e = near_ptr[leaf]; e < near_ptr[leaf + 1]; e++) {
         const int nl = near_leaf[e];
         // integer offset of the adjacent leaf, added exactly to the hi parts
@@ -1514,46 +1543,47 @@ __device__ __forceinline__ void p2p_repeat_pass(int lane, int leaf, int tb, cons
         for (int s = s0 + lane; s < s1; s += 32) {
             const float4 h = sh4[s], l = sl4[s];
             const float sx = h.x + ox, sy = h.y + oy, sz = h.z + oz;
-            float qh[NQ], ql[NQ];
-            qh[0] = h.w;
-            ql[0] = l.w;
+            const u64 SX = pk2(sx, sx), SY = pk2(sy, sy), SZ = pk2(sz, sz);
+            const u64 LX = pk2(l.x, l.x), LY = pk2(l.y, l.y), LZ = pk2(l.z, l.z);
+            u64 qh[NQ], ql[NQ];
+            qh[0] = pk2(h.w, h.w);
+            ql[0] = pk2(l.w, l.w);
             if constexpr (NQ == 2) {
-                qh[1] = q2h[s];
-                ql[1] = q2l[s];
+                const float a = q2h[s], b = q2l[s];
+                qh[1] = pk2(a, a);
+                ql[1] = pk2(b, b);
             }
 #pragma unroll
-            for (int j = 0; j < NT; j++) {
-                const float d1x = thx[j] - sx, d1y = thy[j] - sy, d1z = thz[j] - sz;  // exact
-                const float d2x = tlx[j] - l.x, d2y = tly[j] - l.y, d2z = tlz[j] - l.z;
+            for (int j = 0; j < NP; j++) {
+                const u64 d1x = sub2(thx[j], SX), d1y = sub2(thy[j], SY), d1z = sub2(thz[j], SZ);  // exact
+                const u64 d2x = sub2(tlx[j], LX), d2y = sub2(tly[j], LY), d2z = sub2(tlz[j], LZ);
                 // squares: d^2 = d1^2 + d2 (2 d1 + d2), leading products exact
-                const float px = d1x * d1x, py = d1y * d1y, pz = d1z * d1z;
-                float ex = fmaf(d1x, d1x, -px), ey = fmaf(d1y, d1y, -py), ez = fmaf(d1z, d1z, -pz);
-                ex = fmaf(d2x, 2.f * d1x + d2x, ex);
-                ey = fmaf(d2y, 2.f * d1y + d2y, ey);
-                ez = fmaf(d2z, 2.f * d1z + d2z, ez);
-                float s1_, e1, s2_, e2;
-                ds_two_sum(px, py, s1_, e1);
-                ds_two_sum(s1_, pz, s2_, e2);
-                const float el = (e1 + e2) + (ex + ey + ez);
-                const float Sh = s2_ + el, Sl = el - (Sh - s2_);
+                const u64 px = mul2(d1x, d1x), py = mul2(d1y, d1y), pz = mul2(d1z, d1z);
+                u64 ex = fma2(d1x, d1x, neg2(px)), ey = fma2(d1y, d1y, neg2(py)), ez = fma2(d1z, d1z, neg2(pz));
+                ex = fma2(d2x, fma2(two, d1x, d2x), ex);
+                ey = fma2(d2y, fma2(two, d1y, d2y), ey);
+                ez = fma2(d2z, fma2(two, d1z, d2z), ez);
+                const ds2 r1 = ds2_two_sum(px, py), r2 = ds2_two_sum(r1.h, pz);
+                const u64 el = add2(add2(r1.l, r2.l), add2(add2(ex, ey), ez));
+                const u64 Sh = add2(r2.h, el), Sl = sub2(el, sub2(Sh, r2.h));
                 // 1/sqrt(S): SFU estimate y, then y (1 + (1 - S y^2) / 2) with S y^2 in
                 // double-single (1 - S y^2 is small and exact to ~2^-46)
-                float y;
-                asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(Sh));
-                const float t1_ = y * y, t2_ = fmaf(y, y, -t1_);
-                const float u1 = Sh * t1_;
-                const float u2 = fmaf(Sh, t1_, -u1) + fmaf(Sh, t2_, Sl * t1_);
-                const float delta = (1.f - u1) - u2;
-                const float yl = 0.5f * y * delta;
+                float S0, S1;
+                upk2(Sh, S0, S1);
+                const u64 y = pk2(rsqrt_p<float>(S0), rsqrt_p<float>(S1));
+                const u64 t1 = mul2(y, y), t2 = fma2(y, y, neg2(t1));
+                const u64 u1 = mul2(Sh, t1);
+                const u64 u2 = add2(fma2(Sh, t1, neg2(u1)), fma2(Sh, t2, mul2(Sl, t1)));
+                const u64 delta = sub2(sub2(one, u1), u2);
+                const u64 yl = mul2(mul2(half, y), delta);
                 // q / r = (qh + ql)(y + yl), accumulated with two-sum
 #pragma unroll
                 for (int k = 0; k < NQ; k++) {
-                    const float c1 = qh[k] * y;
-                    const float c2 = fmaf(qh[k], y, -c1) + fmaf(qh[k], yl, ql[k] * y);
-                    float sn, en;
-                    ds_two_sum(ah[k][j], c1, sn, en);
-                    ah[k][j] = sn;
-                    al[k][j] += en + c2;
+                    const u64 c1 = mul2(qh[k], y);
+                    const u64 c2 = add2(fma2(qh[k], y, neg2(c1)), fma2(qh[k], yl, mul2(ql[k], y)));
+                    const ds2 sn = ds2_two_sum(ah[k][j], c1);
+                    ah[k][j] = sn.h;
+                    al[k][j] = add2(al[k][j], add2(sn.l, c2));
                 }
             }
         }
@@ -1561,10 +1591,13 @@ __device__ __forceinline__ void p2p_repeat_pass(int lane, int leaf, int tb, cons
 #pragma unroll
     for (int k = 0; k < NQ; k++)
 #pragma unroll
-        for (int j = 0; j < NT; j++) {
-            double v = double(ah[k][j]) + double(al[k][j]);
+        for (int j = 0; j < 2 * NP; j++) {
+            float h[2], l[2];
+            upk2(ah[k][j / 2], h[0], h[1]);
+            upk2(al[k][j / 2], l[0], l[1]);
+            double v = double(h[j % 2]) + double(l[j % 2]);
             for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == j) (k ? pot1 : pot0)[tgt_node[tb + j]] = v;
+            if (lane == j && j < nt) (k ? pot1 : pot0)[tgt_node[tb + j]] = v;
         }
 }
 
@@ -1580,11 +1613,11 @@ __global__ void __launch_bounds__(128, 4)
     const int4 t = task[w];
 #define FG_P2P(N)                                                                                                   \
     case N:                                                                                                         \
-        p2p_repeat_pass<N, NQ>(lane, t.x, t.y, leaf_src, tgt_node, th4, tl4, sh4, sl4, q2h, q2l, leaf_ijk, near_ptr, \
-                               near_leaf, pot0, pot1);                                                              \
+        p2p_repeat_pass<N, NQ>(lane, t.x, t.y, t.z, leaf_src, tgt_node, th4, tl4, sh4, sl4, q2h, q2l, leaf_ijk,      \
+                               near_ptr, near_leaf, pot0, pot1);                                                    \
         break;
-    switch (t.z) {
-        FG_P2P(1) FG_P2P(2) FG_P2P(3) FG_P2P(4) FG_P2P(5) FG_P2P(6) FG_P2P(7) FG_P2P(8)
+    switch ((t.z + 1) / 2) {
+        FG_P2P(1) FG_P2P(2) FG_P2P(3) FG_P2P(4)
     }
 #undef FG_P2P
 }
@@ -2432,7 +2465,7 @@ static int fmm_build_forest(Ctx &c, int L) {
         std::vector<float4> sh, sl, th, tl;
         split(sloc, sh, sl);
         split(tloc, th, tl);
-        FCK(near_tasks(P2P_NT, 1, 40, t->repeat));
+        FCK(near_tasks(P2P_NT, t->repeat ? 2 : 1, 40, t->repeat));
         FCK(up(&t->ds_src_hi, sh));
         FCK(up(&t->ds_src_lo, sl));
         FCK(up(&t->ds_tgt_hi, th));
