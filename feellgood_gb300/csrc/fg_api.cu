@@ -762,10 +762,7 @@ int fg_set_state(fg_ctx *h, const double *u, const double *v, const double *phi,
     else CK(cudaMemsetAsync(c.phi[0], 0, n1, c.stream));
     if (phiv) CK(cudaMemcpyAsync(c.phiv[0], phiv, n1, cudaMemcpyHostToDevice, c.stream));
     else CK(cudaMemsetAsync(c.phiv[0], 0, n1, c.stream));
-    CK(cudaMemcpyAsync(c.u[1], c.u[0], n3, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.v[1], c.v[0], n3, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.phi[1], c.phi[0], n1, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.phiv[1], c.phiv[0], n1, cudaMemcpyDeviceToDevice, c.stream));
+    CK(launch_copy_state(c, 1, 0));
     CK(cudaStreamSynchronize(c.stream));
     // given potentials are those of the given fields (v = 0 has phiv = 0)
     c.dinc_valid[0] = phi != nullptr;
@@ -913,7 +910,7 @@ static int demag_into(fg_ctx *h, const double *m, double *phi_out) {
 static int energy_impl(fg_ctx *h, const double Hext[3], double E[4], double avg[3]) {
     Ctx &c = h->c;
     CK(launch_energy(c, Hext));
-    c.launches += 1;
+    c.launches += 2;  // and the evolution's copy
     CK(cudaMemcpyAsync(c.hepart, c.epart, 7 * sizeof(double) * c.epart_blocks, cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));
     double s[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -998,11 +995,7 @@ int fg_compute_all(fg_ctx *h, const double Hext[3], double energies[4]) {
     CK(cudaMemcpyAsync(c.hepart, c.epart, 7 * sizeof(double) * c.epart_blocks, cudaMemcpyDeviceToHost, c.stream));
     // Fem::evolution: CURRENT <- NEXT
     if (c.mlp) CK(mlp_before_evolution(c));
-    const size_t n3 = 3 * sizeof(double) * c.nn, n1 = sizeof(double) * c.nn;
-    CK(cudaMemcpyAsync(c.u[0], c.u[1], n3, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.v[0], c.v[1], n3, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.phi[0], c.phi[1], n1, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.phiv[0], c.phiv[1], n1, cudaMemcpyDeviceToDevice, c.stream));
+    CK(launch_copy_state(c, 0, 1));
     CK(cudaEventRecord(c.ev[5], c.stream));
     if (int *fl = fmm_error_flag(c)) CK(cudaMemcpyAsync(c.hflag, fl, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));

@@ -261,17 +261,12 @@ static cudaError_t run_body(Ctx &c) {
     if (e != cudaSuccess) return e;
     if ((e = batch_demag_all(c)) != cudaSuccess) return e;
     if (use && (e = mlp_before_evolution(c)) != cudaSuccess) return e;
-    const size_t n3 = 3 * sizeof(double) * c.nn, n1 = sizeof(double) * c.nn;
-    if ((e = cudaMemcpyAsync(c.u[0], c.u[1], n3, cudaMemcpyDeviceToDevice, c.stream)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(c.v[0], c.v[1], n3, cudaMemcpyDeviceToDevice, c.stream)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(c.phi[0], c.phi[1], n1, cudaMemcpyDeviceToDevice, c.stream)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(c.phiv[0], c.phiv[1], n1, cudaMemcpyDeviceToDevice, c.stream)) != cudaSuccess)
-        return e;
+    if ((e = launch_copy_state(c, 0, 1)) != cudaSuccess) return e;
     return launch_advance(c);
 }
 
 static int body_launches(const Ctx &c) {
-    return 5 + demag_launches(c) + (batch_use_mlp(c) ? 1 : 0);
+    return 6 + demag_launches(c) + (batch_use_mlp(c) ? 1 : 0);
 }
 
 static void try_capture(Ctx &c) {
@@ -440,12 +435,9 @@ int fg_batch_compute_all(fg_ctx *h, const double *Hext, double *energies) {
         c.launches += 2;
         CK(cudaMemcpyAsync(c.hseg_energy, c.seg_energy, 7 * sizeof(double) * ns, cudaMemcpyDeviceToHost, c.stream));
     }
-    const size_t n3 = 3 * sizeof(double) * c.nn, n1 = sizeof(double) * c.nn;
     if (c.mlp) CK(mlp_before_evolution(c));  // v_prev2 of the learned guess's extrapolation
-    CK(cudaMemcpyAsync(c.u[0], c.u[1], n3, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.v[0], c.v[1], n3, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.phi[0], c.phi[1], n1, cudaMemcpyDeviceToDevice, c.stream));
-    CK(cudaMemcpyAsync(c.phiv[0], c.phiv[1], n1, cudaMemcpyDeviceToDevice, c.stream));
+    CK(launch_copy_state(c, 0, 1));
+    c.launches += 1;
     CK(cudaEventRecord(c.ev[5], c.stream));
     if (int *fl = fmm_error_flag(c)) CK(cudaMemcpyAsync(c.hflag, fl, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));

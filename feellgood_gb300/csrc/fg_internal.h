@@ -386,6 +386,7 @@ cudaError_t launch_phi_final(Ctx &c, double *phi0, double *phi1 = nullptr, const
 cudaError_t launch_state_diff(Ctx &c);  // dstate32 = NEXT - CURRENT for u and v (FP32)
 cudaError_t launch_charges32(Ctx &c, int nq);  // FP32 charges of dstate32 (incremental demag)
 cudaError_t launch_energy(Ctx &c, const double Hext[3]);
+cudaError_t launch_copy_state(Ctx &c, int to, int from);  // u, v, phi, phiv
 cudaError_t launch_energy_into(Ctx &c, const double Hext[3], double *partial);
 int bicg_grid_size(Ctx &c);  // and c.bicg_block
 cudaError_t morton_sort(Ctx &c, int n, int L, int nseg, const double *xyz, const int *seg,
