@@ -114,7 +114,7 @@ struct FmmTree {
     int *oz_cells = nullptr, *oz_codes = nullptr, *oz_wexp = nullptr, *oz_leaves = nullptr;
     int4 *oz_units = nullptr;
     int2 *oz_fin = nullptr;
-    double *oz_scratch = nullptr;
+    float2 *oz_scratch = nullptr;
     unsigned char *oz_digits = nullptr;          // of M up to M2L, of F from there
     float *oz_scale = nullptr;
     unsigned char *oz_img[3] = {nullptr, nullptr, nullptr};  // M2M, M2L, L2L
@@ -2367,7 +2367,7 @@ static int fmm_build_forest(Ctx &c, int L) {
             FCK(up(&t->oz_fin, fin));
             FCK(up(&t->oz_wexp, wexp));
             FCK(up(&t->oz_leaves, leaves));
-            FCK(cudaMalloc(&t->oz_scratch, sizeof(double) * std::max(1, nslot) * OZ_TILE * NR * t->nq));
+            FCK(cudaMalloc(&t->oz_scratch, sizeof(float2) * std::max(1, nslot) * OZ_TILE * NR * t->nq));
             FCK(cudaMalloc(&t->oz_digits, (size_t)ncell * t->nq * OZ_CELL_BYTES));
             FCK(cudaMemset(t->oz_digits, 0, (size_t)ncell * t->nq * OZ_CELL_BYTES));
             FCK(cudaMalloc(&t->oz_scale, sizeof(float) * ncell * t->nq));

@@ -29,7 +29,9 @@
 //               the 48 ns expansions (160 contiguous bytes per expansion and stage);
 //   warps 4-15  drain finished accumulators: warp w owns the coefficient rows 32 (w % 4).. and the
 //               columns 32 (w / 4 - 1).., loads the five sums, combines them, scales by
-//               rs_i cs and adds to its double-single sums; at the end FP64 partial sums to scratch;
+//               rs_i cs and adds to its double-single sums; at the end the pairs to scratch (their
+//               conversion to FP64 here, 1/64 of the FP32 rate, took a third of the short launches: M2M
+//               and L2L of the wire 0.185 and 0.164 ms, converted in k_oz_finish 0.162 and 0.133);
 //   warp 3      one lane issues the MMAs.
 // Bound by shared-memory reads of the MMA operands (7 KB per MMA of 128x96x16) and the drain,
 // which the single accumulator set puts in series with the next code's MMAs.
@@ -257,7 +259,7 @@ __global__ void __launch_bounds__(NTHREAD, 1) k_translate_oz(OzArgs a) {
                 upk2(ah[j / 2], h0, h1);
                 upk2(al[j / 2], l0, l1);
                 a.scratch[(((size_t)unit.w * ns + y) * NCELL + col - NCELL * y) * NRC + row] =
-                    (j & 1) ? (double)h1 + (double)l1 : (double)h0 + (double)l0;
+                    (j & 1) ? make_float2(h1, l1) : make_float2(h0, l0);
             }
         }
     }
@@ -282,15 +284,21 @@ __global__ void __launch_bounds__(256) k_oz_finish(OzFinish a) {
     const int cell = a.cells[k];
     if (cell < 0) return;
     double *io = a.io + ((size_t)y * a.ncell + cell) * NRC;
-    double v[4];
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
     const int2 fin = a.fin ? a.fin[k / NCELL] : make_int2(0, 0);
+#pragma unroll 4
+    for (int s = 0; s < fin.y; s++) {
+        const float2 *p = a.scratch + (((size_t)(fin.x + s) * ns + y) * NCELL + k % NCELL) * NRC;
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const float2 x = lane + 32 * m < NRC ? p[lane + 32 * m] : make_float2(0.f, 0.f);
+            v[m] += (double)x.x + (double)x.y;
+        }
+    }
 #pragma unroll
     for (int m = 0; m < 4; m++) {
         const int r = lane + 32 * m;
-        v[m] = 0.0;
         if (r < NRC) {
-            for (int s = 0; s < fin.y; s++)
-                v[m] += a.scratch[(((size_t)(fin.x + s) * ns + y) * NCELL + k % NCELL) * NRC + r];
             if (a.accumulate) v[m] = fin.y ? io[r] + v[m] : io[r];
             if (a.fin && (fin.y || !a.accumulate)) io[r] = v[m];
         }

@@ -464,14 +464,14 @@ struct OzArgs {
     const float *in_scale;        // [set][cell]
     const int4 *units;            // per CTA: tile, first and end index into codes, scratch slot
     int nunits;
-    double *scratch;              // [slot][set][48][100] partial results
+    float2 *scratch;              // [slot][set][48][100] partial results, high and low parts
     int *err;                     // FG_ETIMEDOUT after an expired wait
 };
 struct OzFinish {
     int nlist, ncell, nset;
     const int *cells;       // listed cells (48 per tile) or -1
     const int2 *fin;        // per tile: first slot, number of slots (null: split only)
-    const double *scratch;
+    const float2 *scratch;
     double *io;             // expansions [set][cell][100]
     int accumulate;         // 1: io += result
     int split;              // write digits and scales of the first split listed cells
