@@ -619,10 +619,12 @@ __global__ void k_field_pairs(size_t n3, const double *__restrict__ u, const dou
 // time, the column nodes' fields staged in shared memory in tiles of TILE entries (once where one
 // tile holds them), two entries of a row per 16-byte load. 12 FP32 operations per entry and field
 // (product with its rounding error and cross terms, two-sum), 8 bytes of the block: HBM bounds
-// it. Row r goes to out[rows ? rows[first + r] : first + r].
+// it. The next two steps' loads are issued before a step is used, the first ones before the staging,
+// in 64 registers (near field and L2P of the film 0.93 -> 0.83 ms, wire 0.57 -> 0.50; the same in 80
+// registers 0.90, the loop unrolled by four without it 0.86 but P2M 0.48 -> 0.53). Row r goes to out[rows ? rows[first + r] : first + r].
 constexpr int TILE = 1536;
 template <int NQ>
-__global__ void __launch_bounds__(256) k_block_mv(const int4 *__restrict__ task, const int *__restrict__ rows,
+__global__ void __launch_bounds__(256, 4) k_block_mv(const int4 *__restrict__ task, const int *__restrict__ rows,
                                                   const int *__restrict__ cptr, const int *__restrict__ col,
                                                   const size_t *__restrict__ boff, const float2 *__restrict__ B,
                                                   const float4 *__restrict__ m, double *__restrict__ out0,
@@ -647,7 +649,19 @@ __global__ void __launch_bounds__(256) k_block_mv(const int4 *__restrict__ task,
 #pragma unroll
         for (int q = 0; q < NQ; q++) h[0][q] = h[1][q] = l[0][q] = l[1][q] = 0.f;
         for (int base = 0; base < ne; base += TILE) {
-            const int len = min(TILE, ne - base);
+            const int len = min(TILE, ne - base), n = on0 ? len / 2 : 0;
+            const float4 *p0 = reinterpret_cast<const float4 *>(b0 + base), *p1 = reinterpret_cast<const float4 *>(b1 + base);
+            // two steps of both rows in flight, the first ones while the fields are staged
+            float4 x[2][2];
+            auto load = [&](int e) {
+#pragma unroll
+                for (int k = 0; k < 2; k++)
+                    if (e + 32 * k < n) {
+                        x[k][0] = __ldcs(p0 + e + 32 * k);
+                        x[k][1] = __ldcs(p1 + e + 32 * k);
+                    }
+            };
+            load(lane);
             if (r0 == 0 || ne > TILE) {
                 __syncthreads();
                 for (int e = threadIdx.x; e < len; e += 256) {
@@ -656,20 +670,23 @@ __global__ void __launch_bounds__(256) k_block_mv(const int4 *__restrict__ task,
                 }
                 __syncthreads();
             }
-            if (!on0) continue;
-            const float4 *p0 = reinterpret_cast<const float4 *>(b0 + base), *p1 = reinterpret_cast<const float4 *>(b1 + base);
-#pragma unroll 2
-            for (int e = lane; e < len / 2; e += 32) {
-                const float4 x0 = __ldcs(p0 + e), x1 = __ldcs(p1 + e), ma = sm[2 * e], mb = sm[2 * e + 1];
-                add(h[0][0], l[0][0], x0.x, x0.y, ma.x, ma.y);
-                add(h[1][0], l[1][0], x1.x, x1.y, ma.x, ma.y);
-                add(h[0][0], l[0][0], x0.z, x0.w, mb.x, mb.y);
-                add(h[1][0], l[1][0], x1.z, x1.w, mb.x, mb.y);
-                if constexpr (NQ == 2) {
-                    add(h[0][1], l[0][1], x0.x, x0.y, ma.z, ma.w);
-                    add(h[1][1], l[1][1], x1.x, x1.y, ma.z, ma.w);
-                    add(h[0][1], l[0][1], x0.z, x0.w, mb.z, mb.w);
-                    add(h[1][1], l[1][1], x1.z, x1.w, mb.z, mb.w);
+            for (int e = lane; e < n; e += 64) {
+                const float4 y[2][2] = {{x[0][0], x[0][1]}, {x[1][0], x[1][1]}};
+                load(e + 64);
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    if (e + 32 * k >= n) break;
+                    const float4 x0 = y[k][0], x1 = y[k][1], ma = sm[2 * (e + 32 * k)], mb = sm[2 * (e + 32 * k) + 1];
+                    add(h[0][0], l[0][0], x0.x, x0.y, ma.x, ma.y);
+                    add(h[1][0], l[1][0], x1.x, x1.y, ma.x, ma.y);
+                    add(h[0][0], l[0][0], x0.z, x0.w, mb.x, mb.y);
+                    add(h[1][0], l[1][0], x1.z, x1.w, mb.x, mb.y);
+                    if constexpr (NQ == 2) {
+                        add(h[0][1], l[0][1], x0.x, x0.y, ma.z, ma.w);
+                        add(h[1][1], l[1][1], x1.x, x1.y, ma.z, ma.w);
+                        add(h[0][1], l[0][1], x0.z, x0.w, mb.z, mb.w);
+                        add(h[1][1], l[1][1], x1.z, x1.w, mb.z, mb.w);
+                    }
                 }
             }
         }
