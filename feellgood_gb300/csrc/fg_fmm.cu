@@ -81,7 +81,7 @@ struct FmmTree {
     // hi (on a 2^-20 grid of leaf units) + lo, the charge as hi + lo; (x, y, z, q) per part
     bool ds = false;
     // The FP64 tree of an FP32 + refinement context (full evaluations, where CURRENT has no valid
-    // potentials) keeps the kernels and the order of sums that such runs have always started
+    // potentials) keeps the arithmetic and the order of the sums that such runs have always started
     // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9
     // in phiv two steps later (film), so runs repeat bit for bit only with the same last bits
     bool repeat = false;
@@ -1145,9 +1145,9 @@ __device__ __forceinline__ void l2p_p2p_pass(int leaf, int tb, int nt, int lane,
 // two SFU reciprocal square roots and one fused multiply-add per charge set, the pair
 // arithmetic of the scalar pass. The terms go straight into the pass sums (no per-leaf
 // partial sums as in the scalar pass): 128 registers, so four blocks fit on an SM, or one
-// beside a tensor-core translation CTA (1.61 -> 1.49 ms on the film; the FP32 FMM's error
-// against the FP64 FMM stays 4.7e-7 for the potential of m, 1.1e-6 instead of 7e-7 for the
-// potential of v).
+// beside a tensor-core translation CTA (1.61 -> 1.49 ms on the film, 1.26 with evenly shared
+// tasks; the FP32 FMM's error against the FP64 FMM stays 4.7e-7 for the potential of m, 1.1e-6
+// instead of 7e-7 for the potential of v).
 template <int NT, int NQ>
 __device__ __forceinline__ void l2p_p2p_pass_x2(int leaf, int tb, int nt, int lane, int li, int lj, int lk,
                                                 const int *__restrict__ leaf_src, const int *__restrict__ tgt_node,

@@ -101,9 +101,12 @@ typedef struct {
                              0 on the CUDA cores */
     int mlp_train_every;  /* learned guess: after the first mlp_train_steps solves, train on every
                              n-th successful solve only (1, the default: on every one) */
-    int fmm_native_fp64;  /* FP64 FMM: 0 (default) P2M, near field and translations in
-                             double-single arithmetic on the FP32 pipes (relative error
-                             ~1e-13); 1 all three on the FP64 pipe */
+    int fmm_native_fp64;  /* FP64 FMM: 0 (default) translations as exact digit products on the
+                             tensor cores, P2M and near field as dense double-single blocks
+                             (up to 1/8 of the device memory, else as sums over the Gauss
+                             points), relative error 1e-14 to 1e-13; 1 all three on the FP64
+                             pipe. The full FP64 evaluations of an FP32 + refinement context
+                             run all three in double-single arithmetic on the FP32 pipes */
     int solver_lpr;       /* FP32 + refinement solver: lanes sharing one row of the operator
                              (1 thread per row, 4, 8); 0 (default): the fastest, timed on the
                              first step */
