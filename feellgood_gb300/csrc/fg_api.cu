@@ -1118,14 +1118,14 @@ int fg_mlp_debug_infer(fg_ctx *h, int n, const float *feat, float *out) {
 }
 
 int fg_debug_wait_timeout(fg_ctx *h, int which) {
-    if (!h || which < 0 || which > 1) return FG_EINVAL;
+    if (!h || which < 0 || which > 2) return FG_EINVAL;
     Ctx &c = h->c;
     int *flag = nullptr;
     CK(cudaMalloc(&flag, sizeof(int)));
     int hv = 0;
     cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), c.stream);
     if (e == cudaSuccess)
-        e = which == 0 ? launch_barrier_timeout_probe(c, flag) : launch_mbar_timeout_probe(c.stream, flag);
+        e = which != 1 ? launch_barrier_timeout_probe(c, which == 2, flag) : launch_mbar_timeout_probe(c.stream, flag);
     if (e == cudaSuccess) e = cudaMemcpyAsync(&hv, flag, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c.stream);
     cudaFree(flag);
@@ -1134,8 +1134,8 @@ int fg_debug_wait_timeout(fg_ctx *h, int which) {
         c.err = std::string("fg_debug_wait_timeout: ") + cudaGetErrorString(e);
         return FG_ECUDA;
     }
-    if (hv) {
-        c.err = which == 0 ? "grid barrier: bounded wait expired" : "mbarrier: bounded wait expired";
+    if (which == 2 ? hv == 2 : hv != 0) {
+        c.err = which != 1 ? "grid barrier: bounded wait expired" : "mbarrier: bounded wait expired";
         return FG_ETIMEDOUT;
     }
     return FG_OK;

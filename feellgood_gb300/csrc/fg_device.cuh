@@ -19,9 +19,11 @@ __device__ __forceinline__ unsigned long long gtimer() {
 // counter that only grows, then a wait (acquire) until the last block's arrival is counted. That is
 // two trips to L2 where there was one for each of a generation read, the arrival, its reset and
 // release, the wait and a read of the error flag by every thread (solve of 7.7k tets, 18 barriers,
-// 127 -> 108 us; of the 1.2M-tet film in FP64 0.48 -> 0.46 ms). The wait is bounded: after 2 s
-// without progress it records FG_ETIMEDOUT and returns false; every block then leaves the kernel, so
-// no launch can hang the GPU.
+// 127 -> 108 us; of the 1.2M-tet film in FP64 0.48 -> 0.46 ms). The wait is bounded: a block that saw no
+// progress for 2 s takes the round back (the counter returns to the round's begin, marked expired)
+// and returns false. It can do so only while an arrival is missing, and a marked round never
+// completes: a block that arrives late, or still waits, returns false too. So every block passes a
+// round or none does, each leaves the kernel at the same barrier, and no launch can hang the GPU.
 __device__ inline bool grid_sync(GridBar *gb) {
     if (gridDim.x == 1) {  // a single block meets itself
         __syncthreads();
@@ -30,21 +32,19 @@ __device__ inline bool grid_sync(GridBar *gb) {
     int ok = 1;
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned int ticket, seen;
-        asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(&gb->count) : "memory");
-        const unsigned int last = ticket - ticket % gridDim.x + gridDim.x;  // the counter after the round
+        constexpr unsigned long long EXPIRED = 1ull << 63;
+        unsigned long long ticket, seen;
+        asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(ticket) : "l"(&gb->count) : "memory");
+        const unsigned long long part = ticket >> 32 ? ticket % gridDim.x : (unsigned)ticket % gridDim.x;
+        const unsigned long long begin = ticket - part, last = begin + gridDim.x;  // of the round
         const unsigned long long t0 = gtimer();
-        for (int k = 1;; k++) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&gb->count) : "memory");
-            if ((int)(seen - last) >= 0) break;
-            if (k % 32 == 0) {
-                if (*(volatile int *)&gb->err) ok = 0;
-                else if (gtimer() - t0 > 2000000000ull) {
-                    atomicExch(&gb->err, FG_ETIMEDOUT);
-                    ok = 0;
-                }
-                if (!ok) break;
-            }
+        if (ticket & EXPIRED) ok = 0;
+        for (int k = 1; ok; k++) {
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(&gb->count) : "memory");
+            if ((seen & ~EXPIRED) >= last) break;  // also where a later round has expired
+            if (seen & EXPIRED) ok = 0;
+            else if (k % 32 == 0 && gtimer() - t0 > 2000000000ull && atomicCAS(&gb->count, seen, EXPIRED | begin) == seen)
+                ok = 0;
         }
     }
     return __syncthreads_and(ok);

@@ -95,8 +95,7 @@ struct SegAcc {
 
 // Grid-wide barrier state of the persistent kernels (bounded wait, no hang), zero at each launch.
 struct GridBar {
-    unsigned int count;  // arrivals since the launch
-    int err;             // FG_ETIMEDOUT once a wait expired
+    unsigned long long count;  // arrivals since the launch; the top bit once a wait has expired
 };
 
 // Arguments of the FP64 BiCGSTAB persistent kernel (bicg_dir, src/algebra/bicg.h:163-234).
@@ -400,7 +399,7 @@ int mixed_max_blocks(Ctx &c);
 // co-resident blocks, 2 or 1 per SM); the node kernel is rerun before each timing.
 cudaError_t mixed_autotune(Ctx &c, double dt, double prefactor, double angle);
 // failure-path probes: a bounded device wait that nothing ends (*out / *err set on expiry)
-cudaError_t launch_barrier_timeout_probe(Ctx &c, int *out);
+cudaError_t launch_barrier_timeout_probe(Ctx &c, int late, int *out);
 cudaError_t launch_mbar_timeout_probe(cudaStream_t st, int *err);
 // throughput probe of tcgen05.mma kind::tf32 (M = 128, N = n, K = 8), one CTA per SM
 cudaError_t launch_peak_mma_tf32(cudaStream_t st, int grid, int n, int iters, long long *cyc, int *err);

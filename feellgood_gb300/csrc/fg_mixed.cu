@@ -584,15 +584,23 @@ cudaError_t launch_mixed(Ctx &c, double dt, double prefactor) {
     return cudaLaunchKernelEx(&cfg, k_mixed<1>, a);
 }
 
-// Failure-path probe: block 0 leaves without arriving at the grid barrier, so block 1's
-// bounded wait must expire (about 2 s), set the barrier's error and return false.
-__global__ void k_barrier_timeout_probe(GridBar *bar, int *out) {
-    if (blockIdx.x == 0) return;
+// Failure-path probe: block 0 leaves without arriving at the grid barrier, or (late) arrives once
+// block 1 has given up (a bounded wait as well), so block 1's bounded wait must expire (about 2 s)
+// and every block that arrives must be told: out counts those that were.
+__global__ void k_barrier_timeout_probe(GridBar *bar, int late, int *out) {
+    if (blockIdx.x == 0) {
+        if (!late) return;
+        const unsigned long long t0 = gtimer();
+        if (threadIdx.x == 0)
+            while (*(volatile int *)out == 0 && gtimer() - t0 < 4000000000ull) {
+            }
+        __syncthreads();
+    }
     const bool ok = grid_sync(bar);
-    if (threadIdx.x == 0 && !ok) atomicExch(out, 1);
+    if (threadIdx.x == 0 && !ok) atomicAdd(out, 1);
 }
 
-cudaError_t launch_barrier_timeout_probe(Ctx &c, int *out) {
+cudaError_t launch_barrier_timeout_probe(Ctx &c, int late, int *out) {
     cudaError_t e = cudaMemsetAsync(c.bar, 0, sizeof(GridBar), c.stream);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -604,7 +612,7 @@ cudaError_t launch_barrier_timeout_probe(Ctx &c, int *out) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_barrier_timeout_probe, c.bar, out);
+    return cudaLaunchKernelEx(&cfg, k_barrier_timeout_probe, c.bar, late, out);
 }
 
 // Co-resident blocks per SM of the variant with LPR lanes per row at the given block size.

@@ -24,3 +24,11 @@ def test_bounded_wait_expires_and_context_survives(which):
     c.compute_all(np.zeros(3))
     st = c.get_state(0)
     assert np.all(np.isfinite(st["u"])) and np.allclose(np.linalg.norm(st["u"], axis=1), 1.0)
+
+
+def test_a_round_of_the_grid_barrier_is_passed_by_all_blocks_or_by_none():
+    """A block that reaches the barrier after another has given up is told so as well: were it let
+    through, the node update behind a solver's last barrier would run for some rows only."""
+    m = cases.cuboid(3, 3, 3)
+    c = fg.Context(m, cases.regions())
+    assert c.debug_wait_timeout(2) == fg.FG_ETIMEDOUT
