@@ -809,8 +809,7 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
         cols += nc;
         if (cols > 0x7fffffff || (own && (size_t)t.nleaf * NRM > 0x7fffffff)) return done(cudaSuccess);
         cptr[l + 1] = (int)cols;
-        boff[l] = entries;
-        if (nc == 0 && !own) continue;
+        boff[l] = entries;  // a leaf without columns has tasks too: its rows are zero
         entries += (size_t)nt * 3 * nc;
         // near field: up to 16 rows; P2M: all rows of a leaf (few columns), or 16 where a tile of
         // columns does not hold them

@@ -98,3 +98,24 @@ def test_not_a_number_propagates():
     c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=-3)
     c.set_state(u)
     assert np.isnan(c.demag(0)).all()
+
+
+# a coarse mesh at a large depth: interior nodes with no Gauss point in the leaves around them, whose
+# near field is zero
+@pytest.mark.parametrize("shape,leaf", [((2, 2, 2), -6), ((4, 3, 2), -7)])
+@pytest.mark.parametrize("first_order", [0, 1])
+def test_fp64_fmm_targets_without_near_sources(shape, leaf, first_order):
+    m = cases.cuboid(*shape)
+    u = cases.perturbed_state(m["xyz"], seed=25, sigma=0.3)
+    v = cases.tangent_field(u, seed=26)
+    pot = []
+    for native in (0, 1):
+        c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=leaf, fmm_native_fp64=native,
+                       first_order=first_order)
+        c.set_state(u, v)
+        c.compute_all(np.zeros(3))
+        s = c.get_state(0)
+        pot.append((s["phi"], s["phiv"], c.demag(0), c.demag(1)))
+    # as test_fp64_fmm_edges
+    for k in (0, 2, 3) if first_order else range(4):
+        assert _rel(pot[0][k], pot[1][k]) < (2e-13 if k % 2 == 0 else 1e-12)
