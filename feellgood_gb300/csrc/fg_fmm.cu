@@ -2807,13 +2807,9 @@ cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f) {
 
 int fmm_eval_fp64(Ctx &c, int nq) {
     FmmTree *t32 = static_cast<FmmTree *>(c.fmm);
-    if (!t32) {
-        c.err = "fmm: no tree";
+    if (!t32 || !t32->fp32) {
+        c.err = "fmm: no FP32 tree";
         return FG_EINVAL;
-    }
-    if (!t32->fp32) {
-        FCK(fmm_eval_t<double>(c, *t32, nq, FmmFields{}));
-        return FG_OK;
     }
     if (!c.fmm64) {
         // the same depth (and so the same source order, src_dst) as the FP32 tree

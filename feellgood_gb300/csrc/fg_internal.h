@@ -414,8 +414,8 @@ struct FmmFields {
 bool fmm_whole(const Ctx &c);
 bool fmm_charges(const Ctx &c);  // the evaluation reads charges (else it starts from the fields)
 cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f);  // nq 2: c.src_q2 -> c.pot2 beside c.src_q -> c.pot
-// The same evaluation with an FP64 tree of the FP32 tree's depth (built on first use; the
-// FP32 tree itself when the context is FP64); FG_* status
+// The evaluation of an FP32 tree's charges with an FP64 tree of the same depth (built on first
+// use); FG_* status
 int fmm_eval_fp64(Ctx &c, int nq);
 void fmm64_free(Ctx &c);
 int fmm_launches_per_eval(const Ctx &c, int nq = 1);  // kernels one FMM evaluation launches  // device int: FG_ETIMEDOUT after an expired wait (or nullptr)
