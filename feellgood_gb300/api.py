@@ -62,7 +62,7 @@ class fg_opts(C.Structure):
                 ("mlp_train_every", C.c_int), ("fmm_native_fp64", C.c_int),
                 ("solver_lpr", C.c_int), ("solver_blocks", C.c_int), ("spin_acc", C.c_int), ("spin_tol", C.c_double),
                 ("spin_max_iter", C.c_int), ("demag_increment", C.c_int), ("fmm_overlap", C.c_int),
-                ("fmm_tree_host", C.c_int), ("solver_threads", C.c_int)]
+                ("fmm_tree_host", C.c_int), ("solver_threads", C.c_int), ("demag_blocks", C.c_int)]
 
 
 class fg_step_report(C.Structure):
@@ -125,6 +125,7 @@ SIGNATURES = {
     "fg_mlp_nparam": (C.c_int, []),
     "fg_mlp_debug_infer": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "fg_solver_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
+    "fg_demag_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_longlong)]),
     "fg_debug_wait_timeout": (C.c_int, [C.c_void_p, C.c_int]),
     "fg_gauss_points": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.c_void_p]),
     "fg_spin_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int), C.c_void_p, C.POINTER(C.c_int),
@@ -209,7 +210,8 @@ def rng_seed(seed):
 
 class fg_checkpoint_shape(C.Structure):
     _fields_ = [("n_nodes", C.c_int), ("n_mag_tets", C.c_int), ("precision", C.c_int), ("solver_lpr", C.c_int),
-                ("solver_blocks", C.c_int), ("fmm_depth", C.c_int), ("solver_threads", C.c_int)]
+                ("solver_blocks", C.c_int), ("fmm_depth", C.c_int), ("solver_threads", C.c_int),
+                ("demag_blocks", C.c_int)]
 
 
 class fg_checkpoint_meta(C.Structure):
@@ -453,6 +455,12 @@ class Context:
         if s == FG_ETIMEDOUT or s > FG_ETIMEDOUT:
             self._check(s)
         return s, [{k: getattr(r, k) for k, _ in fg_batch_report._fields_} for r in reps]
+
+    def demag_info(self):
+        """fg_demag_info: (form of the demag: 0, 1 sums, 2 or 3 blocks; device bytes of the blocks)."""
+        v, b = C.c_int(), C.c_longlong()
+        self._check(self.L.fg_demag_info(self.h, C.byref(v), C.byref(b)))
+        return v.value, b.value
 
     def debug_wait_timeout(self, which):
         """fg_debug_wait_timeout: the status a deliberately unended bounded device wait reports."""

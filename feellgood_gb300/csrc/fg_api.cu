@@ -139,6 +139,7 @@ void fg_opts_default(fg_opts *o) {
     o->fmm_overlap = 0;
     o->fmm_tree_host = 0;
     o->solver_threads = 0;
+    o->demag_blocks = 0;
 }
 
 const char *fg_strerror(int s) {
@@ -181,6 +182,10 @@ static int create_impl(fg_ctx *h, const fg_mesh *m, const fg_region *regs, int n
     }
     if (c.opts.solver_threads != 0 && c.opts.solver_threads != 256 && c.opts.solver_threads != 512) {
         c.err = "fg_create: solver_threads must be 0, 256 or 512";
+        return FG_EINVAL;
+    }
+    if (c.opts.demag_blocks < 0 || c.opts.demag_blocks > 3) {
+        c.err = "fg_create: demag_blocks must be 0, 1, 2 or 3";
         return FG_EINVAL;
     }
     if (!m || !regs || nreg <= 0 || m->n_nodes <= 0 || m->n_tets <= 0 || !m->xyz || !m->tet4 || !m->tet_region) {
@@ -584,6 +589,10 @@ static int create_impl(fg_ctx *h, const fg_mesh *m, const fg_region *regs, int n
         if (s != FG_OK) return s;
     } else {
         CK(dense_build(c, R));
+        if (!c.direct_mat && c.opts.demag_blocks >= 2 && c.n_mag_nodes > 0) {
+            c.err = "fg_create: the direct sum's matrix of demag_blocks does not fit in the device's memory";
+            return FG_ENOMEM;
+        }
         if (!c.direct_mat) {
             c.direct_nsplit = direct_splits(c);
             CK(dalloc(&c.direct_part, (c.opts.first_order ? 1 : 2) * (size_t)c.direct_nsplit * std::max(1, c.n_mag_nodes)));
@@ -1093,6 +1102,20 @@ int fg_counters(const fg_ctx *h, long long out[4]) {
     out[1] = L;
     out[2] = (long long)a;
     out[3] = (long long)b;
+    return FG_OK;
+}
+
+int fg_demag_info(const fg_ctx *h, int *blocks, long long *bytes) {
+    if (!h) return FG_EINVAL;
+    const Ctx &c = h->c;
+    size_t b = 0;
+    int form = fmm_blocks(c, &b);
+    if (c.opts.demag == FG_DEMAG_DIRECT) {
+        form = c.direct_mat ? 3 : 1;
+        b = c.direct_mat ? 24 * (size_t)c.n_mag_nodes * c.n_mag_nodes : 0;
+    }
+    if (blocks) *blocks = form;
+    if (bytes) *bytes = (long long)b;
     return FG_OK;
 }
 

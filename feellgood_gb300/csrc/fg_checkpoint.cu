@@ -3,7 +3,8 @@
 //
 // File layout (little-endian, fields written one by one, no padding):
 //   "FGGPUCK1" | u32 version | i32 n_nodes, n_mag_tets, precision, solver_lpr,
-//   solver_blocks, fmm_depth, solver_threads (version 2; version 1 ends at fmm_depth) |
+//   solver_blocks, fmm_depth, solver_threads (from version 2 on), demag_blocks (version 4; there
+//   is no version 3) |
 //   meta: f64 t0, t, dt, dt_soft_max | i64 steps,
 //   output_index | u32 rng_seed | i64 rng_draws | f64 E[4] | f64 u[3n], v[3n], phi[n],
 //   phiv[n] (CURRENT, node order of the set-up mesh) | u64 FNV-1a of all preceding bytes
@@ -22,7 +23,7 @@ int fmm_info(const Ctx &c, int *L, int *nleaf, double *n_m2l, double *n_p2p);
 namespace {
 
 constexpr char MAGIC[8] = {'F', 'G', 'G', 'P', 'U', 'C', 'K', '1'};
-constexpr uint32_t VERSION = 2;  // 2: solver_threads after fmm_depth (1 is still read)
+constexpr uint32_t VERSION = 4;  // 1 and 2 are still read
 
 struct Writer {
     std::vector<unsigned char> buf;
@@ -69,7 +70,7 @@ void put_header(Writer &w, const fg_checkpoint_shape &s, const fg_checkpoint_met
     w.put(VERSION);
     w.put<int32_t>(s.n_nodes); w.put<int32_t>(s.n_mag_tets); w.put<int32_t>(s.precision);
     w.put<int32_t>(s.solver_lpr); w.put<int32_t>(s.solver_blocks); w.put<int32_t>(s.fmm_depth);
-    w.put<int32_t>(s.solver_threads);
+    w.put<int32_t>(s.solver_threads); w.put<int32_t>(s.demag_blocks);
     w.put(m.t0); w.put(m.t); w.put(m.dt); w.put(m.dt_soft_max);
     w.put<int64_t>(m.steps); w.put<int64_t>(m.output_index);
     w.put<uint32_t>(m.rng_seed); w.put<int64_t>(m.rng_draws);
@@ -96,10 +97,11 @@ int get_header(const std::string &path, std::vector<unsigned char> &buf, Reader 
     r.get_bytes(magic, 8);
     if (std::memcmp(magic, MAGIC, 8) != 0) return FG_EIO;
     const uint32_t version = r.get<uint32_t>();
-    if (version != 1 && version != VERSION) return FG_EIO;
+    if (version != 1 && version != 2 && version != VERSION) return FG_EIO;
     s.n_nodes = r.get<int32_t>(); s.n_mag_tets = r.get<int32_t>(); s.precision = r.get<int32_t>();
     s.solver_lpr = r.get<int32_t>(); s.solver_blocks = r.get<int32_t>(); s.fmm_depth = r.get<int32_t>();
     s.solver_threads = version >= 2 ? r.get<int32_t>() : 0;
+    s.demag_blocks = version >= 4 ? r.get<int32_t>() : 0;
     m.t0 = r.get<double>(); m.t = r.get<double>(); m.dt = r.get<double>(); m.dt_soft_max = r.get<double>();
     m.steps = r.get<int64_t>(); m.output_index = r.get<int64_t>();
     m.rng_seed = r.get<uint32_t>(); m.rng_draws = r.get<int64_t>();
@@ -133,6 +135,7 @@ int fg_checkpoint_save(fg_ctx *h, const char *path, const fg_checkpoint_meta *me
         fg::fmm_info(c, &L, &nl, &a, &b);
         s.fmm_depth = L;
     }
+    fg_demag_info(h, &s.demag_blocks, nullptr);
     const size_t n = (size_t)c.nn;
     std::vector<double> u(3 * n), v(3 * n), phi(n), phiv(n);
     int st = fg_get_state(h, 0, u.data(), v.data(), phi.data(), phiv.data());

@@ -162,14 +162,16 @@ __global__ void k_dense_sum(int n, const int *__restrict__ nodes, int nshare, co
 }  // namespace
 
 // Forms B where it fits: at most 1/16 of the device's memory (12,000 nodes take 3.5 GB) and half of
-// what is free. Without it (direct_mat null) the sum over Gauss points runs.
+// what is free, unless fg_opts.demag_blocks asks for it or against it. Without it (direct_mat null)
+// the sum over Gauss points runs.
 cudaError_t dense_build(Ctx &c, const Rules &R) {
     const int n = c.n_mag_nodes;
     size_t free_b = 0, total_b = 0;
     cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
     if (e != cudaSuccess) return e;
     const size_t bytes = 24 * (size_t)n * n, ncol = (size_t)c.nmt + 3 * (size_t)c.nft;
-    if (n == 0 || bytes > std::min(total_b / 16, free_b / 2)) return cudaSuccess;
+    if (n == 0 || c.opts.demag_blocks == 1) return cudaSuccess;
+    if (c.opts.demag_blocks == 0 && bytes > std::min(total_b / 16, free_b / 2)) return cudaSuccess;
     double *G = nullptr;
     // shares of the columns: 8 blocks per SM in all (the last wave costs little and the FP64 pipe of
     // every SM is busy), at least 32 nodes in each
@@ -763,9 +765,10 @@ __global__ void __launch_bounds__(128) k_l2p_apply(int ntgt, const int *__restri
 
 }  // namespace
 
-// Forms the blocks of one kind (own: P2M, else near field) where they fit: at most 1/8 of the
-// device's memory, half of what is free, MAX_NODE columns and MAX_ELEM (MAX_OWN) elements per leaf.
-// Without them (N.B null) the sums over Gauss points run.
+// Forms the blocks of one kind (own: P2M, else near field) where they fit: MAX_NODE columns and
+// MAX_ELEM (MAX_OWN) elements per leaf and, unless fg_opts.demag_blocks asks for them, at most 1/8 of
+// the device's memory and half of what is free. Without them (N.B null) the sums over Gauss points
+// run; N.why then tells whether memory (FG_ENOMEM) or a leaf (FG_EINVAL) was the reason.
 static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool own, DenseBlocks &N) {
     size_t free_b = 0, total_b = 0;
     cudaError_t e = cudaMemGetInfo(&free_b, &total_b);
@@ -779,7 +782,11 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
     auto done = [&](cudaError_t r) {
         if (ncol) cudaFree(ncol);
         if (scratch) cudaFree(scratch);
-        if (r != cudaSuccess || !N.B) blocks_free(N);
+        if (r != cudaSuccess || !N.B) {
+            const int why = r == cudaErrorMemoryAllocation ? FG_ENOMEM : N.why;
+            blocks_free(N);
+            N.why = why;
+        }
         cudaGetLastError();
         // what does not fit is no error: the sums over Gauss points need none of it
         return r == cudaErrorMemoryAllocation ? cudaSuccess : r;
@@ -799,6 +806,7 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
     std::vector<int> hn(t.nleaf + 1);
     NCK(cudaMemcpyAsync(hn.data(), ncol, sizeof(int) * (t.nleaf + 1), cudaMemcpyDeviceToHost, c.stream));
     NCK(cudaStreamSynchronize(c.stream));
+    N.why = FG_EINVAL;
     if (hn[t.nleaf]) return done(cudaSuccess);
     std::vector<int> cptr(t.nleaf + 1, 0);
     std::vector<size_t> boff(t.nleaf, 0);
@@ -819,7 +827,10 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
             task.push_back(make_int4(l, b, f - b, (own ? NRM * l : t.h_leaf_tgt[l]) + b));
         }
     }
-    if (entries == 0 || entries * sizeof(float2) > std::min(total_b / 8, free_b / 2)) return done(cudaSuccess);
+    if (entries == 0) return done(cudaSuccess);
+    N.why = FG_ENOMEM;
+    N.bytes = entries * sizeof(float2);
+    if (c.opts.demag_blocks == 0 && N.bytes > std::min(total_b / 8, free_b / 2)) return done(cudaSuccess);
     N.ntask = (int)task.size();
     NCK(cudaMalloc(&scratch, sizeof(double) * (own ? (size_t)OWN_HASH * NRM : (size_t)HASH * TG) * blocks));
     NCK(cudaMalloc(&N.cptr, sizeof(int) * (t.nleaf + 1)));
@@ -857,12 +868,13 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
 cudaError_t near_build(Ctx &c, const Rules &R, const NearTree &t, NearMat &N) {
     cudaError_t e = blocks_build(c, R, t, false, N.near);
     if (e != cudaSuccess || !N.near.B) return e;
-    e = blocks_build(c, R, t, true, N.p2m);
+    if (c.opts.demag_blocks != 2) e = blocks_build(c, R, t, true, N.p2m);
     if (e != cudaSuccess) return e;
     if (cudaMalloc(&N.field, sizeof(float4) * 3 * (size_t)c.nn) != cudaSuccess ||
         cudaMalloc(&N.l2p, sizeof(double) * NRM * (size_t)std::max(1, t.ntgt)) != cudaSuccess) {
         cudaGetLastError();
         near_free(N);
+        N.near.why = FG_ENOMEM;
         return cudaSuccess;
     }
     if (t.ntgt > 0) k_l2p_table<<<(t.ntgt + 127) / 128, 128, 0, c.stream>>>(t.ntgt, t.tloc, N.l2p);

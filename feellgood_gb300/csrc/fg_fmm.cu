@@ -1845,6 +1845,16 @@ static std::vector<SamplePts> split_samples(const Ctx &c) {
     return S;
 }
 
+// The tree has not the blocks that fg_opts.demag_blocks asks for: the reason, with c.err (else FG_OK).
+static int blocks_missing(Ctx &c, const FmmTree &t) {
+    const int want = t.oz ? c.opts.demag_blocks : 0;
+    const DenseBlocks *none = want >= 2 && !t.near.near.B ? &t.near.near : want == 3 && !t.near.p2m.B ? &t.near.p2m : nullptr;
+    if (!none) return FG_OK;
+    c.err = none->why == FG_ENOMEM ? "fmm: the blocks of demag_blocks do not fit in the device's memory"
+                                   : "fmm: demag_blocks: a leaf of the tree has too many elements for a block";
+    return none->why == FG_ENOMEM ? FG_ENOMEM : FG_EINVAL;
+}
+
 int fmm_build(Ctx &c) {
     const bool fp32 = (c.opts.precision == FG_PREC_FP32_REFINE);
     if (c.opts.fmm_order != 0 && c.opts.fmm_order != FMM_P) {
@@ -1917,7 +1927,7 @@ int fmm_build(Ctx &c) {
     }
     cudaMemsetAsync(c.src_q, 0, sizeof(double) * std::max(1, c.nsrc), c.stream);
     if (c.src_q2) cudaMemsetAsync(c.src_q2, 0, sizeof(double) * std::max(1, c.nsrc), c.stream);
-    int bestL = cands[0];
+    int bestL = cands[0], missing = FG_OK;
     double bestms = 1e300;
     for (size_t k = 0; k < cands.size(); k++) {
         fmm_free(c);
@@ -1926,6 +1936,11 @@ int fmm_build(Ctx &c) {
         t->fp32 = fp32;
         int s = fmm_build_forest(c, cands[k]);
         if (s != FG_OK) return s;
+        if (const int why = blocks_missing(c, *t)) {
+            if (cands.size() == 1) return why;
+            missing = why;
+            continue;  // another depth may have them
+        }
         if (cands.size() == 1) {
             c.fmm_setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_begin).count();
             return FG_OK;
@@ -1948,6 +1963,7 @@ int fmm_build(Ctx &c) {
         if (c.opts.verbose) fprintf(stderr, "fmm autotune: L=%d %.3f ms/eval\n", cands[k], ms / 2);
         if (ms < bestms) { bestms = ms; bestL = cands[k]; }
     }
+    if (bestms == 1e300) return missing;
     fmm_free(c);
     FmmTree *t = new FmmTree();
     c.fmm = t;
@@ -2479,7 +2495,7 @@ static int fmm_build_forest(Ctx &c, int L) {
     if (c.src_dst) cudaFree(c.src_dst);
     c.src_dst = nullptr;
     FCK(up(&c.src_dst, src_dst));
-    if (t->oz) {
+    if (t->oz && c.opts.demag_blocks != 1) {
         std::vector<int> orig(c.nsrc);
         for (int k = 0; k < c.nsrc; k++) orig[src_dst[k]] = k;
         int *d_orig = nullptr;
@@ -2787,6 +2803,15 @@ static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f) {
     }
     const cudaError_t e = cudaGetLastError();
     return terr != cudaSuccess ? terr : e;
+}
+
+int fmm_blocks(const Ctx &c, size_t *bytes) {
+    const FmmTree *t = static_cast<const FmmTree *>(c.fmm);
+    *bytes = 0;
+    if (!t || !t->oz) return 0;
+    if (!t->near.near.B) return 1;
+    *bytes = t->near.near.bytes + t->near.p2m.bytes;
+    return t->near.p2m.B ? 3 : 2;
 }
 
 bool fmm_whole(const Ctx &c) {

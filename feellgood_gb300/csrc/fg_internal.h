@@ -355,6 +355,8 @@ struct DenseBlocks {
     float2 *B = nullptr;                  // [row][3 columns] double-single; null: no blocks
     int4 *task = nullptr;                 // leaf, first row, rows, first output
     int ntask = 0;
+    size_t bytes = 0;                     // of B
+    int why = 0;                          // B null: FG_ENOMEM, or FG_EINVAL where a leaf is too large
 };
 struct NearMat {
     DenseBlocks near, p2m;
@@ -412,6 +414,7 @@ struct FmmFields {
     double *phi[2];
 };
 bool fmm_whole(const Ctx &c);
+int fmm_blocks(const Ctx &c, size_t *bytes);  // fg_demag_info of the FMM's tree
 bool fmm_charges(const Ctx &c);  // the evaluation reads charges (else it starts from the fields)
 cudaError_t fmm_eval(Ctx &c, int nq, const FmmFields &f);  // nq 2: c.src_q2 -> c.pot2 beside c.src_q -> c.pot
 // The evaluation of an FP32 tree's charges with an FP64 tree of the same depth (built on first

@@ -251,11 +251,13 @@ int run_impl(Run &R, const char *settings_path, unsigned int seed, int verbose, 
     o.solver_blocks = S.solver_blocks;
     o.solver_threads = S.solver_threads;
     if (S.fmm_depth > 0) o.fmm_leaf = -S.fmm_depth;
+    o.demag_blocks = S.demag_blocks;
     if (resume) {
         o.solver_lpr = ck.solver_lpr;
         o.solver_blocks = ck.solver_blocks;
         o.solver_threads = ck.solver_threads;
         if (ck.fmm_depth > 0) o.fmm_leaf = -ck.fmm_depth;
+        if (ck.demag_blocks > 0) o.demag_blocks = ck.demag_blocks;
     }
     o.tol = S.tol;
     o.max_iter = S.max_iter;
@@ -268,6 +270,14 @@ int run_impl(Run &R, const char *settings_path, unsigned int seed, int verbose, 
     fg_mesh m;
     fg_mesh_view(R.md, &m);
     s = fg_create(&m, regs.data(), (int)regs.size(), tregs.data(), R.md->n_surf_regions, &o, &R.ctx);
+    if (s != FG_OK && resume && ck.demag_blocks > 1) {  // e.g. less memory than the original run had
+        const std::string why = fg_last_error(nullptr);
+        o.demag_blocks = S.demag_blocks;
+        s = fg_create(&m, regs.data(), (int)regs.size(), tregs.data(), R.md->n_surf_regions, &o, &R.ctx);
+        if (s == FG_OK)
+            std::fprintf(stderr, "warning: %s; the continuation does not repeat the uninterrupted run bit for bit\n",
+                         why.c_str());
+    }
     if (s != FG_OK) return fail(s, fg_last_error(nullptr));
     const int nn = R.md->n_nodes;
     if (S.spin_acc && S.V_file) {  // electrostatSolver::save (src/electrostatSolver.cpp:133-152)

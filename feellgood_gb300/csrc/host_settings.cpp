@@ -451,6 +451,7 @@ void apply_yaml(Settings &S, const std::shared_ptr<YNode> &y) {
         count("solver_blocks", S.solver_blocks);
         count("solver_threads", S.solver_threads);
         count("fmm_depth", S.fmm_depth);
+        count("demag_blocks", S.demag_blocks);
     }
 }
 

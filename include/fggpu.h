@@ -103,8 +103,8 @@ typedef struct {
                              n-th successful solve only (1, the default: on every one) */
     int fmm_native_fp64;  /* FP64 FMM: 0 (default) translations as exact digit products on the
                              tensor cores, P2M and near field as dense double-single blocks
-                             (up to 1/8 of the device memory, else as sums over the Gauss
-                             points), relative error 1e-14 to 1e-13; 1 all three on the FP64
+                             where they fit (demag_blocks), else as sums over the Gauss
+                             points, relative error 1e-14 to 1e-13; 1 all three on the FP64
                              pipe. The full FP64 evaluations of an FP32 + refinement context
                              run all three in double-single arithmetic on the FP32 pipes */
     int solver_lpr;       /* FP32 + refinement solver: lanes sharing one row of the operator
@@ -112,8 +112,8 @@ typedef struct {
                              first step */
     int solver_blocks;    /* FP32 + refinement solver with solver_lpr set: persistent blocks
                              (0: all co-resident blocks). Fixing both, solver_threads (and
-                             fmm_leaf = -depth) makes runs repeat bit for bit: the timed
-                             choices decide the order of the solver's reductions */
+                             fmm_leaf = -depth, demag_blocks) makes runs repeat bit for bit:
+                             the timed choices decide the order of the solver's reductions */
     int spin_acc;         /* 1: spin accumulation coupling (spin_accumulation.enable): the
                              electrostatic potential is solved once, the spin accumulation s
                              in every fg_compute_all, and its field Hst enters the next
@@ -140,6 +140,18 @@ typedef struct {
                              block, 256 or 512 (one block per SM: twice the warps to hide the
                              operator's gathers, the same number of grid-barrier participants);
                              0: 256 */
+    int demag_blocks;     /* direct sum and FP64 FMM (fmm_native_fp64 = 0): what the fields are
+                             multiplied with. 0 (default): dense blocks over the nodes where they
+                             fit (the direct sum's matrix in 1/16 of the device's memory, the FMM's
+                             near-field and P2M blocks in 1/8 each, none in more than half of what
+                             is free at creation), else sums over the Gauss points; 1 sums over the
+                             Gauss points (least memory); 2 the matrix, or near-field blocks and P2M
+                             as sums; 3 the matrix, or both kinds of blocks. With 2 and 3 creation
+                             fails (FG_ENOMEM, or FG_EINVAL where a leaf of the tree is too large
+                             for a block) instead of choosing otherwise. The forms round
+                             differently (a relative 1e-14 to 1e-12): fix the option where runs
+                             have to repeat bit for bit beside other users of the memory;
+                             fg_demag_info tells the form in use */
 } fg_opts;
 
 typedef struct {
@@ -237,9 +249,9 @@ int fg_set_drift(fg_ctx *ctx, int direction, double vdrift);
  * keeps u and phi to 7 digits and loses v and phiv, src/save.cpp:164-186). The file holds the
  * CURRENT state (u, v, phi, phiv in FP64), the caller's run metadata below, and the choices
  * that fix the order of the solver's and the FMM's arithmetic (solver lanes per row and
- * blocks and threads, FMM depth), so that a run resumed from it with those choices
- * (fg_opts.solver_lpr, solver_blocks, solver_threads, fmm_leaf = -depth) repeats the
- * uninterrupted run bit for bit (the learned
+ * blocks and threads, FMM depth, blocks or sums of the demag), so that a run resumed from it
+ * with those choices (fg_opts.solver_lpr, solver_blocks, solver_threads, fmm_leaf = -depth,
+ * demag_blocks) repeats the uninterrupted run bit for bit (the learned
  * guess's network is not saved: with it the resumed run agrees to the solver tolerance).
  * Binary, little-endian, with an FNV-1a checksum; fg_checkpoint_peek reads the header
  * without a context. Call fg_checkpoint_save after fg_compute_all. */
@@ -256,6 +268,7 @@ typedef struct {
     int n_nodes, n_mag_tets, precision;
     int solver_lpr, solver_blocks, fmm_depth; /* 0 where not used */
     int solver_threads;                       /* 0 where not used (and in version-1 files) */
+    int demag_blocks;                         /* 0 where not used (and in files before version 4) */
 } fg_checkpoint_shape;
 int fg_checkpoint_save(fg_ctx *ctx, const char *path, const fg_checkpoint_meta *meta);
 int fg_checkpoint_peek(const char *path, fg_checkpoint_shape *shape, fg_checkpoint_meta *meta);
@@ -288,6 +301,12 @@ int fg_timings(const fg_ctx *ctx, double ms[5]);
 /* Counters: [0] kernels launched by the context so far, [1] FMM tree depth (0 without FMM),
  * [2] M2L (cell, cell) pairs, [3] P2P (target, source) pairs per evaluation. */
 int fg_counters(const fg_ctx *ctx, long long out[4]);
+
+/* What the demag is formed from (fg_opts.demag_blocks): *blocks 1 sums over Gauss points, 2
+ * near-field blocks and P2M as sums, 3 the direct sum's matrix or both kinds of blocks, 0 an FMM
+ * that has no such choice (FP32, or fmm_native_fp64); *bytes of device memory that the matrix or
+ * the blocks take. Either may be NULL. */
+int fg_demag_info(const fg_ctx *ctx, int *blocks, long long *bytes);
 
 /* Failure-path check (no reference counterpart): runs a device wait that nothing ends —
  * which 0: the persistent solvers' grid barrier with one block that never arrives (about

@@ -210,3 +210,27 @@ def test_settings_spin_accumulation(tmp_path):
     assert surf["ground"]["V"] == 0 and surf["ground"]["s"] == [0, 0, 0] and surf["ground"]["jn"] is None
     assert surf["contact"]["jn"] == 1e11 and surf["contact"]["uP"] == [0, 1, 0] and surf["contact"]["V"] is None
     assert fg.settings_dump(p)["recentering"] == {"enable": True, "direction": 1, "threshold": 0.2}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("demag", ["direct", "fmm"])
+def test_checkpoint_resume_keeps_the_form_of_the_demag(tmp_path, golden_dir, demag):
+    """A run whose demag ran as sums over Gauss points (as where the blocks do not fit in the memory
+    that is free) is resumed with the same sums where the blocks would fit: it repeats the
+    uninterrupted run to the last printed digit."""
+    g, st = _full_test_settings(golden_dir, tmp_path)
+    gpu = {"demag": demag, "demag_blocks": 1, "fmm_depth": 3}
+    out = dict(st["outputs"], evol_columns=["t", "<Mx>", "<My>", "<Mz>", "E_ex", "E_demag", "E_zeeman", "E_tot"])
+
+    def run(name, until, **gpu):
+        s = dict(st, gpu=gpu, outputs=dict(out, file_basename=name, final_time=until * g["evol_time_step"]))
+        (tmp_path / f"{name}.json").write_text(json.dumps(s))
+        fg.run(tmp_path / f"{name}.json", seed=5)
+        return [l for l in open(tmp_path / f"{name}.evol") if not l.startswith("#")]
+
+    run("split", 3, checkpoint_every=4, **gpu)
+    head = fg.checkpoint_peek(tmp_path / "split.ckpt")
+    assert head["demag_blocks"] == 1 and head["output_index"] == 4
+    b = run("split", 6, resume=str(tmp_path / "split.ckpt"), demag=demag)
+    a = run("full", 6, **gpu)
+    assert len(a) == len(b) == 7 and a == b

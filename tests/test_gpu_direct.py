@@ -53,3 +53,25 @@ def test_direct_sum_over_gauss_points_where_the_matrix_does_not_fit():
         ref = np.array([((q / np.linalg.norm(pts - m["xyz"][i], axis=1)).sum() + corr[i]) / (4 * np.pi) for i in pick])
         # 1.4 million FP64 terms on either side, summed in shares of thousands
         assert np.linalg.norm(got[pick] - ref) < 1e-11 * np.linalg.norm(ref) * (1 if which == 0 else 10)
+
+
+def test_demag_blocks_of_the_direct_sum():
+    """The matrix and the sum over Gauss points by choice, and what a context reports."""
+    m = cases.cuboid(5, 4, 4)
+    u = cases.perturbed_state(m["xyz"], seed=15, sigma=0.3)
+    v = cases.tangent_field(u, seed=16)
+    o = fgo.Oracle(m, cases.oracle_regions())
+    o.set_state(u, v)
+    n = len(m["xyz"])
+    for blocks, form in ((0, 3), (1, 1), (2, 3), (3, 3)):
+        c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_DIRECT, demag_blocks=blocks)
+        assert c.demag_info() == (form, 24 * n * n if form == 3 else 0)
+        c.set_state(u, v)
+        c.compute_all(np.zeros(3))
+        s = c.get_state(0)
+        # as test_direct_sum_edges
+        assert np.linalg.norm(s["phi"] - o.demag(0)) < 4e-12 * np.linalg.norm(o.demag(0))
+        assert np.linalg.norm(s["phiv"] - o.demag(1)) < 1e-11 * np.linalg.norm(o.demag(1))
+    for blocks in (-1, 4):
+        with pytest.raises(fg.FgError):
+            fg.Context(m, cases.regions(), demag_blocks=blocks)

@@ -119,3 +119,43 @@ def test_fp64_fmm_targets_without_near_sources(shape, leaf, first_order):
     # as test_fp64_fmm_edges
     for k in (0, 2, 3) if first_order else range(4):
         assert _rel(pot[0][k], pot[1][k]) < (2e-13 if k % 2 == 0 else 1e-12)
+
+
+# every form of the near field and P2M, and those that a tree cannot have. At depth 2 a leaf of
+# (15, 14, 13) has more than 6,144 elements around it: no blocks. Of a bar of 520 cells it has 5,500, but
+# 1,048 of its own (five Gauss points), more than the 1,024 of a P2M block, or 653 (one) on 525 nodes,
+# whose columns take two tiles, as those of 506 cells do with five
+@pytest.mark.parametrize("shape,leaf,one_point,auto", [
+    ((3, 3, 3), -2, 0, 3), ((3, 3, 3), -2, 1, 3), ((11, 7, 5), -3, 0, 3), ((11, 7, 5), -3, 1, 3),
+    ((15, 14, 13), -2, 0, 1), ((15, 14, 13), -2, 1, 1), ((1, 1, 520), -2, 0, 2), ((1, 1, 520), -2, 1, 3),
+    ((1, 1, 506), -2, 0, 3)])
+def test_demag_blocks_forms(shape, leaf, one_point, auto):
+    m = cases.cuboid(*shape)
+    u = cases.perturbed_state(m["xyz"], seed=27, sigma=0.3)
+    v = cases.tangent_field(u, seed=28)
+
+    def potentials(**o):
+        c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=leaf, one_gauss_point=one_point, **o)
+        c.set_state(u, v)
+        c.compute_all(np.zeros(3))
+        s = c.get_state(0)
+        return c.demag_info(), (s["phi"], s["phiv"], c.demag(0), c.demag(1))
+
+    (form, _), ref = potentials(fmm_native_fp64=1)
+    assert form == 0
+    (form, n0), default = potentials()
+    assert form == auto and (n0 > 0) == (form > 1)
+    for blocks in (1, 2, 3):
+        if blocks > auto:
+            with pytest.raises(fg.FgError) as e:
+                potentials(demag_blocks=blocks)
+            assert "too many elements" in str(e.value)
+            continue
+        (form, n), pot = potentials(demag_blocks=blocks)
+        assert form == blocks and (n > 0) == (blocks > 1)
+        if blocks == 1 and shape[2] > 500:
+            continue  # the sums hold coordinates to 2^-45 of a leaf's width, here 130 cells
+        for k in range(4):  # as test_fp64_fmm_edges
+            assert _rel(pot[k], ref[k]) < (2e-13 if k % 2 == 0 else 1e-12)
+            if blocks == auto:
+                assert np.array_equal(pot[k], default[k])

@@ -152,3 +152,22 @@ def test_checkpoint_version2_header(tmp_path):
     p.write_bytes(raw3)
     with pytest.raises(fg.FgError):
         fg.checkpoint_peek(p)
+
+
+def test_checkpoint_version4_header(tmp_path):
+    """Version 4 adds the form of the demag after the solver's threads; earlier files report 0."""
+    import struct
+    raw, m = _checkpoint_bytes(version=2)
+    at = 8 + 4 + 7 * 4
+    body = raw[:8] + struct.pack("<I", 4) + raw[12:at] + struct.pack("<i", 2) + raw[at:-8]
+    h = 1469598103934665603
+    for x in body:
+        h = ((h ^ x) * 1099511628211) & 0xFFFFFFFFFFFFFFFF
+    p = tmp_path / "c.ckpt"
+    p.write_bytes(body + struct.pack("<Q", h))
+    got = fg.checkpoint_peek(p)
+    assert (got["solver_threads"], got["demag_blocks"], got["fmm_depth"]) == (512, 2, 6)
+    for k in ("t", "steps", "rng_draws", "E"):
+        assert got[k] == m[k], k
+    p.write_bytes(raw)
+    assert fg.checkpoint_peek(p)["demag_blocks"] == 0
