@@ -309,7 +309,8 @@ __device__ __forceinline__ void near_tables(const NearArgs &a, int leaf, int *no
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(256) k_near_count(NearArgs a, int *ncol, int *over) {
+// Columns of every leaf, and the most elements of one (the largest int where a leaf has too many nodes).
+__global__ void __launch_bounds__(256) k_near_count(NearArgs a, int *ncol, int *most) {
     extern __shared__ int tab[];
     __shared__ int nn, ne;
     const int leaf = blockIdx.x;
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(256) k_near_count(NearArgs a, int *ncol, int *
     near_tables(a, leaf, tab, tab + HASH, &nn, &ne);
     if (threadIdx.x == 0) {
         ncol[leaf] = nn;
-        if (nn > MAX_NODE || ne > (a.own ? MAX_OWN : MAX_ELEM)) *over = 1;
+        atomicMax(most, nn > MAX_NODE ? 0x7fffffff : ne);
     }
 }
 
@@ -475,23 +476,23 @@ __global__ void __launch_bounds__(256) k_near_fill(NearArgs a, Rules R, const in
 
 // The multipoles of a leaf as a block [100][3 columns] over the nodes of its own sources' elements:
 // W[slot][k] = sum over the element's Gauss points in the leaf of w_g conj(Ups_k)(y_g) (a triangle
-// counts as three elements, one per shape function), then a warp per column node gathers its
-// elements, lanes = coefficients. One thread forms one harmonic column of one element.
-constexpr int OWN_HASH = 4096;
+// counts as three elements, one per shape function; a block's scratch holds `rows` of them), then a
+// warp per column node gathers its elements, lanes = coefficients. One thread forms one harmonic
+// column of one element.
 __global__ void __launch_bounds__(256) k_p2m_fill(NearArgs a, Rules R, const int *__restrict__ cptr,
                                                   const int *__restrict__ col, const size_t *__restrict__ boff,
                                                   const int *__restrict__ src_pos, const double4 *__restrict__ sloc,
                                                   const double *__restrict__ da, const double *__restrict__ detJ,
                                                   const int *__restrict__ treg, const DevRegion *__restrict__ regs,
                                                   const int *__restrict__ inc_ptr, const int *__restrict__ inc,
-                                                  const DevTri *__restrict__ tc, double *__restrict__ scratch,
-                                                  float2 *__restrict__ B) {
+                                                  const DevTri *__restrict__ tc, int rows,
+                                                  double *__restrict__ scratch, float2 *__restrict__ B) {
     constexpr int P = 9;
     extern __shared__ int tab[];
     int *mask = tab + HASH, *list = mask + HASH;  // the table, its masks, the occupied slots
     __shared__ int ne, nl;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double *W = scratch + (size_t)blockIdx.x * OWN_HASH * NRM;
+    double *W = scratch + (size_t)blockIdx.x * rows * NRM;
     for (int leaf = blockIdx.x; leaf < a.nleaf; leaf += gridDim.x) {
         const int c0 = cptr[leaf], nc = cptr[leaf + 1] - c0;
         if (nc == 0) continue;
@@ -807,7 +808,8 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
     NCK(cudaMemcpyAsync(hn.data(), ncol, sizeof(int) * (t.nleaf + 1), cudaMemcpyDeviceToHost, c.stream));
     NCK(cudaStreamSynchronize(c.stream));
     N.why = FG_EINVAL;
-    if (hn[t.nleaf]) return done(cudaSuccess);
+    if (hn[t.nleaf] > (own ? MAX_OWN : MAX_ELEM)) return done(cudaSuccess);
+    const int rows = 3 * hn[t.nleaf];  // P2M: the most that a leaf's elements take, all triangles
     std::vector<int> cptr(t.nleaf + 1, 0);
     std::vector<size_t> boff(t.nleaf, 0);
     std::vector<int4> task;
@@ -832,7 +834,7 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
     N.bytes = entries * sizeof(float2);
     if (c.opts.demag_blocks == 0 && N.bytes > std::min(total_b / 8, free_b / 2)) return done(cudaSuccess);
     N.ntask = (int)task.size();
-    NCK(cudaMalloc(&scratch, sizeof(double) * (own ? (size_t)OWN_HASH * NRM : (size_t)HASH * TG) * blocks));
+    NCK(cudaMalloc(&scratch, sizeof(double) * (own ? (size_t)rows * NRM : (size_t)HASH * TG) * blocks));
     NCK(cudaMalloc(&N.cptr, sizeof(int) * (t.nleaf + 1)));
     NCK(cudaMalloc(&N.boff, sizeof(size_t) * t.nleaf));
     NCK(cudaMalloc(&N.task, sizeof(int4) * N.ntask));
@@ -848,7 +850,8 @@ static cudaError_t blocks_build(Ctx &c, const Rules &R, const NearTree &t, bool 
         k_near_cols<<<t.nleaf, 256, smem, c.stream>>>(a, N.cptr, ncol, N.col);
         if (own)
             k_p2m_fill<<<blocks, 256, smem_own, c.stream>>>(a, R, N.cptr, N.col, N.boff, t.src_pos, t.sloc, c.da, c.detJ,
-                                                            c.treg, c.regs, c.inc_ptr, c.inc, c.tri_c, scratch, N.B);
+                                                            c.treg, c.regs, c.inc_ptr, c.inc, c.tri_c, rows, scratch,
+                                                            N.B);
         else
             k_near_fill<<<blocks, 256, smem, c.stream>>>(a, R, N.cptr, N.col, N.boff, c.xyz, c.src_xyz, c.da, c.detJ, c.treg,
                                                          c.regs, c.inc_ptr, c.inc, c.tri_c, scratch, N.B);
