@@ -1790,6 +1790,7 @@ static void oz_weights(int *wM, int *wF) {
 }
 
 void fmm_free(Ctx &c);
+static void harvest_set(FmmTree &t, int k);
 static int fmm_build_forest(Ctx &c, int L);
 template <typename T>
 static cudaError_t fmm_eval_t(Ctx &c, FmmTree &t, int nq, const FmmFields &f);
@@ -1854,6 +1855,39 @@ static int blocks_missing(Ctx &c, const FmmTree &t) {
                                    : "fmm: demag_blocks: a leaf of the tree has too many elements for a block";
     return none->why == FG_ENOMEM ? FG_ENOMEM : FG_EINVAL;
 }
+
+// The tree of the fastest depth so far (and its source order) while others are tried.
+struct KeptTree {
+    Ctx &c;
+    FmmTree *t = nullptr;
+    int *src_dst = nullptr;
+    explicit KeptTree(Ctx &ctx) : c(ctx) {}
+    ~KeptTree() { drop(); }
+    void drop() {
+        if (!t) return;
+        void *current = c.fmm;
+        c.fmm = t;
+        fmm_free(c);
+        c.fmm = current;
+        if (src_dst) cudaFree(src_dst);
+        t = nullptr;
+        src_dst = nullptr;
+    }
+    void take() {  // the context's tree
+        drop();
+        t = static_cast<FmmTree *>(c.fmm);
+        src_dst = c.src_dst;
+        c.fmm = nullptr;
+        c.src_dst = nullptr;
+    }
+    void give() {  // back to the context
+        if (c.src_dst) cudaFree(c.src_dst);
+        c.fmm = t;
+        c.src_dst = src_dst;
+        t = nullptr;
+        src_dst = nullptr;
+    }
+};
 
 int fmm_build(Ctx &c) {
     const bool fp32 = (c.opts.precision == FG_PREC_FP32_REFINE);
@@ -1929,13 +1963,17 @@ int fmm_build(Ctx &c) {
     if (c.src_q2) cudaMemsetAsync(c.src_q2, 0, sizeof(double) * std::max(1, c.nsrc), c.stream);
     int bestL = cands[0], missing = FG_OK;
     double bestms = 1e300;
+    KeptTree best(c);
     for (size_t k = 0; k < cands.size(); k++) {
         fmm_free(c);
+        size_t before = 0, after = 0, total = 0;
+        FCK(cudaMemGetInfo(&before, &total));
         FmmTree *t = new FmmTree();
         c.fmm = t;
         t->fp32 = fp32;
         int s = fmm_build_forest(c, cands[k]);
         if (s != FG_OK) return s;
+        FCK(cudaMemGetInfo(&after, &total));
         if (const int why = blocks_missing(c, *t)) {
             if (cands.size() == 1) return why;
             missing = why;
@@ -1961,14 +1999,28 @@ int fmm_build(Ctx &c) {
         cudaEventDestroy(a);
         cudaEventDestroy(b);
         if (c.opts.verbose) fprintf(stderr, "fmm autotune: L=%d %.3f ms/eval\n", cands[k], ms / 2);
-        if (ms < bestms) { bestms = ms; bestL = cands[k]; }
+        if (ms >= bestms) continue;
+        bestms = ms;
+        bestL = cands[k];
+        // the fastest tree is kept rather than made again, which would be a quarter of the set-up,
+        // unless the next one might want its memory
+        best.drop();
+        if (8 * (before - std::min(before, after)) < after) best.take();
     }
     if (bestms == 1e300) return missing;
     fmm_free(c);
-    FmmTree *t = new FmmTree();
-    c.fmm = t;
-    t->fp32 = fp32;
-    const int s = fmm_build_forest(c, bestL);
+    int s = FG_OK;
+    if (best.t) {
+        for (int k = 0; k < 2; k++) harvest_set(*best.t, k);  // the stage times of the trials do not count
+        for (double &x : best.t->stage_sum) x = 0.0;
+        best.t->stage_n = 0;
+        best.give();
+    } else {
+        FmmTree *t = new FmmTree();
+        c.fmm = t;
+        t->fp32 = fp32;
+        s = fmm_build_forest(c, bestL);
+    }
     c.fmm_setup_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_begin).count();
     return s;
 }

@@ -159,3 +159,23 @@ def test_demag_blocks_forms(shape, leaf, one_point, auto):
             assert _rel(pot[k], ref[k]) < (2e-13 if k % 2 == 0 else 1e-12)
             if blocks == auto:
                 assert np.array_equal(pot[k], default[k])
+
+
+@pytest.mark.parametrize("o", [dict(), dict(first_order=1), dict(precision=fg.FG_PREC_FP32_REFINE),
+                               dict(fmm_native_fp64=1)])
+def test_the_depth_search_leaves_the_tree_of_its_depth(o):
+    """A tree kept from the search over depths gives the bits of one made for that depth alone, whichever
+    of the candidates it was, and its stage times do not count the trials."""
+    for shape in ((6, 5, 4), (14, 13, 12), (40, 36, 1)):
+        m = cases.cuboid(*shape)
+        u = cases.perturbed_state(m["xyz"], seed=29, sigma=0.3)
+        v = cases.tangent_field(u, seed=30)
+        a = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, profile=1, **o)
+        assert np.all(np.array(a.fmm_timings()) == 0)
+        b = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_FMM, fmm_leaf=-a.counters()[1], **o)
+        for c in (a, b):
+            c.set_state(u, v)
+            c.compute_all(np.zeros(3))
+        sa, sb = a.get_state(0), b.get_state(0)
+        assert np.array_equal(sa["phi"], sb["phi"]) and np.array_equal(sa["phiv"], sb["phiv"])
+        assert np.array_equal(a.demag(0), b.demag(0)) and np.array_equal(a.demag(1), b.demag(1))
