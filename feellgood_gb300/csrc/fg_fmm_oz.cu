@@ -1,18 +1,26 @@
 // FMM translations of the FP64 path on the 5th-generation tensor cores (tcgen05).
 //
 // A translation applies a fixed 100x100 operator to 100-coefficient expansions held in FP64.
-// The FP16 tensor pipe evaluates it exactly by digits (the error-free splitting of Ozaki, Ogita,
+// The FP16 tensor pipe evaluates it by digits (the error-free splitting of Ozaki, Ogita,
 // Oishi and Rump, "Error-free transformations of matrix multiplication by using fast routines of
 // matrix multiplication and its applications", 2012): every operator row and every expansion is
 // scaled by a power of two of its own and written as five signed digits of 10 bits,
 //     a_ij = rs_i sum_s A_s[i][j] 2^-10s,    x_j = cs sum_t X_t[j] 2^-10t,
 // |A_0| <= 512, |X_0| <= 1024 and |A_s|, |X_s| <= 512 for s >= 1: integers that FP16 holds. The
 // digit products of equal weight s + t = l <= 4 are summed by MMAs with FP32 accumulation into one
-// accumulator per l; the sums are integers below 2^24, so every MMA is exact. The
+// accumulator per l. A sum of integers is exact there while it stays below 2^24. For l = 0 the
+// operators' scales see to it for every input; for l >= 1 nothing does, the sizes do: were all
+// the lower digits' signs to agree, the worst rows (M2L) would reach 2.1, 3.0, 3.7 and 4.5 x 2^24
+// for l = 1 to 4 (M2M at most 1.5, L2L 2.7), but digits spread over their range with the signs of
+// a number's low digits add up to an rms of 0.12 to 0.15 x 2^24, so 2^24 is 8.5 standard
+// deviations off for l = 1 and 6.6 for l = 4 (over all rows of the operators). A sum beyond it
+// would be rounded to a multiple of 2 to 8 units of 2^-10l. The
 // five accumulators of each operator are combined and added up in double-single arithmetic (about
 // 48 bits). Neglected: digit products of weight 2^-50 and less of the largest ones. Before the
 // splitting each coefficient is weighted by a power of two (and the operator column by its
-// inverse) that makes typical coefficients of all degrees alike. Against FP64 sums the
+// inverse) that makes typical coefficients of all degrees alike: the 50 bits of an expansion share
+// one exponent, so a coefficient far below the largest weighted one keeps fewer significant bits
+// (the pairs of FP32 before had 48 bits each), with an error relative to the largest. Against FP64 sums the
 // potentials differ by 2e-16 to 2e-14, less than the double-single products on the FP32 pipes
 // that this replaces (2e-14 to 7e-14, simulated on the same multipoles).
 //
@@ -357,7 +365,7 @@ cudaError_t launch_oz_finish(cudaStream_t st, const OzFinish &a) {
 
 // Digits of the operators as the MMA reads them, and the scale of every row: column j carries the
 // inverse 2^-wexp[j] of the weight of input coefficient j. The sum of a row's leading digits stays
-// below 2^14, so that with |X_0| <= 1024 no sum of leading products reaches 2^24.
+// below 2^14, so that with |X_0| <= 1024 no sum of leading products (l = 0) reaches 2^24.
 OzImages oz_images(const std::vector<double> &ops, int ncode, const int *wexp) {
     OzImages im;
     im.img.assign((size_t)ncode * IPC * A_BYTES, 0);
