@@ -82,8 +82,9 @@ struct FmmTree {
     bool ds = false;
     // The FP64 tree of an FP32 + refinement context (full evaluations, where CURRENT has no valid
     // potentials) keeps the arithmetic and the order of the sums that such runs have always started
-    // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9
-    // in phiv two steps later (film), so runs repeat bit for bit only with the same last bits
+    // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9 in
+    // phiv two steps later (film). Other deterministic kernels would repeat bit for bit as well; these
+    // also agree with the results of builds before them to the last bit
     bool repeat = false;
     NearMat near;              // oz: P2M and near field as dense blocks, where they fit
     int4 *p2p_task = nullptr;  // leaf, first target, targets of a near-field task
