@@ -32,6 +32,19 @@ def cuboid(nx, ny, nz, h=2.5):
     return om.setup(msh, ["volume"], [], 1e-9, Ms=[MS])
 
 
+def layered_cuboid(nx, ny, nz, Ms, h=2.5):
+    """cuboid() cut along z into one volume region per entry of Ms (0: not magnetic), with the charged
+    interface triangles between them."""
+    msh = cuboid_msh(nx, ny, nz, nx * h, ny * h, nz * h)
+    tets = msh["blocks"][0][4]
+    z = msh["nodes"][tets - 1][:, :, 2].mean(1) / (nz * h)
+    layer = np.minimum((z * len(Ms)).astype(int), len(Ms) - 1)
+    names = [f"layer{k}" for k in range(len(Ms))]
+    msh["names"] = {(3, 300 + k): n for k, n in enumerate(names)}
+    msh["blocks"] = [(3, 1 + k, (300 + k,), 4, tets[layer == k]) for k in range(len(Ms))]
+    return om.setup(msh, names, [], 1e-9, Ms=list(Ms))
+
+
 def regions(alpha=0.5, K=0.0, uk=(0, 0, 1), K3=0.0):
     return [dict(Ae=1e-11, Ms=795774.7, alpha=0.5),
             dict(Ae=AE, Ms=MS, alpha=alpha, K=K, uk=uk, K3=K3)]

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 import feellgood_gb300 as fg
+from oracle import fgo
 from tests import cases
 
 pytestmark = pytest.mark.gpu
@@ -179,3 +180,37 @@ def test_the_depth_search_leaves_the_tree_of_its_depth(o):
         sa, sb = a.get_state(0), b.get_state(0)
         assert np.array_equal(sa["phi"], sb["phi"]) and np.array_equal(sa["phiv"], sb["phiv"])
         assert np.array_equal(a.demag(0), b.demag(0)) and np.array_equal(a.demag(1), b.demag(1))
+
+
+# layers of two magnetisations, with charged triangles between them, beside or around one that is not
+# magnetic: nodes, elements and regions that the blocks have to leave out
+@pytest.mark.parametrize("Ms", [(cases.MS, 3e5, 0.0), (0.0, cases.MS, 0.0, 3e5)])
+@pytest.mark.parametrize("one_point", [0, 1])
+def test_blocks_of_several_regions(Ms, one_point):
+    m = cases.layered_cuboid(7, 6, 9, Ms)
+    reg = [cases.regions()[0]] + [dict(cases.regions()[1], Ms=x) for x in Ms]
+    u = cases.perturbed_state(m["xyz"], seed=31, sigma=0.3)
+    v = cases.tangent_field(u, seed=32)
+    mag = np.unique(m["tets"][np.array((0.0,) + Ms)[m["tet_reg"]] > 0])
+    o = fgo.Oracle(m, [fgo.make_region()] + [fgo.make_region(A=cases.AE, Ms=x, alpha=0.5) for x in Ms],
+                   one_gauss_point=bool(one_point))
+    o.set_state(u, v)
+    exact = [o.demag(0)[mag], o.demag(1)[mag]]
+
+    def potentials(**k):
+        c = fg.Context(m, reg, one_gauss_point=one_point, **k)
+        c.set_state(u, v)
+        c.compute_all(np.zeros(3))
+        s = c.get_state(0)
+        return [s["phi"][mag], s["phiv"][mag]]
+
+    # FP64 sums of at most 15,000 terms on either side (15,000 x 2^-53 = 2e-12 of the summed
+    # magnitudes, an order of magnitude more for the cancelling sums of v)
+    for blocks in (1, 3):
+        p = potentials(demag=fg.FG_DEMAG_DIRECT, demag_blocks=blocks)
+        assert _rel(p[0], exact[0]) < 1e-11 and _rel(p[1], exact[1]) < 3e-11
+    ref = potentials(demag=fg.FG_DEMAG_FMM, fmm_leaf=-3, fmm_native_fp64=1)
+    assert _rel(ref[0], exact[0]) < 1e-4 and _rel(ref[1], exact[1]) < 1e-3  # the expansions' truncation
+    for blocks in (1, 2, 3):
+        p = potentials(demag=fg.FG_DEMAG_FMM, fmm_leaf=-3, demag_blocks=blocks)
+        assert _rel(p[0], ref[0]) < 2e-13 and _rel(p[1], ref[1]) < 1e-12  # as test_fp64_fmm_edges
