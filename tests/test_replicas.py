@@ -50,3 +50,18 @@ def test_reference_arm_runs_on_rank_zero_only(monkeypatch, capsys):
         gpus, steps, warmup = 2, 3, 3
     bench.reference_arm(A())
     assert capsys.readouterr().out == ""
+
+
+def test_reference_arm_says_that_the_reference_is_unavailable(monkeypatch, capsys):
+    """No figure of this library appears under the reference's name."""
+    import json
+    sys.path.insert(0, ROOT)
+    import bench
+    monkeypatch.setattr(bench, "dist_setup", lambda n: (0, 1, None))
+    monkeypatch.setattr(bench, "cpu_leg", lambda *a, **k: pytest.fail("the restatement was timed as the reference"))
+
+    class A:
+        gpus, steps, warmup = 1, 3, 3
+    bench.reference_arm(A())
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
