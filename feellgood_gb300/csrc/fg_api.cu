@@ -549,7 +549,7 @@ static int create_impl(fg_ctx *h, const fg_mesh *m, const fg_region *regs, int n
     CK(dalloc(&c.fv, 23 * (size_t)nn));
     c.bicg_grid = bicg_grid_size(c);
     c.mixed_grid = mixed_grid_size(c);
-    c.partial_len = 8 * std::max(c.bicg_grid, 1024);
+    c.partial_len = 8 * std::max(std::max(c.bicg_grid, c.mixed_grid), 1024);
     CK(dalloc(&c.partial, c.partial_len));
     CK(dalloc(&c.bar, 1));
     CK(cudaMemset(c.bar, 0, sizeof(GridBar)));

@@ -78,6 +78,8 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
         dt = a.seg[sv.g].dt;
     }
     const float c32 = (float)(c0 * a.scale);
+    // consecutive reductions use two buffers in turn, as in k_bicg64
+    double *part[2] = {a.partial, a.partial + 4 * (size_t)G};
     // phase 0: FP32 copies of the per-step operator, FP64 tangent vectors of x, |b|^2, and
     // the learned guess's candidate when its network outputs are given
     {
@@ -125,12 +127,12 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
             if (m) bb += a.b[2 * i] * a.b[2 * i] + a.b[2 * i + 1] * a.b[2 * i + 1];
         }
         double v1[1] = {bb};
-        block_store<1>(v1, a.partial, G);
+        block_store<1>(v1, part[0], G);
     }
     if (!grid_sync(a.bar)) goto timeout;
     {
         double s1[1];
-        range_sum<1>(a.partial, G, sv.b0, sv.b1, s1);
+        range_sum<1>(part[0], G, sv.b0, sv.b1, s1);
         const double rhsn = sqrt(fabs(s1[0]));
         int status = -1, nit = 0, nref = 0;
         double res = 0.0, res0 = 0.0;
@@ -171,12 +173,12 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
                     GROUP_ROWS(row)
                 }
                 double v3[3] = {rr, rc, rx};
-                block_store<3>(v3, a.partial, G);
+                block_store<3>(v3, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s3[3];
-                range_sum<3>(a.partial, G, sv.b0, sv.b1, s3);
+                range_sum<3>(part[1], G, sv.b0, sv.b1, s3);
                 double s2 = s3[0];
                 if (judge && !done) {
                     // x = x_prev + t (x_cand - x_prev) with the t in [0, 1] that minimises the
@@ -237,15 +239,15 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
                     }
                 }
                 float v2[2] = {rr, (threadIdx.x == 0 && !done) ? 1.0f : 0.0f};
-                block_store_f<2>(v2, a.partial, G);
+                block_store_f<2>(v2, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s2[1];
-                range_sum<1>(a.partial, G, sv.b0, sv.b1, s2);
+                range_sum<1>(part[0], G, sv.b0, sv.b1, s2);
                 if (multi) {
                     double f[1];
-                    grid_sum<1>(a.partial + G, G, f);
+                    grid_sum<1>(part[0] + G, G, f);
                     if (f[0] == 0.0) break;  // every sample has ended
                 }
                 double rr = s2[0], rtr = s2[0];
@@ -322,15 +324,15 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
                             GROUP_ROWS(row)
                         }
                         float v2[2] = {vr, (threadIdx.x == 0 && act) ? 1.0f : 0.0f};
-                        block_store_f<2>(v2, a.partial, G);
+                        block_store_f<2>(v2, part[1], G);
                     }
                     if (!grid_sync(a.bar)) goto timeout;
                     {
                         double s1b[1];
-                        range_sum<1>(a.partial, G, sv.b0, sv.b1, s1b);
+                        range_sum<1>(part[1], G, sv.b0, sv.b1, s1b);
                         if (multi) {
                             double f[1];
-                            grid_sum<1>(a.partial + G, G, f);
+                            grid_sum<1>(part[1] + G, G, f);
                             if (f[0] == 0.0) break;
                         }
                         if (act) alpha = block_once([=] { return rho1 / s1b[0]; });
@@ -351,13 +353,13 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
                             }
                         }
                         float v1[1] = {ss};
-                        block_store_f<1>(v1, a.partial, G);
+                        block_store_f<1>(v1, part[0], G);
                     }
                     if (!grid_sync(a.bar)) goto timeout;
                     double ssum = 0.0;
                     {
                         double s1c[1];
-                        range_sum<1>(a.partial, G, sv.b0, sv.b1, s1c);
+                        range_sum<1>(part[0], G, sv.b0, sv.b1, s1c);
                         ssum = s1c[0];
                         if (act && ssum <= target2) {
                             const float fa = (float)alpha;
@@ -394,12 +396,12 @@ __global__ void __launch_bounds__(512, 1) k_mixed(MixedArgs a) {
                             GROUP_ROWS(row)
                         }
                         float v4[4] = {ts, tt, rts, rtt};
-                        block_store_f<4>(v4, a.partial, G);
+                        block_store_f<4>(v4, part[1], G);
                     }
                     if (!grid_sync(a.bar)) goto timeout;
                     {
                         double s4[4];
-                        range_sum<4>(a.partial, G, sv.b0, sv.b1, s4);
+                        range_sum<4>(part[1], G, sv.b0, sv.b1, s4);
                         if (act) {
                             omega = block_once([=] { return s4[0] / s4[1]; });
                             rr = fmax(0.0, ssum - 2.0 * omega * s4[0] + omega * omega * s4[1]);

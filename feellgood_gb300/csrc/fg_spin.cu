@@ -115,6 +115,8 @@ __global__ void __launch_bounds__(256) k_spin_bicg(SpinArgs a) {
     const int G = gridDim.x, nn = a.nn;
     const int stride = G * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int gstride = G * (int)blockDim.x / SPIN_LPR;
+    // consecutive reductions use two buffers in turn, as in k_bicg64
+    double *part[2] = {a.partial, a.partial + 4 * (size_t)G};
     // b = rhs - K xd (masked); x = 0 (the reference starts from a zero vector), r = rt = p = b
     {
         double bb = 0.0;
@@ -136,12 +138,12 @@ __global__ void __launch_bounds__(256) k_spin_bicg(SpinArgs a) {
         };
         SPIN_ROWS(row)
         double v1[1] = {bb};
-        block_store<1>(v1, a.partial, G);
+        block_store<1>(v1, part[0], G);
     }
     if (!grid_sync(a.bar)) goto timeout;
     {
         double s1[1];
-        grid_sum<1>(a.partial, G, s1);
+        grid_sum<1>(part[0], G, s1);
         const double rhsn = sqrt(fabs(s1[0]));
         double rr = s1[0], rtr = s1[0];
         double rho1 = 0.0, rho2 = 0.0, alpha = 0.0, beta = 0.0, omega = 0.0;
@@ -195,12 +197,12 @@ __global__ void __launch_bounds__(256) k_spin_bicg(SpinArgs a) {
                 };
                 SPIN_ROWS(row)
                 double v1[1] = {vr};
-                block_store<1>(v1, a.partial, G);
+                block_store<1>(v1, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s1b[1];
-                grid_sum<1>(a.partial, G, s1b);
+                grid_sum<1>(part[1], G, s1b);
                 alpha = rho1 / s1b[0];
             }
             {
@@ -217,12 +219,12 @@ __global__ void __launch_bounds__(256) k_spin_bicg(SpinArgs a) {
                     }
                 }
                 double v1[1] = {ss};
-                block_store<1>(v1, a.partial, G);
+                block_store<1>(v1, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s1c[1];
-                grid_sum<1>(a.partial, G, s1c);
+                grid_sum<1>(part[0], G, s1c);
                 if (finished(sqrt(fabs(s1c[0])))) {
                     for (int i = i0; i < nn; i += stride)
 #pragma unroll
@@ -247,12 +249,12 @@ __global__ void __launch_bounds__(256) k_spin_bicg(SpinArgs a) {
                 };
                 SPIN_ROWS(row)
                 double v2[2] = {ts, tt};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[1], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s2[2];
-                grid_sum<2>(a.partial, G, s2);
+                grid_sum<2>(part[1], G, s2);
                 omega = s2[0] / s2[1];
             }
             {
@@ -270,12 +272,12 @@ __global__ void __launch_bounds__(256) k_spin_bicg(SpinArgs a) {
                         rtr2 += a.rt[k] * rv;
                     }
                 double v2[2] = {r2, rtr2};
-                block_store<2>(v2, a.partial, G);
+                block_store<2>(v2, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s2c[2];
-                grid_sum<2>(a.partial, G, s2c);
+                grid_sum<2>(part[0], G, s2c);
                 rr = s2c[0];
                 rtr = s2c[1];
             }
@@ -318,6 +320,8 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
     const int G = gridDim.x, nn = a.nn;
     const int stride = G * blockDim.x, i0 = blockIdx.x * blockDim.x + threadIdx.x;
     const int gstride = G * (int)blockDim.x / SPIN_LPR;
+    // consecutive reductions use two buffers in turn, as in k_bicg64
+    double *part[2] = {a.partial, a.partial + 4 * (size_t)G};
     // FP32 CURRENT m; b = rhs - K xd (FP64, masked) = the first refinement residual; x = 0
     for (int k = i0; k < 3 * nn; k += stride) {
         a.m32[k] = (float)a.m0[k];
@@ -341,12 +345,12 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
         };
         SPIN_ROWS(row)
         double v1[1] = {bb};
-        block_store<1>(v1, a.partial, G);
+        block_store<1>(v1, part[1], G);
     }
     if (!grid_sync(a.bar)) goto timeout;
     {
         double s1[1];
-        grid_sum<1>(a.partial, G, s1);
+        grid_sum<1>(part[1], G, s1);
         const double rhsn = sqrt(fabs(s1[0]));
         double res = rhsn;
         const double res0 = res;
@@ -368,10 +372,10 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
                 };
                 SPIN_ROWS(row)
                 double v1[1] = {rr};
-                block_store<1>(v1, a.partial, G);
+                block_store<1>(v1, part[1], G);
                 if (!grid_sync(a.bar)) goto timeout;
                 double s1r[1];
-                grid_sum<1>(a.partial, G, s1r);
+                grid_sum<1>(part[1], G, s1r);
                 res = block_once([=] { return sqrt(fabs(s1r[0])); });
             }
             if (isnan(res)) { status = 2; break; }
@@ -391,12 +395,12 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
                     rr += rv * rv;
                 }
                 float v1[1] = {rr};
-                block_store_f<1>(v1, a.partial, G);
+                block_store_f<1>(v1, part[0], G);
             }
             if (!grid_sync(a.bar)) goto timeout;
             {
                 double s1i[1];
-                grid_sum<1>(a.partial, G, s1i);
+                grid_sum<1>(part[0], G, s1i);
                 double rr = s1i[0], rtr = s1i[0];
                 double rho1 = 0.0, rho2 = 0.0, alpha = 0.0, beta = 0.0, omega = 0.0;
                 // four grid barriers per iteration, as k_mixed: the update d += alpha phat +
@@ -474,12 +478,12 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
                         };
                         SPIN_ROWS(row)
                         float v1[1] = {vr};
-                        block_store_f<1>(v1, a.partial, G);
+                        block_store_f<1>(v1, part[1], G);
                     }
                     if (!grid_sync(a.bar)) goto timeout;
                     {
                         double s1b[1];
-                        grid_sum<1>(a.partial, G, s1b);
+                        grid_sum<1>(part[1], G, s1b);
                         alpha = block_once([=] { return rho1 / s1b[0]; });
                     }
                     double ssum = 0.0;
@@ -499,12 +503,12 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
                             ss += sv.x * sv.x + sv.y * sv.y + sv.z * sv.z + sv.w * sv.w;
                         }
                         float v1[1] = {ss};
-                        block_store_f<1>(v1, a.partial, G);
+                        block_store_f<1>(v1, part[0], G);
                     }
                     if (!grid_sync(a.bar)) goto timeout;
                     {
                         double s1c[1];
-                        grid_sum<1>(a.partial, G, s1c);
+                        grid_sum<1>(part[0], G, s1c);
                         ssum = s1c[0];
                         if (ssum <= target2) {
                             const float fa = (float)alpha;
@@ -539,12 +543,12 @@ __global__ void __launch_bounds__(1024, 1) k_spin_mixed(SpinArgs a) {
                         };
                         SPIN_ROWS(row)
                         float v4[4] = {ts, tt, rts, rtt};
-                        block_store_f<4>(v4, a.partial, G);
+                        block_store_f<4>(v4, part[1], G);
                     }
                     if (!grid_sync(a.bar)) goto timeout;
                     {
                         double s4[4];
-                        grid_sum<4>(a.partial, G, s4);
+                        grid_sum<4>(part[1], G, s4);
                         omega = block_once([=] { return s4[0] / s4[1]; });
                         rr = fmax(0.0, ssum - 2.0 * omega * s4[0] + omega * omega * s4[1]);
                         rtr = s4[2] - omega * s4[3];
@@ -974,7 +978,7 @@ int spin_setup(Ctx &c, const fg_mesh *m, const fg_region *regs, int nreg, const 
     int bps = S->mixed ? 4 : 2;
     if (const char *env = std::getenv("FG_SPIN_BLOCKS_PER_SM")) bps = std::max(1, std::atoi(env));
     S->grid = std::max(1, std::min(std::min(std::max(1, per_sm), bps) * c.nsm, (nn + S->threads - 1) / S->threads));
-    if (cudaMalloc(&S->partial, 4 * sizeof(double) * std::max(1024, S->grid)) != cudaSuccess) return FG_ECUDA;
+    if (cudaMalloc(&S->partial, 8 * sizeof(double) * std::max(1024, S->grid)) != cudaSuccess) return FG_ECUDA;
     c.spin_s = S->out;
     return FG_OK;
 }
