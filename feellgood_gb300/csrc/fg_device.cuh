@@ -37,14 +37,20 @@ __device__ inline bool grid_sync(GridBar *gb) {
         asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(ticket) : "l"(&gb->count) : "memory");
         const unsigned long long part = ticket >> 32 ? ticket % gridDim.x : (unsigned)ticket % gridDim.x;
         const unsigned long long begin = ticket - part, last = begin + gridDim.x;  // of the round
-        const unsigned long long t0 = gtimer();
         if (ticket & EXPIRED) ok = 0;
-        for (int k = 1; ok; k++) {
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(&gb->count) : "memory");
-            if ((seen & ~EXPIRED) >= last) break;  // also where a later round has expired
-            if (seen & EXPIRED) ok = 0;
-            else if (k % 32 == 0 && gtimer() - t0 > 2000000000ull && atomicCAS(&gb->count, seen, EXPIRED | begin) == seen)
-                ok = 0;
+        else if (ticket + 1 != last) {
+            // the timer is read every 32 polls (reading it before the first cost 0.1 us per barrier)
+            unsigned long long t0 = 0;
+            for (int k = 1; ok; k++) {
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(&gb->count) : "memory");
+                if ((seen & ~EXPIRED) >= last) break;  // also where a later round has expired
+                if (seen & EXPIRED) ok = 0;
+                else if (k % 32 == 0) {
+                    const unsigned long long t = gtimer();
+                    if (t0 == 0) t0 = t;
+                    else if (t - t0 > 2000000000ull && atomicCAS(&gb->count, seen, EXPIRED | begin) == seen) ok = 0;
+                }
+            }
         }
     }
     return __syncthreads_and(ok);
