@@ -772,6 +772,7 @@ int fg_set_state(fg_ctx *h, const double *u, const double *v, const double *phi,
     if (phiv) CK(cudaMemcpyAsync(c.phiv[0], phiv, n1, cudaMemcpyHostToDevice, c.stream));
     else CK(cudaMemsetAsync(c.phiv[0], 0, n1, c.stream));
     CK(launch_copy_state(c, 1, 0));
+    c.launches += 1;
     CK(cudaStreamSynchronize(c.stream));
     // given potentials are those of the given fields (v = 0 has phiv = 0)
     c.dinc_valid[0] = phi != nullptr;
@@ -919,7 +920,7 @@ static int demag_into(fg_ctx *h, const double *m, double *phi_out) {
 static int energy_impl(fg_ctx *h, const double Hext[3], double E[4], double avg[3]) {
     Ctx &c = h->c;
     CK(launch_energy(c, Hext));
-    c.launches += 2;  // and the evolution's copy
+    c.launches += 1;
     CK(cudaMemcpyAsync(c.hepart, c.epart, 7 * sizeof(double) * c.epart_blocks, cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));
     double s[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -1005,6 +1006,7 @@ int fg_compute_all(fg_ctx *h, const double Hext[3], double energies[4]) {
     // Fem::evolution: CURRENT <- NEXT
     if (c.mlp) CK(mlp_before_evolution(c));
     CK(launch_copy_state(c, 0, 1));
+    c.launches += 1;
     CK(cudaEventRecord(c.ev[5], c.stream));
     if (int *fl = fmm_error_flag(c)) CK(cudaMemcpyAsync(c.hflag, fl, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
     CK(cudaStreamSynchronize(c.stream));

@@ -75,3 +75,20 @@ def test_demag_blocks_of_the_direct_sum():
     for blocks in (-1, 4):
         with pytest.raises(fg.FgError):
             fg.Context(m, cases.regions(), demag_blocks=blocks)
+
+
+def test_launches_are_counted():
+    """fg_counters: the kernels that each call launches (8 nodes: the matrix in one share)."""
+    m = cases.cuboid(1, 1, 1)
+    u = cases.perturbed_state(m["xyz"], seed=17)
+    c = fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_DIRECT)
+
+    def count(call):
+        n = c.counters()[0]
+        call()
+        return c.counters()[0] - n
+
+    assert count(lambda: c.set_state(u)) == 1                    # the copy to CURRENT
+    assert count(lambda: c.energy(np.zeros(3))) == 1
+    assert count(lambda: c.compute_all(np.zeros(3))) == 3        # demag, energies, evolution
+    assert count(lambda: c.demag(0)) == 1
