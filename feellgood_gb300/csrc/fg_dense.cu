@@ -7,9 +7,9 @@
 // phi_i = sum_j B_ij . m_j with one 3-vector per pair of magnetic nodes. A context of the direct
 // sum forms B once, in FP64 and in the order of the charges' own sums over Gauss points, and an
 // evaluation is one pass over it for both fields: 24 bytes and 6 FP64 fused multiply-adds per pair
-// of nodes instead of 26 (Gauss point, node) pairs of 13 operations each. Measured per evaluation
+// of nodes instead of 26 (Gauss point, node) pairs of 15 operations' time each. Measured per evaluation
 // of both fields: 9,261 nodes (48,000 tetrahedra, B 2.06 GB) 0.93 ms, of which the FP64 pipe (2 per
-// clock and SM) needs 0.82 and HBM 0.30; the sum over Gauss points took 58 ms on that pipe. 1,680
+// clock and SM) needs 0.82 and HBM 0.30; the sum over Gauss points takes 59 ms on that pipe. 1,680
 // nodes 0.061 ms, 180 nodes 0.013. Forming B costs about one such sum. Against quadruple
 // precision the potentials are as exact as those sums (6e-16 for a smooth field of 1,680 nodes).
 #include <algorithm>

@@ -84,7 +84,7 @@ struct FmmTree {
     // potentials) keeps the arithmetic and the order of the sums that such runs have always started
     // from: the FP32 Krylov body turns a difference of 1e-13 in the first potentials into 3e-9 in
     // phiv two steps later (film). Other deterministic kernels would repeat bit for bit as well; these
-    // also agree with the results of builds before them to the last bit
+    // also agree with the results of earlier versions to the last bit
     bool repeat = false;
     NearMat near;              // oz: P2M and near field as dense blocks, where they fit
     int4 *p2p_task = nullptr;  // leaf, first target, targets of a near-field task
