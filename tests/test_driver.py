@@ -234,3 +234,31 @@ def test_checkpoint_resume_keeps_the_form_of_the_demag(tmp_path, golden_dir, dem
     b = run("split", 6, resume=str(tmp_path / "split.ckpt"), demag=demag)
     a = run("full", 6, **gpu)
     assert len(a) == len(b) == 7 and a == b
+
+
+@pytest.mark.gpu
+def test_resume_without_the_recorded_form_of_the_demag_says_so(tmp_path, golden_dir, capfd):
+    """A checkpoint whose form of the demag cannot be had (here one that does not exist) is continued
+    with the form that fits, and a warning."""
+    import struct
+    g, st = _full_test_settings(golden_dir, tmp_path)
+
+    def run(name, until, **gpu):
+        s = dict(st, gpu=gpu, outputs=dict(st["outputs"], file_basename=name, final_time=until * g["evol_time_step"]))
+        (tmp_path / f"{name}.json").write_text(json.dumps(s))
+        fg.run(tmp_path / f"{name}.json", seed=6)
+        return [l for l in open(tmp_path / f"{name}.evol") if not l.startswith("#")]
+
+    run("split", 2, checkpoint_every=3)
+    ck = tmp_path / "split.ckpt"
+    assert fg.checkpoint_peek(ck)["demag_blocks"] == 3
+    raw = ck.read_bytes()
+    body = raw[:40] + struct.pack("<i", 7) + raw[44:-8]
+    h = 1469598103934665603
+    for x in body:
+        h = ((h ^ x) * 1099511628211) & 0xFFFFFFFFFFFFFFFF
+    ck.write_bytes(body + struct.pack("<Q", h))
+    capfd.readouterr()
+    b = run("split", 3, resume=str(ck))
+    assert "does not repeat the uninterrupted run" in capfd.readouterr().err
+    assert b == run("full", 3)

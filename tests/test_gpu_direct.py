@@ -92,3 +92,12 @@ def test_launches_are_counted():
     assert count(lambda: c.energy(np.zeros(3))) == 1
     assert count(lambda: c.compute_all(np.zeros(3))) == 3        # demag, energies, evolution
     assert count(lambda: c.demag(0)) == 1
+
+
+def test_a_matrix_that_does_not_fit_is_an_error_where_it_is_asked_for():
+    """117,000 nodes: a matrix of 328 GB. Creation fails with its own status, and works without it."""
+    m = fg.cuboid(16, 16, 400, 40.0, 40.0, 1000.0, 1e-9, cases.MS)
+    with pytest.raises(fg.FgError) as e:
+        fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_DIRECT, demag_blocks=3)
+    assert e.value.status == 6 and "does not fit" in str(e.value)  # FG_ENOMEM
+    assert fg.Context(m, cases.regions(), demag=fg.FG_DEMAG_DIRECT).demag_info() == (1, 0)
